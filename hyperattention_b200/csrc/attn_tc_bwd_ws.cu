@@ -148,13 +148,7 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
     uint32_t dyn;
     asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
     if ((uint32_t)(smem - smem_raw) + (uint32_t)SMEM_USED > dyn) {      // uniform over the grid
-      if (tid == 0) {
-        if (p.status) atomicExch(p.status, HA_DEV_BAD_LAUNCH);
-        if (p.status_host) {
-          *reinterpret_cast<volatile int32_t*>(p.status_host) = HA_DEV_BAD_LAUNCH;
-          __threadfence_system();
-        }
-      }
+      if (tid == 0) report_status(p.status, p.status_host, HA_DEV_BAD_LAUNCH);
       return;
     }
   }

@@ -1,524 +1,773 @@
-// Attention forward on 5th-generation tensor cores (tcgen05 + TMEM), bf16/fp16, head dims 64 and 128.
+// Attention forward on 5th-generation tensor cores (tcgen05 + TMEM), bf16 / fp16, head dims 64 and 128: one persistent,
+// warp-specialised kernel for both patterns (sorted block windows + sampled rows; exact attention with or without mask).
 //
-// One CTA of 128 threads owns one tile of 128 queries; thread i owns query row i = TMEM lane i.
-//   * Operand rows are gathered straight from the caller's q/k/v by row index with 16-byte cp.async copies into
-//     128-byte-swizzled shared-memory tiles (a 128-byte row is one full line, so a random row gather still moves
-//     whole lines; 8 neighbouring lanes fetch one row).  K/V tiles are double buffered: tile j+1 is in flight while
-//     tile j is computed.
-//   * S = Q K^T: tcgen05.mma, both operands K-major in shared memory, fp32 accumulator in TMEM.
-//   * softmax: each thread reads its row of S with tcgen05.ld (32x32b: one lane per thread, no shuffles), keeps the
-//     running max / sum in base-2, rounds P to the input dtype and writes it back to TMEM with tcgen05.st.
-//   * PV = P V: tcgen05.mma with P as the TMEM A operand and V as MN-major B in shared memory; the product of one
-//     key tile lands in its own TMEM columns and is folded into the fp32 output registers with the rescale factor,
-//     so TMEM is never read-modified-written.
-//   * epilogue: normalise, optionally merge with the (o, lse) already stored for the row (the causal schedule's
-//     in-place combine), round, stage through shared memory and store whole rows coalesced.
-// The same kernel serves both patterns; only the list of key tiles of a query tile differs:
-//   hyper: block-window tiles through k_idx, then the sampled rows;   flash: contiguous tiles, causal mask.
-// TMEM budget per CTA: two regions of 128 columns (S; P in place; PV in the freed half) -> 256 for DV = 64, two CTAs
-// per SM; the MMAs of one key tile and the S MMA of the next are issued as one batch (one commit per key tile).
+// One CTA of 640 threads per SM walks work items; an item is a PAIR of 128-row query tiles of one segment and the list of
+// key tiles the two pair with (FwdItem): every key tile is fetched once for both.  Roles:
+//   * softmax groups 0 / 1 (128 threads each; thread = query row = TMEM lane) of the pair's two query tiles: maximum of the row's 128
+//     scores, then P = exp2(S - reference) back to TMEM in the input dtype and the row's sum.  The reference only moves when
+//     the running maximum has grown by more than 8 (powers of two) beyond it -- any reference gives the same quotient, and
+//     P <= 2^8 is far from either dtype's limits -- so that the accumulator, which lives in TMEM, is hardly ever rescaled; the
+//     group whose reference moved does it, row by row.
+//   * epilogue group (128 threads): O of a finished query tile -> registers -> normalised, merged with the rows already stored
+//     if the call asks for it, stored.  The softmax groups are meanwhile in the next item.
+//   * four MMA warps, S = Q K^T and O += P V of either group, one elected lane issuing from warp-uniform code (descriptors in
+//     uniform registers: an N = 128 step is accepted every 64 cycles, the tensor pipe's own rate; the same instructions from
+//     a divergent lane cost 126).
+//   * four loader warps: contiguous rows by TMA boxes, rows named by an index by tile::gather4 (K) or cp.async (V, Q) -- the two
+//     paths run side by side (gather4: about 2200 cycles per tile of 128 rows of 128 bytes; one warp's cp.async: about 3000).
+//     One of them works out the items and hands their descriptors to everybody through a small ring: the index arithmetic is
+//     done once per item and exists once in the code.
+// The roles' loops are kept small (rolled over column chunks and groups) because their code shares the SM's instruction caches:
+// the same kernel with everything unrolled spent more warp time waiting for instructions than executing them.
+// A unit of the chain S -> softmax -> P V is half a key tile (64 keys).  TMEM (512 columns): group g has score buffers of 64
+// columns from 256 g on, three (DV = 64) or two (DV = 128), and O behind them; P takes the place of its scores.  S of the
+// next units is there before a group asks for it, so a group goes from one unit to the next without waiting.
+// What bounds it: the exponential unit (16 a clock and SM: 1024 cycles per 128 x 128 tile), which is why a part of the exponentials
+// is computed on the FMA pipe (poly_exp2_2), and at head dim 128 the tensor pipe.
 #include "attn_index.cuh"
+#include "tensor_map.cuh"
 
 #include <type_traits>
 
 namespace ha {
 
 template <int D, int DV> struct FwdCfg {
-  static constexpr int Q_BYTES = TILE * D * 2;
-  static constexpr int K_BYTES = TILE * D * 2;
-  static constexpr int V_BYTES = TILE * DV * 2;
-  static constexpr int O_BYTES = TILE * DV * 2;
-  static constexpr int OFF_Q = 0;
-  static constexpr int OFF_K = OFF_Q + Q_BYTES;            // two stages
-  static constexpr int OFF_V = OFF_K + 2 * K_BYTES;        // two stages
-  static constexpr int OFF_OLD = OFF_V + 2 * V_BYTES;      // previous o rows (merge) / output staging
-  static constexpr int SMEM = OFF_OLD + O_BYTES + 1024;    // + alignment slack
-  // TMEM: two regions (key tiles alternate).  A region holds S (128 fp32 columns); P is written in place over its first
-  // 64 columns as S is consumed; the P.V product lands in the columns S no longer needs (DV = 64: the upper half of the
-  // same 128 columns; DV = 128: 128 further columns).
-  static constexpr int REGION = DV <= 64 ? 128 : 256;
-  static constexpr int PV_OFF = DV <= 64 ? 64 : 128;
-  static constexpr int TMEM_COLS = 2 * REGION;
+  static constexpr int NB = DV == 64 ? 3 : 2;                    // score buffers (64 keys each) per group
+  static constexpr int W = D > DV ? D : DV;
+  static constexpr int Q_TILE = TILE * D * 2, KV_TILE = TILE * W * 2;
+  static constexpr int NQ = D == 64 ? 4 : 3;                     // query-tile slots
+  static constexpr int NKV = W == 64 ? 8 : 4;                    // key/value slots: K tiles in the even, V tiles in the odd ones
+  static constexpr int OFF_Q = 0, OFF_KV = NQ * Q_TILE;
+  static constexpr int OFF_STAT = OFF_KV + NKV * KV_TILE;        // [group][row]: (reference, sum) of a finished row
+  static constexpr int SMEM_USED = OFF_STAT + 2 * TILE * 8;      // from the first 1 KB boundary after the static variables
+  static constexpr int COL_O = NB * 64;                          // group g: score buffers at 256 g + 64 b, O behind them
 };
 
-// 128 rows x COLS elements (2 bytes each) gathered by row index into swizzled slabs; 8 lanes per row.
-// my_row = source row of smem row (warp*32 + lane), or -1 to zero-fill.
-template <int COLS>
-__device__ __forceinline__ void gather_tile(uint32_t smem_base, const uint16_t* __restrict__ base, int64_t row_stride, int my_row,
-                                            int warp, int lane) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int rl = 4 * i + (lane >> 3);
-    const int src_row = __shfl_sync(0xffffffffu, my_row, rl);
-    const int row = warp * 32 + rl;
-    const int chunk = lane & 7;
-    const uint32_t dst = smem_base + row * 128 + ((chunk ^ (row & 7)) << 4);
-#pragma unroll
-    for (int s = 0; s < COLS / 64; ++s) {
-      const uint16_t* src = base + (int64_t)(src_row < 0 ? 0 : src_row) * row_stride + s * 64 + chunk * 8;
-      cp_async16(dst + s * (TILE * 128), src, src_row >= 0 ? 16u : 0u);
+namespace fw {
+constexpr int THREADS = 640;
+constexpr int W_EPI = 8, W_S = 12, W_PV = 14, W_Q = 16, W_K = 17;   // first warp of each role (S, P V, V: two each)
+constexpr int ND = 4;                 // descriptor ring
+constexpr int CONSUMERS = 19;         // warps that read every descriptor (all but the one that writes it)
+enum { B_KV_FULL = 0, B_KV_EMPTY = 8, B_Q_FULL = 16, B_Q_EMPTY = 20, B_S_READY = 24, B_PV_DONE = 30, B_O_FULL = 36, B_P_READY = 38, B_O_FREE = 44,
+       B_STAT = 46, B_D_FULL = 48, B_D_EMPTY = 48 + ND, N_BARS = 48 + 2 * ND };      // (S ready, P ready, product done: 3 g + buffer)
+constexpr float REF_SLACK = 8.f;
+}  // namespace fw
+
+struct FwdMaps { CUtensorMap tile[3], rows[2]; };    // tiles of q, k, v; rows of q, k
+struct FwdPlan {
+  FastDiv by_pairs, by_segs, by_heads, by_group, by_block;     // pairs, segs_per_head, H, kv_group, window tiles per block
+  int n_items, pairs;                 // items = pairs of query tiles x segments
+  int tiles, rows;                    // contiguous rows may be loaded as TMA boxes / indexed rows of q (1) and k (2) by gather4
+  int row_sb[2], row_sh[2], row_sn[2];   // row maps of q, k: steps of the row number per batch, head and row
+};
+
+// One item: query tiles qt0, qt0 + 1 (has1) of segment seg and their common list of key tiles.  Entries [lo_g, hi_g) of the list are
+// window (or contiguous) tiles of query tile g; entries n_win .. n_list - 1 are sampled tiles, which both take.  n_list = 0: the end.
+struct FwdItem {
+  int seg, qt0, has1, n_list;
+  int n_win, lo1, hi0, hi1;           // (lo of query tile 0 is 0)
+  int first, b, h, hk;                // sorted position of list entry 0 (hyper)
+  int q_row0, k_row0, kseg, pad;
+  __device__ __forceinline__ int lo(int g) const { return g ? lo1 : 0; }
+  __device__ __forceinline__ int hi(int g) const { return g ? hi1 : hi0; }
+  __device__ __forceinline__ bool active(int g, int e) const { return (g == 0 || has1) && ((e >= lo(g) && e < hi(g)) || e >= n_win); }
+  __device__ __forceinline__ int first_entry(int g) const { return hi(g) > lo(g) ? lo(g) : n_win; }
+  __device__ __forceinline__ int last_entry(int g) const { return n_list > n_win ? n_list - 1 : hi(g) - 1; }
+  __device__ __forceinline__ int count(int g) const { return (g == 0 || has1) ? hi(g) - lo(g) + n_list - n_win : 0; }
+};
+
+__device__ __forceinline__ FwdItem fwd_item(const ha_attn_params& p, const FwdPlan& pl, int item, bool flash) {
+  FwdItem it;
+  it.pad = 0;
+  it.seg = pl.by_pairs(item);
+  int pr = item - it.seg * pl.pairs;
+  const int n_qt = (p.m_q + TILE - 1) / TILE;
+  if (flash && (p.flags & HA_FLAG_CAUSAL)) {
+    // Items grow with the pair.  Long pairs first; with few pairs the order is turned by the segment, so that a CTA, which
+    // takes every 148th item, meets all lengths.
+    pr = pl.pairs - 1 - pr;
+    if (pl.pairs <= 32) pr += it.seg - pl.by_pairs(pr + it.seg) * pl.pairs;
+  }
+  it.qt0 = 2 * pr;
+  it.has1 = it.qt0 + 1 < n_qt;
+  it.first = 0;
+  it.lo1 = 0;
+  if (flash) {
+    const int n_kt = (p.m_k + TILE - 1) / TILE;
+    const bool causal = p.flags & HA_FLAG_CAUSAL;
+    it.hi0 = causal ? min(it.qt0 + 1, n_kt) : n_kt;
+    it.hi1 = causal ? min(it.qt0 + 2, n_kt) : n_kt;
+    it.n_win = it.has1 ? it.hi1 : it.hi0;
+    it.n_list = it.n_win;
+  } else {
+    // block windows (block_window) of both tiles
+    const int bs = (p.block_size + TILE - 1) / TILE, tiles = p.m_k / TILE;
+    const bool smooth = p.flags & HA_FLAG_SMOOTH;
+    const int beta0 = pl.by_block(it.qt0), beta1 = pl.by_block(it.qt0 + 1);
+    if (smooth) {
+      it.first = TILE * it.qt0 - (TILE / 2) * (bs - 1);
+      while (it.first < 0) it.first += p.m_k;
+    } else {
+      it.first = beta0 * bs * TILE;
     }
+    it.hi0 = min(bs, tiles - beta0 * bs);
+    it.hi1 = it.n_win = it.hi0;
+    if (it.has1) {
+      // second window: the same one (both tiles in one block), one tile further on (smooth), or the next block's
+      it.lo1 = smooth ? 1 : beta1 > beta0 ? it.hi0 : 0;
+      it.hi1 = it.lo1 + min(bs, tiles - beta1 * bs);
+      it.n_win = max(it.hi0, it.hi1);
+    }
+    it.n_list = it.n_win + p.sample_size / TILE;
+  }
+  const int bh = pl.by_segs(it.seg), part = it.seg - bh * p.segs_per_head;
+  const int group = p.kv_group > 1 ? p.kv_group : 1;
+  it.b = pl.by_heads(bh);
+  it.h = bh - it.b * p.H;
+  it.hk = pl.by_group(it.h);
+  it.q_row0 = part * p.span + p.q_off;
+  it.k_row0 = part * p.span + p.k_off;
+  it.kseg = group > 1 ? (it.b * pl.by_group(p.H) + it.hk) * p.segs_per_head + part : it.seg;
+  return it;
+}
+
+// Rows of list entry e: key row of tile row r inside the segment (-1: none).
+__device__ __forceinline__ int fwd_key_row(const ha_attn_params& p, const FwdItem& it, int e, int r, bool flash) {
+  if (flash) {
+    const int row = e * TILE + r;
+    return row < p.m_k ? row : -1;
+  }
+  if (e < it.n_win) {
+    int pos = it.first + e * TILE + r;
+    while (pos >= p.m_k) pos -= p.m_k;
+    return p.k_idx[(long long)it.kseg * p.m_k + pos];
+  }
+  const int s = (e - it.n_win) * TILE + r;
+  return p.sample_idx ? p.sample_idx[(long long)it.kseg * p.sample_size + s] : s;
+}
+
+// 128 rows of 64 * slabs elements gathered by ONE warp with cp.async: rows[q] = source row of tile row 32 q + lane (-1: zero fill)
+__device__ __forceinline__ void warp_gather_tile(uint32_t smem_base, const uint16_t* __restrict__ base, int64_t row_stride, int slabs, int (&rows)[4], int lane) {
+  const int chunk = lane & 7;
+#pragma unroll 1
+  for (int q = 0; q < 4; ++q) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int rl = 4 * i + (lane >> 3);
+      const int src_row = __shfl_sync(0xffffffffu, rows[0], rl);
+      const int row = q * 32 + rl;
+      const uint32_t dst = smem_base + row * 128 + ((chunk ^ (row & 7)) << 4);
+      const uint16_t* src = base + (int64_t)(src_row < 0 ? 0 : src_row) * row_stride + chunk * 8;
+      cp_async16(dst, src, src_row >= 0 ? 16u : 0u);
+      if (slabs > 1) cp_async16(dst + TILE * 128, src + 64, src_row >= 0 ? 16u : 0u);
+    }
+    rows[0] = rows[1]; rows[1] = rows[2]; rows[2] = rows[3];
   }
 }
 
-// rows staged in swizzled slabs -> global rows by index, coalesced; my_row = destination row or -1 to skip
-template <int COLS>
-__device__ __forceinline__ void scatter_tile(const uint8_t* smem_base, uint16_t* __restrict__ base, int64_t row_stride, int my_row,
-                                             int warp, int lane) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int rl = 4 * i + (lane >> 3);
-    const int dst_row = __shfl_sync(0xffffffffu, my_row, rl);
-    const int row = warp * 32 + rl;
-    const int chunk = lane & 7;
-#pragma unroll
-    for (int s = 0; s < COLS / 64; ++s) {
-      const uint4 v = *reinterpret_cast<const uint4*>(smem_base + s * (TILE * 128) + row * 128 + ((chunk ^ (row & 7)) << 4));
-      if (dst_row >= 0) *reinterpret_cast<uint4*>(base + (int64_t)dst_row * row_stride + s * 64 + chunk * 8) = v;
-    }
-  }
-}
-
-struct TileList {
-  int n_tiles;      // key tiles of this query tile
-  int n_blk;        // hyper: how many of them are block-window tiles
-  Window w;
-};
-
-// WT: weighted sampling (sample_logw / sample_mask given); a template flag so that the plain instantiation carries none of it
-template <typename T, int D, int DV, bool WT>
-__global__ void __launch_bounds__(128) attn_tc_fwd_kernel(const ha_attn_params p, const int pf_dist) {
+// KIND: the plain hyper pattern, exact attention, or any call (merging calls, weighted sampling): the code of an instance is what the
+// instruction caches have to hold, so the two frequent kinds carry nothing they do not use.
+enum { FWD_HYPER = 0, FWD_FLASH = 1, FWD_ANY = 2 };
+template <typename T, int D, int DV, int KIND>
+__global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_attn_params p, const FwdPlan pl, const __grid_constant__ FwdMaps maps) {
+  using namespace fw;
   using Cfg = FwdCfg<D, DV>;
+  constexpr int NQ = Cfg::NQ, NKV = Cfg::NKV, NB = Cfg::NB;
+  const bool flash = KIND == FWD_FLASH || (KIND == FWD_ANY && p.mode == HA_MODE_FLASH);
+  constexpr bool WT = KIND == FWD_ANY;                 // weighted sampling / merging possible
+  // Pairs of every eight whose exponentials go to the FMA pipe.  It pays where the chain is bound by the exponential unit, i.e. in exact
+  // attention (32 x 2048-row leaves, head dim 64: 1.67 -> 1.60 ms); the hyper pattern is bound by its gathers and by the
+  // instruction caches before that (0.79 ms without, 0.83 ms with).
+  constexpr int POLY = KIND == FWD_FLASH ? 2 : 0;
+  const bool merge = KIND == FWD_ANY && (p.flags & HA_FLAG_MERGE);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t s_base = smem_u32(smem);
-  __shared__ uint64_t mma_bar;
+  __shared__ __align__(16) FwdItem s_item[ND];
+  __shared__ uint64_t bars[N_BARS];
   __shared__ uint32_t tmem_slot;
+  __shared__ int s_abort;
   __shared__ int s_bail;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool hyper = p.mode == HA_MODE_HYPER;
-  const bool causal = p.flags & HA_FLAG_CAUSAL;
-  const int n_qt = (p.m_q + TILE - 1) / TILE;
-  // heavy (late) causal tiles first
-  const int qt = causal ? n_qt - 1 - (int)blockIdx.x : (int)blockIdx.x;
-  const int seg = blockIdx.y;
-  const SegInfo si = seg_info(p, seg);
-  const uint32_t bar = smem_u32(&mma_bar);
-  HA_T_DECL(8)
-
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   if (cta_sees_failure(p.status, &s_bail)) return;   // an earlier CTA gave up: drain quickly (uniform over the CTA)
+  {
+    // should the window start somewhere else than assumed, do nothing rather than run over its end
+    uint32_t dyn;
+    asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+    if ((uint32_t)(smem - smem_raw) + (uint32_t)Cfg::SMEM_USED > dyn) {      // uniform over the grid
+      if (tid == 0) report_status(p.status, p.status_host, HA_DEV_BAD_LAUNCH);
+      return;
+    }
+  }
+  float2* s_stat = reinterpret_cast<float2*>(smem + Cfg::OFF_STAT);
+  const uint32_t bar0 = smem_u32(bars);
+  auto bar = [&](int i) -> uint32_t { return bar0 + 8 * i; };
   if (tid == 0) {
-    mbar_init(bar, 2);      // one arrival from each of the two MMA-issuing threads per batch
+    // arrivals per phase: 32 (every lane of the tile's loader) on the tiles' "full" barriers, 128 (a group) on the hand-offs of the
+    // thread groups, one per reading warp on "descriptor empty", 2 (both groups' MMA warps) on the tiles' "empty" barriers, 1 (a
+    // tcgen05.commit, the scheduler) elsewhere
+    for (int i = 0; i < N_BARS; ++i) {
+      const bool loader = (i >= B_KV_FULL && i < B_KV_EMPTY) || (i >= B_Q_FULL && i < B_Q_EMPTY);
+      const bool group = i >= B_P_READY && i < B_D_FULL;
+      mbar_init(bar(i), loader ? 32 : group ? 128 : i >= B_D_EMPTY ? CONSUMERS : i >= B_KV_EMPTY && i < B_Q_FULL ? 2 : 1);
+    }
+    s_abort = 0;
     mbar_fence_init();
   }
-  if (warp == 0) tmem_alloc(smem_u32(&tmem_slot), Cfg::TMEM_COLS);
-
-  // ---- this thread's query row ----
-  const int qpos = qt * TILE + tid;
-  int qrow = -1;
-  if (qpos < p.m_q) qrow = hyper ? p.q_idx[(long long)seg * p.m_q + qpos] : qpos;
-
-  TileList tl;
-  if (hyper) {
-    const int bs = (p.block_size + TILE - 1) / TILE;
-    tl.w = block_window(qt, bs, p.m_k, p.flags & HA_FLAG_SMOOTH);
-    tl.n_blk = tl.w.count / TILE;
-    tl.n_tiles = tl.n_blk + p.sample_size / TILE;
-  } else {
-    const int n_kt = (p.m_k + TILE - 1) / TILE;
-    tl.n_blk = 0;
-    tl.w = Window{0, 0};
-    tl.n_tiles = causal ? min(qt + 1, n_kt) : n_kt;
-  }
-  // local key row that thread `tid` fetches for key tile j (-1: none)
-  auto key_row = [&](int j) -> int {
-    if (j >= tl.n_tiles) return -1;
-    if (!hyper) {
-      const int r = j * TILE + tid;
-      return r < p.m_k ? r : -1;
-    }
-    if (j < tl.n_blk) {
-      int pos = tl.w.first + j * TILE + tid;
-      if (pos >= p.m_k) pos -= p.m_k;
-      return p.k_idx[kseg_of(p, seg) * p.m_k + pos];
-    }
-    const int s = (j - tl.n_blk) * TILE + tid;
-    return p.sample_idx ? p.sample_idx[kseg_of(p, seg) * p.sample_size + s] : s;
-  };
-
-  const uint16_t* qbase = (const uint16_t*)p.q + si.b * p.q_sb + si.h * p.q_sh + si.q_row0 * p.q_sn;
-  const uint16_t* kbase = (const uint16_t*)p.k + si.b * p.k_sb + si.hk * p.k_sh + si.k_row0 * p.k_sn;
-  const uint16_t* vbase = (const uint16_t*)p.v + si.b * p.v_sb + si.hk * p.v_sh + si.k_row0 * p.v_sn;
-  uint16_t* obase = (uint16_t*)p.o + si.b * p.o_sb + si.h * p.o_sh + si.q_row0 * p.o_sn;
-  const bool merge = p.flags & HA_FLAG_MERGE;
-
-  // ---- prologue: Q, previous o rows (merge), key tile 0 ----
-  int krow_cur = key_row(0);
-  gather_tile<D>(s_base + Cfg::OFF_Q, qbase, p.q_sn, qrow, warp, lane);
-  if (merge) gather_tile<DV>(s_base + Cfg::OFF_OLD, obase, p.o_sn, qrow, warp, lane);
-  gather_tile<D>(s_base + Cfg::OFF_K, kbase, p.k_sn, krow_cur, warp, lane);
-  gather_tile<DV>(s_base + Cfg::OFF_V, vbase, p.v_sn, krow_cur, warp, lane);
-  cp_async_commit();
-  int krow_next = key_row(1);
-
-  // ---- rows of the query tile that runs pf_dist CTAs later (one wave ahead): pulled into L2 while this CTA computes,
-  //      so that tile's dependent index -> row gathers hit L2 instead of HBM.  Index loads are issued here, the prefetches
-  //      after the first key tile, when the indices have arrived.
-  constexpr int PF_TILES = 4;
-  int pf_q = -1, pf_k[PF_TILES];
-#pragma unroll
-  for (int i = 0; i < PF_TILES; ++i) pf_k[i] = -1;
-  SegInfo pf_si = si;
-  {
-    const long long lin = (long long)blockIdx.y * gridDim.x + blockIdx.x + pf_dist;
-    if (hyper && pf_dist > 0 && lin < (long long)gridDim.x * gridDim.y) {
-      const int pseg = (int)(lin / gridDim.x), pqt = (int)(lin - (long long)pseg * gridDim.x);
-      pf_si = seg_info(p, pseg);
-      const int bs = (p.block_size + TILE - 1) / TILE;
-      const Window pw = block_window(pqt, bs, p.m_k, p.flags & HA_FLAG_SMOOTH);
-      const int pn_blk = pw.count / TILE;
-      pf_q = p.q_idx[(long long)pseg * p.m_q + pqt * TILE + tid];
-#pragma unroll
-      for (int i = 0; i < PF_TILES; ++i) {
-        if (i < pn_blk) {
-          int pos = pw.first + i * TILE + tid;
-          if (pos >= p.m_k) pos -= p.m_k;
-          pf_k[i] = p.k_idx[kseg_of(p, pseg) * p.m_k + pos];
-        } else if (p.sample_idx && (i - pn_blk) * TILE < p.sample_size) {
-          pf_k[i] = p.sample_idx[kseg_of(p, pseg) * p.sample_size + (i - pn_blk) * TILE + tid];
-        }
-      }
-    }
-  }
-
+  if (warp == W_S) tmem_alloc(smem_u32(&tmem_slot), 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = tmem_slot;
-  const uint32_t lane_sel = (uint32_t)(warp * 32) << 16;
-  constexpr int AB_FMT = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
-  const uint32_t idesc_s = mma_idesc(TILE, TILE, AB_FMT, 0, 0);
-  const uint32_t idesc_pv = mma_idesc(TILE, DV, AB_FMT, 0, 1);
-
-  __align__(8) float o_acc[DV];
-#pragma unroll
-  for (int i = 0; i < DV; ++i) o_acc[i] = 0.f;
-  float m_run = -INFINITY, l_run = 0.f;
-  const float scale2 = p.scale * 1.4426950408889634f;
-  uint32_t phase = 0;
-  bool failed = false;
-
-  auto issue_s = [&](int stg, uint32_t t_s) {
-#pragma unroll
-    for (int kk = 0; kk < D / 16; ++kk) {
-      const uint32_t a_addr = s_base + Cfg::OFF_Q + (kk >> 2) * (TILE * 128) + (kk & 3) * 32;
-      const uint32_t b_addr = s_base + Cfg::OFF_K + stg * Cfg::K_BYTES + (kk >> 2) * (TILE * 128) + (kk & 3) * 32;
-      mma_ss(t_s, smem_desc(a_addr, 16, 1024), smem_desc(b_addr, 16, 1024), idesc_s, kk > 0);
-    }
-  };
-  auto issue_pv = [&](int stg, uint32_t t_p, uint32_t t_pv) {
-#pragma unroll
-    for (int kk = 0; kk < TILE / 16; ++kk) {
-      const uint32_t b_addr = s_base + Cfg::OFF_V + stg * Cfg::V_BYTES + kk * 2048;
-      mma_ts(t_pv, t_p + kk * 8, smem_desc(b_addr, TILE * 128, 1024), idesc_pv, kk > 0);
-    }
-  };
-  auto accumulate_pv = [&](uint32_t t_pv, float alpha) {
-    const uint64_t al2 = pack_f2(alpha, alpha);
-    uint64_t* o2 = reinterpret_cast<uint64_t*>(o_acc);
-#pragma unroll
-    for (int c = 0; c < DV / 32; ++c) {
-      uint32_t r[32];
-      tmem_ld32(t_pv + lane_sel + c * 32, r);
-      tmem_ld_fence(r);
-#pragma unroll
-      for (int i = 0; i < 32; i += 2) o2[(c * 32 + i) >> 1] = ffma2(o2[(c * 32 + i) >> 1], al2, pack_u2(r[i], r[i + 1]));
-    }
+  // A wait that gives up (or finds the abort flag up) ends the role's loop; the status word is set once, at the end.  Called by whole
+  // warps; one answer for the warp.
+  auto wait = [&](int b, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait_or_abort(bar(b), parity, &s_abort)); };
+  uint32_t n_item = 0;       // descriptors this warp has taken
+  // the next item's descriptor; false: no more items (or a wait gave up)
+  auto next_item = [&](FwdItem& it) -> bool {
+    const int slot = n_item % ND;
+    if (!wait(B_D_FULL + slot, (n_item / ND) & 1)) return false;
+    it = s_item[slot];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar(B_D_EMPTY + slot));
+    ++n_item;
+    return it.n_list != 0;
   };
 
-  // Schedule: batch(j) = { P.V of key tile j ; S of key tile j+1 } is one commit; while it runs, the other CTA on the SM
-  // has the pipes.  The product of tile j-1 is folded into the output registers at the top of iteration j.
-  cp_async_wait<0>();
-  fence_async_smem();
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  // Two threads issue the MMAs of a batch: thread 0 the P V product of key tile j, thread 32 S of key tile j + 1.  One thread
-  // gets a tcgen05.mma accepted only about every 110-130 cycles whatever its shape (measured), so the 12 instructions of a
-  // batch from one thread cost more than the tensor pipe needs for them; each thread arrives once per batch (a commit
-  // after its instructions, or a plain arrival when it has none).
-  if (tid == 0) mbar_arrive(bar);
-  if (tid == 32) {
-    issue_s(0, tmem);
-    mma_commit(bar);
-  }
-  float alpha_prev = 0.f;
-  HA_T_MARK(7)
-  for (int j = 0; j < tl.n_tiles; ++j) {
-    HA_T_MARK(0)
-    const int st = j & 1;
-    const uint32_t tS = tmem + st * Cfg::REGION, tP = tS, tPV = tS + Cfg::PV_OFF;
-    if (!mbar_wait(bar, phase)) { failed = true; }     // batch(j-1): S of this tile (and P.V of the previous one) landed
-    phase ^= 1;
-    tc_fence_after();
-    if (__syncthreads_or(failed)) { failed = true; break; }
-    HA_T_MARK(1)
-    // the other stage is free now: fetch key tile j+1
-    if (j + 1 < tl.n_tiles) {
-      gather_tile<D>(s_base + Cfg::OFF_K + (st ^ 1) * Cfg::K_BYTES, kbase, p.k_sn, krow_next, warp, lane);
-      gather_tile<DV>(s_base + Cfg::OFF_V + (st ^ 1) * Cfg::V_BYTES, vbase, p.v_sn, krow_next, warp, lane);
-    }
-    cp_async_commit();
-    const int krow_after = key_row(j + 2);   // index load for the tile after next, consumed next iteration
-    if (j >= 1) accumulate_pv(tmem + (st ^ 1) * Cfg::REGION + Cfg::PV_OFF, alpha_prev);
-    HA_T_MARK(2)
-    // ---- softmax over this tile's 128 columns ----
-    // visible columns of this row: all of them, except on a causal diagonal tile or a ragged last tile
-    int limit = TILE;
-    bool masked = false;   // uniform over the CTA
-    // weighted sampling: a sampled tile's scores get the tile's log weight, and its dropped slots are masked
-    uint32_t wm[4] = {0u, 0u, 0u, 0u};
-    float bias2 = 0.f;
-    if (WT && hyper && j >= tl.n_blk) {
-      const long long qtile = (long long)seg * n_qt + qt;
-      const uint32_t* mw = p.sample_mask + qtile * (p.sample_size / 32) + (j - tl.n_blk) * 4;
-      wm[0] = mw[0]; wm[1] = mw[1]; wm[2] = mw[2]; wm[3] = mw[3];
-      bias2 = p.sample_logw[qtile] * 1.4426950408889634f;
-      masked = (wm[0] | wm[1] | wm[2] | wm[3]) != 0u;
-    }
-    if (!hyper) {
-      limit = min(TILE, p.m_k - j * TILE);
-      masked = limit < TILE;
-      if (causal) {
-        limit = min(limit, qpos - j * TILE + 1);
-        masked = masked || (j == qt);
-      }
-    }
-    float mx;
-    {
-      float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
-      uint32_t ra[32], rb[32];
-      tmem_ld32(tS + lane_sel, ra);
-      tmem_ld_fence(ra);
+  // Register budget: 640 threads x 96 at launch = 61440 = 256 x 120 (softmax) + 128 x 96 (epilogue) + 256 x 72 (the rest).
+  if (warp < W_EPI) {
+    // =====================================================================================================
+    // softmax groups
+    // =====================================================================================================
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 120;");
+    const int g = warp >> 2, row = tid & 127;
+    const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t tG = tmem + g * 256 + lane_sel, tO = tG + Cfg::COL_O;
+    const float scale2 = p.scale * 1.4426950408889634f;
+    const bool causal = flash && (p.flags & HA_FLAG_CAUSAL);
+    uint32_t buf = 0, par = 0;          // score buffer of the next unit, parity of its barriers
+    uint32_t it_g = 0;                  // items this group has taken part in
+    bool ok = true;
+    HA_T_DECL(8)
+    FwdItem it;
+    while (ok && next_item(it)) {
+      const int n_act = 2 * it.count(g);
+      if (n_act == 0) continue;
+      const int n_w = 2 * (it.hi(g) - it.lo(g)), lo = 2 * it.lo(g), qt = it.qt0 + g;
+      float m_ref = -INFINITY, l_run = 0.f;
+#pragma unroll 1
+      for (int a = 0; a < n_act; ++a) {
+        const int u = a < n_w ? lo + a : 2 * it.n_win + a - n_w;     // unit: half (u & 1) of list entry u / 2
+        const uint32_t tS = tG + buf * 64;
+        HA_T_MARK(0)
+        if (!(ok = wait(B_S_READY + 3 * g + buf, par))) break;
+        HA_T_MARK(1)
+        tc_fence_after();
+        uint32_t s[64];
+        {
+          uint32_t(&s0)[32] = *reinterpret_cast<uint32_t(*)[32]>(s);
+          uint32_t(&s1)[32] = *reinterpret_cast<uint32_t(*)[32]>(s + 32);
+          tmem_ld32(tS, s0);
+          tmem_ld32(tS + 32, s1);
+          tmem_ld_fence(s0);
+          tmem_ld_fence(s1);
+        }
+        // ---- columns this row does not see: past the diagonal, past a ragged last tile, dropped slots of the sample ----
+        float bias2 = 0.f;
+        if (flash) {
+          int limit = p.m_k - u * 64;
+          const bool diag = causal && (u >> 1) == qt;
+          if (diag) limit = min(limit, row + 1 - (u & 1) * 64);
+          if (diag || limit < 64) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t(&cur)[32] = (c & 1) ? rb : ra;
-        uint32_t(&nxt)[32] = (c & 1) ? ra : rb;
-        if (c + 1 < 4) tmem_ld32(tS + lane_sel + (c + 1) * 32, nxt);
-        if (!masked) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            m0 = fmax3(m0, __uint_as_float(cur[i]), __uint_as_float(cur[i + 1]));
-            m1 = fmax3(m1, __uint_as_float(cur[i + 2]), __uint_as_float(cur[i + 3]));
-            m2 = fmax3(m2, __uint_as_float(cur[i + 4]), __uint_as_float(cur[i + 5]));
-            m3 = fmax3(m3, __uint_as_float(cur[i + 6]), __uint_as_float(cur[i + 7]));
+            for (int i = 0; i < 64; ++i)
+              if (i >= limit) s[i] = 0xff800000u;
           }
-        } else {
+        } else if (WT && p.sample_logw && u >= 2 * it.n_win) {
+          const long long qtile = (long long)it.seg * (p.m_q / TILE) + qt;
+          const uint32_t* drop = p.sample_mask + qtile * (p.sample_size / 32) + (u - 2 * it.n_win) * 2;
+          const uint32_t d0 = drop[0], d1 = drop[1];
+          bias2 = p.sample_logw[qtile] * 1.4426950408889634f;
+          if ((d0 | d1) != 0u) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i)
-            if (c * 32 + i < limit && !(WT && ((wm[c] >> i) & 1u))) m0 = fmaxf(m0, __uint_as_float(cur[i]));
-        }
-        if (c + 1 < 4) tmem_ld_fence(nxt);
-      }
-      mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
-    }
-    const float m_new = fmaxf(m_run, WT ? mx * scale2 + bias2 : mx * scale2);
-    const float m_use = m_new == -INFINITY ? 0.f : m_new;
-    const float alpha = fast_exp2(m_run - m_use);   // m_run = -inf -> 0
-    float psum;
-    {
-      const uint64_t sc2 = pack_f2(scale2, scale2), negm = WT ? pack_f2(bias2 - m_use, bias2 - m_use) : pack_f2(-m_use, -m_use);
-      uint64_t ps_a = pack_f2(0.f, 0.f), ps_b = ps_a;
-      uint32_t ra[32], rb[32];
-      tmem_ld32(tS + lane_sel, ra);
-      tmem_ld_fence(ra);
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t(&cur)[32] = (c & 1) ? rb : ra;
-        uint32_t(&nxt)[32] = (c & 1) ? ra : rb;
-        // P chunk c below overwrites columns [16c, 16c+16), part of S chunk c/2, which is already in registers; the
-        // chunk being loaded (c+1) lies in columns >= 32(c+1), disjoint from them
-        if (c + 1 < 4) tmem_ld32(tS + lane_sel + (c + 1) * 32, nxt);
-        uint32_t pk[16];
-#pragma unroll
-        for (int i = 0; i < 32; i += 4) {
-          float p0, p1, p2, p3;
-          unpack_f2(ffma2(pack_u2(cur[i], cur[i + 1]), sc2, negm), p0, p1);
-          unpack_f2(ffma2(pack_u2(cur[i + 2], cur[i + 3]), sc2, negm), p2, p3);
-          p0 = fast_exp2(p0); p1 = fast_exp2(p1); p2 = fast_exp2(p2); p3 = fast_exp2(p3);
-          if (masked) {
-            if (c * 32 + i >= limit || (WT && ((wm[c] >> i) & 1u))) p0 = 0.f;
-            if (c * 32 + i + 1 >= limit || (WT && ((wm[c] >> (i + 1)) & 1u))) p1 = 0.f;
-            if (c * 32 + i + 2 >= limit || (WT && ((wm[c] >> (i + 2)) & 1u))) p2 = 0.f;
-            if (c * 32 + i + 3 >= limit || (WT && ((wm[c] >> (i + 3)) & 1u))) p3 = 0.f;
+            for (int i = 0; i < 64; ++i)
+              if (((i < 32 ? d0 : d1) >> (i & 31)) & 1u) s[i] = 0xff800000u;
           }
-          ps_a = fadd2(ps_a, pack_f2(p0, p1));
-          ps_b = fadd2(ps_b, pack_f2(p2, p3));
-          pk[i >> 1] = pack2<T>(p0, p1);
-          pk[(i >> 1) + 1] = pack2<T>(p2, p3);
         }
-        tmem_st16(tP + lane_sel + c * 16, pk);
-        if (c + 1 < 4) tmem_ld_fence(nxt);
-      }
-      float s0, s1;
-      unpack_f2(fadd2(ps_a, ps_b), s0, s1);
-      psum = s0 + s1;
-    }
-    tmem_st_wait();
-    l_run = l_run * alpha + psum;
-    m_run = m_new;
-    alpha_prev = alpha;
-    HA_T_MARK(3)
-    cp_async_wait<0>();                        // key tile j+1 has landed
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    if (tid == 0) {
-      issue_pv(st, tP, tPV);
-      mma_commit(bar);
-    }
-    if (tid == 32) {
-      if (j + 1 < tl.n_tiles) {
-        issue_s(st ^ 1, tmem + (st ^ 1) * Cfg::REGION);
-        mma_commit(bar);
-      } else {
-        mbar_arrive(bar);
-      }
-    }
-    HA_T_MARK(4)
-    krow_cur = krow_next;
-    krow_next = krow_after;
-    if (j == 0 && pf_q >= 0) {
-      const uint16_t* pq = (const uint16_t*)p.q + pf_si.b * p.q_sb + pf_si.h * p.q_sh + (pf_si.q_row0 + pf_q) * p.q_sn;
-      const uint16_t* pk = (const uint16_t*)p.k + pf_si.b * p.k_sb + pf_si.hk * p.k_sh + pf_si.k_row0 * p.k_sn;
-      const uint16_t* pv = (const uint16_t*)p.v + pf_si.b * p.v_sb + pf_si.hk * p.v_sh + pf_si.k_row0 * p.v_sn;
-      prefetch_l2(pq);
-      if (D > 64) prefetch_l2(pq + 64);
-      if (merge) {
-        const uint16_t* po = (const uint16_t*)p.o + pf_si.b * p.o_sb + pf_si.h * p.o_sh + (pf_si.q_row0 + pf_q) * p.o_sn;
-        prefetch_l2(po);
-        if (DV > 64) prefetch_l2(po + 64);
-      }
+        float mx;
+        {
+          float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int i = 0; i < PF_TILES; ++i) {
-        if (pf_k[i] >= 0) {
-          prefetch_l2(pk + (int64_t)pf_k[i] * p.k_sn);
-          if (D > 64) prefetch_l2(pk + (int64_t)pf_k[i] * p.k_sn + 64);
-          prefetch_l2(pv + (int64_t)pf_k[i] * p.v_sn);
-          if (DV > 64) prefetch_l2(pv + (int64_t)pf_k[i] * p.v_sn + 64);
+          for (int i = 0; i < 64; i += 2) m4[(i >> 1) & 3] = fmax3(m4[(i >> 1) & 3], __uint_as_float(s[i]), __uint_as_float(s[i + 1]));
+          mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
         }
+        const float m_cand = WT ? mx * scale2 + bias2 : mx * scale2;
+        const bool move = m_cand > m_ref + REF_SLACK;        // (the first visible unit always: -inf + 8)
+        float alpha = 1.f;
+        if (__any_sync(0xffffffffu, move)) {
+          const float m_new = move ? m_cand : m_ref;
+          if (move) alpha = fast_exp2(m_ref - m_new);        // m_ref = -inf -> 0
+          m_ref = m_new;
+          if (a > 0) {
+            // O is complete up to the previous unit: rescale it
+            const uint32_t pb = buf == 0 ? NB - 1 : buf - 1;
+            if (!(ok = wait(B_PV_DONE + 3 * g + pb, buf == 0 ? par ^ 1 : par))) break;
+            tc_fence_after();
+            const uint64_t al2 = pack_f2(alpha, alpha);
+#pragma unroll 1
+            for (int c = 0; c < DV / 16; ++c) {
+              uint32_t r[16];
+              tmem_ld16(tO + c * 16, r);
+              tmem_ld_fence16(r);
+#pragma unroll
+              for (int i = 0; i < 16; i += 2) {
+                float x, y;
+                unpack_f2(fmul2(pack_u2(r[i], r[i + 1]), al2), x, y);
+                r[i] = __float_as_uint(x);
+                r[i + 1] = __float_as_uint(y);
+              }
+              tmem_st16(tO + c * 16, r);
+            }
+          }
+        }
+        HA_T_MARK(2)
+        const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
+        const uint64_t sc2 = pack_f2(scale2, scale2), negm = WT ? pack_f2(bias2 - m_use, bias2 - m_use) : pack_f2(-m_use, -m_use);
+        uint64_t ps_a = pack_f2(0.f, 0.f), ps_b = ps_a;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t pk[8];
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) {
+            // of every eight pairs POLY go to the FMA pipe, the others to the exponential unit
+            const uint64_t x = ffma2(pack_u2(s[c * 16 + i], s[c * 16 + i + 1]), sc2, negm);
+            float p0, p1;
+            if ((i >> 1) % 3 == 1 && (i >> 1) / 3 < POLY) {
+              poly_exp2_2(x, p0, p1);
+            } else {
+              unpack_f2(x, p0, p1);
+              p0 = fast_exp2(p0);
+              p1 = fast_exp2(p1);
+            }
+            uint64_t& ps = (i & 2) ? ps_b : ps_a;
+            ps = fadd2(ps, pack_f2(p0, p1));
+            pk[i >> 1] = pack2<T>(p0, p1);
+          }
+          tmem_st8(tS + c * 8, pk);
+        }
+        HA_T_MARK(3)
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive(bar(B_P_READY + 3 * g + buf));
+        float s0, s1;
+        unpack_f2(fadd2(ps_a, ps_b), s0, s1);
+        l_run = l_run * alpha + (s0 + s1);
+        if (++buf == NB) { buf = 0; par ^= 1; }
+        HA_T_MARK(4)
+      }
+      if (!ok) break;
+      // The epilogue has read the previous item's values (long ago, except where items are a single key tile).
+      if (it_g >= 1 && !(ok = wait(B_O_FREE + g, (it_g - 1) & 1))) break;
+      s_stat[g * TILE + row] = make_float2(m_ref, l_run);
+      mbar_arrive(bar(B_STAT + g));
+      ++it_g;
+    }
+    HA_T_DUMP(8, (int)blockIdx.x * 8, tid == 0)
+  } else if (warp < W_S) {
+    // =====================================================================================================
+    // epilogue group
+    // =====================================================================================================
+    const int row = tid & 127;
+    const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
+    uint32_t n_out[2] = {0, 0};
+    bool ok = true;
+    HA_T_DECL(8)
+    FwdItem it;
+    while (ok && next_item(it)) {
+#pragma unroll 1
+      for (int g = 0; g < 1 + it.has1; ++g) {
+        const int qpos = (it.qt0 + g) * TILE + row;
+        int qrow = -1;
+        if (qpos < p.m_q) qrow = flash ? qpos : p.q_idx[(long long)it.seg * p.m_q + qpos];
+        const long long o_row = (long long)it.q_row0 + (qrow < 0 ? 0 : qrow);
+        const long long lse_at = ((long long)(it.b * p.H + it.h)) * p.n + o_row;
+        const long long o_at = it.b * p.o_sb + it.h * p.o_sh + o_row * p.o_sn;
+        const float lse_old = merge ? p.lse[lse_at] : 0.f;          // requested ahead of the waits
+        const uint32_t par = (g ? n_out[1] : n_out[0]) & 1;
+        HA_T_MARK(0)
+        if (!(ok = wait(B_STAT + g, par) && wait(B_O_FULL + g, par))) break;
+        HA_T_MARK(1)
+        tc_fence_after();
+        const float2 st = s_stat[g * TILE + row];
+        const float inv = st.y > 0.f ? 1.f / st.y : 0.f;
+        const float lse_own = st.y > 0.f ? (st.x + log2f(st.y)) * 0.6931471805599453f : -INFINITY;
+        float lse = lse_own, w1 = 0.f, w2 = 1.f;
+        if (merge) {
+          const float l1 = lse_old, l2 = lse_own;
+          if (p.flags & HA_FLAG_MERGE_EXACT) {
+            const float m2 = fmaxf(l1, l2);
+            const float e1 = __expf(l1 - m2), e2 = __expf(l2 - m2);
+            w1 = e1 / (e1 + e2);
+            w2 = e2 / (e1 + e2);
+            lse = m2 + __logf(e1 + e2);
+          } else {
+            const float cf = round_to<T>(1.f / (1.f + __expf(l2 - l1)));
+            w1 = cf;
+            w2 = round_to<T>(1.f - cf);
+            lse = l1 - __logf(cf + 1.1920929e-07f);
+          }
+        }
+        const uint64_t inv2 = pack_f2(inv, inv);
+        // 64 columns at a time.  A thread stores its own row, 16 bytes a piece: staging the tile for row-coalesced stores measured
+        // no faster.
+#pragma unroll 1
+        for (int hf = 0; hf < DV / 64; ++hf) {
+          uint32_t ra[32], rb[32];
+          tmem_ld32(tmem + g * 256 + Cfg::COL_O + lane_sel + hf * 64, ra);
+          tmem_ld32(tmem + g * 256 + Cfg::COL_O + lane_sel + hf * 64 + 32, rb);
+          tmem_ld_fence(ra);
+          tmem_ld_fence(rb);
+          if (hf == DV / 64 - 1) {
+            tc_fence_before();
+            mbar_arrive(bar(B_O_FREE + g));
+            HA_T_MARK(2)
+          }
+          uint32_t w[32];      // the row, normalised and rounded
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            float x, y;
+            unpack_f2(fmul2(pack_u2(ra[i], ra[i + 1]), inv2), x, y);
+            w[i >> 1] = pack2<T>(x, y);
+            unpack_f2(fmul2(pack_u2(rb[i], rb[i + 1]), inv2), x, y);
+            w[16 + (i >> 1)] = pack2<T>(x, y);
+          }
+          if (qrow >= 0) {
+            if (WT && p.part_o) {      // the un-merged result of this call
+              uint4* part = reinterpret_cast<uint4*>((T*)p.part_o + o_at + hf * 64);
+#pragma unroll
+              for (int e = 0; e < 8; ++e) part[e] = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
+            }
+            uint4* out = reinterpret_cast<uint4*>((T*)p.o + o_at + hf * 64);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              uint4 v = make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
+              if (merge) {
+                const uint4 ov = out[e];
+                const uint32_t ow[4] = {ov.x, ov.y, ov.z, ov.w}, nw[4] = {v.x, v.y, v.z, v.w};
+                uint32_t z[4];
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                  const float2 old = unpack2<T>(ow[h]), mine = unpack2<T>(nw[h]);
+                  z[h] = pack2<T>(w1 * old.x + w2 * mine.x, w1 * old.y + w2 * mine.y);
+                }
+                v = make_uint4(z[0], z[1], z[2], z[3]);
+              }
+              out[e] = v;
+            }
+          }
+        }
+        if (g) ++n_out[1];
+        else ++n_out[0];
+        if (qrow >= 0) {
+          if (WT && p.part_o && p.part_lse) p.part_lse[lse_at] = lse_own;
+          p.lse[lse_at] = lse;
+        }
+        HA_T_MARK(3)
       }
     }
-    HA_T_MARK(5)
-  }
-  cp_async_wait<0>();
-  if (!failed) {
-    if (!mbar_wait(bar, phase)) failed = true;          // the last P.V
-    phase ^= 1;
-    tc_fence_after();
-    failed = __syncthreads_or(failed);
-    if (!failed) accumulate_pv(tmem + ((tl.n_tiles - 1) & 1) * Cfg::REGION + Cfg::PV_OFF, alpha_prev);
-  }
-
-  if (failed) {
-    if (tid == 0) report_timeout(p.status, p.status_host);
+    HA_T_DUMP(8, (int)blockIdx.x * 8 + 5, row == 0)
   } else {
-    // ---- epilogue ----
-    const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-    float lse = l_run > 0.f ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
-    const long long lse_at = ((long long)(si.b * p.H + si.h)) * p.n + si.q_row0 + (qrow < 0 ? 0 : qrow);
-    uint8_t* stage = smem + Cfg::OFF_OLD;
-    float w1 = 0.f, w2 = 1.f;
-    if (merge && qrow >= 0) {
-      const float l1 = p.lse[lse_at], l2 = lse;
-      if (p.flags & HA_FLAG_MERGE_EXACT) {
-        const float m2 = fmaxf(l1, l2);
-        const float e1 = __expf(l1 - m2), e2 = __expf(l2 - m2);
-        w1 = e1 / (e1 + e2);
-        w2 = e2 / (e1 + e2);
-        lse = m2 + __logf(e1 + e2);
-      } else {
-        const float c = round_to<T>(1.f / (1.f + __expf(l2 - l1)));
-        w1 = c;
-        w2 = round_to<T>(1.f - c);
-        lse = l1 - __logf(c + 1.1920929e-07f);
-      }
-    }
-    if (merge) {
-      // merge (the causal schedule's rectangles): rows staged in shared memory and stored row-coalesced; measured faster
-      // here than per-thread row stores (two output tensors per tile and the read of the previous rows)
-      if (p.part_o) {
-        // un-merged result of this call, staged over the (now idle) Q tile
-        uint8_t* st2 = smem + Cfg::OFF_Q;
-        __syncthreads();   // all S MMAs reading Q have completed (waited above); make the reuse explicit
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    if (warp < W_Q) {
+      // ===================================================================================================
+      // MMA issue, one warp per product and group.  These warps run few instructions between two hand-offs, and every one counts:
+      // the chain of a unit passes through them.
+      // ===================================================================================================
+      constexpr int AB = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
+      const int g = warp & 1;
+      const uint32_t tG = tmem + g * 256;
+      bool ok = true;
+      uint32_t slot = warp < W_PV ? 0 : 1, full_par = 0;       // ring slot of the next K (V) tile, parity of its "full" barrier
+      uint32_t buf = 0, par = 0;                               // score buffer of the next unit, parity of its barriers
+      const bool fence_copies = !(flash && pl.tiles);          // tiles that came by cp.async
+      HA_T_DECL(8)
+      FwdItem it;
+      if (warp < W_PV) {
+        // S = Q K^T: 64 keys at a time
+        const uint32_t idesc = mma_idesc(TILE, 64, AB, 0, 0);
+        uint32_t q_seq = 0;                   // query tiles of the items so far
+        bool reused = false;                  // every score buffer has been used once
+        while (ok && next_item(it)) {
+          const uint32_t qs = q_seq + g, qslot = qs % NQ;
+          const uint64_t dQ = smem_desc(s_base + Cfg::OFF_Q + qslot * Cfg::Q_TILE, 16, 1024);
+          const bool mine = g == 0 || it.has1;
+          const int last = mine ? it.last_entry(g) : -1;
+          if (mine) ok = wait(B_Q_FULL + qslot, (qs / NQ) & 1);       // (its fence: the K tile's below)
+#pragma unroll 1
+          for (int e = 0; e < it.n_list && ok; ++e) {
+            HA_T_MARK(0)
+            // (waited for by a group the tile is not meant for, too: it may not run ahead of the ring)
+            if (!(ok = wait(B_KV_FULL + slot, full_par))) break;
+            if (fence_copies) fence_async_smem();
+            HA_T_MARK(1)
+            if (it.active(g, e)) {
+              const uint64_t dK = smem_desc(s_base + Cfg::OFF_KV + slot * Cfg::KV_TILE, 16, 1024);
 #pragma unroll
-        for (int e = 0; e < DV; e += 2)
-          *reinterpret_cast<uint32_t*>(st2 + swz_off(TILE, tid, e)) = pack2<T>(o_acc[e] * inv, o_acc[e + 1] * inv);
-        __syncwarp();
-        uint16_t* pbase = (uint16_t*)p.part_o + si.b * p.o_sb + si.h * p.o_sh + si.q_row0 * p.o_sn;
-        scatter_tile<DV>(st2, pbase, p.o_sn, qrow, warp, lane);
-        if (p.part_lse && qrow >= 0) p.part_lse[lse_at] = l_run > 0.f ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
-      }
+              for (int hf = 0; hf < 2; ++hf) {
+                // the product that read P out of this buffer has completed
+                if (reused && !(ok = wait(B_PV_DONE + 3 * g + buf, par ^ 1))) break;
+                HA_T_MARK(2)
+                tc_fence_after();
+                if (elect_one()) {
 #pragma unroll
-      for (int e = 0; e < DV; e += 2) {
-        float a = o_acc[e] * inv, b = o_acc[e + 1] * inv;
-        uint32_t* slot = reinterpret_cast<uint32_t*>(stage + swz_off(TILE, tid, e));
-        const float2 old = unpack2<T>(*slot);
-        a = w1 * old.x + w2 * round_to<T>(a);
-        b = w1 * old.y + w2 * round_to<T>(b);
-        *slot = pack2<T>(a, b);
-      }
-      __syncwarp();
-      scatter_tile<DV>(stage, obase, p.o_sn, qrow, warp, lane);
-    } else {
-      // each thread stores its own row: DV contiguous elements in 16-byte pieces straight from registers (whole 32-byte
-      // sectors pair up in L2); much less code than staging, and this code runs once per tile
-      if (p.part_o && qrow >= 0) {
-        // un-merged result of this call
-        uint4* prow = reinterpret_cast<uint4*>((uint16_t*)p.part_o + si.b * p.o_sb + si.h * p.o_sh + (si.q_row0 + qrow) * p.o_sn);
-#pragma unroll
-        for (int e = 0; e < DV; e += 8)
-          prow[e >> 3] = make_uint4(pack2<T>(o_acc[e] * inv, o_acc[e + 1] * inv), pack2<T>(o_acc[e + 2] * inv, o_acc[e + 3] * inv),
-                                    pack2<T>(o_acc[e + 4] * inv, o_acc[e + 5] * inv), pack2<T>(o_acc[e + 6] * inv, o_acc[e + 7] * inv));
-        if (p.part_lse) p.part_lse[lse_at] = l_run > 0.f ? (m_run + log2f(l_run)) * 0.6931471805599453f : -INFINITY;
-      }
-      if (qrow >= 0) {
-        uint4* orow = reinterpret_cast<uint4*>(obase + (int64_t)qrow * p.o_sn);
-#pragma unroll
-        for (int e = 0; e < DV; e += 8) {
-          uint32_t w[4];
-#pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            w[h] = pack2<T>(o_acc[e + 2 * h] * inv, o_acc[e + 2 * h + 1] * inv);
+                  for (int kk = 0; kk < D / 16; ++kk) {
+                    const uint32_t off = ((kk >> 2) * (TILE * 128) + (kk & 3) * 32) >> 4;
+                    mma_ss(tG + buf * 64, dQ + off, dK + off + hf * (8192 >> 4), idesc, kk > 0);
+                  }
+                  mma_commit(bar(B_S_READY + 3 * g + buf));
+                }
+                __syncwarp();
+                if (++buf == NB) { buf = 0; par ^= 1; reused = true; }
+                HA_T_MARK(3)
+              }
+              if (!ok) break;
+            }
+            if (elect_one()) {
+              mma_commit(bar(B_KV_EMPTY + slot));                    // this group's last read of the tile
+              if (e == last) mma_commit(bar(B_Q_EMPTY + qslot));     // ... and of the query tile
+            }
+            __syncwarp();
+            slot += 2;
+            if (slot == NKV) { slot = 0; full_par ^= 1; }
+            HA_T_MARK(4)
           }
-          orow[e >> 3] = make_uint4(w[0], w[1], w[2], w[3]);
+          q_seq += 1 + it.has1;
         }
+        HA_T_DUMP(8, (int)blockIdx.x * 8 + 1, lane == 0 && g == 0)
+      } else {
+        // O += P V
+        const uint32_t idesc = mma_idesc(TILE, DV, AB, 0, 1);
+        uint32_t n_o = 0;                     // items begun
+        while (ok && next_item(it)) {
+          const bool mine = g == 0 || it.has1;
+          const int first = it.first_entry(g), last = mine ? it.last_entry(g) : -1;
+          if (mine) {
+            if (n_o >= 1) ok = wait(B_O_FREE + g, (n_o - 1) & 1);      // the previous item's O is out
+            ++n_o;
+          }
+#pragma unroll 1
+          for (int e = 0; e < it.n_list && ok; ++e) {
+            HA_T_MARK(0)
+            if (!(ok = wait(B_KV_FULL + slot, full_par))) break;
+            if (fence_copies) fence_async_smem();
+            HA_T_MARK(1)
+            if (it.active(g, e)) {
+              const uint64_t dV = smem_desc(s_base + Cfg::OFF_KV + slot * Cfg::KV_TILE, TILE * 128, 1024);
+#pragma unroll
+              for (int hf = 0; hf < 2; ++hf) {
+                if (!(ok = wait(B_P_READY + 3 * g + buf, par))) break;
+                HA_T_MARK(2)
+                tc_fence_after();
+                if (elect_one()) {
+#pragma unroll
+                  for (int kk = 0; kk < 4; ++kk)
+                    mma_ts(tG + Cfg::COL_O, tG + buf * 64 + kk * 8, dV + hf * (8192 >> 4) + kk * (2048 >> 4), idesc, (hf + kk > 0) | (e != first));
+                  mma_commit(bar(B_PV_DONE + 3 * g + buf));
+                }
+                __syncwarp();
+                if (++buf == NB) { buf = 0; par ^= 1; }
+                HA_T_MARK(3)
+              }
+              if (!ok) break;
+            }
+            if (elect_one()) {
+              if (e == last) mma_commit(bar(B_O_FULL + g));
+              mma_commit(bar(B_KV_EMPTY + slot));                    // this group's last read of the tile
+            }
+            __syncwarp();
+            slot += 2;
+            if (slot > NKV) { slot = 1; full_par ^= 1; }
+            HA_T_MARK(4)
+          }
+        }
+        HA_T_DUMP(8, (int)blockIdx.x * 8 + 6, lane == 0 && g == 0)
       }
+    } else {
+      // ===================================================================================================
+      // loaders: query tiles, K tiles, V tiles (a warp each for the even and the odd list entries).  The copies of a tile signal its "full"
+      // barrier themselves (TMA by their bytes, cp.async by an arrival of every lane), so a loader only waits for free slots and
+      // runs ahead across items; the row numbers of its next tile are requested before it waits for this one's slot.
+      // The query loader is the scheduler too: it works out the items and publishes their descriptors two items ahead.
+      // ===================================================================================================
+      const bool is_q = warp == W_Q, is_k = warp == W_K;
+      const CUtensorMap* map = &maps.tile[is_q ? 0 : is_k ? 1 : 2];
+      const uint16_t* tensor = (const uint16_t*)(is_q ? p.q : is_k ? p.k : p.v);
+      const int64_t sb = is_q ? p.q_sb : is_k ? p.k_sb : p.v_sb, sh = is_q ? p.q_sh : is_k ? p.k_sh : p.v_sh, sn = is_q ? p.q_sn : is_k ? p.k_sn : p.v_sn;
+      const int slabs = is_q || is_k ? D / 64 : DV / 64;
+      const int b_full = is_q ? B_Q_FULL : B_KV_FULL, b_empty = is_q ? B_Q_EMPTY : B_KV_EMPTY;
+      const uint32_t ring = is_q ? NQ : NKV;
+      const uint32_t s_ring = s_base + (is_q ? Cfg::OFF_Q : Cfg::OFF_KV), s_step = is_q ? Cfg::Q_TILE : Cfg::KV_TILE;
+      const int stride = is_q || is_k ? 1 : 2;      // list entries from one tile of this warp to the next
+      uint32_t n = is_q || is_k ? 0 : 2 * (warp & 1) + 1;      // ring position of this warp's next tile
+      int published = 0;
+      auto take = [&](FwdItem& it) -> bool {        // the next item's descriptor; n_list = 0 past the last one
+        if (!is_q) return next_item(it);
+#pragma unroll 1
+        for (; published <= (int)n_item + 2; ++published) {
+          const uint32_t slot = published % ND;
+          it.n_list = 0;
+          const int item = blockIdx.x + published * gridDim.x;
+          if (item < pl.n_items) it = fwd_item(p, pl, item, flash);
+          if (published >= ND && !wait(B_D_EMPTY + slot, (published / ND - 1) & 1)) return false;
+          if (lane == 0) {
+            s_item[slot] = it;
+            mbar_arrive(bar(B_D_FULL + slot));
+          }
+          __syncwarp();
+        }
+        it = s_item[n_item % ND];
+        ++n_item;
+        return it.n_list != 0;
+      };
+      // indexed tiles by TMA: all of K, and the first query tile -- what is left for the cp.async warps then is a tile each per item
+      auto by_gather4 = [&](int e) -> bool { return is_k ? pl.rows & 2 : is_q && e == 0 && (pl.rows & 1); };
+      auto row_numbers = [&](const FwdItem& it, int e, int (&rows)[4]) {
+        const bool gathered = by_gather4(e);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int r = gathered ? 4 * lane + q : 32 * q + lane;
+          if (is_q) {
+            const int pos = (it.qt0 + e) * TILE + r;
+            rows[q] = pos >= p.m_q ? -1 : flash ? pos : p.q_idx[(long long)it.seg * p.m_q + pos];
+          } else {
+            rows[q] = fwd_key_row(p, it, e, r, flash);
+          }
+        }
+      };
+      auto is_boxed = [&](const FwdItem& it, int e) -> bool { return pl.tiles && (flash || (!is_q && e >= it.n_win && !p.sample_idx)); };
+      HA_T_DECL(8)
+      FwdItem it;
+      int e = is_q || is_k ? 0 : warp & 1;
+      // moves (it, e) to this warp's next tile; e may lie past the end of the item
+      auto settle = [&]() -> bool {
+        while (true) {
+          const int cnt = is_q ? 1 + it.has1 : it.n_list;
+          if (e < cnt) return true;
+          e -= cnt;
+          if (!take(it)) return false;
+        }
+      };
+      bool more = take(it) && settle();
+      int rows[4] = {0, 0, 0, 0};
+      if (more && !is_boxed(it, e)) row_numbers(it, e, rows);
+      while (more) {
+        // this tile
+        const bool boxed = is_boxed(it, e), gathered = !boxed && by_gather4(e);
+        const int hd = is_q ? it.h : it.hk, b = it.b, row0 = is_q ? it.q_row0 : it.k_row0;
+        const int tile0 = row0 + (is_q ? it.qt0 + e : flash ? e : e - it.n_win) * TILE;
+        // the next one
+        e += stride;
+        more = settle();
+        int ahead[4] = {0, 0, 0, 0};
+        if (more && !is_boxed(it, e)) row_numbers(it, e, ahead);
+        const uint32_t slot = n % ring, dst = s_ring + slot * s_step, full = bar(b_full + slot);
+        HA_T_MARK(0)
+        if (n >= ring && !wait(b_empty + slot, (n / ring - 1) & 1)) break;
+        HA_T_MARK(1)
+        if (boxed) {
+          const int ur = __shfl_sync(0xffffffffu, tile0, 0), uh = __shfl_sync(0xffffffffu, hd, 0), ub = __shfl_sync(0xffffffffu, b, 0);
+          if (elect_one()) {
+            mbar_expect_tx(full, TILE * 128 * slabs);
+#pragma unroll
+            for (int s = 0; s < Cfg::W / 64; ++s)
+              if (s < slabs) tma_tile(dst + s * TILE * 128, map, s * 64, ur, uh, ub, full);
+          } else {
+            mbar_arrive(full);
+          }
+          __syncwarp();
+        } else if (gathered) {
+          const int x = is_k, step = pl.row_sn[x], base = b * pl.row_sb[x] + hd * pl.row_sh[x] + row0 * step;
+          mbar_expect_tx(full, 512 * slabs);     // this lane's four rows
+#pragma unroll 1
+          for (int s = 0; s < slabs; ++s)
+            tma_gather4(dst + s * TILE * 128 + lane * 512, &maps.rows[x], s * 64, base + rows[0] * step, base + rows[1] * step,
+                        base + rows[2] * step, base + rows[3] * step, full);
+        } else {
+          warp_gather_tile(dst, tensor + b * sb + hd * sh + row0 * sn, sn, slabs, rows, lane);
+          asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(full) : "memory");
+        }
+        // the next tile's rows into L2 (a copy that finds them there holds its place in the queue for half the time)
+        if (!flash && more && !is_boxed(it, e) && (is_q || e < it.n_win)) {
+          const uint16_t* base = tensor + it.b * sb + (is_q ? it.h : it.hk) * sh + (int64_t)(is_q ? it.q_row0 : it.k_row0) * sn;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            prefetch_l2(base + (int64_t)ahead[q] * sn);
+            if (slabs > 1) prefetch_l2(base + (int64_t)ahead[q] * sn + 64);
+          }
+        }
+        HA_T_MARK(2)
+        n += is_q ? 1 : 2 * stride;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) rows[q] = ahead[q];
+      }
+      HA_T_DUMP(8, (int)blockIdx.x * 8 + (is_k ? 2 : is_q ? 4 : 3), lane == 0 && (warp <= W_K + 1))
+      cp_async_commit();
+      cp_async_wait<0>();      // nothing of this warp is in flight when the CTA retires
     }
-    if (qrow >= 0) p.lse[lse_at] = lse;
   }
-
-  HA_T_MARK(6)
-  HA_T_DUMP(8, (int)(blockIdx.y * gridDim.x + blockIdx.x), tid == 0)
+  // every role is done (or has given up); TMEM goes back
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, Cfg::TMEM_COLS);
+  if (tid == 0 && s_abort) report_timeout(p.status, p.status_host);
+  if (warp == W_S) tmem_dealloc(tmem, 512);
 }
 
-template <typename T, int D, int DV, bool WT>
+template <typename T, int D, int DV, int KIND>
 static int launch_fwd(const ha_attn_params& p, cudaStream_t st) {
   using Cfg = FwdCfg<D, DV>;
   const long long segs = (long long)p.B * p.H * p.segs_per_head;
-  const int n_qt = (p.m_q + TILE - 1) / TILE;
-  if (segs == 0 || n_qt == 0) return HA_OK;
-  if (segs > 65535) return HA_ERR_INVALID;
-  HA_SMEM_ATTR_ONCE((attn_tc_fwd_kernel<T, D, DV, WT>), Cfg::SMEM, "ha_attn_fwd smem attribute");
-  // CTAs resident at once (shared memory and TMEM allow two per SM at head dim 64, one otherwise) = prefetch distance
+  FwdPlan pl;
+  pl.pairs = ((p.m_q + TILE - 1) / TILE + 1) / 2;
+  const long long items = segs * pl.pairs;
+  if (items == 0) return HA_OK;
+  if (items > 0x7fffffffLL) return HA_ERR_TOO_LARGE;
+  pl.n_items = (int)items;
+  pl.by_pairs = FastDiv(pl.pairs);
+  pl.by_segs = FastDiv(p.segs_per_head);
+  pl.by_heads = FastDiv(p.H);
+  pl.by_group = FastDiv(p.kv_group > 1 ? p.kv_group : 1);
+  pl.by_block = FastDiv(p.mode == HA_MODE_HYPER ? (p.block_size + TILE - 1) / TILE : 1);
+  FwdMaps maps;
+  const int Hk = p.kv_group > 1 ? p.H / p.kv_group : p.H;
+  // rows a head really has on either side (a single-segment call may have fewer or more keys than queries)
+  const long long n_q = p.segs_per_head > 1 ? (long long)p.segs_per_head * p.span : p.q_off + p.m_q;
+  const long long n_k = p.segs_per_head > 1 ? (long long)p.segs_per_head * p.span : p.k_off + p.m_k;
+  pl.tiles = encode_tile_map(&maps.tile[0], p.dtype, p.q, D, n_q, p.H, p.B, p.q_sn, p.q_sh, p.q_sb, TILE) &&
+             encode_tile_map(&maps.tile[1], p.dtype, p.k, D, n_k, Hk, p.B, p.k_sn, p.k_sh, p.k_sb, TILE) &&
+             encode_tile_map(&maps.tile[2], p.dtype, p.v, DV, n_k, Hk, p.B, p.v_sn, p.v_sh, p.v_sb, TILE);
+  pl.rows = 0;
+  for (int x = 0; x < 2 && p.mode == HA_MODE_HYPER; ++x) {
+    const int heads = x ? Hk : p.H;
+    const int64_t sn = x ? p.k_sn : p.q_sn, sh = x ? p.k_sh : p.q_sh, sb = x ? p.k_sb : p.q_sb;
+    int64_t pitch = 1;
+    if (!encode_row_map(&maps.rows[x], p.dtype, x ? p.k : p.q, D, x ? n_k : n_q, heads, p.B, sn, sh, sb, &pitch)) continue;
+    pl.rows |= 1 << x;
+    pl.row_sn[x] = (int)(sn / pitch);
+    pl.row_sh[x] = heads > 1 ? (int)(sh / pitch) : 0;      // (the encoder has seen that every row number fits)
+    pl.row_sb[x] = p.B > 1 ? (int)(sb / pitch) : 0;
+  }
+  // the tiles start at the first 1 KB boundary after the static variables; at head dim 128 they end with the CTA's last byte
+  static int dyn_bytes = 0;
+  if (dyn_bytes == 0) {
+    cudaFuncAttributes fa;
+    HA_CUDA_OK(cudaFuncGetAttributes(&fa, attn_tc_fwd_kernel<T, D, DV, KIND>), "ha_attn_fwd kernel attributes");
+    const int stat = ((int)fa.sharedSizeBytes + 15) / 16 * 16;
+    dyn_bytes = (1024 - stat % 1024) % 1024 + Cfg::SMEM_USED;
+  }
+  HA_SMEM_ATTR_ONCE((attn_tc_fwd_kernel<T, D, DV, KIND>), dyn_bytes, "ha_attn_fwd smem attribute");
   const int sms = sm_count();
-  const int pf_dist = p.mode == HA_MODE_HYPER ? sms * (Cfg::TMEM_COLS == 256 ? 2 : 1) : 0;
-  attn_tc_fwd_kernel<T, D, DV, WT><<<dim3(n_qt, (unsigned)segs), 128, Cfg::SMEM, st>>>(p, pf_dist);
+  attn_tc_fwd_kernel<T, D, DV, KIND><<<(unsigned)(items < sms ? items : sms), fw::THREADS, dyn_bytes, st>>>(p, pl, maps);
   HA_LAUNCHED("ha_attn_fwd (tcgen05)");
   return HA_OK;
 }
@@ -527,7 +776,7 @@ bool tc_supported(const ha_attn_params& p) {
   if (p.dtype != HA_BF16 && p.dtype != HA_FP16) return false;
   if (!(p.scale > 0.f)) return false;   // the running max is taken before scaling
   if (!((p.d == 64 || p.d == 128) && (p.dv == 64 || p.dv == 128))) return false;
-  // 16-byte row alignment for the cp.async gathers and vector stores
+  // 16-byte row alignment for the copies and vector stores
   auto ok = [](const void* ptr, int64_t sb, int64_t sh, int64_t sn) {
     return ((uintptr_t)ptr % 16 == 0) && sb % 8 == 0 && sh % 8 == 0 && sn % 8 == 0;
   };
@@ -535,26 +784,26 @@ bool tc_supported(const ha_attn_params& p) {
       !ok(p.o, p.o_sb, p.o_sh, p.o_sn))
     return false;
   if (p.part_o && (uintptr_t)p.part_o % 16 != 0) return false;
-  if ((long long)p.B * p.H * p.segs_per_head > 65535) return false;
   return true;
 }
 
-int tc_attn_fwd(const ha_attn_params& p, cudaStream_t st) {
-#define HA_FWD_CASE(TT, DD, DDV) \
-  if (p.d == DD && p.dv == DDV) return p.sample_logw ? launch_fwd<TT, DD, DDV, true>(p, st) : launch_fwd<TT, DD, DDV, false>(p, st);
-  if (p.dtype == HA_BF16) {
-    HA_FWD_CASE(__nv_bfloat16, 64, 64)
-    HA_FWD_CASE(__nv_bfloat16, 128, 128)
-    HA_FWD_CASE(__nv_bfloat16, 128, 64)
-    HA_FWD_CASE(__nv_bfloat16, 64, 128)
-  } else {
-    HA_FWD_CASE(__half, 64, 64)
-    HA_FWD_CASE(__half, 128, 128)
-    HA_FWD_CASE(__half, 128, 64)
-    HA_FWD_CASE(__half, 64, 128)
-  }
+template <typename T>
+static int tc_fwd_typed(const ha_attn_params& p, cudaStream_t st) {
+  const bool any = (p.flags & HA_FLAG_MERGE) || p.part_o || (p.mode == HA_MODE_HYPER && p.sample_logw && p.sample_size > 0);
+#define HA_FWD_CASE(DD, DDV)                                                              \
+  if (p.d == DD && p.dv == DDV)                                                           \
+    return any ? launch_fwd<T, DD, DDV, FWD_ANY>(p, st)                                   \
+               : p.mode == HA_MODE_FLASH ? launch_fwd<T, DD, DDV, FWD_FLASH>(p, st) : launch_fwd<T, DD, DDV, FWD_HYPER>(p, st);
+  HA_FWD_CASE(64, 64)
+  HA_FWD_CASE(128, 128)
+  HA_FWD_CASE(128, 64)
+  HA_FWD_CASE(64, 128)
 #undef HA_FWD_CASE
   return HA_ERR_INVALID;
+}
+
+int tc_attn_fwd(const ha_attn_params& p, cudaStream_t st) {
+  return p.dtype == HA_BF16 ? tc_fwd_typed<__nv_bfloat16>(p, st) : tc_fwd_typed<__half>(p, st);
 }
 
 }  // namespace ha

@@ -36,6 +36,17 @@ void set_cuda_error(cudaError_t e, const char* where);
 
 inline int dtype_size(int dtype) { return dtype == HA_FP32 ? 4 : 2; }
 
+// n / d for 0 <= n < 2^31 by one wide multiplication and a shift (m = ceil(2^(31 + s) / d), s = ceil(log2 d): the round-up method).
+struct FastDiv {
+  uint32_t m = 1u << 31, s = 0;
+  FastDiv() = default;
+  explicit FastDiv(uint32_t d) {
+    while ((1ull << s) < d) ++s;
+    m = (uint32_t)(((1ull << (31 + s)) + d - 1) / d);
+  }
+  __host__ __device__ __forceinline__ int operator()(int n) const { return (int)(((unsigned long long)(uint32_t)n * m) >> (31 + s)); }
+};
+
 // Number of SMs of the current device, looked up once per device.
 inline int sm_count() {
   static std::atomic<int> cache[64];
@@ -109,6 +120,14 @@ __device__ __forceinline__ void mbar_fence_init() { asm volatile("fence.mbarrier
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("{\n .reg .b64 st;\n mbarrier.arrive.shared::cta.b64 st, [%0];\n}\n" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+               : "=r"(ok)
+               : "r"(bar), "r"(parity)
+               : "memory");
+  return ok != 0;
+}
 // Bounded wait: returns false when the phase did not complete within SPIN_LIMIT polls or WAIT_CYCLES cycles.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
   const long long t0 = clock64();
@@ -123,6 +142,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     if (clock64() - t0 > WAIT_CYCLES) return false;
   }
   return false;
+}
+
+// The same inside a kernel whose roles share an abort flag: whoever gives up raises it, everybody else leaves at the next wait.
+// (A poll may itself suspend the thread for a while; the time cap, about a second, is what bounds the wait.)
+__device__ __forceinline__ bool mbar_wait_or_abort(uint32_t bar, uint32_t parity, int* abort_flag) {
+  if (__builtin_expect(mbar_try_wait(bar, parity), 1)) return true;
+  const uint32_t t0 = (uint32_t)clock();
+#pragma unroll 1
+  while (!mbar_try_wait(bar, parity)) {
+    if ((uint32_t)clock() - t0 > (uint32_t)WAIT_CYCLES) *reinterpret_cast<volatile int*>(abort_flag) = 1;
+    if (*reinterpret_cast<volatile int*>(abort_flag)) return false;
+  }
+  return true;
 }
 
 // 16-byte async copy global -> shared; src_bytes = 0 zero-fills the destination.
@@ -182,6 +214,13 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d_tmem),
       "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+// One lane of the (converged) warp, always the same one.  Around tcgen05 instructions in warp-uniform code it lets the compiler keep
+// descriptors in uniform registers; a `lane == 0` branch does not (measured: 64 against 126 cycles per N = 128 instruction).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n .reg .pred P;\n .reg .b32 R;\n elect.sync R|P, 0xFFFFFFFF;\n selp.u32 %0, 1, 0, P;\n}\n" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -294,13 +333,14 @@ static __device__ unsigned long long* g_timing_buf = nullptr;   // one per trans
 #endif
 
 // A bounded wait gave up: record it in the device status word and, if the caller gave one, in the host-visible word.
-__device__ __forceinline__ void report_timeout(int32_t* status, int32_t* status_host) {
-  if (status) atomicExch(status, HA_DEV_TIMEOUT);
+__device__ __forceinline__ void report_status(int32_t* status, int32_t* status_host, int32_t code) {
+  if (status) atomicExch(status, code);
   if (status_host) {
-    *reinterpret_cast<volatile int32_t*>(status_host) = HA_DEV_TIMEOUT;
+    *reinterpret_cast<volatile int32_t*>(status_host) = code;
     __threadfence_system();
   }
 }
+__device__ __forceinline__ void report_timeout(int32_t* status, int32_t* status_host) { report_status(status, status_host, HA_DEV_TIMEOUT); }
 // Did an earlier CTA of this (or a previous) launch give up?  One thread reads the word and the whole CTA branches on
 // the shared copy, so the answer is the same for every thread even while another CTA is writing the word.
 // Contains a __syncthreads(): call it from every thread of the CTA.
@@ -317,6 +357,31 @@ __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// 2^x of two values on the FMA and integer pipes, for the share of a softmax's exponentials that the exponential unit (four lanes a clock
+// and scheduler) cannot take: x = n + f with n the nearest integer (Cody-Waite, by adding and subtracting 1.5 * 2^23),
+// 2^f on [-1/2, 1/2] by a degree 5 polynomial with value 1 at 0 whose largest relative error is minimal (found as a linear
+// programme over 4001 Chebyshev points; 1.7e-7 in fp32 arithmetic, the exponential unit's own bound is 2.4e-7), n added to the
+// exponent field.  Arguments below -127, -infinity among them, give 0; arguments are at most about 8 here, 127 in general.
+__device__ __forceinline__ void poly_exp2_2(uint64_t x2, float& lo, float& hi) {
+  float a, b;
+  unpack_f2(x2, a, b);
+  x2 = pack_f2(fmaxf(a, -127.f), fmaxf(b, -127.f));
+  const uint64_t magic = pack_f2(12582912.f, 12582912.f), nmagic = pack_f2(-12582912.f, -12582912.f), mone = pack_f2(-1.f, -1.f);
+  const uint64_t r = fadd2(x2, magic);
+  const uint64_t f = ffma2(fadd2(r, nmagic), mone, x2);
+  auto c = [](float v) { return pack_f2(v, v); };
+  uint64_t q = ffma2(f, c(0x1.5bba14p-10f), c(0x1.3cea88p-7f));
+  q = ffma2(f, q, c(0x1.c6b752p-5f));
+  q = ffma2(f, q, c(0x1.ebf9bcp-3f));
+  q = ffma2(f, q, c(0x1.62e42ap-1f));
+  q = ffma2(f, q, c(1.f));
+  float ra, rb;
+  unpack_f2(r, ra, rb);
+  unpack_f2(q, a, b);
+  lo = __uint_as_float(__float_as_uint(a) + (__float_as_uint(ra) << 23));
+  hi = __uint_as_float(__float_as_uint(b) + (__float_as_uint(rb) << 23));
 }
 
 }  // namespace ha

@@ -30,17 +30,32 @@ ROLES = {0: ('elementwise group 0', ['wait S^T/dP^T ready', 'wait lse/delta (+ s
          6: ('dQ issuer', ['loop', 'wait dS slabs full', 'wait dQ drained', 'fences, 8 MMAs, commits']),
          7: ('Q / dO loader warp', ['index loads, L2 prefetch', 'wait stage empty', 'issuing the copies of two tiles'])}
 
-# attn_tc_fwd_ws_kernel, softmax group 0: (counter slot, phase)
-FWD_PHASES = [(0, 'item set-up, loop (row index, accumulator clear)'), (1, 'wait S ready'),
-              (3, 'max pass, previous product (wait + fold), exp pass, P store'), (4, "the item's last product: wait + fold"),
-              (6, 'epilogue: normalise, pack, row stores'), (5, 'lse store')]
+# attn_tc_fwd_kernel
+FWD_ROLES = {0: ('softmax group 0', ['loop, item set-up', 'wait S ready', 'scores out of TMEM, maximum, rescale', 'exponentials, P, sum',
+                                     'P store wait, arrival']),
+             1: ('S warp of group 0', ['loop, item set-up', 'wait K tile', 'wait score buffer free', 'issue', 'tile done']),
+             6: ('P V warp of group 0', ['loop, item set-up', 'wait V tile', 'wait P ready', 'issue', 'tile done']),
+             2: ('K loader', ['index loads', 'wait slot free', 'issue copies']), 3: ('V loader', ['index loads', 'wait slot free', 'issue copies']),
+             4: ('Q loader', ['index loads', 'wait slot free', 'issue copies']),
+             5: ('epilogue group', ['item set-up', 'wait O complete', 'O out of TMEM', 'merge, stores'])}
+
+
+def report(b, roles):
+    for r, (name, phases) in roles.items():
+        bb = b[:, r]
+        tot = bb[:, :8].sum(1).mean().item()
+        print(f'{name}: {round(tot)} cycles per CTA')
+        for i, ph in enumerate(phases):
+            print(f'   {ph:46s} {bb[:, i].mean().item():11.0f} {100 * bb[:, i].mean().item() / max(tot, 1):5.1f}%')
 
 
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument('--heads', type=int, default=32)
     ap.add_argument('--seq-len', type=int, default=131072)
-    ap.add_argument('--forward', action='store_true', help='the forward kernel (attn_tc_fwd_ws_kernel) instead of the backward')
+    ap.add_argument('--forward', action='store_true', help='the forward kernel (attn_tc_fwd_kernel) instead of the backward')
+    ap.add_argument('--dim', type=int, default=64)
+    ap.add_argument('--causal', action='store_true', help='(forward) the last launch of a causal call; exact attention when --seq-len <= 2048')
     a = ap.parse_args()
     path = os.path.join(os.path.dirname(os.path.abspath(__file__)), 'libhyperattn_b200_timing.so')
     assert os.path.exists(path), 'build the instrumented library first: python hyperattention_b200/csrc/build.py --timing'
@@ -48,24 +63,21 @@ def main():
     lib = _lib.load()
     from .module import HyperAttention
     torch.manual_seed(0)
-    q, k, v, do = [torch.randn(1, a.heads, a.seq_len, 64, device='cuda', dtype=torch.bfloat16) for _ in range(4)]
-    mod = HyperAttention(input_dim=64).to(device='cuda', dtype=torch.bfloat16)
+    q, k, v, do = [torch.randn(1, a.heads, a.seq_len, a.dim, device='cuda', dtype=torch.bfloat16) for _ in range(4)]
+    mod = HyperAttention(input_dim=a.dim).to(device='cuda', dtype=torch.bfloat16)
     buf = torch.zeros(4096 * 16, dtype=torch.int64, device='cuda')
     n_cta = min(148, a.heads * a.seq_len // 256)
     if a.forward:
         with torch.no_grad():
-            mod(q, k, v)
+            mod(q, k, v, causal=a.causal)
             torch.cuda.synchronize()
-            setter = lib.ha_debug_set_timing_buffer_fwd_ws
+            setter = lib.ha_debug_set_timing_buffer_fwd
             setter.restype, setter.argtypes = C.c_int, [C.c_void_p]
             setter(C.c_void_p(buf.data_ptr()))
-            mod(q, k, v)
+            mod(q, k, v, causal=a.causal)
             torch.cuda.synchronize()
-        b = buf.view(4096, 16).cpu().float()[:n_cta, :8]
-        tot = b.sum(1).mean().item()
-        print(f'softmax group 0 (thread 0): {round(tot)} cycles per CTA, {round(tot / max(1, a.heads * a.seq_len // 256 / n_cta))} per work item')
-        for i, ph in FWD_PHASES:
-            print(f'   {ph:58s} {b[:, i].mean().item():11.0f} {100 * b[:, i].mean().item() / max(tot, 1):5.1f}%')
+        print(f'{a.heads * a.seq_len // 256 / n_cta:.1f} work items per CTA (non-causal call)')
+        report(buf.view(4096, 16).cpu().float()[:n_cta * 8].view(n_cta, 8, 16), FWD_ROLES)
         return
     qg, kg, vg = [t.clone().requires_grad_() for t in (q, k, v)]
     for rep in range(2):
@@ -77,12 +89,7 @@ def main():
         o.backward(do)
         torch.cuda.synchronize()
     b = buf.view(4096, 16).cpu().float()[:n_cta * 8].view(n_cta, 8, 16)
-    for r, (name, phases) in ROLES.items():
-        bb = b[:, r]
-        tot = bb[:, :8].sum(1).mean().item()
-        print(f'{name}: {round(tot)} cycles per CTA')
-        for i, ph in enumerate(phases):
-            print(f'   {ph:46s} {bb[:, i].mean().item():11.0f} {100 * bb[:, i].mean().item() / max(tot, 1):5.1f}%')
+    report(b, ROLES)
 
 
 if __name__ == '__main__':

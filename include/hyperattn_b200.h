@@ -47,8 +47,8 @@ enum {
   HA_FLAG_MERGE_EXACT = 8,   /* with MERGE: plain log-sum-exp combine instead of the reference's rounded formula */
   HA_FLAG_BWD_REF_SMOOTH = 16,/* backward + SMOOTH: enumerate pairs per key tile as the reference backward does */
   HA_FLAG_FORCE_SIMT = 32,   /* use the fp32 CUDA-core kernels even where a tensor-core kernel exists */
-  HA_FLAG_NO_WS = 128,       /* keep the earlier kernels (forward: one tile per CTA; backward: one thread-block role) where the
-                                persistent warp-specialised ones apply */
+  HA_FLAG_NO_WS = 128,       /* backward: keep the earlier kernel (one thread-block role) where the warp-specialised one applies
+                                (the forward has one kernel and takes no notice) */
   HA_FLAG_CHECK_INDICES = 256,/* HA_MODE_HYPER, needs `status`: a checking kernel runs first and looks at every entry of q_idx, k_idx
                                 and sample_idx; an entry outside [0, rows of the segment) sets the status words to
                                 HA_DEV_BAD_INDEX, and the attention kernel that follows returns at once instead of reading

@@ -1,0 +1,102 @@
+"""The attention kernels where their tiles, lists of key tiles and loaders change shape, forward and backward, against the oracle."""
+import pytest
+import torch
+
+from oracle import hyper_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+T = lambda x: x.transpose(1, 2)
+TOL = {torch.float32: (1e-4, 2e-4), torch.bfloat16: (2e-2, 3e-2), torch.float16: (2e-2, 3e-2)}
+
+
+def rel(a, b):
+    a, b = a.detach().float().cpu(), b.detach().float().cpu()
+    return ((a - b).norm() / b.norm().clamp_min(1e-30)).item()
+
+
+def _check(got, want, dtype):
+    t_out, t_grad = TOL[dtype]
+    errs = [rel(g, w) for g, w in zip(got, want)]
+    assert max(errs[:2]) < t_out and max(errs[2:], default=0.) < t_grad, errs
+
+
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize('cfg', [
+    # B, H, n, d, dv, block, sample, smooth
+    (1, 2, 128, 64, 64, 256, 128, False),      # a single query tile, a window cut to one tile
+    (2, 1, 640, 64, 64, 128, 128, False),      # one-tile blocks: the two tiles of a pair have windows of their own
+    (1, 3, 896, 64, 64, 384, 0, False),        # three-tile blocks: pairs that straddle two blocks; nothing sampled
+    (1, 2, 1152, 128, 128, 384, 128, False),   # ... at head dim 128, last block cut
+    (1, 2, 896, 64, 64, 512, 384, True),       # smooth windows of four tiles, an odd number of query tiles
+    (1, 2, 640, 128, 128, 256, 256, True),
+    (1, 1, 512, 64, 128, 256, 128, False),     # dv != d, both ways
+    (1, 1, 512, 128, 64, 256, 128, False),
+    (1, 160, 256, 64, 64, 256, 256, False),    # more items than CTAs: every ring wraps
+    (1, 84, 512, 128, 128, 256, 256, False),
+])
+def test_hyper_pattern_edges(dtype, cfg):
+    import hyperattention_b200 as ha
+    from hyperattention_b200 import _lib as L
+    B, H, n, d, dv, block, sample, smooth = cfg
+    torch.manual_seed(70)
+    q, k, do = torch.randn(B, H, n, d).to(dtype), torch.randn(B, H, n, d).to(dtype), torch.randn(B, H, n, dv).to(dtype)
+    v = torch.randn(B, H, n, dv).to(dtype)
+    qi, ki = [torch.sort(torch.randint(0, 16, (B, H, n)), dim=2, stable=True)[1] for _ in range(2)]
+    qg, kg, vg = [t.cuda().requires_grad_() for t in (q, k, v)]
+    o, lse = ha.hyper_attn_func(T(qg), T(kg), T(vg), T(qi.cuda()), T(ki.cuda()), block, sample, None, smooth, None,
+                                L.FLAG_BWD_REF_SMOOTH if smooth else 0)
+    T(o).backward(do.cuda())
+    h = slice(0, 2) if H > 4 else slice(None)           # heads are independent: two of many are enough
+    qc, kc, vc = [t[:, h].float().requires_grad_() for t in (q, k, v)]
+    ow, lw = O.hyper_attn_func(T(qc), T(kc), T(vc), T(qi[:, h]), T(ki[:, h]), block, sample, None, smooth, None, False)
+    T(ow).backward(do[:, h].float())
+    _check((T(o)[:, h], lse[:, h], qg.grad[:, h], kg.grad[:, h], vg.grad[:, h]), (T(ow), lw, qc.grad, kc.grad, vc.grad), dtype)
+
+
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize('n', [1, 63, 64, 65, 127, 128, 129, 191, 257, 385, 700])
+@pytest.mark.parametrize('causal', [True, False])
+@pytest.mark.parametrize('d', [64, 128])
+def test_exact_attention_lengths(dtype, n, causal, d):
+    import hyperattention_b200 as ha
+    torch.manual_seed(71)
+    B, H = 2, 2
+    q, k, v, do = [torch.randn(B, n, H, d).to(dtype) for _ in range(4)]
+    qg, kg, vg = [t.cuda().requires_grad_() for t in (q, k, v)]
+    o, lse = ha.flash_attn_func(qg, kg, vg, None, causal, None)
+    o.backward(do.cuda())
+    qc, kc, vc = [t.float().requires_grad_() for t in (q, k, v)]
+    ow, lw = O.flash_attn_func(qc, kc, vc, None, causal, None)
+    ow.backward(do.float())
+    g = 3 if n > 1 else 1          # one key: dq and dk are zero but for rounding
+    _check((o, lse[:, :, :n]) + (vg.grad, qg.grad, kg.grad)[:g], (ow, lw[:, :, :n]) + (vc.grad, qc.grad, kc.grad)[:g], dtype)
+
+
+@pytest.mark.parametrize('nq,nk', [(300, 77), (77, 300), (128, 1000)])
+def test_exact_attention_unequal_lengths_and_layouts(nq, nk):
+    """fewer / more keys than queries; K/V heads expanded with stride 0, which no tensor map can describe; sequence-major tensors"""
+    import hyperattention_b200 as ha
+    torch.manual_seed(72)
+    B, H, d = 2, 3, 64
+    q = torch.randn(B, nq, H, d).bfloat16()
+    k, v = [torch.randn(B, nk, 1, d).bfloat16().expand(-1, -1, H, -1) for _ in range(2)]
+    o, lse = ha.flash_attn_func(q.cuda(), k.cuda()[:, :, :1].expand(-1, -1, H, -1), v.cuda()[:, :, :1].expand(-1, -1, H, -1))
+    ow, lw = O.flash_attn_func(q.float(), k.float(), v.float())
+    assert rel(o, ow) < 2e-2 and rel(lse[:, :, :nq], lw[:, :, :nq]) < 2e-2
+    qs, ks, vs = [t.contiguous().permute(1, 0, 2, 3).contiguous().cuda().permute(1, 0, 2, 3) for t in (q, k, v)]     # [n, B, H, d] memory
+    o2, lse2 = ha.flash_attn_func(qs, ks, vs)
+    assert torch.equal(o2, o) and torch.equal(lse2, lse)
+
+
+def test_rows_that_see_no_key_of_a_tile():
+    """weighted sampling in which whole sampled tiles are dropped for a query tile (every sampled key lies in its window)"""
+    import hyperattention_b200 as ha
+    torch.manual_seed(73)
+    B, H, n, d = 1, 2, 512, 64
+    q, k, v = [torch.randn(B, H, n, d).bfloat16() for _ in range(3)]
+    qi, ki = [torch.sort(torch.randint(0, 4, (B, H, n)), dim=2, stable=True)[1] for _ in range(2)]
+    sidx = ki[:, :, :128].contiguous()                  # the first window tile's keys: dropped for the first block, kept for the second
+    o, lse = ha.hyper_attn_func(T(q.cuda()), T(k.cuda()), T(v.cuda()), T(qi.cuda()), T(ki.cuda()), 256, 128, None, False, sidx.cuda(), 0, True)
+    ow, lw = O.hyper_attn_func(T(q.float()), T(k.float()), T(v.float()), T(qi), T(ki), 256, 128, None, False, sidx, False, True)
+    assert rel(o, ow) < 2e-2 and rel(lse, lw) < 2e-2
