@@ -2,7 +2,7 @@
 // warp-specialised kernel for both patterns (sorted block windows + sampled rows; exact attention with or without mask).
 //
 // One CTA of 640 threads per SM walks work items; an item is a PAIR of 128-row query tiles of one segment and the list of
-// key tiles the two pair with (FwdItem): every key tile is fetched once for both.  Roles:
+// key tiles the two pair with (AttnItem): every key tile is fetched once for both.  Roles:
 //   * softmax groups 0 / 1 (128 threads each; thread = query row = TMEM lane) of the pair's two query tiles: maximum of the row's 128
 //     scores, then P = exp2(S - reference) back to TMEM in the input dtype and the row's sum.  The reference only moves when
 //     the running maximum has grown by more than 8 (powers of two) beyond it -- any reference gives the same quotient, and
@@ -24,8 +24,7 @@
 // next units is there before a group asks for it, so a group goes from one unit to the next without waiting.
 // What bounds it: the exponential unit (16 a clock and SM: 1024 cycles per 128 x 128 tile), which is why a part of the exponentials
 // is computed on the FMA pipe (poly_exp2_2), and at head dim 128 the tensor pipe.
-#include "attn_index.cuh"
-#include "tensor_map.cuh"
+#include "attn_items.cuh"
 
 #include <type_traits>
 
@@ -54,122 +53,12 @@ constexpr float REF_SLACK = 8.f;
 }  // namespace fw
 
 struct FwdMaps { CUtensorMap tile[3], rows[2]; };    // tiles of q, k, v; rows of q, k
-struct FwdPlan {
-  FastDiv by_pairs, by_segs, by_heads, by_group, by_block;     // pairs, segs_per_head, H, kv_group, window tiles per block
-  int n_items, pairs;                 // items = pairs of query tiles x segments
-  int tiles, rows;                    // contiguous rows may be loaded as TMA boxes / indexed rows of q (1) and k (2) by gather4
-  int row_sb[2], row_sh[2], row_sn[2];   // row maps of q, k: steps of the row number per batch, head and row
-};
-
-// One item: query tiles qt0, qt0 + 1 (has1) of segment seg and their common list of key tiles.  Entries [lo_g, hi_g) of the list are
-// window (or contiguous) tiles of query tile g; entries n_win .. n_list - 1 are sampled tiles, which both take.  n_list = 0: the end.
-struct FwdItem {
-  int seg, qt0, has1, n_list;
-  int n_win, lo1, hi0, hi1;           // (lo of query tile 0 is 0)
-  int first, b, h, hk;                // sorted position of list entry 0 (hyper)
-  int q_row0, k_row0, kseg, pad;
-  __device__ __forceinline__ int lo(int g) const { return g ? lo1 : 0; }
-  __device__ __forceinline__ int hi(int g) const { return g ? hi1 : hi0; }
-  __device__ __forceinline__ bool active(int g, int e) const { return (g == 0 || has1) && ((e >= lo(g) && e < hi(g)) || e >= n_win); }
-  __device__ __forceinline__ int first_entry(int g) const { return hi(g) > lo(g) ? lo(g) : n_win; }
-  __device__ __forceinline__ int last_entry(int g) const { return n_list > n_win ? n_list - 1 : hi(g) - 1; }
-  __device__ __forceinline__ int count(int g) const { return (g == 0 || has1) ? hi(g) - lo(g) + n_list - n_win : 0; }
-};
-
-__device__ __forceinline__ FwdItem fwd_item(const ha_attn_params& p, const FwdPlan& pl, int item, bool flash) {
-  FwdItem it;
-  it.pad = 0;
-  it.seg = pl.by_pairs(item);
-  int pr = item - it.seg * pl.pairs;
-  const int n_qt = (p.m_q + TILE - 1) / TILE;
-  if (flash && (p.flags & HA_FLAG_CAUSAL)) {
-    // Items grow with the pair.  Long pairs first; with few pairs the order is turned by the segment, so that a CTA, which
-    // takes every 148th item, meets all lengths.
-    pr = pl.pairs - 1 - pr;
-    if (pl.pairs <= 32) pr += it.seg - pl.by_pairs(pr + it.seg) * pl.pairs;
-  }
-  it.qt0 = 2 * pr;
-  it.has1 = it.qt0 + 1 < n_qt;
-  it.first = 0;
-  it.lo1 = 0;
-  if (flash) {
-    const int n_kt = (p.m_k + TILE - 1) / TILE;
-    const bool causal = p.flags & HA_FLAG_CAUSAL;
-    it.hi0 = causal ? min(it.qt0 + 1, n_kt) : n_kt;
-    it.hi1 = causal ? min(it.qt0 + 2, n_kt) : n_kt;
-    it.n_win = it.has1 ? it.hi1 : it.hi0;
-    it.n_list = it.n_win;
-  } else {
-    // block windows (block_window) of both tiles
-    const int bs = (p.block_size + TILE - 1) / TILE, tiles = p.m_k / TILE;
-    const bool smooth = p.flags & HA_FLAG_SMOOTH;
-    const int beta0 = pl.by_block(it.qt0), beta1 = pl.by_block(it.qt0 + 1);
-    if (smooth) {
-      it.first = TILE * it.qt0 - (TILE / 2) * (bs - 1);
-      while (it.first < 0) it.first += p.m_k;
-    } else {
-      it.first = beta0 * bs * TILE;
-    }
-    it.hi0 = min(bs, tiles - beta0 * bs);
-    it.hi1 = it.n_win = it.hi0;
-    if (it.has1) {
-      // second window: the same one (both tiles in one block), one tile further on (smooth), or the next block's
-      it.lo1 = smooth ? 1 : beta1 > beta0 ? it.hi0 : 0;
-      it.hi1 = it.lo1 + min(bs, tiles - beta1 * bs);
-      it.n_win = max(it.hi0, it.hi1);
-    }
-    it.n_list = it.n_win + p.sample_size / TILE;
-  }
-  const int bh = pl.by_segs(it.seg), part = it.seg - bh * p.segs_per_head;
-  const int group = p.kv_group > 1 ? p.kv_group : 1;
-  it.b = pl.by_heads(bh);
-  it.h = bh - it.b * p.H;
-  it.hk = pl.by_group(it.h);
-  it.q_row0 = part * p.span + p.q_off;
-  it.k_row0 = part * p.span + p.k_off;
-  it.kseg = group > 1 ? (it.b * pl.by_group(p.H) + it.hk) * p.segs_per_head + part : it.seg;
-  return it;
-}
-
-// Rows of list entry e: key row of tile row r inside the segment (-1: none).
-__device__ __forceinline__ int fwd_key_row(const ha_attn_params& p, const FwdItem& it, int e, int r, bool flash) {
-  if (flash) {
-    const int row = e * TILE + r;
-    return row < p.m_k ? row : -1;
-  }
-  if (e < it.n_win) {
-    int pos = it.first + e * TILE + r;
-    while (pos >= p.m_k) pos -= p.m_k;
-    return p.k_idx[(long long)it.kseg * p.m_k + pos];
-  }
-  const int s = (e - it.n_win) * TILE + r;
-  return p.sample_idx ? p.sample_idx[(long long)it.kseg * p.sample_size + s] : s;
-}
-
-// 128 rows of 64 * slabs elements gathered by ONE warp with cp.async: rows[q] = source row of tile row 32 q + lane (-1: zero fill)
-__device__ __forceinline__ void warp_gather_tile(uint32_t smem_base, const uint16_t* __restrict__ base, int64_t row_stride, int slabs, int (&rows)[4], int lane) {
-  const int chunk = lane & 7;
-#pragma unroll 1
-  for (int q = 0; q < 4; ++q) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int rl = 4 * i + (lane >> 3);
-      const int src_row = __shfl_sync(0xffffffffu, rows[0], rl);
-      const int row = q * 32 + rl;
-      const uint32_t dst = smem_base + row * 128 + ((chunk ^ (row & 7)) << 4);
-      const uint16_t* src = base + (int64_t)(src_row < 0 ? 0 : src_row) * row_stride + chunk * 8;
-      cp_async16(dst, src, src_row >= 0 ? 16u : 0u);
-      if (slabs > 1) cp_async16(dst + TILE * 128, src + 64, src_row >= 0 ? 16u : 0u);
-    }
-    rows[0] = rows[1]; rows[1] = rows[2]; rows[2] = rows[3];
-  }
-}
 
 // KIND: the plain hyper pattern, exact attention, or any call (merging calls, weighted sampling): the code of an instance is what the
 // instruction caches have to hold, so the two frequent kinds carry nothing they do not use.
 enum { FWD_HYPER = 0, FWD_FLASH = 1, FWD_ANY = 2 };
 template <typename T, int D, int DV, int KIND>
-__global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_attn_params p, const FwdPlan pl, const __grid_constant__ FwdMaps maps) {
+__global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_attn_params p, const AttnPlan pl, const __grid_constant__ FwdMaps maps) {
   using namespace fw;
   using Cfg = FwdCfg<D, DV>;
   constexpr int NQ = Cfg::NQ, NKV = Cfg::NKV, NB = Cfg::NB;
@@ -183,7 +72,7 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t s_base = smem_u32(smem);
-  __shared__ __align__(16) FwdItem s_item[ND];
+  __shared__ __align__(16) AttnItem s_item[ND];
   __shared__ uint64_t bars[N_BARS];
   __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
@@ -225,7 +114,7 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
   auto wait = [&](int b, uint32_t parity) -> bool { return __all_sync(0xffffffffu, mbar_wait_or_abort(bar(b), parity, &s_abort)); };
   uint32_t n_item = 0;       // descriptors this warp has taken
   // the next item's descriptor; false: no more items (or a wait gave up)
-  auto next_item = [&](FwdItem& it) -> bool {
+  auto next_item = [&](AttnItem& it) -> bool {
     const int slot = n_item % ND;
     if (!wait(B_D_FULL + slot, (n_item / ND) & 1)) return false;
     it = s_item[slot];
@@ -250,7 +139,7 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
     uint32_t it_g = 0;                  // items this group has taken part in
     bool ok = true;
     HA_T_DECL(8)
-    FwdItem it;
+    AttnItem it;
     while (ok && next_item(it)) {
       const int n_act = 2 * it.count(g);
       if (n_act == 0) continue;
@@ -383,7 +272,7 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
     uint32_t n_out[2] = {0, 0};
     bool ok = true;
     HA_T_DECL(8)
-    FwdItem it;
+    AttnItem it;
     while (ok && next_item(it)) {
 #pragma unroll 1
       for (int g = 0; g < 1 + it.has1; ++g) {
@@ -492,7 +381,7 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
       uint32_t buf = 0, par = 0;                               // score buffer of the next unit, parity of its barriers
       const bool fence_copies = !(flash && pl.tiles);          // tiles that came by cp.async
       HA_T_DECL(8)
-      FwdItem it;
+      AttnItem it;
       if (warp < W_PV) {
         // S = Q K^T: 64 keys at a time
         const uint32_t idesc = mma_idesc(TILE, 64, AB, 0, 0);
@@ -611,14 +500,14 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
       const int stride = is_q || is_k ? 1 : 2;      // list entries from one tile of this warp to the next
       uint32_t n = is_q || is_k ? 0 : 2 * (warp & 1) + 1;      // ring position of this warp's next tile
       int published = 0;
-      auto take = [&](FwdItem& it) -> bool {        // the next item's descriptor; n_list = 0 past the last one
+      auto take = [&](AttnItem& it) -> bool {        // the next item's descriptor; n_list = 0 past the last one
         if (!is_q) return next_item(it);
 #pragma unroll 1
         for (; published <= (int)n_item + 2; ++published) {
           const uint32_t slot = published % ND;
           it.n_list = 0;
           const int item = blockIdx.x + published * gridDim.x;
-          if (item < pl.n_items) it = fwd_item(p, pl, item, flash);
+          if (item < pl.n_items) it = attn_item(p, pl, item, flash);
           if (published >= ND && !wait(B_D_EMPTY + slot, (published / ND - 1) & 1)) return false;
           if (lane == 0) {
             s_item[slot] = it;
@@ -632,7 +521,7 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
       };
       // indexed tiles by TMA: all of K, and the first query tile -- what is left for the cp.async warps then is a tile each per item
       auto by_gather4 = [&](int e) -> bool { return is_k ? pl.rows & 2 : is_q && e == 0 && (pl.rows & 1); };
-      auto row_numbers = [&](const FwdItem& it, int e, int (&rows)[4]) {
+      auto row_numbers = [&](const AttnItem& it, int e, int (&rows)[4]) {
         const bool gathered = by_gather4(e);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -641,13 +530,13 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
             const int pos = (it.qt0 + e) * TILE + r;
             rows[q] = pos >= p.m_q ? -1 : flash ? pos : p.q_idx[(long long)it.seg * p.m_q + pos];
           } else {
-            rows[q] = fwd_key_row(p, it, e, r, flash);
+            rows[q] = item_key_row(p, it, e, r, flash);
           }
         }
       };
-      auto is_boxed = [&](const FwdItem& it, int e) -> bool { return pl.tiles && (flash || (!is_q && e >= it.n_win && !p.sample_idx)); };
+      auto is_boxed = [&](const AttnItem& it, int e) -> bool { return pl.tiles && (flash || (!is_q && e >= it.n_win && !p.sample_idx)); };
       HA_T_DECL(8)
-      FwdItem it;
+      AttnItem it;
       int e = is_q || is_k ? 0 : warp & 1;
       // moves (it, e) to this warp's next tile; e may lie past the end of the item
       auto settle = [&]() -> bool {
@@ -726,18 +615,9 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
 template <typename T, int D, int DV, int KIND>
 static int launch_fwd(const ha_attn_params& p, cudaStream_t st) {
   using Cfg = FwdCfg<D, DV>;
-  const long long segs = (long long)p.B * p.H * p.segs_per_head;
-  FwdPlan pl;
-  pl.pairs = ((p.m_q + TILE - 1) / TILE + 1) / 2;
-  const long long items = segs * pl.pairs;
-  if (items == 0) return HA_OK;
-  if (items > 0x7fffffffLL) return HA_ERR_TOO_LARGE;
-  pl.n_items = (int)items;
-  pl.by_pairs = FastDiv(pl.pairs);
-  pl.by_segs = FastDiv(p.segs_per_head);
-  pl.by_heads = FastDiv(p.H);
-  pl.by_group = FastDiv(p.kv_group > 1 ? p.kv_group : 1);
-  pl.by_block = FastDiv(p.mode == HA_MODE_HYPER ? (p.block_size + TILE - 1) / TILE : 1);
+  AttnPlan pl;
+  if (!plan_items(pl, p)) return HA_ERR_TOO_LARGE;
+  if (pl.n_items == 0) return HA_OK;
   FwdMaps maps;
   const int Hk = p.kv_group > 1 ? p.H / p.kv_group : p.H;
   // rows a head really has on either side (a single-segment call may have fewer or more keys than queries)
@@ -746,17 +626,7 @@ static int launch_fwd(const ha_attn_params& p, cudaStream_t st) {
   pl.tiles = encode_tile_map(&maps.tile[0], p.dtype, p.q, D, n_q, p.H, p.B, p.q_sn, p.q_sh, p.q_sb, TILE) &&
              encode_tile_map(&maps.tile[1], p.dtype, p.k, D, n_k, Hk, p.B, p.k_sn, p.k_sh, p.k_sb, TILE) &&
              encode_tile_map(&maps.tile[2], p.dtype, p.v, DV, n_k, Hk, p.B, p.v_sn, p.v_sh, p.v_sb, TILE);
-  pl.rows = 0;
-  for (int x = 0; x < 2 && p.mode == HA_MODE_HYPER; ++x) {
-    const int heads = x ? Hk : p.H;
-    const int64_t sn = x ? p.k_sn : p.q_sn, sh = x ? p.k_sh : p.q_sh, sb = x ? p.k_sb : p.q_sb;
-    int64_t pitch = 1;
-    if (!encode_row_map(&maps.rows[x], p.dtype, x ? p.k : p.q, D, x ? n_k : n_q, heads, p.B, sn, sh, sb, &pitch)) continue;
-    pl.rows |= 1 << x;
-    pl.row_sn[x] = (int)(sn / pitch);
-    pl.row_sh[x] = heads > 1 ? (int)(sh / pitch) : 0;      // (the encoder has seen that every row number fits)
-    pl.row_sb[x] = p.B > 1 ? (int)(sb / pitch) : 0;
-  }
+  plan_row_maps(pl, p, maps.rows, n_q, n_k);
   // the tiles start at the first 1 KB boundary after the static variables; at head dim 128 they end with the CTA's last byte
   static int dyn_bytes = 0;
   if (dyn_bytes == 0) {
@@ -767,7 +637,7 @@ static int launch_fwd(const ha_attn_params& p, cudaStream_t st) {
   }
   HA_SMEM_ATTR_ONCE((attn_tc_fwd_kernel<T, D, DV, KIND>), dyn_bytes, "ha_attn_fwd smem attribute");
   const int sms = sm_count();
-  attn_tc_fwd_kernel<T, D, DV, KIND><<<(unsigned)(items < sms ? items : sms), fw::THREADS, dyn_bytes, st>>>(p, pl, maps);
+  attn_tc_fwd_kernel<T, D, DV, KIND><<<(unsigned)(pl.n_items < sms ? pl.n_items : sms), fw::THREADS, dyn_bytes, st>>>(p, pl, maps);
   HA_LAUNCHED("ha_attn_fwd (tcgen05)");
   return HA_OK;
 }

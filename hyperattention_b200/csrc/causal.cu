@@ -16,6 +16,8 @@
 namespace ha {
 
 bool tc_bwd_supported(const ha_attn_params& p);   // attn_tc_bwd.cu
+bool ws_bwd_supported(const ha_attn_params& p);   // attn_tc_bwd_ws.cu
+int ws_attn_bwd(const ha_attn_params& p, bool store_dq, cudaStream_t st);
 
 // One helper stream and two events per device, created on first use and kept for the life of the process.
 // `mu` serialises the callers of one device over the fork .. join section (the two events are shared).
@@ -452,18 +454,20 @@ int ha_causal_bwd(const ha_causal_params* pp, void* stream) {
   ha_attn_params a;
   fill_attn(p, a);
   a.delta = delta; a.dq_acc = dq_acc; a.dk_acc = dk_acc; a.dv_acc = dv_acc;
-  // The leaves run first and cover every key row; on the tensor-core kernel one work item owns a key tile's whole
-  // dK/dV there (leaves of up to 2048 rows), so it stores them and the two accumulators need no zero-fill.
-  bool kv_init = false;
+  // The leaves run first and cover every row.  The warp-specialised kernel holds a query row's whole sum in one item there: it stores
+  // dQ, whose accumulator needs no zero-fill.  In the earlier kernel an item owns a key tile's whole dK / dV (leaves of up
+  // to 2048 rows) and stores those.
+  bool q_init = false, kv_init = false;
   {
     ha_attn_params probe = a;
     probe.mode = HA_MODE_FLASH;
     probe.flags = HA_FLAG_CAUSAL | (p.flags & HA_FLAG_FORCE_SIMT);
     probe.segs_per_head = 1 << p.levels;
     probe.span = pl.leaf; probe.m_q = pl.leaf; probe.m_k = pl.leaf;
-    kv_init = pl.leaf <= 16 * TILE && !(p.flags & HA_FLAG_FORCE_SIMT) && p.kv_group <= 1 && tc_bwd_supported(probe);
+    q_init = !(p.flags & HA_FLAG_FORCE_SIMT) && ws_bwd_supported(probe);
+    kv_init = !q_init && pl.leaf <= 16 * TILE && !(p.flags & HA_FLAG_FORCE_SIMT) && p.kv_group <= 1 && tc_bwd_supported(probe);
   }
-  HA_CUDA_OK(cudaMemsetAsync(dq_acc, 0, pl.rows * p.d * 4, st), "ha_causal_bwd memset");
+  if (!q_init) HA_CUDA_OK(cudaMemsetAsync(dq_acc, 0, pl.rows * p.d * 4, st), "ha_causal_bwd memset");
   if (!kv_init) {
     HA_CUDA_OK(cudaMemsetAsync(dk_acc, 0, pl.rows_k * p.d * 4, st), "ha_causal_bwd memset");
     HA_CUDA_OK(cudaMemsetAsync(dv_acc, 0, pl.rows_k * p.dv * 4, st), "ha_causal_bwd memset");
@@ -501,7 +505,7 @@ int ha_causal_bwd(const ha_causal_params* pp, void* stream) {
   a.flags = HA_FLAG_CAUSAL | (p.flags & HA_FLAG_FORCE_SIMT) | (kv_init ? HA_FLAG_BWD_KV_INIT : 0);
   a.segs_per_head = 1 << p.levels;
   a.span = pl.leaf; a.q_off = 0; a.k_off = 0; a.m_q = pl.leaf; a.m_k = pl.leaf;
-  rc = ha_attn_bwd(&a, stream);
+  rc = q_init ? ws_attn_bwd(a, true, st) : ha_attn_bwd(&a, stream);
   if (rc != HA_OK) return rc;
   for (int l = p.levels - 1; l >= 0; --l) {
     const int span = p.n >> l, m = span / 2;
@@ -553,14 +557,20 @@ static void noncausal_attn(const ha_causal_params& p, ha_attn_params& a, long lo
   a.k_idx = (const int32_t*)((const uint8_t*)p.saved + align256(rows * 4));
 }
 
-// what the backward needs beyond delta: 2 = slot buffers only, 1 = slot buffers + fp32 dQ, 0 = three fp32 accumulators
+// what the backward needs beyond delta: 3 = fp32 dK and dV (typed dQ), 2 = slot buffers only, 1 = slot buffers + fp32 dQ, 0 = three fp32
+// accumulators
 static int noncausal_bwd_level(const ha_causal_params& p, long long rows) {
   ha_attn_params a;
   noncausal_attn(p, a, rows);
   float dummy = 0.f;
   a.delta = &dummy;                               // (only looked at for being there)
   a.dq_acc = a.dk_acc = a.dv_acc = nullptr;
-  return p.dtype == HA_FP32 ? 0 : ha_attn_bwd_direct_level(&a);
+  const int level = p.dtype == HA_FP32 ? 0 : ha_attn_bwd_direct_level(&a);
+  if (level == 2 || p.dtype == HA_FP32 || (p.flags & HA_FLAG_FORCE_SIMT) || (uintptr_t)p.dq % 16 != 0) return level;
+  // key rows that several items add to, on the kernel that sums a query row inside one item
+  a.dq_out = (void*)256;                          // (the outputs are only looked at for being there, and for their alignment)
+  a.dk_acc = a.dv_acc = (float*)256;
+  return ws_bwd_supported(a) ? 3 : level;
 }
 
 int64_t ha_noncausal_saved_bytes(const ha_causal_params* p) {
@@ -576,7 +586,8 @@ int64_t ha_noncausal_scratch_bytes(const ha_causal_params* p, int32_t backward) 
   const int level = noncausal_bwd_level(*p, rows);
   const long long sacc = align256((long long)p->B * p->H * p->sample_size * (p->d + p->dv) * 4);
   long long bytes = align256(rows * 4);
-  if (level == 2) bytes += sacc;
+  if (level == 3) bytes += align256(rows_k * p->d * 4) + align256(rows_k * p->dv * 4);
+  else if (level == 2) bytes += sacc;
   else if (level == 1) bytes += sacc + align256(rows * p->d * 4);
   else bytes += align256(rows * p->d * 4) + align256(rows_k * p->d * 4) + align256(rows_k * p->dv * 4);
   return bytes;
@@ -634,6 +645,17 @@ int ha_noncausal_bwd(const ha_causal_params* pp, void* stream) {
   rc = ha_delta(p.o, a.o_sb, a.o_sh, a.o_sn, p.d_o, a.do_sb, a.do_sh, a.do_sn, p.B, p.H, p.n, p.dv, p.dtype, delta, stream);
   if (rc != HA_OK) return rc;
   const int level = noncausal_bwd_level(p, rows);
+  if (level == 3) {
+    a.dk_acc = (float*)s;                    s += align256(rows_k * p.d * 4);
+    a.dv_acc = (float*)s;
+    a.dq_out = p.dq;
+    HA_CUDA_OK(cudaMemsetAsync(a.dk_acc, 0, align256(rows_k * p.d * 4) + rows_k * p.dv * 4, st), "ha_noncausal_bwd memset");
+    rc = ws_attn_bwd(a, false, st);
+    if (rc != HA_OK) return rc;
+    rc = ha_cast_from_f32(a.dk_acc, p.dk, rows_k * p.d, p.dtype, stream);
+    if (rc != HA_OK) return rc;
+    return ha_cast_from_f32(a.dv_acc, p.dv_out, rows_k * p.dv, p.dtype, stream);
+  }
   if (level >= 1) {
     const long long segs = (long long)p.B * p.H;
     const long long sacc_bytes = segs * p.sample_size * (p.d + p.dv) * 4;

@@ -18,6 +18,10 @@ static EncodeFn encode_fn() {
   return fn;
 }
 
+static CUtensorMapDataType map_type(int dtype) {
+  return dtype == HA_FP32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : dtype == HA_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+}
+
 static bool encode(CUtensorMap* map, int dtype, const void* base, int rank, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box,
                    CUtensorMapL2promotion promo) {
   const EncodeFn fn = encode_fn();
@@ -27,7 +31,7 @@ static bool encode(CUtensorMap* map, int dtype, const void* base, int rank, cons
   for (int i = 0; i < rank; ++i)
     if (dims[i] == 0 || dims[i] > 0x7fffffffull) return false;
   const cuuint32_t ones[4] = {1, 1, 1, 1};
-  return fn(map, dtype == HA_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, (cuuint32_t)rank, const_cast<void*>(base), dims,
+  return fn(map, map_type(dtype), (cuuint32_t)rank, const_cast<void*>(base), dims,
             strides, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, promo,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -42,6 +46,13 @@ bool encode_tile_map(CUtensorMap* map, int dtype, const void* base, int width, l
   const cuuint64_t strides[3] = {(cuuint64_t)sn * 2, (cuuint64_t)sh * 2, (cuuint64_t)sb * 2};
   const cuuint32_t box[4] = {64, (cuuint32_t)box_rows, 1, 1};
   return encode(map, dtype, base, 4, dims, strides, box, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+}
+
+bool encode_acc_map(CUtensorMap* map, float* base, int width, long long rows, long long heads) {
+  const cuuint64_t dims[3] = {(cuuint64_t)width, (cuuint64_t)rows, (cuuint64_t)heads};
+  const cuuint64_t strides[2] = {(cuuint64_t)width * 4, (cuuint64_t)width * 4 * (cuuint64_t)rows};
+  const cuuint32_t box[3] = {32, TILE, 1};
+  return encode(map, HA_FP32, base, 3, dims, strides, box, CU_TENSOR_MAP_L2_PROMOTION_NONE);
 }
 
 bool encode_row_map(CUtensorMap* map, int dtype, const void* base, int width, long long rows, int H, int B, int64_t sn, int64_t sh, int64_t sb,

@@ -17,18 +17,12 @@ import torch
 
 from . import _lib
 
-ROLES = {0: ('elementwise group 0', ['wait S^T/dP^T ready', 'wait lse/delta (+ scaling)', 'wait dS buffer free', 'loads + math + stores',
-                                       'store-wait, fences, arrivals']),
-         1: ('elementwise group 1', ['wait S^T/dP^T ready', 'wait lse/delta (+ scaling)', 'wait dS buffer free', 'loads + math + stores',
-                                       'store-wait, fences, arrivals']),
-         2: ('drain group', ['wait accumulators full', 'index loads, staging writes, coalesced stores / reductions', 'wait dQ full', 'dQ rows',
-                             'accumulator -> registers (issuers blocked)', 'wait staging tile free (whole-tile additions)', 'proxy fence',
-                             'whole-tile additions: barrier, issue (thread 0 of the group: + the read of the tile)']),
-         3: ('K loader warp', ['index loads, L2 prefetch', 'wait stage empty', 'issuing the copies of a tile']),
-         4: ('S^T issuer', ['loop', 'wait stage columns free (dV of the previous pair)', 'wait K / Q tiles', 'fences, 4 MMAs, commits']),
-         5: ('dV issuer', ['loop', 'wait P^T ready', 'wait accumulator drained', 'fences, 4 MMAs, commits']),
-         6: ('dQ issuer', ['loop', 'wait dS slabs full', 'wait dQ drained', 'fences, 8 MMAs, commits']),
-         7: ('Q / dO loader warp', ['index loads, L2 prefetch', 'wait stage empty', 'issuing the copies of two tiles'])}
+EW = ['loop, item set-up', 'wait S^T / dP^T ready', 'lse / delta scaling, wait dS buffer free', 'loads, math, stores', 'store wait, fences, arrivals']
+ISSUE = ['loop, item set-up', 'wait operand tile', 'wait inputs / accumulator', 'issue', 'tile done']
+LOAD = ['row numbers', 'wait slot free', 'issue copies']
+ROLES = {0: ('elementwise group 0', EW), 1: ('elementwise group 1', EW),
+         2: ('drain group', ['loop, item set-up', 'row numbers, wait staging tile', 'wait accumulator complete', 'out of TMEM, staged, stored']),
+         3: ('K loader', LOAD), 4: ('S^T warp', ISSUE), 5: ('dV warp', ISSUE), 6: ('dQ warp', ISSUE), 7: ('Q / dO loader', LOAD)}
 
 # attn_tc_fwd_kernel
 FWD_ROLES = {0: ('softmax group 0', ['loop, item set-up', 'wait S ready', 'scores out of TMEM, maximum, rescale', 'exponentials, P, sum',
@@ -81,7 +75,7 @@ def main():
         return
     qg, kg, vg = [t.clone().requires_grad_() for t in (q, k, v)]
     for rep in range(2):
-        o = mod(qg, kg, vg)
+        o = mod(qg, kg, vg, causal=a.causal)
         if rep == 1:
             setter = lib.ha_debug_set_timing_buffer_bwd_ws
             setter.restype, setter.argtypes = C.c_int, [C.c_void_p]
