@@ -4,6 +4,9 @@
 namespace ha {
 int simt_attn_fwd(const ha_attn_params& p, cudaStream_t st);
 int simt_attn_bwd(const ha_attn_params& p, cudaStream_t st);
+bool f32_tiled_supported(const ha_attn_params& p, bool backward);
+int f32_tiled_fwd(const ha_attn_params& p, cudaStream_t st);
+int f32_tiled_bwd(const ha_attn_params& p, cudaStream_t st);
 int tc_attn_fwd(const ha_attn_params& p, cudaStream_t st);
 bool tc_supported(const ha_attn_params& p);
 bool tc_bwd_supported(const ha_attn_params& p);
@@ -155,6 +158,7 @@ int ha_attn_fwd(const ha_attn_params* p, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   if ((p->flags & HA_FLAG_CHECK_INDICES) && p->mode == HA_MODE_HYPER && (rc = check_indices(*p, st)) != HA_OK) return rc;
   if (!(p->flags & HA_FLAG_FORCE_SIMT) && tc_supported(*p)) return tc_attn_fwd(*p, st);
+  if (f32_tiled_supported(*p, false)) return f32_tiled_fwd(*p, st);
   return simt_attn_fwd(*p, st);
 }
 
@@ -171,6 +175,7 @@ int ha_attn_bwd(const ha_attn_params* p, void* stream) {
   if (!(p->flags & HA_FLAG_FORCE_SIMT) && ws_bwd_supported(*p)) return ws_attn_bwd(*p, false, st);
   if (!(p->flags & HA_FLAG_FORCE_SIMT) && tc_bwd_supported(*p)) return tc_attn_bwd(*p, st);
   if (p->dk_out || (p->flags & HA_FLAG_BWD_KV_INIT)) return HA_ERR_INVALID;   // tensor-core kernel only
+  if (f32_tiled_supported(*p, true)) return f32_tiled_bwd(*p, st);
   return simt_attn_bwd(*p, st);
 }
 

@@ -535,9 +535,11 @@ __global__ void __launch_bounds__(256) attn_tc_bwd_kernel(const ha_attn_params p
       float* dv_base = p.dv_acc + (si.khead0 + si.k_row0) * DV;
       if (p.flags & HA_FLAG_BWD_KV_INIT) {   // (exact attention only) this item is the only writer of its key rows: store, nothing to add to
         reduce_rows<DV / 2, 1>(stg, tDV + lane_sel + wg * (DV / 2), dv_base + wg * (DV / 2), DV, kr, row);
+        if constexpr (D != DV) __syncthreads();      // rows of another pitch: a warp's share of the staging tile lies elsewhere
         reduce_rows<D / 2, 1>(stg, tDK + lane_sel + wg * (D / 2), dk_base + wg * (D / 2), D, kr, row);
       } else {
         reduce_rows<DV / 2>(stg, tDV + lane_sel + wg * (DV / 2), dv_base + wg * (DV / 2), DV, kr, row);
+        if constexpr (D != DV) __syncthreads();      // rows of another pitch: a warp's share of the staging tile lies elsewhere
         reduce_rows<D / 2>(stg, tDK + lane_sel + wg * (D / 2), dk_base + wg * (D / 2), D, kr, row);
       }
     } else if (!sampled_tile) {
@@ -550,6 +552,7 @@ __global__ void __launch_bounds__(256) attn_tc_bwd_kernel(const ha_attn_params p
       float* dk_base = p.dk_sacc + kseg_of(p, seg) * p.sample_size * D;
       float* dv_base = p.dv_sacc + kseg_of(p, seg) * p.sample_size * DV;
       reduce_rows<DV / 2>(stg, tDV + lane_sel + wg * (DV / 2), dv_base + wg * (DV / 2), DV, slot, row);
+      if constexpr (D != DV) __syncthreads();
       reduce_rows<D / 2>(stg, tDK + lane_sel + wg * (D / 2), dk_base + wg * (D / 2), D, slot, row);
     }
   };

@@ -329,7 +329,8 @@ int64_t ha_causal_scratch_bytes(const ha_causal_params* p, int32_t backward) {
   CausalPlan pl;
   if (!p || make_plan(*p, pl) != HA_OK) return -1;
   if (!backward) return 2 * align256(pl.rows * 4) + align256(pl.sort_ws) + scratch_part_bytes(*p, pl);
-  return align256(pl.rows * p->d * 4) + align256(pl.rows_k * p->d * 4) + align256(pl.rows_k * p->dv * 4) + align256(pl.rows * 4 * (p->levels + 1));
+  const long long acc = p->dtype == HA_FP32 ? 0 : align256(pl.rows * p->d * 4) + align256(pl.rows_k * p->d * 4) + align256(pl.rows_k * p->dv * 4);
+  return acc + align256(pl.rows * 4 * (p->levels + 1));
 }
 
 int ha_causal_fwd(const ha_causal_params* pp, void* stream) {
@@ -447,9 +448,12 @@ int ha_causal_bwd(const ha_causal_params* pp, void* stream) {
   if (!p.scratch || p.scratch_bytes < ha_causal_scratch_bytes(pp, 1)) return HA_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   uint8_t* s = (uint8_t*)p.scratch;
-  float* dq_acc = (float*)s;                 s += align256(pl.rows * p.d * 4);
-  float* dk_acc = (float*)s;                 s += align256(pl.rows_k * p.d * 4);
-  float* dv_acc = (float*)s;                 s += align256(pl.rows_k * p.dv * 4);
+  float *dq_acc = (float*)p.dq, *dk_acc = (float*)p.dk, *dv_acc = (float*)p.dv_out;      // fp32 gradients are their own accumulators
+  if (p.dtype != HA_FP32) {
+    dq_acc = (float*)s;                      s += align256(pl.rows * p.d * 4);
+    dk_acc = (float*)s;                      s += align256(pl.rows_k * p.d * 4);
+    dv_acc = (float*)s;                      s += align256(pl.rows_k * p.dv * 4);
+  }
   float* delta = (float*)s;
   ha_attn_params a;
   fill_attn(p, a);
@@ -520,6 +524,7 @@ int ha_causal_bwd(const ha_causal_params* pp, void* stream) {
     rc = ha_attn_bwd(&a, stream);
     if (rc != HA_OK) return rc;
   }
+  if (p.dtype == HA_FP32) return HA_OK;
   rc = ha_cast_from_f32(dq_acc, p.dq, pl.rows * p.d, p.dtype, stream);
   if (rc != HA_OK) return rc;
   rc = ha_cast_from_f32(dk_acc, p.dk, pl.rows_k * p.d, p.dtype, stream);
@@ -589,7 +594,7 @@ int64_t ha_noncausal_scratch_bytes(const ha_causal_params* p, int32_t backward) 
   if (level == 3) bytes += align256(rows_k * p->d * 4) + align256(rows_k * p->dv * 4);
   else if (level == 2) bytes += sacc;
   else if (level == 1) bytes += sacc + align256(rows * p->d * 4);
-  else bytes += align256(rows * p->d * 4) + align256(rows_k * p->d * 4) + align256(rows_k * p->dv * 4);
+  else if (p->dtype != HA_FP32) bytes += align256(rows * p->d * 4) + align256(rows_k * p->d * 4) + align256(rows_k * p->dv * 4);
   return bytes;
 }
 
@@ -678,20 +683,18 @@ int ha_noncausal_bwd(const ha_causal_params* pp, void* stream) {
     if (level == 1) rc = ha_cast_from_f32(a.dq_acc, p.dq, rows * p.d, p.dtype, stream);
     return rc;
   }
-  a.dq_acc = (float*)s;                      s += align256(rows * p.d * 4);
-  a.dk_acc = (float*)s;                      s += align256(rows_k * p.d * 4);
-  a.dv_acc = (float*)s;
+  a.dq_acc = (float*)p.dq; a.dk_acc = (float*)p.dk; a.dv_acc = (float*)p.dv_out;         // fp32 gradients are their own accumulators
+  if (p.dtype != HA_FP32) {
+    a.dq_acc = (float*)s;                    s += align256(rows * p.d * 4);
+    a.dk_acc = (float*)s;                    s += align256(rows_k * p.d * 4);
+    a.dv_acc = (float*)s;
+  }
   HA_CUDA_OK(cudaMemsetAsync(a.dq_acc, 0, rows * p.d * 4, st), "ha_noncausal_bwd memset");
   HA_CUDA_OK(cudaMemsetAsync(a.dk_acc, 0, rows_k * p.d * 4, st), "ha_noncausal_bwd memset");
   HA_CUDA_OK(cudaMemsetAsync(a.dv_acc, 0, rows_k * p.dv * 4, st), "ha_noncausal_bwd memset");
   rc = ha_attn_bwd(&a, stream);
   if (rc != HA_OK) return rc;
-  if (p.dtype == HA_FP32) {
-    HA_CUDA_OK(cudaMemcpyAsync(p.dq, a.dq_acc, rows * p.d * 4, cudaMemcpyDeviceToDevice, st), "ha_noncausal_bwd copy");
-    HA_CUDA_OK(cudaMemcpyAsync(p.dk, a.dk_acc, rows_k * p.d * 4, cudaMemcpyDeviceToDevice, st), "ha_noncausal_bwd copy");
-    HA_CUDA_OK(cudaMemcpyAsync(p.dv_out, a.dv_acc, rows_k * p.dv * 4, cudaMemcpyDeviceToDevice, st), "ha_noncausal_bwd copy");
-    return HA_OK;
-  }
+  if (p.dtype == HA_FP32) return HA_OK;
   rc = ha_cast_from_f32(a.dq_acc, p.dq, rows * p.d, p.dtype, stream);
   if (rc != HA_OK) return rc;
   rc = ha_cast_from_f32(a.dk_acc, p.dk, rows_k * p.d, p.dtype, stream);
