@@ -212,8 +212,8 @@ struct SavedLayout {
 // One lane per 16-byte chunk of a row; part = depth, leaves last, as in the saved layout.
 template <typename T>
 __global__ void __launch_bounds__(256) merge_parts_kernel(const uint8_t* __restrict__ parts0, long long part_stride_bytes, long long lse_off_bytes,
-                                                          int levels, int n, int lpr, T* __restrict__ o, float* __restrict__ lse,
-                                                          long long total_rows, int exact, int log2n) {
+                                                          int levels, int n, int lpr, T* __restrict__ o, int64_t o_sb, int64_t o_sh, int64_t o_sn,
+                                                          FastDiv by_heads, int H, float* __restrict__ lse, long long total_rows, int exact, int log2n) {
   const int lane = threadIdx.x & 31;
   const int rpw = 32 / lpr, chunk = lane % lpr, sub = lane / lpr;
   const long long warp_id = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -221,9 +221,12 @@ __global__ void __launch_bounds__(256) merge_parts_kernel(const uint8_t* __restr
   const int dv = lpr * 8;
   const int step = (int)((n_warps * rpw) % n);
   int i = (int)((warp_id * rpw + sub) % n) - step;
+  const int step_bh = (int)((n_warps * rpw) / n);
+  int bh = (int)((warp_id * rpw + sub) / n) - step_bh;
   for (long long base = warp_id * rpw; base < total_rows; base += n_warps * rpw) {
     i += step;
-    if (i >= n) i -= n;
+    bh += step_bh;
+    if (i >= n) { i -= n; ++bh; }
     const long long row = base + sub;
     if (row >= total_rows) continue;
     auto part_row = [&](int part) { return __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(parts0 + part * part_stride_bytes) + row * dv + chunk * 8)); };
@@ -273,25 +276,50 @@ __global__ void __launch_bounds__(256) merge_parts_kernel(const uint8_t* __restr
         l1 = lm;
       }
     }
-    *reinterpret_cast<uint4*>(o + row * dv + chunk * 8) = cur;
+    const int b = by_heads(bh);
+    *reinterpret_cast<uint4*>(o + b * o_sb + (bh - b * H) * o_sh + i * o_sn + chunk * 8) = cur;
     if (chunk == 0) lse[row] = l1;
   }
 }
 
-static void fill_attn(const ha_causal_params& p, ha_attn_params& a) {
+// Element strides (batch, head, row) of q, k, v, o, dO; the gradients are contiguous.
+struct Layout {
+  int64_t q[3], k[3], v[3], o[3], g[3];
+  Layout(const ha_causal_params& p, const int64_t* strides) {
+    if (strides) {
+      for (int i = 0; i < 3; ++i) { q[i] = strides[i]; k[i] = strides[3 + i]; v[i] = strides[6 + i]; o[i] = strides[9 + i]; g[i] = strides[12 + i]; }
+      return;
+    }
+    const int Hk = p.kv_group > 1 ? p.H / p.kv_group : p.H;
+    auto set = [&](int64_t (&s)[3], int heads, int width) {
+      s[2] = width;
+      s[1] = (int64_t)p.n * width;
+      s[0] = s[1] * heads;
+    };
+    set(q, p.H, p.d);
+    set(k, Hk, p.d);
+    set(v, Hk, p.dv);
+    set(o, p.H, p.dv);
+    set(g, p.H, p.dv);
+  }
+  static bool contiguous(const int64_t (&s)[3], const ha_causal_params& p) {
+    return s[2] == p.dv && (p.H == 1 || s[1] == (int64_t)p.n * p.dv) && (p.B == 1 || s[0] == (int64_t)p.n * p.dv * p.H);
+  }
+};
+
+static void fill_attn(const ha_causal_params& p, const Layout& lay, ha_attn_params& a) {
   a = ha_attn_params{};
   a.dtype = p.dtype;
   a.B = p.B; a.H = p.H; a.n = p.n; a.d = p.d; a.dv = p.dv;
   a.block_size = p.block_size; a.sample_size = p.sample_size; a.scale = p.scale;
   a.q = p.q; a.k = p.k; a.v = p.v;
-  a.q_sn = p.d; a.q_sh = (int64_t)p.n * p.d; a.q_sb = a.q_sh * p.H;
-  const int Hk = p.kv_group > 1 ? p.H / p.kv_group : p.H;
   a.kv_group = p.kv_group;
-  a.k_sn = p.d; a.k_sh = a.q_sh; a.k_sb = a.k_sh * Hk;
-  a.v_sn = p.dv; a.v_sh = (int64_t)p.n * p.dv; a.v_sb = a.v_sh * Hk;
-  a.o = p.o; a.o_sn = p.dv; a.o_sh = a.v_sh; a.o_sb = a.o_sh * p.H;
+  a.q_sb = lay.q[0]; a.q_sh = lay.q[1]; a.q_sn = lay.q[2];
+  a.k_sb = lay.k[0]; a.k_sh = lay.k[1]; a.k_sn = lay.k[2];
+  a.v_sb = lay.v[0]; a.v_sh = lay.v[1]; a.v_sn = lay.v[2];
+  a.o = p.o; a.o_sb = lay.o[0]; a.o_sh = lay.o[1]; a.o_sn = lay.o[2];
   a.lse = p.lse;
-  a.d_o = p.d_o; a.do_sn = p.dv; a.do_sh = a.v_sh; a.do_sb = a.o_sb;
+  a.d_o = p.d_o; a.do_sb = lay.g[0]; a.do_sh = lay.g[1]; a.do_sn = lay.g[2];
   a.status = p.status;
   a.status_host = p.status_host;
 }
@@ -333,7 +361,7 @@ int64_t ha_causal_scratch_bytes(const ha_causal_params* p, int32_t backward) {
   return acc + align256(pl.rows * 4 * (p->levels + 1));
 }
 
-int ha_causal_fwd(const ha_causal_params* pp, void* stream) {
+int ha_causal_fwd_strided(const ha_causal_params* pp, const int64_t* strides, void* stream) {
   if (!pp) return HA_ERR_INVALID;
   const ha_causal_params& p = *pp;
   CausalPlan pl;
@@ -347,10 +375,10 @@ int ha_causal_fwd(const ha_causal_params* pp, void* stream) {
   int32_t* codes_k = (int32_t*)((uint8_t*)p.scratch + align256(pl.rows * 4));
   void* sort_ws = (uint8_t*)p.scratch + 2 * align256(pl.rows * 4);
 
-  const int64_t sn = p.d, sh = (int64_t)p.n * p.d, sb = sh * p.H;
-  rc = ha_lsh_hash(p.q, sb, sh, sn, p.B, p.H, p.n, p.d, p.dtype, p.proj, p.lsh_bits, codes_q, stream);
+  const Layout lay(p, strides);
+  rc = ha_lsh_hash(p.q, lay.q[0], lay.q[1], lay.q[2], p.B, p.H, p.n, p.d, p.dtype, p.proj, p.lsh_bits, codes_q, stream);
   if (rc != HA_OK) return rc;
-  rc = ha_lsh_hash(p.k, sh * pl.Hk, sh, sn, p.B, pl.Hk, p.n, p.d, p.dtype, p.proj, p.lsh_bits, codes_k, stream);
+  rc = ha_lsh_hash(p.k, lay.k[0], lay.k[1], lay.k[2], p.B, pl.Hk, p.n, p.d, p.dtype, p.proj, p.lsh_bits, codes_k, stream);
   if (rc != HA_OK) return rc;
 
   // The sorts of every depth depend on the codes only: they run on a side stream (forked here, joined before the first
@@ -382,7 +410,7 @@ int ha_causal_fwd(const ha_causal_params* pp, void* stream) {
   }
 
   ha_attn_params a;
-  fill_attn(p, a);
+  fill_attn(p, lay, a);
   // leaves: exact causal attention on 2^levels spans per head
   a.mode = HA_MODE_FLASH;
   a.flags = HA_FLAG_CAUSAL | (p.flags & HA_FLAG_FORCE_SIMT);
@@ -397,7 +425,12 @@ int ha_causal_fwd(const ha_causal_params* pp, void* stream) {
   const long long slot_stride = align256(pl.part_o_bytes) + align256(pl.part_lse_bytes), slot_lse = align256(pl.part_o_bytes);
   auto slot_o = [&](int part) -> void* { return slots + part * slot_stride; };
   auto slot_lse_of = [&](int part) -> float* { return (float*)(slots + part * slot_stride + slot_lse); };
-  if (deferred) { a.o = slot_o(p.levels); a.lse = slot_lse_of(p.levels); }
+  // (un-merged rows beside the merged ones have the layout of o: only where that is the slots' own)
+  if (p.keep_parts && !deferred && !Layout::contiguous(lay.o, p)) {
+    if (side) { cudaStreamWaitEvent(main_st, side->join, 0); side_lock.unlock(); }
+    return HA_ERR_INVALID;
+  }
+  if (deferred) { a.o = slot_o(p.levels); a.lse = slot_lse_of(p.levels); a.o_sn = p.dv; a.o_sh = (int64_t)p.n * p.dv; a.o_sb = a.o_sh * p.H; }
   else if (p.keep_parts) { a.part_o = sv.part_o(p.levels); a.part_lse = sv.part_lse(p.levels); }
   rc = ha_attn_fwd(&a, stream);
   if (side) HA_CUDA_OK(cudaStreamWaitEvent(main_st, side->join, 0), "ha_causal_fwd join");
@@ -427,16 +460,18 @@ int ha_causal_fwd(const ha_causal_params* pp, void* stream) {
     const int exact_merge = (p.flags & HA_FLAG_MERGE_EXACT) ? 1 : 0;
     if (p.dtype == HA_BF16)
       merge_parts_kernel<__nv_bfloat16><<<grid, 256, 0, main_st>>>((const uint8_t*)slots, part_stride, lse_off, p.levels, p.n, lpr,
-                                                                  (__nv_bfloat16*)p.o, p.lse, pl.rows, exact_merge, log2_if_pow2(p.n));
+                                                                  (__nv_bfloat16*)p.o, lay.o[0], lay.o[1], lay.o[2], FastDiv(p.H), p.H, p.lse, pl.rows, exact_merge, log2_if_pow2(p.n));
     else
       merge_parts_kernel<__half><<<grid, 256, 0, main_st>>>((const uint8_t*)slots, part_stride, lse_off, p.levels, p.n, lpr, (__half*)p.o,
-                                                           p.lse, pl.rows, exact_merge, log2_if_pow2(p.n));
+                                                           lay.o[0], lay.o[1], lay.o[2], FastDiv(p.H), p.H, p.lse, pl.rows, exact_merge, log2_if_pow2(p.n));
     HA_LAUNCHED("ha_causal_fwd merge");
   }
   return HA_OK;
 }
 
-int ha_causal_bwd(const ha_causal_params* pp, void* stream) {
+int ha_causal_fwd(const ha_causal_params* p, void* stream) { return ha_causal_fwd_strided(p, nullptr, stream); }
+
+int ha_causal_bwd_strided(const ha_causal_params* pp, const int64_t* strides, void* stream) {
   if (!pp) return HA_ERR_INVALID;
   const ha_causal_params& p = *pp;
   CausalPlan pl;
@@ -456,7 +491,8 @@ int ha_causal_bwd(const ha_causal_params* pp, void* stream) {
   }
   float* delta = (float*)s;
   ha_attn_params a;
-  fill_attn(p, a);
+  const Layout lay(p, strides);
+  fill_attn(p, lay, a);
   a.delta = delta; a.dq_acc = dq_acc; a.dk_acc = dk_acc; a.dv_acc = dv_acc;
   // The leaves run first and cover every row.  The warp-specialised kernel holds a query row's whole sum in one item there: it stores
   // dQ, whose accumulator needs no zero-fill.  In the earlier kernel an item owns a key tile's whole dK / dV (leaves of up
@@ -479,7 +515,7 @@ int ha_causal_bwd(const ha_causal_params* pp, void* stream) {
   // reference gradient convention: every part uses sum(o_part * dO) of its own output (its d(lse) is dropped);
   // exact convention: sum(o * dO) of the merged output, computed once
   bool fused_parts = false;
-  if (p.keep_parts) {
+  if (p.keep_parts && Layout::contiguous(lay.g, p)) {
     const int es = dtype_size(p.dtype), epc = 16 / es, lpr = p.dv / epc;
     if (p.dv % epc == 0 && (lpr == 2 || lpr == 4 || lpr == 8 || lpr == 16 || lpr == 32) && (uintptr_t)p.d_o % 16 == 0) {
       const long long part_stride = (uint8_t*)sv.part_o(1) - (uint8_t*)sv.part_o(0);
@@ -501,7 +537,9 @@ int ha_causal_bwd(const ha_causal_params* pp, void* stream) {
     if (!p.keep_parts && part != p.levels) return HA_OK;   // one delta from the merged output serves every part
     const void* o_src = p.keep_parts ? sv.part_o(part) : p.o;
     a.delta = delta;
-    return ha_delta(o_src, a.o_sb, a.o_sh, a.o_sn, p.d_o, a.do_sb, a.do_sh, a.do_sn, p.B, p.H, p.n, p.dv, p.dtype, delta, stream);
+    const int64_t sh = (int64_t)p.n * p.dv;          // (the parts are contiguous)
+    const bool kept = p.keep_parts;
+    return ha_delta(o_src, kept ? sh * p.H : a.o_sb, kept ? sh : a.o_sh, kept ? p.dv : a.o_sn, p.d_o, a.do_sb, a.do_sh, a.do_sn, p.B, p.H, p.n, p.dv, p.dtype, delta, stream);
   };
   rc = part_delta(p.levels);
   if (rc != HA_OK) return rc;
@@ -532,6 +570,8 @@ int ha_causal_bwd(const ha_causal_params* pp, void* stream) {
   return ha_cast_from_f32(dv_acc, p.dv_out, pl.rows_k * p.dv, p.dtype, stream);
 }
 
+int ha_causal_bwd(const ha_causal_params* p, void* stream) { return ha_causal_bwd_strided(p, nullptr, stream); }
+
 
 /* ---------------------------------------------------------------------------------------------------------------
  * The non-causal module call (forward_no_causal_mask, hyper_attention.py:103-132, on sequences of at least min_seq_len)
@@ -552,8 +592,8 @@ static int noncausal_check(const ha_causal_params& p, long long& rows, long long
   return HA_OK;
 }
 
-static void noncausal_attn(const ha_causal_params& p, ha_attn_params& a, long long rows) {
-  fill_attn(p, a);
+static void noncausal_attn(const ha_causal_params& p, const Layout& lay, ha_attn_params& a, long long rows) {
+  fill_attn(p, lay, a);
   a.mode = HA_MODE_HYPER;
   a.flags = p.flags & (HA_FLAG_SMOOTH | HA_FLAG_BWD_REF_SMOOTH | HA_FLAG_FORCE_SIMT | HA_FLAG_NO_WS);
   a.segs_per_head = 1;
@@ -564,9 +604,9 @@ static void noncausal_attn(const ha_causal_params& p, ha_attn_params& a, long lo
 
 // what the backward needs beyond delta: 3 = fp32 dK and dV (typed dQ), 2 = slot buffers only, 1 = slot buffers + fp32 dQ, 0 = three fp32
 // accumulators
-static int noncausal_bwd_level(const ha_causal_params& p, long long rows) {
+static int noncausal_bwd_level(const ha_causal_params& p, const Layout& lay, long long rows) {
   ha_attn_params a;
-  noncausal_attn(p, a, rows);
+  noncausal_attn(p, lay, a, rows);
   float dummy = 0.f;
   a.delta = &dummy;                               // (only looked at for being there)
   a.dq_acc = a.dk_acc = a.dv_acc = nullptr;
@@ -584,11 +624,11 @@ int64_t ha_noncausal_saved_bytes(const ha_causal_params* p) {
   return 2 * align256(rows * 4);
 }
 
-int64_t ha_noncausal_scratch_bytes(const ha_causal_params* p, int32_t backward) {
+int64_t ha_noncausal_scratch_bytes_strided(const ha_causal_params* p, const int64_t* strides, int32_t backward) {
   long long rows, rows_k;
   if (!p || noncausal_check(*p, rows, rows_k) != HA_OK) return -1;
   if (!backward) return 2 * align256(rows * 4) + align256(ha_seg_sort_workspace_bytes(2 * p->B * p->H, p->n, p->n, p->n, p->lsh_bits));
-  const int level = noncausal_bwd_level(*p, rows);
+  const int level = noncausal_bwd_level(*p, Layout(*p, strides), rows);
   const long long sacc = align256((long long)p->B * p->H * p->sample_size * (p->d + p->dv) * 4);
   long long bytes = align256(rows * 4);
   if (level == 3) bytes += align256(rows_k * p->d * 4) + align256(rows_k * p->dv * 4);
@@ -598,7 +638,9 @@ int64_t ha_noncausal_scratch_bytes(const ha_causal_params* p, int32_t backward) 
   return bytes;
 }
 
-int ha_noncausal_fwd(const ha_causal_params* pp, void* stream) {
+int64_t ha_noncausal_scratch_bytes(const ha_causal_params* p, int32_t backward) { return ha_noncausal_scratch_bytes_strided(p, nullptr, backward); }
+
+int ha_noncausal_fwd_strided(const ha_causal_params* pp, const int64_t* strides, void* stream) {
   if (!pp) return HA_ERR_INVALID;
   const ha_causal_params& p = *pp;
   long long rows, rows_k;
@@ -612,11 +654,11 @@ int ha_noncausal_fwd(const ha_causal_params* pp, void* stream) {
   int32_t* codes = (int32_t*)p.scratch;
   void* sort_ws = (uint8_t*)p.scratch + 2 * align256(rows * 4);
   const long long sort_ws_bytes = p.scratch_bytes - 2 * align256(rows * 4);
-  const int64_t sn = p.d, sh = (int64_t)p.n * p.d, sb = sh * p.H;
-  rc = ha_lsh_hash(p.q, sb, sh, sn, p.B, p.H, p.n, p.d, p.dtype, p.proj, p.lsh_bits, codes, stream);
+  const Layout lay(p, strides);
+  rc = ha_lsh_hash(p.q, lay.q[0], lay.q[1], lay.q[2], p.B, p.H, p.n, p.d, p.dtype, p.proj, p.lsh_bits, codes, stream);
   if (rc != HA_OK) return rc;
   const int Hk = p.kv_group > 1 ? p.H / p.kv_group : p.H;
-  rc = ha_lsh_hash(p.k, sh * Hk, sh, sn, p.B, Hk, p.n, p.d, p.dtype, p.proj, p.lsh_bits, codes + rows, stream);
+  rc = ha_lsh_hash(p.k, lay.k[0], lay.k[1], lay.k[2], p.B, Hk, p.n, p.d, p.dtype, p.proj, p.lsh_bits, codes + rows, stream);
   if (rc != HA_OK) return rc;
   if (align256(rows * 4) == rows * 4 && Hk == p.H) {
     rc = ha_seg_sort(codes, 2 * p.B * p.H, p.n, p.n, 0, p.n, p.lsh_bits, (int32_t*)p.saved, sort_ws, sort_ws_bytes, stream);
@@ -628,11 +670,13 @@ int ha_noncausal_fwd(const ha_causal_params* pp, void* stream) {
   }
   if (rc != HA_OK) return rc;
   ha_attn_params a;
-  noncausal_attn(p, a, rows);
+  noncausal_attn(p, lay, a, rows);
   return ha_attn_fwd(&a, stream);
 }
 
-int ha_noncausal_bwd(const ha_causal_params* pp, void* stream) {
+int ha_noncausal_fwd(const ha_causal_params* p, void* stream) { return ha_noncausal_fwd_strided(p, nullptr, stream); }
+
+int ha_noncausal_bwd_strided(const ha_causal_params* pp, const int64_t* strides, void* stream) {
   if (!pp) return HA_ERR_INVALID;
   const ha_causal_params& p = *pp;
   long long rows, rows_k;
@@ -640,16 +684,17 @@ int ha_noncausal_bwd(const ha_causal_params* pp, void* stream) {
   if (rc != HA_OK) return rc;
   if (!p.q || !p.k || !p.v || !p.o || !p.lse || !p.d_o || !p.dq || !p.dk || !p.dv_out) return HA_ERR_INVALID;
   if (!p.saved || p.saved_bytes < ha_noncausal_saved_bytes(pp)) return HA_ERR_WORKSPACE;
-  if (!p.scratch || p.scratch_bytes < ha_noncausal_scratch_bytes(pp, 1)) return HA_ERR_WORKSPACE;
+  if (!p.scratch || p.scratch_bytes < ha_noncausal_scratch_bytes_strided(pp, strides, 1)) return HA_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   uint8_t* s = (uint8_t*)p.scratch;
   float* delta = (float*)s;                  s += align256(rows * 4);
   ha_attn_params a;
-  noncausal_attn(p, a, rows);
+  const Layout lay(p, strides);
+  noncausal_attn(p, lay, a, rows);
   a.delta = delta;
   rc = ha_delta(p.o, a.o_sb, a.o_sh, a.o_sn, p.d_o, a.do_sb, a.do_sh, a.do_sn, p.B, p.H, p.n, p.dv, p.dtype, delta, stream);
   if (rc != HA_OK) return rc;
-  const int level = noncausal_bwd_level(p, rows);
+  const int level = noncausal_bwd_level(p, lay, rows);
   if (level == 3) {
     a.dk_acc = (float*)s;                    s += align256(rows_k * p.d * 4);
     a.dv_acc = (float*)s;
@@ -701,5 +746,7 @@ int ha_noncausal_bwd(const ha_causal_params* pp, void* stream) {
   if (rc != HA_OK) return rc;
   return ha_cast_from_f32(a.dv_acc, p.dv_out, rows_k * p.dv, p.dtype, stream);
 }
+
+int ha_noncausal_bwd(const ha_causal_params* p, void* stream) { return ha_noncausal_bwd_strided(p, nullptr, stream); }
 
 }  // extern "C"

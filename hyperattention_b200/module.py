@@ -9,9 +9,9 @@ Additional keyword arguments (all optional, accepted through **kwargs like the r
   rng         torch.Generator used to draw proj_dir (the reference's AngularLSHTriton has the same argument).
   fused_causal  True (default): run regular causal shapes through the single-call schedule; False: always use the
               per-level path built from the individual operators.
-  fused_calls True (default): a non-causal call on contiguous inputs is one library call each way (hash, sort and attention;
-              delta, backward and finishing pass); False: one call per operator, as strided inputs and the uniform
-              sampling mode always do.
+  fused_calls True (default): a non-causal call is one library call each way (hash, sort and attention;
+              delta, backward and finishing pass); False: one call per operator, as the uniform sampling mode always
+              does.
 """
 import math
 
@@ -130,9 +130,11 @@ class HyperAttention(torch.nn.Module):
         return levels
 
     def _regular_causal(self, n):
-        """True when the single-call schedule applies: n halves evenly down to leaves <= min_seq_len, every rectangle is
+        """True when the single-call schedule applies: n (an odd n with the row it is padded by) halves evenly down to leaves <= min_seq_len, every rectangle is
         a whole number of 128-row tiles and those on the hyper pattern hold the sampled rows.  (Rectangles shorter than
         min_seq_len -- only the deepest ones can be -- are exact, hyper_attention.py:109-113; the schedule does the same.)"""
+        if n % 2 and self.grad_mode == 'reference':
+            n += 1
         levels = self._causal_levels(n)
         leaf = n >> levels
         smallest_hyper = 2 * leaf if self.min_seq_len > leaf else leaf
@@ -144,9 +146,9 @@ class HyperAttention(torch.nn.Module):
         """query, key [B, H, n, d]; value [B, H, n, dv]; returns attn [B, H, n, dv] (and lse, float32 [B, H, n, 1];
         [B, H, ceil(n/128)*128] when a causal call is short enough to be a single exact leaf, as in the reference)."""
         # The reference copies its inputs here (hyper_attention.py:38-40).  The kernels take (batch, head, row) strides,
-        # so only a tensor whose rows are not contiguous is copied; the causal schedule below, which addresses
-        # [B, H, n, d] memory directly, makes its own copies where it needs them.
-        query, key, value = [t if t.stride(-1) == 1 else t.contiguous() for t in (query, key, value)]
+        # so only a tensor whose rows are not contiguous is copied.  The output lies in memory in the order of the queries.
+        if query.stride(-1) != 1 or key.stride(-1) != 1 or value.stride(-1) != 1:
+            query, key, value = [t if t.stride(-1) == 1 else t.contiguous() for t in (query, key, value)]
         n_query = query.shape[2]
         batch_size, n_heads, n_key, dim = key.shape
         scale = scale or dim ** (-0.5)
@@ -156,8 +158,7 @@ class HyperAttention(torch.nn.Module):
             # expanded to every query head, chatglm_fast_attention.py:53-58).  The single-call paths hash and sort K once
             # per K/V head and never expand; every other path expands here.
             assert query.shape[1] % n_heads == 0 and value.shape[1] == n_heads, 'query heads must be a multiple of the K/V heads'
-            grouped_ok = self.sampling == 'reference' and n_key >= self.min_seq_len and all(
-                t.is_contiguous() for t in (query, key, value)) and \
+            grouped_ok = self.sampling == 'reference' and n_key >= self.min_seq_len and \
                 ((causal and n_key > self.min_seq_len and self.fused_causal and self._regular_causal(n_key)) or (not causal and self.fused_calls and query.dtype == self.lsh.proj_dir.dtype))
             if not grouped_ok:
                 rep = query.shape[1] // n_heads
@@ -167,12 +168,12 @@ class HyperAttention(torch.nn.Module):
             attn, lse = self.forward_no_causal_mask(query, key, value, scale)
         elif n_key <= self.min_seq_len:
             attn, lse = ops.flash_attn_func(query.transpose(1, 2), key.transpose(1, 2), value.transpose(1, 2), None, True,
-                                            scale, self.kernel_flags & L.FLAG_FORCE_SIMT)
+                                            scale, self.kernel_flags & L.FLAG_FORCE_SIMT, return_lse)
             attn = attn.transpose(1, 2)
         elif self.fused_causal and self.sampling == 'reference' and self._regular_causal(n_key):
-            attn, lse = ops.CausalHyperFunc.apply(query, key, value, self.lsh.proj_f32(), self._causal_levels(n_key),
-                                                  self.block_size, self.sample_size, scale, self._flags(),
-                                                  self.grad_mode == 'reference', self.min_seq_len)
+            attn, lse = ops.causal_hyper(query, key, value, self.lsh.proj_f32(), self._causal_levels(n_key + n_key % 2),
+                                         self.block_size, self.sample_size, scale, self._flags(),
+                                         self.grad_mode == 'reference', self.min_seq_len)
             lse = lse.unsqueeze(-1)
         else:
             attn, lse = self._causal_by_levels(query.contiguous(), key.contiguous(), value.contiguous(), scale)
@@ -213,11 +214,10 @@ class HyperAttention(torch.nn.Module):
         if self.min_seq_len > n_query:
             attn, lse = ops.flash_attn_func(query.transpose(1, 2), key.transpose(1, 2), value.transpose(1, 2), None, False,
                                             scale, self.kernel_flags & L.FLAG_FORCE_SIMT)
-        elif self.sampling == 'reference' and self.fused_calls and query.is_contiguous() and key.is_contiguous() \
-                and value.is_contiguous() and query.dtype == self.lsh.proj_dir.dtype:
+        elif self.sampling == 'reference' and self.fused_calls and query.dtype == self.lsh.proj_dir.dtype:
             # hash, sort, attention (and, in the backward, delta, the backward kernel, the finishing pass) in one library call
-            attn, lse = ops.NonCausalHyperFunc.apply(query, key, value, self.lsh.proj_f32(), self.block_size, self.sample_size,
-                                                     scale, self._flags())
+            attn, lse = ops.noncausal_hyper(query, key, value, self.lsh.proj_f32(), self.block_size, self.sample_size,
+                                            scale, self._flags())
             return attn, lse.unsqueeze(-1)
         else:
             bits = self.lsh_num_projs

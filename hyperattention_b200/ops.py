@@ -21,7 +21,45 @@ def _dtype_id(t):
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+
+
+def _call(fn, device, *args):
+    """fn(*args, stream) with `device` current (which it nearly always is: switching and back costs as much as a launch)."""
+    if torch.cuda.current_device() == device.index:
+        return fn(*args, torch._C._cuda_getCurrentRawStream(device.index))
+    with torch.cuda.device(device):
+        return fn(*args, torch._C._cuda_getCurrentRawStream(device.index))
+
+
+def _wants_grad(*ts):
+    return torch.is_grad_enabled() and any(t.requires_grad for t in ts)
+
+
+# Parameter structs of earlier calls by shape, strides and options (everything but the pointers): filling one field by field costs more
+# host time than the launch.  Bounded; entries are immutable bytes.
+_TEMPLATES = {}
+
+
+def _template(cls, key, fill):
+    raw = _TEMPLATES.get(key)
+    if raw is None:
+        p = cls()
+        fill(p)
+        if len(_TEMPLATES) >= 512:
+            _TEMPLATES.clear()
+        raw = _TEMPLATES[key] = bytes(p)
+    return cls.from_buffer_copy(raw)
+
+
+def _rows_like(t, width):
+    """Uninitialised [B, H, n, width] tensor whose dimensions lie in memory in the order of t's (rows contiguous)."""
+    B, H, n, d = t.shape
+    if not t.is_contiguous() and width == d:
+        o = torch.empty_like(t)
+        if o.stride(-1) == 1:
+            return o
+    return torch.empty(B, H, n, width, dtype=t.dtype, device=t.device)
 
 
 def _ptr(t):
@@ -29,6 +67,7 @@ def _ptr(t):
 
 
 _STATUS = {}
+_STATUS_RAW = {}        # the words' addresses, and the host word as the processor sees it
 
 
 def _status_words(device):
@@ -39,6 +78,8 @@ def _status_words(device):
     if key not in _STATUS:
         _STATUS[key] = (torch.zeros(1, dtype=torch.int32, device=f'cuda:{key}'),
                         torch.zeros(1, dtype=torch.int32).pin_memory())
+        dev_w, host_w = _STATUS[key]
+        _STATUS_RAW[key] = (dev_w.data_ptr(), host_w.data_ptr(), C.c_int32.from_address(host_w.data_ptr()))
     return _STATUS[key]
 
 
@@ -50,9 +91,13 @@ def _set_status(p, device):
     """Fills the status pointers of a parameter struct.  Before that, looks at the host-visible word: a timeout
     reported by an earlier launch raises here, at the next call into the library, instead of going unnoticed (the
     outputs of the launch that timed out, and of everything launched since, are undefined)."""
-    dev_w, host_w = _status_words(device)
-    _raise_if_failed(dev_w, host_w)
-    p.status, p.status_host = _ptr(dev_w), C.c_void_p(host_w.data_ptr())
+    raw = _STATUS_RAW.get(device.index)
+    if raw is None:
+        _status_words(device)
+        raw = _STATUS_RAW[device.index]
+    if raw[2].value != 0:
+        _raise_if_failed(*_status_words(device))
+    p.status, p.status_host = raw[0], raw[1]
 
 
 def _status_text(v):
@@ -377,38 +422,42 @@ def hyper_attn_func(q, k, v, q_sort_idx, k_sort_idx, block_size, sample_size=0, 
                                sample_idx, flags, weighted)
 
 
+def _flash_forward(q, k, v, causal, softmax_scale, flags):
+    """Exact attention on [B, n, H, *] views with contiguous rows: o [B, n_q, H, dv] (in the memory order of q) and lse [B, H, n_q]."""
+    _cuda(q, k, v)
+    B, nq, H, d = q.shape
+    nk = k.shape[1]
+    assert k.shape == (B, nk, H, d)
+    assert v.shape[:3] == (B, nk, H)
+    assert q.dtype == k.dtype == v.dtype, 'All tensors must have the same type'
+    o = _rows_like(q.transpose(1, 2), v.shape[-1]).transpose(1, 2)
+    lse = torch.empty(B, H, nq, dtype=torch.float32, device=q.device)
+    p = _flash_params(q, k, v, o, lse, causal, softmax_scale or 1.0 / math.sqrt(d), flags)
+    L.check(_call(L.load().ha_attn_fwd, q.device, C.byref(p)), 'ha_attn_fwd')
+    return o, lse
+
+
 class FlashAttnFunc(torch.autograd.Function):
     """Drop-in for FlashAttnFunc (src/flash_attn_triton.py:995-1042) without the bias branch: q [B, n_q, H, d],
-    k, v [B, n_k, H, d]; returns o [B, n_q, H, d] and lse [B, H, ceil(n_q/128)*128] (rows past n_q are zero)."""
+    k, v [B, n_k, H, d]; returns o [B, n_q, H, d] and lse [B, H, ceil(n_q/128)*128] (rows past n_q are zero;
+    pad_lse=False: lse [B, H, n_q])."""
 
     @staticmethod
-    def forward(ctx, q, k, v, bias=None, causal=False, softmax_scale=None, flags=0):
+    def forward(ctx, q, k, v, bias=None, causal=False, softmax_scale=None, flags=0, pad_lse=True):
         assert bias is None, 'attention bias is not part of the HyperAttention path'
-        _cuda(q, k, v)
         q, k, v = [x if x.stride(-1) == 1 else x.contiguous() for x in (q, k, v)]
-        B, nq, H, d = q.shape
-        nk = k.shape[1]
-        assert k.shape == (B, nk, H, d)
-        assert v.shape[:3] == (B, nk, H)
-        assert q.dtype == k.dtype == v.dtype, 'All tensors must have the same type'
-        dv = v.shape[-1]
-        scale = softmax_scale or 1.0 / math.sqrt(d)
-        o = torch.empty(B, H, nq, dv, dtype=q.dtype, device=q.device).transpose(1, 2)
-        lse = torch.empty(B, H, nq, dtype=torch.float32, device=q.device)
-        p = _flash_params(q, k, v, o, lse, causal, scale, flags)
-        with torch.cuda.device(q.device):
-            rc = L.load().ha_attn_fwd(C.byref(p), _stream())
-        L.check(rc, 'ha_attn_fwd')
+        o, lse = _flash_forward(q, k, v, causal, softmax_scale, flags)
         ctx.save_for_backward(q, k, v, o, lse)
-        ctx.cfg = (causal, scale, flags)
-        nq_r = math.ceil(nq / 128) * 128
-        lse_out = lse if nq_r == nq else torch.nn.functional.pad(lse, (0, nq_r - nq))
-        return o, lse_out
+        ctx.cfg = (causal, softmax_scale or 1.0 / math.sqrt(q.shape[-1]), flags)
+        ctx.set_materialize_grads(False)          # the gradient of lse is never used: no zero tensor for it
+        return o, _pad_lse(lse) if pad_lse else lse
 
     @staticmethod
     def backward(ctx, do, dlse_unused=None):
         q, k, v, o, lse = ctx.saved_tensors
         causal, scale, flags = ctx.cfg
+        if do is None:                            # only lse was used downstream: its gradient is dropped, as in the reference
+            return (None,) * 8
         if do.stride(-1) != 1:
             do = do.contiguous()
         B, nq, H, d = q.shape
@@ -430,173 +479,228 @@ class FlashAttnFunc(torch.autograd.Function):
             rc = lib.ha_attn_bwd(C.byref(p), _stream())
             L.check(rc, 'ha_attn_bwd')
             grads = _cast_grads(lib, acc, q.dtype, B, H, n, d, dv)
-        return grads + (None,) * 4
+        return grads + (None,) * 5
+
+
+def _pad_lse(lse):
+    nq = lse.shape[-1]
+    nq_r = math.ceil(nq / 128) * 128
+    return lse if nq_r == nq else torch.nn.functional.pad(lse, (0, nq_r - nq))
 
 
 def _flash_params(q, k, v, o, lse, causal, scale, flags):
-    B, nq, H, d = q.shape
-    nk, dv = k.shape[1], v.shape[-1]
-    n = nq
-    p = L.AttnParams()
-    p.mode, p.dtype = L.MODE_FLASH, _dtype_id(q)
-    p.flags = (L.FLAG_CAUSAL if causal else 0) | flags
-    p.B, p.H, p.n, p.d, p.dv = B, H, n, d, dv
-    p.segs_per_head, p.span, p.q_off, p.k_off, p.m_q, p.m_k = 1, n, 0, 0, nq, nk
-    p.scale = scale
-    _fill_qkv(p, q, k, v)
-    p.o = _ptr(o)
-    p.o_sb, p.o_sh, p.o_sn = _bhn(o)
-    p.lse = _ptr(lse)
+    def fill(p):
+        B, nq, H, d = q.shape
+        nk, dv = k.shape[1], v.shape[-1]
+        p.mode, p.dtype = L.MODE_FLASH, _dtype_id(q)
+        p.flags = (L.FLAG_CAUSAL if causal else 0) | flags
+        p.B, p.H, p.n, p.d, p.dv = B, H, nq, d, dv
+        p.segs_per_head, p.span, p.q_off, p.k_off, p.m_q, p.m_k = 1, nq, 0, 0, nq, nk
+        p.scale = scale
+        p.q_sb, p.q_sh, p.q_sn = _bhn(q)
+        p.k_sb, p.k_sh, p.k_sn = _bhn(k)
+        p.v_sb, p.v_sh, p.v_sn = _bhn(v)
+        p.o_sb, p.o_sh, p.o_sn = _bhn(o)
+    p = _template(L.AttnParams, (0, q.dtype, q.shape, k.shape[1], v.shape[-1], q.stride(), k.stride(), v.stride(), o.stride(), causal, scale, flags), fill)
+    p.q, p.k, p.v, p.o, p.lse = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr()
     _set_status(p, q.device)
     return p
 
 
-def flash_attn_func(q, k, v, bias=None, causal=False, softmax_scale=None, flags=0):
-    return FlashAttnFunc.apply(q, k, v, bias, causal, softmax_scale, flags)
+def flash_attn_func(q, k, v, bias=None, causal=False, softmax_scale=None, flags=0, pad_lse=True):
+    if bias is None and not _wants_grad(q, k, v):
+        q, k, v = [x if x.stride(-1) == 1 else x.contiguous() for x in (q, k, v)]
+        o, lse = _flash_forward(q, k, v, causal, softmax_scale, flags)
+        return o, _pad_lse(lse) if pad_lse else lse
+    return FlashAttnFunc.apply(q, k, v, bias, causal, softmax_scale, flags, pad_lse)
 
 
 # ------------------------------------------------------------------------------------------------
+# The single-call paths.  Sizes, strides and buffer sizes of a call are worked out once per shape (_PLANS; bounded).
+_PLANS = {}
+
+
+def _plan(causal, backward, q, k, v, o, do, cfg):
+    """(parameter struct with the tensors' pointers set, strides array, bytes of `saved`, bytes of scratch) of one call;
+    cfg = (levels, block_size, sample_size, lsh_bits, keep_parts, min_seq_len, scale, flags)."""
+    ptrs = (q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr() if do is not None else 0)
+    key = (causal, backward, q.dtype, q.shape, k.shape[1], v.shape[-1], q.stride(), k.stride(), v.stride(), o.stride(),
+           do.stride() if do is not None else None, cfg, (ptrs[0] | ptrs[1] | ptrs[2] | ptrs[3] | ptrs[4]) & 15)
+    plan = _PLANS.get(key)
+    if plan is None:
+        p = L.CausalParams()
+        p.dtype = _dtype_id(q)
+        p.B, p.H, p.n, p.d = q.shape
+        p.dv = v.shape[-1]
+        p.levels, p.block_size, p.sample_size, p.lsh_bits, p.keep_parts, p.min_seq_len, p.scale, p.flags = cfg
+        p.kv_group = q.shape[1] // k.shape[1]
+        st = (C.c_int64 * 15)(*q.stride()[:3], *k.stride()[:3], *v.stride()[:3], *o.stride()[:3], *(do.stride()[:3] if do is not None else (0, 0, 0)))
+        raw = bytes(p)
+        p.q, p.k, p.v, p.o, p.d_o = ptrs
+        lib = L.load()
+        if causal:
+            saved, scratch = lib.ha_causal_saved_bytes(C.byref(p)), lib.ha_causal_scratch_bytes(C.byref(p), backward)
+            assert saved >= 0 and scratch >= 0, 'causal schedule: n must be divisible by 2^levels with 128-row multiples at every depth'
+        else:
+            saved, scratch = lib.ha_noncausal_saved_bytes(C.byref(p)), lib.ha_noncausal_scratch_bytes_strided(C.byref(p), st, backward)
+            assert saved >= 0 and scratch >= 0, 'shape not accepted (n and sample_size multiples of 128, sample_size <= n)'
+        if len(_PLANS) >= 512:
+            _PLANS.clear()
+        plan = _PLANS[key] = (raw, st, saved, scratch)
+    raw, st, saved, scratch = plan
+    p = L.CausalParams.from_buffer_copy(raw)
+    p.q, p.k, p.v, p.o, p.d_o = ptrs
+    _set_status(p, q.device)
+    return p, st, saved, scratch
+
+
+def _buffer(p, name, nbytes, device):
+    t = torch.empty(nbytes, dtype=torch.uint8, device=device)
+    setattr(p, name, t.data_ptr())
+    setattr(p, name + '_bytes', nbytes)
+    return t
+
+
+def _call_forward(causal, q, k, v, proj_f32, cfg):
+    """One ha_causal_fwd / ha_noncausal_fwd call on [B, H, n, *] tensors with contiguous rows: (o, lse [B, H, n], saved)."""
+    _cuda(q, k, v, proj_f32)
+    B, H, n, d = q.shape
+    dev = q.device
+    dv = v.shape[-1]
+    # o lies in memory as q does; the causal schedule's merges outside the tensor-core kernels want it contiguous
+    strided_o = not causal or (q.dtype != torch.float32 and dv in (32, 64, 128) and not cfg[7] & L.FLAG_FORCE_SIMT)
+    o = _rows_like(q, dv) if strided_o else torch.empty(B, H, n, dv, dtype=q.dtype, device=dev)
+    lse = torch.empty(B, H, n, dtype=torch.float32, device=dev)
+    p, st, saved_bytes, scratch_bytes = _plan(causal, 0, q, k, v, o, None, cfg)
+    p.proj, p.lse = proj_f32.data_ptr(), lse.data_ptr()
+    saved = _buffer(p, 'saved', saved_bytes, dev)
+    scratch = _buffer(p, 'scratch', scratch_bytes, dev)      # (free once the launches are enqueued: same stream)
+    lib = L.load()
+    if causal:
+        L.check(_call(lib.ha_causal_fwd_strided, dev, C.byref(p), st), 'ha_causal_fwd')
+    else:
+        L.check(_call(lib.ha_noncausal_fwd_strided, dev, C.byref(p), st), 'ha_noncausal_fwd')
+    del scratch
+    return o, lse, saved
+
+
+def _call_backward(causal, q, k, v, proj_f32, o, lse, saved, do, cfg):
+    dev = q.device
+    # one buffer for the three gradients (dq | dk | dv): one allocation per step
+    nq, nk, nv = q.numel(), k.numel(), v.numel()
+    out = torch.empty(nq + nk + nv, dtype=q.dtype, device=dev)
+    dq, dk, dvv = out[:nq].view(q.shape), out[nq:nq + nk].view(k.shape), out[nq + nk:].view(v.shape)
+    p, st, _, scratch_bytes = _plan(causal, 1, q, k, v, o, do, cfg)
+    p.proj, p.lse = proj_f32.data_ptr(), lse.data_ptr()
+    p.saved, p.saved_bytes = saved.data_ptr(), saved.numel()
+    p.dq = out.data_ptr()
+    p.dk, p.dv_out = p.dq + nq * out.element_size(), p.dq + (nq + nk) * out.element_size()
+    scratch = _buffer(p, 'scratch', scratch_bytes, dev)
+    lib = L.load()
+    if causal:
+        L.check(_call(lib.ha_causal_bwd_strided, dev, C.byref(p), st), 'ha_causal_bwd')
+    else:
+        L.check(_call(lib.ha_noncausal_bwd_strided, dev, C.byref(p), st), 'ha_noncausal_bwd')
+    del scratch
+    return dq, dk, dvv
+
+
+def _padded(t, rows):
+    """t [B, H, n, w] with zero rows up to `rows`, contiguous."""
+    B, H, n, w = t.shape
+    out = torch.empty(B, H, rows, w, dtype=t.dtype, device=t.device)
+    out[:, :, :n].copy_(t)
+    out[:, :, n:].zero_()
+    return out
+
+
 class CausalHyperFunc(torch.autograd.Function):
-    """The whole causal recursion (hyper_attention.py:51-96) as one call on contiguous [B, H, n, *] tensors.
+    """The whole causal recursion (hyper_attention.py:51-96) as one call on [B, H, n, *] tensors with contiguous rows.
     grad_reference=True keeps every part's own output so that the backward reproduces the reference's gradient
     convention (each part differentiated with its own rowwise o.do, d(lse) dropped); False gives the gradient of the
-    merged output."""
+    merged output.  An odd n is padded by one zero row, as the reference does at the first split (hyper_attention.py:59-61)."""
 
     @staticmethod
     def forward(ctx, q, k, v, proj_f32, levels, block_size, sample_size, scale, flags, grad_reference, min_seq_len=0):
-        _cuda(q, k, v, proj_f32)
-        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        B, H, n, d = q.shape
-        dv = v.shape[-1]
-        dev = q.device
-        need_grad = any(t.requires_grad for t in (q, k, v))
-        o = torch.empty(B, H, n, dv, dtype=q.dtype, device=dev)
-        lse = torch.empty(B, H, n, dtype=torch.float32, device=dev)
-        p = L.CausalParams()
-        p.dtype, p.flags = _dtype_id(q), flags
-        p.B, p.H, p.n, p.d, p.dv = B, H, n, d, dv
-        p.levels, p.block_size, p.sample_size, p.lsh_bits = levels, block_size, sample_size, proj_f32.shape[1]
-        p.keep_parts = 1 if (grad_reference and need_grad) else 0
-        p.min_seq_len = min_seq_len
-        p.kv_group = H // k.shape[1]
-        p.scale = scale
-        p.q, p.k, p.v, p.proj, p.o, p.lse = _ptr(q), _ptr(k), _ptr(v), _ptr(proj_f32), _ptr(o), _ptr(lse)
-        _set_status(p, dev)
-        lib = L.load()
-        saved_bytes = lib.ha_causal_saved_bytes(C.byref(p))
-        scratch_bytes = lib.ha_causal_scratch_bytes(C.byref(p), 0)
-        assert saved_bytes >= 0 and scratch_bytes >= 0, \
-            'causal schedule: n must be divisible by 2^levels with 128-row multiples at every depth'
-        saved = torch.empty(saved_bytes, dtype=torch.uint8, device=dev)
-        scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=dev)
-        p.saved, p.saved_bytes, p.scratch, p.scratch_bytes = _ptr(saved), saved_bytes, _ptr(scratch), scratch_bytes
-        with torch.cuda.device(dev):
-            rc = lib.ha_causal_fwd(C.byref(p), _stream())
-        L.check(rc, 'ha_causal_fwd')
+        n = q.shape[2]
+        o, lse, saved, (q, k, v), cfg = CausalHyperFunc.run(q, k, v, proj_f32, levels, block_size, sample_size, scale, flags,
+                                                            grad_reference and any(t.requires_grad for t in (q, k, v)), min_seq_len)
         ctx.save_for_backward(q, k, v, o, lse, saved, proj_f32)
-        ctx.cfg = (levels, block_size, sample_size, scale, flags, p.keep_parts, min_seq_len)
-        return o, lse
+        ctx.cfg = cfg
+        ctx.set_materialize_grads(False)
+        return (o, lse) if o.shape[2] == n else (o[:, :, :n], lse[:, :, :n])
+
+    @staticmethod
+    def run(q, k, v, proj_f32, levels, block_size, sample_size, scale, flags, keep_parts, min_seq_len):
+        assert q.dtype == k.dtype == v.dtype, 'All tensors must have the same type'
+        n = q.shape[2]
+        if n % 2:
+            q, k, v = [_padded(t, n + 1) for t in (q, k, v)]
+        cfg = (levels, block_size, sample_size, proj_f32.shape[1], int(keep_parts), min_seq_len, scale, flags)
+        o, lse, saved = _call_forward(True, q, k, v, proj_f32, cfg)
+        return o, lse, saved, (q, k, v), cfg
 
     @staticmethod
     def backward(ctx, do, dlse_unused=None):
+        if do is None:
+            return (None,) * 11
         q, k, v, o, lse, saved, proj_f32 = ctx.saved_tensors
-        levels, block_size, sample_size, scale, flags, keep_parts, min_seq_len = ctx.cfg
-        do = do.contiguous()
-        B, H, n, d = q.shape
-        dv = v.shape[-1]
-        dev = q.device
-        dq, dk, dvv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        p = L.CausalParams()
-        p.dtype, p.flags = _dtype_id(q), flags
-        p.B, p.H, p.n, p.d, p.dv = B, H, n, d, dv
-        p.levels, p.block_size, p.sample_size, p.lsh_bits = levels, block_size, sample_size, proj_f32.shape[1]
-        p.keep_parts, p.scale, p.min_seq_len = keep_parts, scale, min_seq_len
-        p.kv_group = H // k.shape[1]
-        p.q, p.k, p.v, p.proj, p.o, p.lse = _ptr(q), _ptr(k), _ptr(v), _ptr(proj_f32), _ptr(o), _ptr(lse)
-        p.saved, p.saved_bytes = _ptr(saved), saved.numel()
-        _set_status(p, dev)
-        lib = L.load()
-        scratch_bytes = lib.ha_causal_scratch_bytes(C.byref(p), 1)
-        scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=dev)
-        p.scratch, p.scratch_bytes = _ptr(scratch), scratch_bytes
-        p.d_o, p.dq, p.dk, p.dv_out = _ptr(do), _ptr(dq), _ptr(dk), _ptr(dvv)
-        with torch.cuda.device(dev):
-            rc = lib.ha_causal_bwd(C.byref(p), _stream())
-        L.check(rc, 'ha_causal_bwd')
-        return dq, dk, dvv, None, None, None, None, None, None, None, None
+        n, rows = do.shape[2], q.shape[2]
+        do = do.contiguous() if n == rows else _padded(do, rows)
+        dq, dk, dv = _call_backward(True, q, k, v, proj_f32, o, lse, saved, do, ctx.cfg)
+        if n != rows:
+            dq, dk, dv = dq[:, :, :n], dk[:, :, :n], dv[:, :, :n]
+        return (dq, dk, dv) + (None,) * 8
+
+
+def causal_hyper(q, k, v, proj_f32, levels, block_size, sample_size, scale, flags, grad_reference, min_seq_len):
+    """CausalHyperFunc, without the autograd machinery where no gradient is wanted."""
+    if _wants_grad(q, k, v):
+        return CausalHyperFunc.apply(q, k, v, proj_f32, levels, block_size, sample_size, scale, flags, grad_reference, min_seq_len)
+    n = q.shape[2]
+    o, lse = CausalHyperFunc.run(q, k, v, proj_f32, levels, block_size, sample_size, scale, flags, False, min_seq_len)[:2]
+    return (o, lse) if n % 2 == 0 else (o[:, :, :n], lse[:, :, :n])
 
 
 class NonCausalHyperFunc(torch.autograd.Function):
     """forward_no_causal_mask on sequences of at least min_seq_len (hyper_attention.py:116-130: hash, stable sort,
-    hyper_attn_func) as ONE library call each way (ha_noncausal_fwd / ha_noncausal_bwd) on contiguous [B, H, n, *] tensors:
+    hyper_attn_func) as ONE library call each way (ha_noncausal_fwd / ha_noncausal_bwd) on [B, H, n, *] tensors with contiguous rows:
     two calls into the library per training step instead of nine, which is what bounds the step when a rank owns few
     heads.  Returns o [B, H, n, dv] and lse [B, H, n]; the gradient flowing into lse is discarded, as in the reference."""
 
     @staticmethod
-    def _params(q, k, v, proj_f32, block_size, sample_size, scale, flags):
-        B, H, n, d = q.shape
-        p = L.CausalParams()
-        p.dtype, p.flags = _dtype_id(q), flags
-        p.B, p.H, p.n, p.d, p.dv = B, H, n, d, v.shape[-1]
-        p.block_size, p.sample_size, p.lsh_bits, p.scale = block_size, sample_size, proj_f32.shape[1], scale
-        p.kv_group = H // k.shape[1]
-        p.q, p.k, p.v, p.proj = _ptr(q), _ptr(k), _ptr(v), _ptr(proj_f32)
-        _set_status(p, q.device)
-        return p
-
-    @staticmethod
-    def forward(ctx, q, k, v, proj_f32, block_size, sample_size, scale, flags):
-        _cuda(q, k, v, proj_f32)
-        assert q.is_contiguous() and k.is_contiguous() and v.is_contiguous()
+    def run(q, k, v, proj_f32, block_size, sample_size, scale, flags):
         assert q.dtype == k.dtype == v.dtype, 'All tensors must have the same type'
         B, H, n, d = q.shape
         assert k.shape[0] == B and k.shape[2:] == (n, d), 'query and key sequence lengths must be equal'
         assert H % k.shape[1] == 0 and v.shape[:3] == k.shape[:3], 'query heads must be a multiple of the key/value heads'
         assert n % 128 == 0, 'keys sequence length must be divisible by 128'
         assert sample_size % 128 == 0
-        dev = q.device
-        o = torch.empty(B, H, n, v.shape[-1], dtype=q.dtype, device=dev)
-        lse = torch.empty(B, H, n, dtype=torch.float32, device=dev)
-        p = NonCausalHyperFunc._params(q, k, v, proj_f32, block_size, sample_size, scale, flags)
-        p.o, p.lse = _ptr(o), _ptr(lse)
-        lib = L.load()
-        saved_bytes, scratch_bytes = lib.ha_noncausal_saved_bytes(C.byref(p)), lib.ha_noncausal_scratch_bytes(C.byref(p), 0)
-        assert saved_bytes >= 0 and scratch_bytes >= 0, 'shape not accepted (n and sample_size multiples of 128, sample_size <= n)'
-        saved = torch.empty(saved_bytes, dtype=torch.uint8, device=dev)
-        scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=dev)
-        p.saved, p.saved_bytes, p.scratch, p.scratch_bytes = _ptr(saved), saved_bytes, _ptr(scratch), scratch_bytes
-        with torch.cuda.device(dev):
-            rc = lib.ha_noncausal_fwd(C.byref(p), _stream())
-        L.check(rc, 'ha_noncausal_fwd')
+        cfg = (0, block_size, sample_size, proj_f32.shape[1], 0, 0, scale, flags)
+        return _call_forward(False, q, k, v, proj_f32, cfg), cfg
+
+    @staticmethod
+    def forward(ctx, q, k, v, proj_f32, block_size, sample_size, scale, flags):
+        (o, lse, saved), ctx.cfg = NonCausalHyperFunc.run(q, k, v, proj_f32, block_size, sample_size, scale, flags)
         ctx.save_for_backward(q, k, v, o, lse, saved, proj_f32)
-        ctx.cfg = (block_size, sample_size, scale, flags)
         ctx.set_materialize_grads(False)
         return o, lse
 
     @staticmethod
     def backward(ctx, do, dlse_unused=None):
-        q, k, v, o, lse, saved, proj_f32 = ctx.saved_tensors
-        block_size, sample_size, scale, flags = ctx.cfg
         if do is None:
             return (None,) * 8
-        do = do.contiguous()
-        dev = q.device
-        # one buffer for the three gradients (dq | dk | dv): one allocation per step
-        nq, nk, nv = q.numel(), k.numel(), v.numel()
-        out = torch.empty(nq + nk + nv, dtype=q.dtype, device=dev)
-        dq, dk, dvv = out[:nq].view_as(q), out[nq:nq + nk].view_as(k), out[nq + nk:].view_as(v)
-        p = NonCausalHyperFunc._params(q, k, v, proj_f32, block_size, sample_size, scale, flags)
-        p.o, p.lse = _ptr(o), _ptr(lse)
-        p.saved, p.saved_bytes = _ptr(saved), saved.numel()
-        p.d_o, p.dq, p.dk, p.dv_out = _ptr(do), _ptr(dq), _ptr(dk), _ptr(dvv)
-        lib = L.load()
-        scratch_bytes = lib.ha_noncausal_scratch_bytes(C.byref(p), 1)
-        scratch = torch.empty(scratch_bytes, dtype=torch.uint8, device=dev)
-        p.scratch, p.scratch_bytes = _ptr(scratch), scratch_bytes
-        with torch.cuda.device(dev):
-            rc = lib.ha_noncausal_bwd(C.byref(p), _stream())
-        L.check(rc, 'ha_noncausal_bwd')
-        return dq, dk, dvv, None, None, None, None, None
+        q, k, v, o, lse, saved, proj_f32 = ctx.saved_tensors
+        if do.stride(-1) != 1:
+            do = do.contiguous()
+        return _call_backward(False, q, k, v, proj_f32, o, lse, saved, do, ctx.cfg) + (None,) * 5
+
+
+def noncausal_hyper(q, k, v, proj_f32, block_size, sample_size, scale, flags):
+    """NonCausalHyperFunc, without the autograd machinery where no gradient is wanted."""
+    if _wants_grad(q, k, v):
+        return NonCausalHyperFunc.apply(q, k, v, proj_f32, block_size, sample_size, scale, flags)
+    return NonCausalHyperFunc.run(q, k, v, proj_f32, block_size, sample_size, scale, flags)[0][:2]
 
 
 def launch_count():

@@ -260,6 +260,16 @@ int64_t ha_noncausal_scratch_bytes(const ha_causal_params* p, int32_t backward);
 int ha_noncausal_fwd(const ha_causal_params* p, void* stream);
 int ha_noncausal_bwd(const ha_causal_params* p, void* stream);
 
+/* The same calls on strided tensors.  strides: 15 element strides, (batch, head, row) of q, k, v, o, dO in this order, the last
+ * dimension contiguous (dO's are looked at by the backward only); NULL = contiguous.  The gradients stay contiguous.  (A causal
+ * call that keeps its parts on the CUDA-core kernels takes a contiguous o only.)  The reference copies its inputs instead
+ * (hyper_attention.py:38-40). */
+int ha_causal_fwd_strided(const ha_causal_params* p, const int64_t* strides, void* stream);
+int ha_causal_bwd_strided(const ha_causal_params* p, const int64_t* strides, void* stream);
+int64_t ha_noncausal_scratch_bytes_strided(const ha_causal_params* p, const int64_t* strides, int32_t backward);
+int ha_noncausal_fwd_strided(const ha_causal_params* p, const int64_t* strides, void* stream);
+int ha_noncausal_bwd_strided(const ha_causal_params* p, const int64_t* strides, void* stream);
+
 /* Diagnostic for the timeout path.  One warp polls an mbarrier that nothing ever arrives at, `polls` times (1..2^18),
  * gives up and reports HA_DEV_TIMEOUT through status / status_host exactly as the attention kernels do when one of their
  * bounded waits runs out.  No copy and no tensor-core operation is in flight; the kernel returns normally and the

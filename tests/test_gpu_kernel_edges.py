@@ -100,3 +100,54 @@ def test_rows_that_see_no_key_of_a_tile():
     o, lse = ha.hyper_attn_func(T(q.cuda()), T(k.cuda()), T(v.cuda()), T(qi.cuda()), T(ki.cuda()), 256, 128, None, False, sidx.cuda(), 0, True)
     ow, lw = O.hyper_attn_func(T(q.float()), T(k.float()), T(v.float()), T(qi), T(ki), 256, 128, None, False, sidx, False, True)
     assert rel(o, ow) < 2e-2 and rel(lse, lw) < 2e-2
+
+
+@pytest.mark.parametrize('n,dtype,train', [(1023, torch.bfloat16, True), (2047, torch.float32, True), (1535, torch.bfloat16, False)])
+def test_causal_odd_length_runs_the_single_call_schedule(n, dtype, train):
+    """an odd length is padded by one zero row and takes the single-call schedule: against the oracle, which pads as the reference does"""
+    import hyperattention_b200 as ha
+    torch.manual_seed(74)
+    B, H, d = 1, 2, 64
+    proj = torch.randn(1, 1, d, 8).to(dtype).float()
+    q, k, v, do = [torch.randn(B, H, n, d).to(dtype) for _ in range(4)]
+    mod = ha.HyperAttention(input_dim=d, block_size=256, sample_size=256, min_seq_len=512)
+    mod.lsh.proj_dir.copy_(proj)
+    mod = mod.to(device='cuda', dtype=dtype)
+    assert mod._regular_causal(n)
+    qg, kg, vg = [t.cuda().requires_grad_(train) for t in (q, k, v)]
+    o, lse = mod(qg, kg, vg, causal=True, return_lse=True)
+    orc = O.HyperAttentionOracle(proj, 256, 256, 512, False)
+    qc, kc, vc = [t.float().requires_grad_() for t in (q, k, v)]
+    ow, lw = orc(qc, kc, vc, causal=True, return_lse=True)
+    assert o.shape == ow.shape and lse.shape == lw.shape
+    if not train:
+        return _check((o, lse), (ow, lw), dtype)
+    o.backward(do.cuda())
+    ow.backward(do.float())
+    _check((o, lse, qg.grad, kg.grad, vg.grad), (ow, lw, qc.grad, kc.grad, vc.grad), dtype)
+
+
+@pytest.mark.parametrize('causal', [True, False])
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float32])
+def test_strided_tensors_match_contiguous_ones(causal, dtype):
+    """[n, B, H, d] and [B, n, H, d] tensors as [B, H, n, d] views: same results, gradients included; the output keeps the order"""
+    import hyperattention_b200 as ha
+    torch.manual_seed(75)
+    B, H, n, d = 2, 3, 1024, 64
+    mod = ha.HyperAttention(input_dim=d, min_seq_len=256, sample_size=128, rng=torch.Generator().manual_seed(5)).to(device='cuda', dtype=dtype)
+    base = [torch.randn(B, H, n, d, device='cuda').to(dtype) for _ in range(4)]
+    res = []
+    for order in ((0, 1, 2, 3), (2, 0, 1, 3), (0, 2, 1, 3)):
+        inv = tuple(order.index(i) for i in range(4))
+        q, k, v, do = [t.permute(order).contiguous().permute(inv) for t in base]
+        q, k, v = [t.requires_grad_() for t in (q, k, v)]
+        o, lse = mod(q, k, v, causal=causal, return_lse=True)
+        if dtype == torch.bfloat16:
+            assert o.stride() == q.stride()
+        with torch.no_grad():
+            o2 = mod(q, k, v, causal=causal)
+        res.append((o.detach(), lse.detach(), o2) + torch.autograd.grad(o, (q, k, v), do))
+    for r in res[1:]:
+        assert torch.equal(r[0], res[0][0]) and torch.equal(r[1], res[0][1]) and torch.equal(r[2], res[0][2])
+        for a, b in zip(r[3:], res[0][3:]):
+            assert rel(a, b) < 1e-3
