@@ -83,6 +83,8 @@ SIGNATURES = {
     'ha_noncausal_scratch_bytes_strided': (i64, [C.POINTER(CausalParams), vp, i32]),
     'ha_noncausal_fwd_strided': (C.c_int, [C.POINTER(CausalParams), vp, vp]),
     'ha_noncausal_bwd_strided': (C.c_int, [C.POINTER(CausalParams), vp, vp]),
+    'ha_flash_bwd_scratch_bytes': (i64, [C.POINTER(AttnParams), vp]),
+    'ha_flash_bwd': (C.c_int, [C.POINTER(AttnParams), vp, vp, vp, vp, i64, vp]),
     'ha_wait_probe': (C.c_int, [vp, vp, i32, vp]),
     'ha_causal_saved_bytes': (i64, [C.POINTER(CausalParams)]),
     'ha_causal_scratch_bytes': (i64, [C.POINTER(CausalParams), i32]),

@@ -10,6 +10,7 @@
 // which the reference's merges nest (stored value = attn1, rectangle = attn2).  No concatenation, no per-depth
 // copies.
 #include "attn_index.cuh"
+#include "seg_sort.cuh"
 
 #include <mutex>
 
@@ -18,6 +19,8 @@ namespace ha {
 bool tc_bwd_supported(const ha_attn_params& p);   // attn_tc_bwd.cu
 bool ws_bwd_supported(const ha_attn_params& p);   // attn_tc_bwd_ws.cu
 int ws_attn_bwd(const ha_attn_params& p, bool store_dq, cudaStream_t st);
+int hash_pair(const void* q, const int64_t (&qs)[3], int H, int32_t* codes_q, const void* k, const int64_t (&ks)[3], int Hk, int32_t* codes_k, int B, int n,
+              int d, int dtype, const float* proj, int r, cudaStream_t st);   // stream_kernels.cu
 
 // One helper stream and two events per device, created on first use and kept for the life of the process.
 // `mu` serialises the callers of one device over the fork .. join section (the two events are shared).
@@ -50,7 +53,7 @@ struct CausalPlan {
   int Hk;                  // K/V heads
   long long idx_bytes;     // one depth's q_idx or k_idx
   long long part_o_bytes, part_lse_bytes;
-  long long sort_ws;       // largest sort workspace over the depths
+  long long sort_ws;       // sort workspaces of all depths, queries and keys
   int leaf;
 };
 
@@ -76,8 +79,7 @@ static int make_plan(const ha_causal_params& p, CausalPlan& pl) {
   pl.sort_ws = 0;
   for (int l = 0; l < p.levels; ++l) {
     const int span = p.n >> l;
-    const long long ws = ha_seg_sort_workspace_bytes(p.B * p.H, p.n, span, span / 2, p.lsh_bits);
-    if (ws > pl.sort_ws) pl.sort_ws = ws;
+    pl.sort_ws += 2 * ha_seg_sort_workspace_bytes(p.B * p.H, p.n, span, span / 2, p.lsh_bits);
   }
   return HA_OK;
 }
@@ -376,13 +378,11 @@ int ha_causal_fwd_strided(const ha_causal_params* pp, const int64_t* strides, vo
   void* sort_ws = (uint8_t*)p.scratch + 2 * align256(pl.rows * 4);
 
   const Layout lay(p, strides);
-  rc = ha_lsh_hash(p.q, lay.q[0], lay.q[1], lay.q[2], p.B, p.H, p.n, p.d, p.dtype, p.proj, p.lsh_bits, codes_q, stream);
-  if (rc != HA_OK) return rc;
-  rc = ha_lsh_hash(p.k, lay.k[0], lay.k[1], lay.k[2], p.B, pl.Hk, p.n, p.d, p.dtype, p.proj, p.lsh_bits, codes_k, stream);
+  rc = hash_pair(p.q, lay.q, p.H, codes_q, p.k, lay.k, pl.Hk, codes_k, p.B, p.n, p.d, p.dtype, p.proj, p.lsh_bits, (cudaStream_t)stream);
   if (rc != HA_OK) return rc;
 
   // The sorts of every depth depend on the codes only: they run on a side stream (forked here, joined before the first
-  // rectangle) underneath the leaves' kernel, which does not need them.  36 short launches leave the critical path.
+  // rectangle) beside the leaves' kernel, which does not need them.
   SideStream* side = side_stream();
   cudaStream_t main_st = (cudaStream_t)stream;
   const bool exact_deepest = deepest_exact(p, pl);
@@ -395,12 +395,25 @@ int ha_causal_fwd_strided(const ha_causal_params* pp, const int64_t* strides, vo
   }
   void* sort_stream = side ? (void*)side->stream : stream;
   int sort_rc = HA_OK;
+  // the segments of every depth in batches of like length (three launches for the long ones, one for those of a chunk)
+  SortJobs batch[3];
+  uint8_t* ws = (uint8_t*)sort_ws;
+  uint8_t* batch_ws[3] = {nullptr, nullptr, nullptr};
   for (int l = p.levels - 1 - (exact_deepest ? 1 : 0); l >= 0 && sort_rc == HA_OK; --l) {
     const int span = p.n >> l, m = span / 2;
-    sort_rc = ha_seg_sort(codes_q, p.B * p.H, p.n, span, m, m, p.lsh_bits, sv.q_idx(l), sort_ws, pl.sort_ws, sort_stream);
-    if (sort_rc == HA_OK)
-      sort_rc = ha_seg_sort(codes_k, p.B * pl.Hk, p.n, span, 0, m, p.lsh_bits, sv.k_idx(l), sort_ws, pl.sort_ws, sort_stream);
+    const long long bytes = ha_seg_sort_workspace_bytes(p.B * p.H, p.n, span, m, p.lsh_bits);
+    if (SortJobs::fits(m, p.lsh_bits)) {
+      const int b = m <= 2048 ? 0 : m <= 4096 ? 1 : 2;
+      if (!batch_ws[b]) batch_ws[b] = ws;
+      batch[b].add(codes_q, p.B * p.H, p.n, span, m, m, sv.q_idx(l));
+      batch[b].add(codes_k, p.B * pl.Hk, p.n, span, 0, m, sv.k_idx(l));
+    } else {
+      sort_rc = ha_seg_sort(codes_q, p.B * p.H, p.n, span, m, m, p.lsh_bits, sv.q_idx(l), ws, bytes, sort_stream);
+      if (sort_rc == HA_OK) sort_rc = ha_seg_sort(codes_k, p.B * pl.Hk, p.n, span, 0, m, p.lsh_bits, sv.k_idx(l), ws + bytes, bytes, sort_stream);
+    }
+    ws += 2 * bytes;
   }
+  for (int b = 0; b < 3 && sort_rc == HA_OK; ++b) sort_rc = batch[b].run((uint32_t*)batch_ws[b], (cudaStream_t)sort_stream);
   if (side) {   // joined in every case, so that the caller's stream also orders after whatever the side stream holds
     HA_CUDA_OK(cudaEventRecord(side->join, side->stream), "ha_causal_fwd join");
   }
@@ -581,6 +594,13 @@ int ha_causal_bwd(const ha_causal_params* p, void* stream) { return ha_causal_bw
  * saved: q_idx | k_idx.  scratch: forward = codes of q and k + sort workspace; backward = delta + slot buffers / fp32
  * accumulators as the backward kernel needs them.
  * --------------------------------------------------------------------------------------------------------------- */
+// dk | dv accumulators -> typed gradients: one cast where both pairs are adjacent
+static int cast_kv(const float* dk_acc, const float* dv_acc, void* dk, void* dv, long long count_k, long long count_v, int dtype, void* stream) {
+  if (dv_acc == dk_acc + count_k && (uint8_t*)dv == (uint8_t*)dk + count_k * dtype_size(dtype)) return ha_cast_from_f32(dk_acc, dk, count_k + count_v, dtype, stream);
+  const int rc = ha_cast_from_f32(dk_acc, dk, count_k, dtype, stream);
+  return rc != HA_OK ? rc : ha_cast_from_f32(dv_acc, dv, count_v, dtype, stream);
+}
+
 static int noncausal_check(const ha_causal_params& p, long long& rows, long long& rows_k) {
   if (p.dtype != HA_BF16 && p.dtype != HA_FP16 && p.dtype != HA_FP32) return HA_ERR_DTYPE;
   if (p.B <= 0 || p.H <= 0 || p.n <= 0 || p.d <= 0 || p.dv <= 0 || p.d > 256 || p.dv > 256) return HA_ERR_INVALID;
@@ -649,24 +669,22 @@ int ha_noncausal_fwd_strided(const ha_causal_params* pp, const int64_t* strides,
   if (!p.q || !p.k || !p.v || !p.o || !p.lse || !p.proj) return HA_ERR_INVALID;
   if (!p.saved || p.saved_bytes < ha_noncausal_saved_bytes(pp)) return HA_ERR_WORKSPACE;
   if (!p.scratch || p.scratch_bytes < ha_noncausal_scratch_bytes(pp, 0)) return HA_ERR_WORKSPACE;
-  // codes of q and k side by side: one segmented sort call covers both, and its output is q_idx | k_idx -- if the two
-  // halves of `saved` are contiguous, which they are when rows * 4 is a multiple of 256 (n is a multiple of 128)
   int32_t* codes = (int32_t*)p.scratch;
   void* sort_ws = (uint8_t*)p.scratch + 2 * align256(rows * 4);
   const long long sort_ws_bytes = p.scratch_bytes - 2 * align256(rows * 4);
   const Layout lay(p, strides);
-  rc = ha_lsh_hash(p.q, lay.q[0], lay.q[1], lay.q[2], p.B, p.H, p.n, p.d, p.dtype, p.proj, p.lsh_bits, codes, stream);
-  if (rc != HA_OK) return rc;
   const int Hk = p.kv_group > 1 ? p.H / p.kv_group : p.H;
-  rc = ha_lsh_hash(p.k, lay.k[0], lay.k[1], lay.k[2], p.B, Hk, p.n, p.d, p.dtype, p.proj, p.lsh_bits, codes + rows, stream);
+  rc = hash_pair(p.q, lay.q, p.H, codes, p.k, lay.k, Hk, codes + rows, p.B, p.n, p.d, p.dtype, p.proj, p.lsh_bits, (cudaStream_t)stream);
   if (rc != HA_OK) return rc;
-  if (align256(rows * 4) == rows * 4 && Hk == p.H) {
-    rc = ha_seg_sort(codes, 2 * p.B * p.H, p.n, p.n, 0, p.n, p.lsh_bits, (int32_t*)p.saved, sort_ws, sort_ws_bytes, stream);
+  int32_t* k_idx = (int32_t*)((uint8_t*)p.saved + align256(rows * 4));
+  if (SortJobs::fits(p.n, p.lsh_bits)) {
+    SortJobs jobs;
+    jobs.add(codes, p.B * p.H, p.n, p.n, 0, p.n, (int32_t*)p.saved);
+    jobs.add(codes + rows, p.B * Hk, p.n, p.n, 0, p.n, k_idx);
+    rc = jobs.run((uint32_t*)sort_ws, (cudaStream_t)stream);
   } else {
     rc = ha_seg_sort(codes, p.B * p.H, p.n, p.n, 0, p.n, p.lsh_bits, (int32_t*)p.saved, sort_ws, sort_ws_bytes, stream);
-    if (rc == HA_OK)
-      rc = ha_seg_sort(codes + rows, p.B * Hk, p.n, p.n, 0, p.n, p.lsh_bits, (int32_t*)((uint8_t*)p.saved + align256(rows * 4)), sort_ws,
-                       sort_ws_bytes, stream);
+    if (rc == HA_OK) rc = ha_seg_sort(codes + rows, p.B * Hk, p.n, p.n, 0, p.n, p.lsh_bits, k_idx, sort_ws, sort_ws_bytes, stream);
   }
   if (rc != HA_OK) return rc;
   ha_attn_params a;
@@ -702,9 +720,7 @@ int ha_noncausal_bwd_strided(const ha_causal_params* pp, const int64_t* strides,
     HA_CUDA_OK(cudaMemsetAsync(a.dk_acc, 0, align256(rows_k * p.d * 4) + rows_k * p.dv * 4, st), "ha_noncausal_bwd memset");
     rc = ws_attn_bwd(a, false, st);
     if (rc != HA_OK) return rc;
-    rc = ha_cast_from_f32(a.dk_acc, p.dk, rows_k * p.d, p.dtype, stream);
-    if (rc != HA_OK) return rc;
-    return ha_cast_from_f32(a.dv_acc, p.dv_out, rows_k * p.dv, p.dtype, stream);
+    return cast_kv(a.dk_acc, a.dv_acc, p.dk, p.dv_out, rows_k * p.d, rows_k * p.dv, p.dtype, stream);
   }
   if (level >= 1) {
     const long long segs = (long long)p.B * p.H;
@@ -748,5 +764,64 @@ int ha_noncausal_bwd_strided(const ha_causal_params* pp, const int64_t* strides,
 }
 
 int ha_noncausal_bwd(const ha_causal_params* p, void* stream) { return ha_noncausal_bwd_strided(p, nullptr, stream); }
+
+/* Backward of exact attention (HA_MODE_FLASH) as one call: delta, the backward kernel with the outputs it supports, casts. */
+static bool flash_typed_dq(const ha_attn_params& p, const void* dq) {
+  ha_attn_params a = p;
+  a.dq_out = (void*)256;                          // (outputs are only looked at for being there, and for their alignment)
+  a.dq_acc = nullptr;
+  a.dk_acc = a.dv_acc = (float*)256;
+  return p.dtype != HA_FP32 && !(p.flags & HA_FLAG_FORCE_SIMT) && (uintptr_t)dq % 16 == 0 && ws_bwd_supported(a);
+}
+static bool flash_bwd_shape(const ha_attn_params* p, long long& rows, long long& rows_k) {
+  if (!p || p->mode != HA_MODE_FLASH || p->segs_per_head != 1 || p->q_off || p->k_off || p->m_q != p->n || p->m_k != p->n || p->span != p->n) return false;
+  if (p->B <= 0 || p->H <= 0 || p->n <= 0 || p->d <= 0 || p->dv <= 0 || p->kv_group < 0 || (p->kv_group > 1 && p->H % p->kv_group != 0)) return false;
+  if (p->dtype != HA_BF16 && p->dtype != HA_FP16 && p->dtype != HA_FP32) return false;
+  rows = (long long)p->B * p->H * p->n;
+  rows_k = p->kv_group > 1 ? rows / p->kv_group : rows;
+  return true;
+}
+
+int64_t ha_flash_bwd_scratch_bytes(const ha_attn_params* p, const void* dq) {
+  long long rows, rows_k;
+  if (!flash_bwd_shape(p, rows, rows_k)) return -1;
+  long long bytes = align256(rows * 4);
+  if (p->dtype != HA_FP32) bytes += (flash_typed_dq(*p, dq) ? 0 : rows * p->d * 4) + rows_k * (p->d + p->dv) * 4;
+  return align256(bytes);
+}
+
+int ha_flash_bwd(const ha_attn_params* pp, void* dq, void* dk, void* dv, void* scratch, int64_t scratch_bytes, void* stream) {
+  long long rows, rows_k;
+  if (!flash_bwd_shape(pp, rows, rows_k) || !pp->o || !pp->d_o || !pp->lse || !dq || !dk || !dv) return HA_ERR_INVALID;
+  if (!scratch || scratch_bytes < ha_flash_bwd_scratch_bytes(pp, dq)) return HA_ERR_WORKSPACE;
+  cudaStream_t st = (cudaStream_t)stream;
+  ha_attn_params a = *pp;
+  const bool typed = flash_typed_dq(a, dq), f32 = a.dtype == HA_FP32;
+  float* delta = (float*)scratch;
+  float* acc = (float*)((uint8_t*)scratch + align256(rows * 4));
+  int rc = ha_delta(a.o, a.o_sb, a.o_sh, a.o_sn, a.d_o, a.do_sb, a.do_sh, a.do_sn, a.B, a.H, a.n, a.dv, a.dtype, delta, stream);
+  if (rc != HA_OK) return rc;
+  a.delta = delta;
+  a.dk_out = a.dv_out = a.dq_out = nullptr;
+  if (f32) {                                      // fp32 gradients are their own accumulators
+    a.dq_acc = (float*)dq; a.dk_acc = (float*)dk; a.dv_acc = (float*)dv;
+    HA_CUDA_OK(cudaMemsetAsync(dq, 0, rows * a.d * 4, st), "ha_flash_bwd memset");
+    HA_CUDA_OK(cudaMemsetAsync(dk, 0, rows_k * a.d * 4, st), "ha_flash_bwd memset");
+    HA_CUDA_OK(cudaMemsetAsync(dv, 0, rows_k * a.dv * 4, st), "ha_flash_bwd memset");
+    return ha_attn_bwd(&a, stream);
+  }
+  a.dq_acc = typed ? nullptr : acc;
+  a.dk_acc = acc + (typed ? 0 : rows * a.d);
+  a.dv_acc = a.dk_acc + rows_k * a.d;
+  HA_CUDA_OK(cudaMemsetAsync(acc, 0, ((typed ? 0 : rows * a.d) + rows_k * (a.d + a.dv)) * 4, st), "ha_flash_bwd memset");
+  if (typed) {
+    a.dq_out = dq;
+    rc = ws_attn_bwd(a, false, st);
+  } else {
+    rc = ha_attn_bwd(&a, stream);
+    if (rc == HA_OK) rc = ha_cast_from_f32(a.dq_acc, dq, rows * a.d, a.dtype, stream);
+  }
+  return rc != HA_OK ? rc : cast_kv(a.dk_acc, a.dv_acc, dk, dv, rows_k * a.d, rows_k * a.dv, a.dtype, stream);
+}
 
 }  // extern "C"

@@ -147,11 +147,20 @@ __device__ __forceinline__ uint32_t spread4(uint32_t x) {   // bit i -> bit 2i, 
   return (x & 1u) | ((x & 2u) << 1) | ((x & 4u) << 2) | ((x & 8u) << 3);
 }
 
+// One tensor of a call (queries and keys share a launch).
+struct HashSrc {
+  const void* x;
+  int64_t sb, sh, sn;
+  int H;
+  FastDiv by_heads;
+  int32_t* codes;
+  long long rows;
+};
+
 // CH = d / 32 column chunks; NSET = 1 (r <= 8) or 2 (r <= 16)
 template <typename T, int CH, int NSET, int UNROLL>
-__global__ void __launch_bounds__(256, 4) lsh_hash_mma_kernel(const T* __restrict__ x, int64_t sb, int64_t sh, int64_t sn, int H, int n,
-                                                           const float* __restrict__ proj, int r, int32_t* __restrict__ codes,
-                                                           long long total_rows) {
+__global__ void __launch_bounds__(256, 4) lsh_hash_mma_kernel(const HashSrc src0, const HashSrc src1, FastDiv by_n, int n,
+                                                           const float* __restrict__ proj, int r) {
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   // B fragments: for chunk c, MMA m (0/1), register j (0/1): projection column (set*8 + g), rows c*32 + 8t + 4m + 2j + {0,1}
@@ -173,7 +182,14 @@ __global__ void __launch_bounds__(256, 4) lsh_hash_mma_kernel(const T* __restric
   const long long warp_id = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
   const long long step = 16LL * UNROLL;
-  for (long long base = warp_id * step; base < total_rows; base += n_warps * step) {
+  const long long steps0 = (src0.rows + step - 1) / step, steps = steps0 + (src1.rows + step - 1) / step;
+  for (long long at = warp_id; at < steps; at += n_warps) {
+    const HashSrc& src = at < steps0 ? src0 : src1;
+    const T* __restrict__ x = (const T*)src.x;
+    const int64_t sb = src.sb, sh = src.sh, sn = src.sn;
+    const int H = src.H;
+    const long long total_rows = src.rows, base = (at < steps0 ? at : at - steps0) * step;
+    int32_t* __restrict__ codes = src.codes;
     uint4 v[UNROLL][2][CH];
 #pragma unroll
     for (int u = 0; u < UNROLL; ++u)
@@ -181,9 +197,8 @@ __global__ void __launch_bounds__(256, 4) lsh_hash_mma_kernel(const T* __restric
       for (int hrow = 0; hrow < 2; ++hrow) {
         const long long row = base + u * 16 + g + 8 * hrow;
         const bool ok = row < total_rows;
-        const long long bh = ok ? row / n : 0;
-        const int i = ok ? (int)(row - bh * n) : 0;
-        const T* p = x + (bh / H) * sb + (bh % H) * sh + (long long)i * sn + 8 * t;
+        const int bh = ok ? by_n((int)row) : 0, i = ok ? (int)row - bh * n : 0, b = src.by_heads(bh);
+        const T* p = x + b * sb + (bh - b * H) * sh + (long long)i * sn + 8 * t;
 #pragma unroll
         for (int c = 0; c < CH; ++c) v[u][hrow][c] = ok ? __ldg(reinterpret_cast<const uint4*>(p + 32 * c)) : make_uint4(0, 0, 0, 0);
       }
@@ -218,16 +233,39 @@ __global__ void __launch_bounds__(256, 4) lsh_hash_mma_kernel(const T* __restric
 }
 
 template <typename T, int CH>
-static void launch_hash_mma(const T* x, int64_t sb, int64_t sh, int64_t sn, int H, int n, const float* proj, int r, int32_t* codes,
-                            long long total, cudaStream_t st) {
+static void launch_hash_mma(const HashSrc& a, const HashSrc& b, int n, const float* proj, int r, cudaStream_t st) {
   constexpr int UNROLL = CH <= 2 ? 2 : 1;   // 64 registers -> four CTAs (32 warps) per SM, each with its loads in flight
   const long long rows_per_cta = 8LL * 16 * UNROLL;
-  long long want = (total + rows_per_cta - 1) / rows_per_cta;
+  const long long want = (a.rows + rows_per_cta - 1) / rows_per_cta + (b.rows + rows_per_cta - 1) / rows_per_cta;
   const int grid = (int)(want < 148LL * 16 ? want : 148LL * 16);
-  if (r <= 8)
-    lsh_hash_mma_kernel<T, CH, 1, UNROLL><<<grid, 256, 0, st>>>(x, sb, sh, sn, H, n, proj, r, codes, total);
-  else
-    lsh_hash_mma_kernel<T, CH, 2, UNROLL><<<grid, 256, 0, st>>>(x, sb, sh, sn, H, n, proj, r, codes, total);
+  if (r <= 8) lsh_hash_mma_kernel<T, CH, 1, UNROLL><<<grid, 256, 0, st>>>(a, b, FastDiv(n), n, proj, r);
+  else lsh_hash_mma_kernel<T, CH, 2, UNROLL><<<grid, 256, 0, st>>>(a, b, FastDiv(n), n, proj, r);
+}
+
+// Rows the tensor-core path takes: 16-byte aligned, d = 32, 64 or 128.
+static bool hash_mma_ok(const HashSrc& a, int d, int dtype) {
+  return dtype != HA_FP32 && (d == 32 || d == 64 || d == 128) && a.sb % 8 == 0 && a.sh % 8 == 0 && a.sn % 8 == 0 && (uintptr_t)a.x % 16 == 0 &&
+         a.rows < (1LL << 31);
+}
+template <typename T>
+static void run_hash_mma(const HashSrc& a, const HashSrc& b, int n, int d, const float* proj, int r, cudaStream_t st) {
+  if (d == 32) launch_hash_mma<T, 1>(a, b, n, proj, r, st);
+  else if (d == 64) launch_hash_mma<T, 2>(a, b, n, proj, r, st);
+  else launch_hash_mma<T, 4>(a, b, n, proj, r, st);
+}
+
+// Queries and keys (Hk heads) of a call, in one launch where the tensor-core path takes both.
+int hash_pair(const void* q, const int64_t (&qs)[3], int H, int32_t* codes_q, const void* k, const int64_t (&ks)[3], int Hk, int32_t* codes_k, int B, int n,
+              int d, int dtype, const float* proj, int r, cudaStream_t st) {
+  const HashSrc a{q, qs[0], qs[1], qs[2], H, FastDiv(H), codes_q, (long long)B * H * n}, b{k, ks[0], ks[1], ks[2], Hk, FastDiv(Hk), codes_k, (long long)B * Hk * n};
+  if (r >= 1 && r <= 16 && a.rows > 0 && hash_mma_ok(a, d, dtype) && hash_mma_ok(b, d, dtype)) {
+    if (dtype == HA_BF16) run_hash_mma<__nv_bfloat16>(a, b, n, d, proj, r, st);
+    else run_hash_mma<__half>(a, b, n, d, proj, r, st);
+    HA_LAUNCHED("ha_lsh_hash");
+    return HA_OK;
+  }
+  const int rc = ha_lsh_hash(q, qs[0], qs[1], qs[2], B, H, n, d, dtype, proj, r, codes_q, st);
+  return rc != HA_OK ? rc : ha_lsh_hash(k, ks[0], ks[1], ks[2], B, Hk, n, d, dtype, proj, r, codes_k, st);
 }
 
 // Generic path (any d <= 256, any element alignment): one warp per row, lane-strided elements.
@@ -278,12 +316,13 @@ static int launch_hash(const void* x, int64_t sb, int64_t sh, int64_t sn, int B,
                       (sn % EPC == 0) && ((uintptr_t)x % 16 == 0);
   int sms = 148;
   if constexpr (!std::is_same<T, float>::value) {
-    // tensor-core path: 16-byte aligned rows, d a multiple of 32 up to 128.  The projection is rounded to the input
-    // dtype, which is the dtype the reference requires it to have (src/angular_lsh_triton.py:104).
-    if (vec_ok && (d == 32 || d == 64 || d == 128)) {
-      if (d == 32) launch_hash_mma<T, 1>((const T*)x, sb, sh, sn, H, n, proj, r, codes, total, st);
-      else if (d == 64) launch_hash_mma<T, 2>((const T*)x, sb, sh, sn, H, n, proj, r, codes, total, st);
-      else launch_hash_mma<T, 4>((const T*)x, sb, sh, sn, H, n, proj, r, codes, total, st);
+    // tensor-core path.  The projection is rounded to the input dtype, which is the dtype the reference requires it to have
+    // (src/angular_lsh_triton.py:104).
+    const HashSrc a{x, sb, sh, sn, H, FastDiv(H), codes, total};
+    if (hash_mma_ok(a, d, HA_BF16)) {
+      HashSrc none = a;
+      none.rows = 0;
+      run_hash_mma<T>(a, none, n, d, proj, r, st);
       HA_LAUNCHED("ha_lsh_hash");
       return HA_OK;
     }

@@ -158,8 +158,10 @@ class HyperAttention(torch.nn.Module):
             # expanded to every query head, chatglm_fast_attention.py:53-58).  The single-call paths hash and sort K once
             # per K/V head and never expand; every other path expands here.
             assert query.shape[1] % n_heads == 0 and value.shape[1] == n_heads, 'query heads must be a multiple of the K/V heads'
-            grouped_ok = self.sampling == 'reference' and n_key >= self.min_seq_len and \
-                ((causal and n_key > self.min_seq_len and self.fused_causal and self._regular_causal(n_key)) or (not causal and self.fused_calls and query.dtype == self.lsh.proj_dir.dtype))
+            short = n_key <= self.min_seq_len if causal else n_key < self.min_seq_len          # exact attention
+            grouped_ok = short or (self.sampling == 'reference' and
+                                   ((causal and self.fused_causal and self._regular_causal(n_key)) or
+                                    (not causal and self.fused_calls and query.dtype == self.lsh.proj_dir.dtype)))
             if not grouped_ok:
                 rep = query.shape[1] // n_heads
                 key, value = key.repeat_interleave(rep, dim=1), value.repeat_interleave(rep, dim=1)

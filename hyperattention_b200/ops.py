@@ -427,8 +427,9 @@ def _flash_forward(q, k, v, causal, softmax_scale, flags):
     _cuda(q, k, v)
     B, nq, H, d = q.shape
     nk = k.shape[1]
-    assert k.shape == (B, nk, H, d)
-    assert v.shape[:3] == (B, nk, H)
+    Hk = k.shape[2]              # fewer key / value heads: consecutive query heads share one
+    assert k.shape == (B, nk, Hk, d) and H % Hk == 0
+    assert v.shape[:3] == (B, nk, Hk)
     assert q.dtype == k.dtype == v.dtype, 'All tensors must have the same type'
     o = _rows_like(q.transpose(1, 2), v.shape[-1]).transpose(1, 2)
     lse = torch.empty(B, H, nq, dtype=torch.float32, device=q.device)
@@ -460,26 +461,21 @@ class FlashAttnFunc(torch.autograd.Function):
             return (None,) * 8
         if do.stride(-1) != 1:
             do = do.contiguous()
-        B, nq, H, d = q.shape
-        nk, dv = k.shape[1], v.shape[-1]
-        assert nq == nk, 'backward is implemented for equal query/key lengths'
-        dev = q.device
-        n = nq
-        acc = torch.zeros(B * H * n * (2 * d + dv), dtype=torch.float32, device=dev)
-        dq_acc, dk_acc, dv_acc = acc[:B * H * n * d], acc[B * H * n * d:2 * B * H * n * d], acc[2 * B * H * n * d:]
-        delta = torch.empty(B, H, n, dtype=torch.float32, device=dev)
+        B, n, H, d = q.shape
+        Hk, dv = k.shape[2], v.shape[-1]
+        assert n == k.shape[1], 'backward is implemented for equal query/key lengths'
+        nq, nk, nv = B * H * n * d, B * Hk * n * d, B * Hk * n * dv
+        out = torch.empty(nq + nk + nv, dtype=q.dtype, device=q.device)      # dq | dk | dv
+        p = _flash_params(q, k, v, o, lse, causal, scale, flags)
+        p.d_o = do.data_ptr()
+        p.do_sb, p.do_sh, p.do_sn = _bhn(do)
+        dq_ptr, es = out.data_ptr(), out.element_size()
         lib = L.load()
-        with torch.cuda.device(dev):
-            rc = lib.ha_delta(_ptr(o), *_bhn(o), _ptr(do), *_bhn(do), B, H, n, dv, _dtype_id(q), _ptr(delta), _stream())
-            L.check(rc, 'ha_delta')
-            p = _flash_params(q, k, v, o, lse, causal, scale, flags)
-            p.d_o = _ptr(do)
-            p.do_sb, p.do_sh, p.do_sn = _bhn(do)
-            p.delta, p.dq_acc, p.dk_acc, p.dv_acc = _ptr(delta), _ptr(dq_acc), _ptr(dk_acc), _ptr(dv_acc)
-            rc = lib.ha_attn_bwd(C.byref(p), _stream())
-            L.check(rc, 'ha_attn_bwd')
-            grads = _cast_grads(lib, acc, q.dtype, B, H, n, d, dv)
-        return grads + (None,) * 5
+        scratch = torch.empty(lib.ha_flash_bwd_scratch_bytes(C.byref(p), dq_ptr), dtype=torch.uint8, device=q.device)
+        L.check(_call(lib.ha_flash_bwd, q.device, C.byref(p), dq_ptr, dq_ptr + es * nq, dq_ptr + es * (nq + nk), scratch.data_ptr(), scratch.numel()),
+                'ha_flash_bwd')
+        return (out[:nq].view(B, H, n, d).transpose(1, 2), out[nq:nq + nk].view(B, Hk, n, d).transpose(1, 2),
+                out[nq + nk:].view(B, Hk, n, dv).transpose(1, 2)) + (None,) * 5
 
 
 def _pad_lse(lse):
@@ -497,11 +493,12 @@ def _flash_params(q, k, v, o, lse, causal, scale, flags):
         p.B, p.H, p.n, p.d, p.dv = B, H, nq, d, dv
         p.segs_per_head, p.span, p.q_off, p.k_off, p.m_q, p.m_k = 1, nq, 0, 0, nq, nk
         p.scale = scale
+        p.kv_group = H // k.shape[2]
         p.q_sb, p.q_sh, p.q_sn = _bhn(q)
         p.k_sb, p.k_sh, p.k_sn = _bhn(k)
         p.v_sb, p.v_sh, p.v_sn = _bhn(v)
         p.o_sb, p.o_sh, p.o_sn = _bhn(o)
-    p = _template(L.AttnParams, (0, q.dtype, q.shape, k.shape[1], v.shape[-1], q.stride(), k.stride(), v.stride(), o.stride(), causal, scale, flags), fill)
+    p = _template(L.AttnParams, (0, q.dtype, q.shape, k.shape[1:3], v.shape[-1], q.stride(), k.stride(), v.stride(), o.stride(), causal, scale, flags), fill)
     p.q, p.k, p.v, p.o, p.lse = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr()
     _set_status(p, q.device)
     return p

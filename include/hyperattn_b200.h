@@ -270,6 +270,12 @@ int64_t ha_noncausal_scratch_bytes_strided(const ha_causal_params* p, const int6
 int ha_noncausal_fwd_strided(const ha_causal_params* p, const int64_t* strides, void* stream);
 int ha_noncausal_bwd_strided(const ha_causal_params* p, const int64_t* strides, void* stream);
 
+/* Backward of exact attention (HA_MODE_FLASH, one segment, equal lengths) in one call: delta, the backward kernel, casts.  p as for
+ * ha_attn_bwd without delta and outputs; dq [B,H,n,d], dk / dv [B,H/kv_group,n,*] contiguous, in the tensors' dtype.  Replaces
+ * FlashAttnFunc.backward (src/flash_attn_triton.py:1019-1040). */
+int64_t ha_flash_bwd_scratch_bytes(const ha_attn_params* p, const void* dq);
+int ha_flash_bwd(const ha_attn_params* p, void* dq, void* dk, void* dv, void* scratch, int64_t scratch_bytes, void* stream);
+
 /* Diagnostic for the timeout path.  One warp polls an mbarrier that nothing ever arrives at, `polls` times (1..2^18),
  * gives up and reports HA_DEV_TIMEOUT through status / status_host exactly as the attention kernels do when one of their
  * bounded waits runs out.  No copy and no tensor-core operation is in flight; the kernel returns normally and the
