@@ -80,9 +80,11 @@ SIGNATURES = {
     'ha_noncausal_bwd': (C.c_int, [C.POINTER(CausalParams), vp]),
     'ha_causal_fwd_strided': (C.c_int, [C.POINTER(CausalParams), vp, vp]),
     'ha_causal_bwd_strided': (C.c_int, [C.POINTER(CausalParams), vp, vp]),
-    'ha_noncausal_scratch_bytes_strided': (i64, [C.POINTER(CausalParams), vp, i32]),
-    'ha_noncausal_fwd_strided': (C.c_int, [C.POINTER(CausalParams), vp, vp]),
-    'ha_noncausal_bwd_strided': (C.c_int, [C.POINTER(CausalParams), vp, vp]),
+    'ha_noncausal_saved_bytes_ext': (i64, [C.POINTER(CausalParams), vp]),
+    'ha_noncausal_scratch_bytes_ext': (i64, [C.POINTER(CausalParams), vp, vp, i32]),
+    'ha_noncausal_fwd_ext': (C.c_int, [C.POINTER(CausalParams), vp, vp, vp]),
+    'ha_noncausal_bwd_ext': (C.c_int, [C.POINTER(CausalParams), vp, vp, vp]),
+    'ha_uniform_sample': (C.c_int, [i32, i32, i32, C.c_uint64, vp, vp]),
     'ha_flash_bwd_scratch_bytes': (i64, [C.POINTER(AttnParams), vp]),
     'ha_flash_bwd': (C.c_int, [C.POINTER(AttnParams), vp, vp, vp, vp, i64, vp]),
     'ha_wait_probe': (C.c_int, [vp, vp, i32, vp]),

@@ -612,7 +612,11 @@ static int noncausal_check(const ha_causal_params& p, long long& rows, long long
   return HA_OK;
 }
 
-static void noncausal_attn(const ha_causal_params& p, const Layout& lay, ha_attn_params& a, long long rows) {
+// `saved`: q_idx | k_idx and, with sampled rows given (importance-weighted), the query tiles' log weights and dropped-slot masks.
+static long long noncausal_weights_off(long long rows) { return 2 * align256(rows * 4); }
+static long long noncausal_logw_bytes(long long rows) { return align256(rows / TILE * 4); }
+
+static void noncausal_attn(const ha_causal_params& p, const Layout& lay, const int32_t* sample_idx, ha_attn_params& a, long long rows) {
   fill_attn(p, lay, a);
   a.mode = HA_MODE_HYPER;
   a.flags = p.flags & (HA_FLAG_SMOOTH | HA_FLAG_BWD_REF_SMOOTH | HA_FLAG_FORCE_SIMT | HA_FLAG_NO_WS);
@@ -620,13 +624,18 @@ static void noncausal_attn(const ha_causal_params& p, const Layout& lay, ha_attn
   a.span = p.n; a.q_off = 0; a.k_off = 0; a.m_q = p.n; a.m_k = p.n;
   a.q_idx = (const int32_t*)p.saved;
   a.k_idx = (const int32_t*)((const uint8_t*)p.saved + align256(rows * 4));
+  if (sample_idx && p.sample_size > 0) {
+    a.sample_idx = sample_idx;
+    a.sample_logw = (const float*)((const uint8_t*)p.saved + noncausal_weights_off(rows));
+    a.sample_mask = (const uint32_t*)((const uint8_t*)a.sample_logw + noncausal_logw_bytes(rows));
+  }
 }
 
 // what the backward needs beyond delta: 3 = fp32 dK and dV (typed dQ), 2 = slot buffers only, 1 = slot buffers + fp32 dQ, 0 = three fp32
 // accumulators
-static int noncausal_bwd_level(const ha_causal_params& p, const Layout& lay, long long rows) {
+static int noncausal_bwd_level(const ha_causal_params& p, const Layout& lay, const int32_t* sample_idx, long long rows) {
   ha_attn_params a;
-  noncausal_attn(p, lay, a, rows);
+  noncausal_attn(p, lay, sample_idx, a, rows);
   float dummy = 0.f;
   a.delta = &dummy;                               // (only looked at for being there)
   a.dq_acc = a.dk_acc = a.dv_acc = nullptr;
@@ -638,17 +647,20 @@ static int noncausal_bwd_level(const ha_causal_params& p, const Layout& lay, lon
   return ws_bwd_supported(a) ? 3 : level;
 }
 
-int64_t ha_noncausal_saved_bytes(const ha_causal_params* p) {
+int64_t ha_noncausal_saved_bytes_ext(const ha_causal_params* p, const int32_t* sample_idx) {
   long long rows, rows_k;
   if (!p || noncausal_check(*p, rows, rows_k) != HA_OK) return -1;
-  return 2 * align256(rows * 4);
+  if (!sample_idx || p->sample_size == 0) return noncausal_weights_off(rows);
+  if (p->kv_group > 1 || (long long)p->B * p->H > 65535) return -1;
+  return noncausal_weights_off(rows) + noncausal_logw_bytes(rows) + align256(rows / TILE * (p->sample_size / 32) * 4);
 }
+int64_t ha_noncausal_saved_bytes(const ha_causal_params* p) { return ha_noncausal_saved_bytes_ext(p, nullptr); }
 
-int64_t ha_noncausal_scratch_bytes_strided(const ha_causal_params* p, const int64_t* strides, int32_t backward) {
+int64_t ha_noncausal_scratch_bytes_ext(const ha_causal_params* p, const int64_t* strides, const int32_t* sample_idx, int32_t backward) {
   long long rows, rows_k;
   if (!p || noncausal_check(*p, rows, rows_k) != HA_OK) return -1;
   if (!backward) return 2 * align256(rows * 4) + align256(ha_seg_sort_workspace_bytes(2 * p->B * p->H, p->n, p->n, p->n, p->lsh_bits));
-  const int level = noncausal_bwd_level(*p, Layout(*p, strides), rows);
+  const int level = noncausal_bwd_level(*p, Layout(*p, strides), sample_idx, rows);
   const long long sacc = align256((long long)p->B * p->H * p->sample_size * (p->d + p->dv) * 4);
   long long bytes = align256(rows * 4);
   if (level == 3) bytes += align256(rows_k * p->d * 4) + align256(rows_k * p->dv * 4);
@@ -658,16 +670,16 @@ int64_t ha_noncausal_scratch_bytes_strided(const ha_causal_params* p, const int6
   return bytes;
 }
 
-int64_t ha_noncausal_scratch_bytes(const ha_causal_params* p, int32_t backward) { return ha_noncausal_scratch_bytes_strided(p, nullptr, backward); }
+int64_t ha_noncausal_scratch_bytes(const ha_causal_params* p, int32_t backward) { return ha_noncausal_scratch_bytes_ext(p, nullptr, nullptr, backward); }
 
-int ha_noncausal_fwd_strided(const ha_causal_params* pp, const int64_t* strides, void* stream) {
+int ha_noncausal_fwd_ext(const ha_causal_params* pp, const int64_t* strides, const int32_t* sample_idx, void* stream) {
   if (!pp) return HA_ERR_INVALID;
   const ha_causal_params& p = *pp;
   long long rows, rows_k;
   int rc = noncausal_check(p, rows, rows_k);
   if (rc != HA_OK) return rc;
   if (!p.q || !p.k || !p.v || !p.o || !p.lse || !p.proj) return HA_ERR_INVALID;
-  if (!p.saved || p.saved_bytes < ha_noncausal_saved_bytes(pp)) return HA_ERR_WORKSPACE;
+  if (!p.saved || p.saved_bytes < ha_noncausal_saved_bytes_ext(pp, sample_idx)) return HA_ERR_WORKSPACE;
   if (!p.scratch || p.scratch_bytes < ha_noncausal_scratch_bytes(pp, 0)) return HA_ERR_WORKSPACE;
   int32_t* codes = (int32_t*)p.scratch;
   void* sort_ws = (uint8_t*)p.scratch + 2 * align256(rows * 4);
@@ -688,31 +700,37 @@ int ha_noncausal_fwd_strided(const ha_causal_params* pp, const int64_t* strides,
   }
   if (rc != HA_OK) return rc;
   ha_attn_params a;
-  noncausal_attn(p, lay, a, rows);
+  noncausal_attn(p, lay, sample_idx, a, rows);
+  if (a.sample_logw) {
+    // (the codes are used up: their place takes the inverse key permutation)
+    rc = ha_sample_weights(a.k_idx, sample_idx, p.B * p.H, p.n, p.block_size, p.sample_size, (p.flags & HA_FLAG_SMOOTH) ? 1 : 0, codes, (float*)a.sample_logw,
+                           (uint32_t*)a.sample_mask, stream);
+    if (rc != HA_OK) return rc;
+  }
   return ha_attn_fwd(&a, stream);
 }
 
-int ha_noncausal_fwd(const ha_causal_params* p, void* stream) { return ha_noncausal_fwd_strided(p, nullptr, stream); }
+int ha_noncausal_fwd(const ha_causal_params* p, void* stream) { return ha_noncausal_fwd_ext(p, nullptr, nullptr, stream); }
 
-int ha_noncausal_bwd_strided(const ha_causal_params* pp, const int64_t* strides, void* stream) {
+int ha_noncausal_bwd_ext(const ha_causal_params* pp, const int64_t* strides, const int32_t* sample_idx, void* stream) {
   if (!pp) return HA_ERR_INVALID;
   const ha_causal_params& p = *pp;
   long long rows, rows_k;
   int rc = noncausal_check(p, rows, rows_k);
   if (rc != HA_OK) return rc;
   if (!p.q || !p.k || !p.v || !p.o || !p.lse || !p.d_o || !p.dq || !p.dk || !p.dv_out) return HA_ERR_INVALID;
-  if (!p.saved || p.saved_bytes < ha_noncausal_saved_bytes(pp)) return HA_ERR_WORKSPACE;
-  if (!p.scratch || p.scratch_bytes < ha_noncausal_scratch_bytes_strided(pp, strides, 1)) return HA_ERR_WORKSPACE;
+  if (!p.saved || p.saved_bytes < ha_noncausal_saved_bytes_ext(pp, sample_idx)) return HA_ERR_WORKSPACE;
+  if (!p.scratch || p.scratch_bytes < ha_noncausal_scratch_bytes_ext(pp, strides, sample_idx, 1)) return HA_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   uint8_t* s = (uint8_t*)p.scratch;
   float* delta = (float*)s;                  s += align256(rows * 4);
   ha_attn_params a;
   const Layout lay(p, strides);
-  noncausal_attn(p, lay, a, rows);
+  noncausal_attn(p, lay, sample_idx, a, rows);
   a.delta = delta;
   rc = ha_delta(p.o, a.o_sb, a.o_sh, a.o_sn, p.d_o, a.do_sb, a.do_sh, a.do_sn, p.B, p.H, p.n, p.dv, p.dtype, delta, stream);
   if (rc != HA_OK) return rc;
-  const int level = noncausal_bwd_level(p, lay, rows);
+  const int level = noncausal_bwd_level(p, lay, sample_idx, rows);
   if (level == 3) {
     a.dk_acc = (float*)s;                    s += align256(rows_k * p.d * 4);
     a.dv_acc = (float*)s;
@@ -763,7 +781,7 @@ int ha_noncausal_bwd_strided(const ha_causal_params* pp, const int64_t* strides,
   return ha_cast_from_f32(a.dv_acc, p.dv_out, rows_k * p.dv, p.dtype, stream);
 }
 
-int ha_noncausal_bwd(const ha_causal_params* p, void* stream) { return ha_noncausal_bwd_strided(p, nullptr, stream); }
+int ha_noncausal_bwd(const ha_causal_params* p, void* stream) { return ha_noncausal_bwd_ext(p, nullptr, nullptr, stream); }
 
 /* Backward of exact attention (HA_MODE_FLASH) as one call: delta, the backward kernel with the outputs it supports, casts. */
 static bool flash_typed_dq(const ha_attn_params& p, const void* dq) {

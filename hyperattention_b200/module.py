@@ -98,7 +98,8 @@ class HyperAttention(torch.nn.Module):
     # ------------------------------------------------------------------------------------------
     def _counter_u24(self, rows, S, device):
         """24 uniform bits per (row, slot): top bits of the splitmix64 finaliser of (sample_seed, call number, row * S + slot),
-        in int64 arithmetic (wrap-around products; logical right shifts written as arithmetic shift + mask)."""
+        in int64 arithmetic (wrap-around products; logical right shifts written as arithmetic shift + mask): what
+        ops.uniform_sample draws on the device."""
         def c(v):                                   # a 64-bit constant as a signed Python int
             return v - (1 << 64) if v >= (1 << 63) else v
         def shr(x, k):
@@ -209,6 +210,25 @@ class HyperAttention(torch.nn.Module):
             attn, lse = attn[:, :, :-1], lse[:, :, :-1]
         return attn, lse
 
+    def _sampled_rows(self, B, H, key):
+        """int32 [B * H, sample_size] rows of the importance-weighted sampled part, or None (sampling 'reference': rows 0..sample_size-1).
+        Distinct rows with equal inclusion probability per (batch, head): one uniform draw from each of sample_size equal
+        strata of the key range (cheaper than a draw without replacement, lower variance)."""
+        if self.sampling != 'uniform' or self.sample_size == 0:
+            return None
+        n_k, S = key.shape[2], self.sample_size
+        if self.sample_generator is not None:
+            edges = (torch.arange(S + 1, device=key.device, dtype=torch.int64) * n_k) // S
+            size = edges[1:] - edges[:-1]
+            u = torch.rand(B * H, S, device=key.device, generator=self.sample_generator)
+            sample_idx = (edges[:-1] + torch.minimum((u * size).long(), size - 1)).to(torch.int32)
+        else:
+            base = (self.sample_seed * 0x9E3779B97F4A7C15 + self.sample_calls * 0xD1B54A32D192ED03) & ((1 << 64) - 1)
+            sample_idx = ops.uniform_sample(B * H, n_k, S, base, key.device)
+            self.sample_calls += 1
+        self.last_sample_idx = sample_idx.view(B, H, S)
+        return sample_idx
+
     def forward_no_causal_mask(self, query, key, value, scale):
         """hyper_attention.py:103-132: exact attention below min_seq_len, otherwise hash -> stable sort -> fused
         block-diagonal + sampled attention."""
@@ -216,10 +236,10 @@ class HyperAttention(torch.nn.Module):
         if self.min_seq_len > n_query:
             attn, lse = ops.flash_attn_func(query.transpose(1, 2), key.transpose(1, 2), value.transpose(1, 2), None, False,
                                             scale, self.kernel_flags & L.FLAG_FORCE_SIMT)
-        elif self.sampling == 'reference' and self.fused_calls and query.dtype == self.lsh.proj_dir.dtype:
+        elif self.fused_calls and query.dtype == self.lsh.proj_dir.dtype:
             # hash, sort, attention (and, in the backward, delta, the backward kernel, the finishing pass) in one library call
             attn, lse = ops.noncausal_hyper(query, key, value, self.lsh.proj_f32(), self.block_size, self.sample_size,
-                                            scale, self._flags())
+                                            scale, self._flags(), self._sampled_rows(B, H, key))
             return attn, lse.unsqueeze(-1)
         else:
             bits = self.lsh_num_projs
@@ -229,23 +249,10 @@ class HyperAttention(torch.nn.Module):
             self.lsh.hash_cuda(key, codes[1])
             idx = ops.seg_sort(codes.view(2 * B * H, n_query), bits)
             q_idx, k_idx = idx[:B * H].view(B, H, n_query), idx[B * H:].view(B, H, n_query)
-            sample_idx, weighted = None, False
-            if self.sampling == 'uniform' and self.sample_size > 0:
-                # distinct rows with equal inclusion probability per (batch, head): one uniform draw from each of
-                # sample_size equal strata of the key range (cheaper than a draw without replacement, lower variance)
-                n_k, S = key.shape[2], self.sample_size
-                edges = (torch.arange(S + 1, device=key.device, dtype=torch.int64) * n_k) // S
-                size = edges[1:] - edges[:-1]
-                if self.sample_generator is not None:
-                    u = torch.rand(B * H, S, device=key.device, generator=self.sample_generator)
-                    sample_idx = (edges[:-1] + torch.minimum((u * size).long(), size - 1)).to(torch.int32)
-                else:
-                    sample_idx = (edges[:-1] + ((size * self._counter_u24(B * H, S, key.device)) >> 24)).to(torch.int32)
-                    self.sample_calls += 1
-                self.last_sample_idx = sample_idx.view(B, H, self.sample_size)
-                weighted = True
+            sample_idx = self._sampled_rows(B, H, key)
             attn, lse = ops.hyper_attn_func(query.transpose(1, 2), key.transpose(1, 2), value.transpose(1, 2),
                                             q_idx.transpose(1, 2), k_idx.transpose(1, 2), self.block_size, self.sample_size,
-                                            scale, self.smooth_block, sample_idx, self._flags() & ~L.FLAG_SMOOTH, weighted)
+                                            scale, self.smooth_block, sample_idx, self._flags() & ~L.FLAG_SMOOTH,
+                                            sample_idx is not None)
         attn = attn.transpose(1, 2)
         return attn, lse.unsqueeze(-1)

@@ -466,6 +466,8 @@ class FlashAttnFunc(torch.autograd.Function):
         assert n == k.shape[1], 'backward is implemented for equal query/key lengths'
         nq, nk, nv = B * H * n * d, B * Hk * n * d, B * Hk * n * dv
         out = torch.empty(nq + nk + nv, dtype=q.dtype, device=q.device)      # dq | dk | dv
+        if not out.numel():
+            return torch.empty_like(q), torch.empty_like(k), torch.empty_like(v), None, None, None, None, None
         p = _flash_params(q, k, v, o, lse, causal, scale, flags)
         p.d_o = do.data_ptr()
         p.do_sb, p.do_sh, p.do_sn = _bhn(do)
@@ -517,12 +519,12 @@ def flash_attn_func(q, k, v, bias=None, causal=False, softmax_scale=None, flags=
 _PLANS = {}
 
 
-def _plan(causal, backward, q, k, v, o, do, cfg):
+def _plan(causal, backward, q, k, v, o, do, cfg, sample=None):
     """(parameter struct with the tensors' pointers set, strides array, bytes of `saved`, bytes of scratch) of one call;
     cfg = (levels, block_size, sample_size, lsh_bits, keep_parts, min_seq_len, scale, flags)."""
     ptrs = (q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr() if do is not None else 0)
     key = (causal, backward, q.dtype, q.shape, k.shape[1], v.shape[-1], q.stride(), k.stride(), v.stride(), o.stride(),
-           do.stride() if do is not None else None, cfg, (ptrs[0] | ptrs[1] | ptrs[2] | ptrs[3] | ptrs[4]) & 15)
+           do.stride() if do is not None else None, cfg, sample is not None, (ptrs[0] | ptrs[1] | ptrs[2] | ptrs[3] | ptrs[4]) & 15)
     plan = _PLANS.get(key)
     if plan is None:
         p = L.CausalParams()
@@ -539,7 +541,8 @@ def _plan(causal, backward, q, k, v, o, do, cfg):
             saved, scratch = lib.ha_causal_saved_bytes(C.byref(p)), lib.ha_causal_scratch_bytes(C.byref(p), backward)
             assert saved >= 0 and scratch >= 0, 'causal schedule: n must be divisible by 2^levels with 128-row multiples at every depth'
         else:
-            saved, scratch = lib.ha_noncausal_saved_bytes(C.byref(p)), lib.ha_noncausal_scratch_bytes_strided(C.byref(p), st, backward)
+            sp = _ptr(sample)
+            saved, scratch = lib.ha_noncausal_saved_bytes_ext(C.byref(p), sp), lib.ha_noncausal_scratch_bytes_ext(C.byref(p), st, sp, backward)
             assert saved >= 0 and scratch >= 0, 'shape not accepted (n and sample_size multiples of 128, sample_size <= n)'
         if len(_PLANS) >= 512:
             _PLANS.clear()
@@ -558,8 +561,9 @@ def _buffer(p, name, nbytes, device):
     return t
 
 
-def _call_forward(causal, q, k, v, proj_f32, cfg):
-    """One ha_causal_fwd / ha_noncausal_fwd call on [B, H, n, *] tensors with contiguous rows: (o, lse [B, H, n], saved)."""
+def _call_forward(causal, q, k, v, proj_f32, cfg, sample=None):
+    """One ha_causal_fwd / ha_noncausal_fwd call on [B, H, n, *] tensors with contiguous rows: (o, lse [B, H, n], saved).  sample: int32
+    [B * H, sample_size] rows of the importance-weighted sampled part (non-causal calls), or None."""
     _cuda(q, k, v, proj_f32)
     B, H, n, d = q.shape
     dev = q.device
@@ -568,7 +572,7 @@ def _call_forward(causal, q, k, v, proj_f32, cfg):
     strided_o = not causal or (q.dtype != torch.float32 and dv in (32, 64, 128) and not cfg[7] & L.FLAG_FORCE_SIMT)
     o = _rows_like(q, dv) if strided_o else torch.empty(B, H, n, dv, dtype=q.dtype, device=dev)
     lse = torch.empty(B, H, n, dtype=torch.float32, device=dev)
-    p, st, saved_bytes, scratch_bytes = _plan(causal, 0, q, k, v, o, None, cfg)
+    p, st, saved_bytes, scratch_bytes = _plan(causal, 0, q, k, v, o, None, cfg, sample)
     p.proj, p.lse = proj_f32.data_ptr(), lse.data_ptr()
     saved = _buffer(p, 'saved', saved_bytes, dev)
     scratch = _buffer(p, 'scratch', scratch_bytes, dev)      # (free once the launches are enqueued: same stream)
@@ -576,18 +580,18 @@ def _call_forward(causal, q, k, v, proj_f32, cfg):
     if causal:
         L.check(_call(lib.ha_causal_fwd_strided, dev, C.byref(p), st), 'ha_causal_fwd')
     else:
-        L.check(_call(lib.ha_noncausal_fwd_strided, dev, C.byref(p), st), 'ha_noncausal_fwd')
+        L.check(_call(lib.ha_noncausal_fwd_ext, dev, C.byref(p), st, _ptr(sample)), 'ha_noncausal_fwd')
     del scratch
     return o, lse, saved
 
 
-def _call_backward(causal, q, k, v, proj_f32, o, lse, saved, do, cfg):
+def _call_backward(causal, q, k, v, proj_f32, o, lse, saved, do, cfg, sample=None):
     dev = q.device
     # one buffer for the three gradients (dq | dk | dv): one allocation per step
     nq, nk, nv = q.numel(), k.numel(), v.numel()
     out = torch.empty(nq + nk + nv, dtype=q.dtype, device=dev)
     dq, dk, dvv = out[:nq].view(q.shape), out[nq:nq + nk].view(k.shape), out[nq + nk:].view(v.shape)
-    p, st, _, scratch_bytes = _plan(causal, 1, q, k, v, o, do, cfg)
+    p, st, _, scratch_bytes = _plan(causal, 1, q, k, v, o, do, cfg, sample)
     p.proj, p.lse = proj_f32.data_ptr(), lse.data_ptr()
     p.saved, p.saved_bytes = saved.data_ptr(), saved.numel()
     p.dq = out.data_ptr()
@@ -597,7 +601,7 @@ def _call_backward(causal, q, k, v, proj_f32, o, lse, saved, do, cfg):
     if causal:
         L.check(_call(lib.ha_causal_bwd_strided, dev, C.byref(p), st), 'ha_causal_bwd')
     else:
-        L.check(_call(lib.ha_noncausal_bwd_strided, dev, C.byref(p), st), 'ha_noncausal_bwd')
+        L.check(_call(lib.ha_noncausal_bwd_ext, dev, C.byref(p), st, _ptr(sample)), 'ha_noncausal_bwd')
     del scratch
     return dq, dk, dvv
 
@@ -666,7 +670,7 @@ class NonCausalHyperFunc(torch.autograd.Function):
     heads.  Returns o [B, H, n, dv] and lse [B, H, n]; the gradient flowing into lse is discarded, as in the reference."""
 
     @staticmethod
-    def run(q, k, v, proj_f32, block_size, sample_size, scale, flags):
+    def run(q, k, v, proj_f32, block_size, sample_size, scale, flags, sample=None):
         assert q.dtype == k.dtype == v.dtype, 'All tensors must have the same type'
         B, H, n, d = q.shape
         assert k.shape[0] == B and k.shape[2:] == (n, d), 'query and key sequence lengths must be equal'
@@ -674,30 +678,38 @@ class NonCausalHyperFunc(torch.autograd.Function):
         assert n % 128 == 0, 'keys sequence length must be divisible by 128'
         assert sample_size % 128 == 0
         cfg = (0, block_size, sample_size, proj_f32.shape[1], 0, 0, scale, flags)
-        return _call_forward(False, q, k, v, proj_f32, cfg), cfg
+        return _call_forward(False, q, k, v, proj_f32, cfg, sample), cfg
 
     @staticmethod
-    def forward(ctx, q, k, v, proj_f32, block_size, sample_size, scale, flags):
-        (o, lse, saved), ctx.cfg = NonCausalHyperFunc.run(q, k, v, proj_f32, block_size, sample_size, scale, flags)
-        ctx.save_for_backward(q, k, v, o, lse, saved, proj_f32)
+    def forward(ctx, q, k, v, proj_f32, block_size, sample_size, scale, flags, sample=None):
+        (o, lse, saved), ctx.cfg = NonCausalHyperFunc.run(q, k, v, proj_f32, block_size, sample_size, scale, flags, sample)
+        ctx.save_for_backward(q, k, v, o, lse, saved, proj_f32, sample)
         ctx.set_materialize_grads(False)
         return o, lse
 
     @staticmethod
     def backward(ctx, do, dlse_unused=None):
         if do is None:
-            return (None,) * 8
-        q, k, v, o, lse, saved, proj_f32 = ctx.saved_tensors
+            return (None,) * 9
+        q, k, v, o, lse, saved, proj_f32, sample = ctx.saved_tensors
         if do.stride(-1) != 1:
             do = do.contiguous()
-        return _call_backward(False, q, k, v, proj_f32, o, lse, saved, do, ctx.cfg) + (None,) * 5
+        return _call_backward(False, q, k, v, proj_f32, o, lse, saved, do, ctx.cfg, sample) + (None,) * 6
 
 
-def noncausal_hyper(q, k, v, proj_f32, block_size, sample_size, scale, flags):
+def uniform_sample(rows, n, sample_size, base, device):
+    """int32 [rows, sample_size]: one row of [0, n) per stratum, from counters base + row * sample_size + slot (ha_uniform_sample)."""
+    out = torch.empty(rows, sample_size, dtype=torch.int32, device=device)
+    _cuda(out)
+    L.check(_call(L.load().ha_uniform_sample, out.device, rows, n, sample_size, base, out.data_ptr()), 'ha_uniform_sample')
+    return out
+
+
+def noncausal_hyper(q, k, v, proj_f32, block_size, sample_size, scale, flags, sample=None):
     """NonCausalHyperFunc, without the autograd machinery where no gradient is wanted."""
     if _wants_grad(q, k, v):
-        return NonCausalHyperFunc.apply(q, k, v, proj_f32, block_size, sample_size, scale, flags)
-    return NonCausalHyperFunc.run(q, k, v, proj_f32, block_size, sample_size, scale, flags)[0][:2]
+        return NonCausalHyperFunc.apply(q, k, v, proj_f32, block_size, sample_size, scale, flags, sample)
+    return NonCausalHyperFunc.run(q, k, v, proj_f32, block_size, sample_size, scale, flags, sample)[0][:2]
 
 
 def launch_count():

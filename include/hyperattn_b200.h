@@ -266,9 +266,17 @@ int ha_noncausal_bwd(const ha_causal_params* p, void* stream);
  * (hyper_attention.py:38-40). */
 int ha_causal_fwd_strided(const ha_causal_params* p, const int64_t* strides, void* stream);
 int ha_causal_bwd_strided(const ha_causal_params* p, const int64_t* strides, void* stream);
-int64_t ha_noncausal_scratch_bytes_strided(const ha_causal_params* p, const int64_t* strides, int32_t backward);
-int ha_noncausal_fwd_strided(const ha_causal_params* p, const int64_t* strides, void* stream);
-int ha_noncausal_bwd_strided(const ha_causal_params* p, const int64_t* strides, void* stream);
+/* ... and the non-causal one with sampled rows of the caller's choice: sample_idx (int32 [B*H][sample_size], distinct rows) makes the sampled
+ * part the importance-weighted estimate of ha_sample_weights, whose outputs then lie in `saved` as well; NULL = rows
+ * 0..sample_size-1, unweighted.  Not together with shared K/V heads. */
+int64_t ha_noncausal_saved_bytes_ext(const ha_causal_params* p, const int32_t* sample_idx);
+int64_t ha_noncausal_scratch_bytes_ext(const ha_causal_params* p, const int64_t* strides, const int32_t* sample_idx, int32_t backward);
+int ha_noncausal_fwd_ext(const ha_causal_params* p, const int64_t* strides, const int32_t* sample_idx, void* stream);
+int ha_noncausal_bwd_ext(const ha_causal_params* p, const int64_t* strides, const int32_t* sample_idx, void* stream);
+
+/* Distinct sampled rows, one uniform draw from each of sample_size equal strata of [0, n) per row of sample_idx [rows][sample_size]: 24 bits
+ * of the splitmix64 finaliser of base + row * sample_size + slot.  No counterpart in the reference. */
+int ha_uniform_sample(int32_t rows, int32_t n, int32_t sample_size, uint64_t base, int32_t* sample_idx, void* stream);
 
 /* Backward of exact attention (HA_MODE_FLASH, one segment, equal lengths) in one call: delta, the backward kernel, casts.  p as for
  * ha_attn_bwd without delta and outputs; dq [B,H,n,d], dk / dv [B,H/kv_group,n,*] contiguous, in the tensors' dtype.  Replaces

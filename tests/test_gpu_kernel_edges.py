@@ -151,3 +151,47 @@ def test_strided_tensors_match_contiguous_ones(causal, dtype):
         assert torch.equal(r[0], res[0][0]) and torch.equal(r[1], res[0][1]) and torch.equal(r[2], res[0][2])
         for a, b in zip(r[3:], res[0][3:]):
             assert rel(a, b) < 1e-3
+
+
+@pytest.mark.parametrize('rows,n,span,off,length,bits', [
+    (3, 2047, 2047, 0, 2047, 8), (3, 2048, 2048, 0, 2048, 8), (2, 2049, 2049, 0, 2049, 7), (2, 4097, 4097, 0, 4097, 8),
+    (1, 8192, 8192, 0, 8192, 8), (2, 8193, 8193, 0, 8193, 1), (1, 70001, 70001, 0, 70001, 8), (150, 1, 1, 0, 1, 8),
+    (2, 12288, 4096, 2048, 2048, 8), (2, 4100, 2050, 1025, 1025, 8), (2, 3000, 3000, 0, 3000, 10),
+])
+def test_segment_sort_at_the_edges_of_its_chunks(rows, n, span, off, length, bits):
+    """lengths around the chunk sizes, segments that start inside a span, more key bits than a chunk counts: the stable order"""
+    import hyperattention_b200 as ha
+    codes = torch.randint(0, 1 << bits, (rows, n), generator=torch.Generator().manual_seed(76), dtype=torch.int32)
+    idx = ha.seg_sort(codes.cuda(), bits, span=span, seg_off=off, seg_len=length).cpu()
+    segs = codes.view(rows * (n // span), span)[:, off:off + length]
+    assert torch.equal(idx.view(segs.shape).long(), torch.sort(segs, dim=1, stable=True)[1])
+
+
+@pytest.mark.parametrize('dtype,d,n,causal', [(torch.bfloat16, 64, 333, True), (torch.float16, 128, 257, True),
+                                              (torch.bfloat16, 64, 130, False), (torch.float32, 64, 200, True)])
+def test_exact_attention_with_shared_key_value_heads(dtype, d, n, causal):
+    """fewer key/value heads than query heads, never expanded: against the oracle on expanded ones"""
+    import hyperattention_b200 as ha
+    torch.manual_seed(77)
+    B, H, Hk = 2, 6, 2
+    q, do = [torch.randn(B, n, H, d).to(dtype) for _ in range(2)]
+    k, v = [torch.randn(B, n, Hk, d).to(dtype) for _ in range(2)]
+    qg, kg, vg = [t.cuda().requires_grad_() for t in (q, k, v)]
+    o, lse = ha.flash_attn_func(qg, kg, vg, None, causal)
+    o.backward(do.cuda())
+    qc, kc, vc = [t.float().requires_grad_() for t in (q, k, v)]
+    s = (qc.transpose(1, 2) @ kc.repeat_interleave(H // Hk, 2).permute(0, 2, 3, 1)) * d ** -0.5
+    if causal:
+        s = s.masked_fill(torch.ones(n, n, dtype=torch.bool).triu(1), float('-inf'))
+    ow = (s.softmax(-1) @ vc.repeat_interleave(H // Hk, 2).transpose(1, 2)).transpose(1, 2)
+    ow.backward(do.float())
+    _check((o, lse[:, :, :n], qg.grad, kg.grad, vg.grad), (ow, s.logsumexp(-1), qc.grad, kc.grad, vc.grad), dtype)
+
+
+@pytest.mark.parametrize('rows,n,S', [(3, 1000, 256), (1, 128, 128), (5, 131072, 384)])
+def test_uniform_sample_draws_the_oracles_rows(rows, n, S):
+    """one row per stratum, whole numbers equal to the oracle's, at sizes that divide evenly and that do not"""
+    from hyperattention_b200 import ops
+    base = (2024 * 0x9E3779B97F4A7C15 + 3 * 0xD1B54A32D192ED03) & ((1 << 64) - 1)
+    got = ops.uniform_sample(rows, n, S, base, 'cuda').cpu().long()
+    assert torch.equal(got, torch.as_tensor(O.uniform_sample_idx(2024, 3, rows, S, n)).long())
