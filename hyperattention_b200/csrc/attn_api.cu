@@ -14,6 +14,8 @@ int tc_attn_bwd(const ha_attn_params& p, cudaStream_t st);
 int ws_attn_bwd(const ha_attn_params& p, bool store_dq, cudaStream_t st);
 bool ws_bwd_supported(const ha_attn_params& p);
 bool ws_bwd_direct_ok(const ha_attn_params& p);
+int kt_attn_bwd(const ha_attn_params& p, cudaStream_t st);
+bool kt_bwd_supported(const ha_attn_params& p);
 
 static int check_common(const ha_attn_params& p, bool backward) {
   if (p.dtype != HA_BF16 && p.dtype != HA_FP16 && p.dtype != HA_FP32) return HA_ERR_DTYPE;
@@ -173,6 +175,7 @@ int ha_attn_bwd(const ha_attn_params* p, void* stream) {
     if (p->mode != HA_MODE_FLASH || p->m_q > 16 * TILE || p->dk_out) return HA_ERR_INVALID;
   }
   if (!(p->flags & HA_FLAG_FORCE_SIMT) && ws_bwd_supported(*p)) return ws_attn_bwd(*p, false, st);
+  if (!(p->flags & HA_FLAG_FORCE_SIMT) && kt_bwd_supported(*p)) return kt_attn_bwd(*p, st);
   if (!(p->flags & HA_FLAG_FORCE_SIMT) && tc_bwd_supported(*p)) return tc_attn_bwd(*p, st);
   if (p->dk_out || (p->flags & HA_FLAG_BWD_KV_INIT)) return HA_ERR_INVALID;   // tensor-core kernel only
   if (f32_tiled_supported(*p, true)) return f32_tiled_bwd(*p, st);

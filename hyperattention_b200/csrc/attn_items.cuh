@@ -109,6 +109,13 @@ __device__ __forceinline__ int item_key_row(const ha_attn_params& p, const AttnI
   return p.sample_idx ? p.sample_idx[(long long)it.kseg * p.sample_size + s] : s;
 }
 
+__device__ __forceinline__ void red_add_v4(float* addr, float4 v) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+__device__ __forceinline__ void push_copies(uint32_t bar) {      // an arrival once this thread's cp.async copies so far have landed
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+
 // 128 rows of 64 * slabs elements gathered by ONE warp with cp.async: rows[q] = source row of tile row 32 q + lane (-1: zero fill)
 __device__ __forceinline__ void warp_gather_tile(uint32_t smem_base, const uint16_t* __restrict__ base, int64_t row_stride, int slabs, int (&rows)[4], int lane) {
   const int chunk = lane & 7;

@@ -107,13 +107,6 @@ __device__ __forceinline__ void bws_bulk_wait_all() { asm volatile("cp.async.bul
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void bws_red_add_v4(float* addr, float4 v) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
-}
-__device__ __forceinline__ void push_copies(uint32_t bar) {      // an arrival once this thread's cp.async copies so far have landed
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
-
 template <typename T, int KIND>
 __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const ha_attn_params p, const AttnPlan pl, const BwdOut out,
                                                                          const __grid_constant__ BwdMaps maps) {
@@ -420,7 +413,7 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
                 const bool there = __shfl_sync(0xffffffffu, local, rl) >= 0;
                 if (there) {
                   if (mode == TYPED) *reinterpret_cast<float4*>(typed + rr * D + c * 8) = v;
-                  else if (mode == ROWS_ADD) bws_red_add_v4(acc + rr * D + hf * 32 + c * 4, v);
+                  else if (mode == ROWS_ADD) red_add_v4(acc + rr * D + hf * 32 + c * 4, v);
                   else *reinterpret_cast<float4*>(acc + rr * D + hf * 32 + c * 4) = v;
                 }
               }

@@ -24,6 +24,13 @@ ROLES = {0: ('elementwise group 0', EW), 1: ('elementwise group 1', EW),
          2: ('drain group', ['loop, item set-up', 'row numbers, wait staging tile', 'wait accumulator complete', 'out of TMEM, staged, stored']),
          3: ('K loader', LOAD), 4: ('S^T warp', ISSUE), 5: ('dV warp', ISSUE), 6: ('dQ warp', ISSUE), 7: ('Q / dO loader', LOAD)}
 
+# attn_tc_bwd_kt_kernel (head dim 128)
+KT_ISSUE = ['loop, item set-up', 'wait K / V tile', 'wait unit', 'wait stage, accumulator', 'issue']
+KT_ROLES = {0: ('elementwise group 0', ['loop, item set-up', 'wait S^T / dP^T ready', 'wait dS buffer free', 'loads, math, stores', 'store wait, fences, arrival']),
+            2: ('drain group', ['loop, item set-up, row numbers', 'wait dQ', 'dQ out of TMEM, added', 'wait dV / dK', 'dV / dK out of TMEM, staged, stored']),
+            3: ('K / V loader', ['row numbers', 'wait slot free', 'issue copies']), 4: ('S^T warp', KT_ISSUE), 1: ('dP^T warp', KT_ISSUE), 5: ('dV warp', KT_ISSUE),
+            6: ('dQ warp', KT_ISSUE), 7: ('Q loader', LOAD)}
+
 # attn_tc_fwd_kernel
 FWD_ROLES = {0: ('softmax group 0', ['loop, item set-up', 'wait S ready', 'scores out of TMEM, maximum, rescale', 'exponentials, P, sum',
                                      'P store wait, arrival']),
@@ -77,13 +84,13 @@ def main():
     for rep in range(2):
         o = mod(qg, kg, vg, causal=a.causal)
         if rep == 1:
-            setter = lib.ha_debug_set_timing_buffer_bwd_ws
+            setter = lib.ha_debug_set_timing_buffer_bwd_kt if a.dim == 128 else lib.ha_debug_set_timing_buffer_bwd_ws
             setter.restype, setter.argtypes = C.c_int, [C.c_void_p]
             setter(C.c_void_p(buf.data_ptr()))
         o.backward(do)
         torch.cuda.synchronize()
     b = buf.view(4096, 16).cpu().float()[:n_cta * 8].view(n_cta, 8, 16)
-    report(b, ROLES)
+    report(b, KT_ROLES if a.dim == 128 else ROLES)
 
 
 if __name__ == '__main__':

@@ -195,3 +195,46 @@ def test_uniform_sample_draws_the_oracles_rows(rows, n, S):
     base = (2024 * 0x9E3779B97F4A7C15 + 3 * 0xD1B54A32D192ED03) & ((1 << 64) - 1)
     got = ops.uniform_sample(rows, n, S, base, 'cuda').cpu().long()
     assert torch.equal(got, torch.as_tensor(O.uniform_sample_idx(2024, 3, rows, S, n)).long())
+
+
+@pytest.mark.parametrize('n,causal,H', [(1, True, 2), (63, False, 1), (64, True, 2), (65, True, 1), (193, True, 3), (1000, False, 1), (2176, True, 1), (384, True, 80)])
+def test_exact_backward_by_key_tiles(n, causal, H):
+    """head dim 128: steps of 64 query rows and key tiles of 128, cut anywhere; more key tiles than CTAs"""
+    import hyperattention_b200 as ha
+    torch.manual_seed(78)
+    q, k, v, do = [torch.randn(1, n, H, 128).bfloat16() for _ in range(4)]
+    qg, kg, vg = [t.cuda().requires_grad_() for t in (q, k, v)]
+    o, lse = ha.flash_attn_func(qg, kg, vg, None, causal)
+    o.backward(do.cuda())
+    qc, kc, vc = [t.float().requires_grad_() for t in (q, k, v)]
+    s = T(qc) @ T(kc).transpose(2, 3) * 128 ** -0.5
+    if causal:
+        s = s.masked_fill(torch.ones(n, n, dtype=torch.bool).triu(1), float('-inf'))
+    ow = T(s.softmax(-1) @ T(vc))
+    ow.backward(do.float())
+    if n == 1:                                          # (one key: its weight is one, so q and k have no gradient)
+        assert rel(vg.grad, vc.grad) < 2e-2 and qg.grad.abs().max() < 0.1 and kg.grad.abs().max() < 0.1
+    else:
+        _check((o, lse[:, :, :n], qg.grad, kg.grad, vg.grad), (ow, s.logsumexp(-1), qc.grad, kc.grad, vc.grad), torch.bfloat16)
+
+
+@pytest.mark.parametrize('n,block,S,smooth,weighted', [(896, 384, 128, False, False), (512, 256, 128, False, True), (768, 256, 256, True, True)])
+def test_hyper_backward_by_key_tiles(n, block, S, smooth, weighted):
+    """head dim 128: key tiles that one query tile of a pair meets, weighted samples with dropped slots, smooth windows; against the kernel that
+    takes the other shapes"""
+    import hyperattention_b200 as ha
+    from hyperattention_b200 import _lib as L
+    torch.manual_seed(79)
+    B, H, d = 1, 2, 128
+    q, k, v, do = [torch.randn(B, H, n, d).bfloat16() for _ in range(4)]
+    qi, ki = [torch.sort(torch.randint(0, 4, (B, H, n)), dim=2, stable=True)[1] for _ in range(2)]
+    sidx = ki[:, :, 64:64 + S].contiguous() if weighted else None
+    qg, kg, vg = [T(t.cuda()).requires_grad_() for t in (q, k, v)]
+    o, lse = ha.hyper_attn_func(qg, kg, vg, T(qi.cuda()), T(ki.cuda()), block, S, None, smooth, sidx.cuda() if weighted else None,
+                                L.FLAG_BWD_REF_SMOOTH if smooth else 0, weighted)
+    o.backward(T(do.cuda()))
+    want = [t.detach().requires_grad_() for t in (qg, kg, vg)]
+    ow, lw = ha.hyper_attn_func(*want, T(qi.cuda()), T(ki.cuda()), block, S, None, smooth, sidx.cuda() if weighted else None,
+                                (L.FLAG_BWD_REF_SMOOTH if smooth else 0) | L.FLAG_NO_WS, weighted)
+    ow.backward(T(do.cuda()))
+    _check((o, lse, qg.grad, kg.grad, vg.grad), (ow, lw, want[0].grad, want[1].grad, want[2].grad), torch.bfloat16)
