@@ -310,32 +310,31 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
             if (!(ok = wait(B_DQ_FULL + s, (unit >> 1) & 1))) break;
             HA_T_MARK(1)
             tc_fence_after();
-#pragma unroll 1
+            uint32_t r[2][32];
+            tmem_ld32(tmem + 128 * s + 64 + lane_sel, r[0]);
+            tmem_ld32(tmem + 128 * s + 96 + lane_sel, r[1]);
+            tmem_ld_fence(r[0]);
+            tmem_ld_fence(r[1]);
+            tc_fence_before();
+            mbar_arrive(bar(B_DQ_FREE + s));          // (the additions do not hold the stage up)
+#pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
-              uint32_t r[32];
-              tmem_ld32(tmem + 128 * s + 64 + hf * 32 + lane_sel, r);
-              tmem_ld_fence(r);
-              if (hf == 1) {
-                tc_fence_before();
-                mbar_arrive(bar(B_DQ_FREE + s));
-              }
               if (flash) {
                 // consecutive rows, `valid` of them
                 const int pos0 = it.q_pos0 + y * TILE + UQ * s + 32 * hf, valid = p.m_q - pos0;
                 float* to = dq_base + (long long)pos0 * D;
 #pragma unroll
-                for (int i = 0; i < 32; ++i) red_add_f32_if(i < valid, to + i * D, __uint_as_float(r[i]));
+                for (int i = 0; i < 32; ++i) red_add_f32_if(i < valid, to + i * D, __uint_as_float(r[hf][i]));
               } else {
                 // the row numbers eight at a time: one by one, each addition would wait for a shuffle
 #pragma unroll
                 for (int i = 0; i < 32; i += 8) {
                   int to[8];
 #pragma unroll
-                  for (int j = 0; j < 8; ++j) to[j] = __shfl_sync(0xffffffffu, q0, i + j);
+                  for (int j = 0; j < 8; ++j) to[j] = __shfl_sync(0xffffffffu, hf ? q1 : q0, i + j);
 #pragma unroll
-                  for (int j = 0; j < 8; ++j) red_add_f32(dq_base + (long long)to[j] * D, __uint_as_float(r[i + j]));
+                  for (int j = 0; j < 8; ++j) red_add_f32(dq_base + (long long)to[j] * D, __uint_as_float(r[hf][i + j]));
                 }
-                q0 = q1;
               }
             }
             HA_T_MARK(2)
@@ -548,13 +547,11 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
         return it.n_list != 0;
       };
       KtItem it;
-      int e = 0, y = 0, s = 0;
+      int e = 0, y = 0;
       bool more = take(it);
       // (every list starts with a key tile that its first query tile meets)
       if (more) { e = it.e0; y = it.y0; }
       auto advance = [&]() {
-        s ^= 1;
-        if (s) return;
         do {
           if (++y < it.y1) continue;
           y = it.y0;
@@ -564,24 +561,25 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
           return;
         } while (!active(it, y, e));
       };
-      // row numbers of the unit, lse and delta scaled for the elementwise groups
-      auto row_numbers = [&](int& r0, int& r1, float (&ld)[4]) {
-        int pos0 = it.q_pos0 + y * TILE + UQ * s + lane, pos1 = pos0 + 32;
-        if (flash) {
-          r0 = pos0 < p.m_q ? pos0 : -1;
-          r1 = pos1 < p.m_q ? pos1 : -1;
-        } else {
-          if (pos0 >= p.m_q) pos0 -= p.m_q;
-          if (pos1 >= p.m_q) pos1 -= p.m_q;
-          r0 = p.q_idx[(long long)it.seg * p.m_q + pos0];
-          r1 = p.q_idx[(long long)it.seg * p.m_q + pos1];
+      // row numbers of the query tile's two units (-1: none)
+      auto row_numbers = [&](int (&rows)[4]) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          int pos = it.q_pos0 + y * TILE + 32 * q + lane;
+          if (flash) {
+            rows[q] = pos < p.m_q ? pos : -1;
+          } else {
+            if (pos >= p.m_q) pos -= p.m_q;
+            rows[q] = p.q_idx[(long long)it.seg * p.m_q + pos];
+          }
         }
-        if (is_q) {
-          const long long at = ((long long)(it.b * p.H + it.h)) * p.n + it.q_row0;
-          ld[0] = r0 >= 0 ? p.lse[at + r0] : INFINITY;           // no such query: P = 0
-          ld[1] = r1 >= 0 ? p.lse[at + r1] : INFINITY;
-          ld[2] = r0 >= 0 ? p.delta[at + r0] : 0.f;
-          ld[3] = r1 >= 0 ? p.delta[at + r1] : 0.f;
+      };
+      auto lse_delta = [&](const int (&rows)[4], float (&l)[4], float (&dl)[4]) {
+        const long long at = ((long long)(it.b * p.H + it.h)) * p.n + it.q_row0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          l[q] = rows[q] >= 0 ? p.lse[at + rows[q]] : INFINITY;      // no such query: P = 0
+          dl[q] = rows[q] >= 0 ? p.delta[at + rows[q]] : 0.f;
         }
       };
       const uint16_t* tensor = (const uint16_t*)(is_q ? p.q : p.d_o);
@@ -589,45 +587,65 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
       const int b_full = is_q ? B_Q_FULL : B_DO_FULL, b_empty = is_q ? B_Q_EMPTY : B_DO_EMPTY;
       const uint32_t ring = s_base + (is_q ? OFF_Q : OFF_DO);
       uint32_t n = 0, slot = 0, lap = 0;
-      int r0 = 0, r1 = 0;
-      float ld[4] = {0.f, 0.f, 0.f, 0.f};
-      if (more) row_numbers(r0, r1, ld);
+      int rows[4] = {0, 0, 0, 0}, ahead[4] = {0, 0, 0, 0};
+      float l[4], dl[4], l_ahead[4], dl_ahead[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) l[q] = dl[q] = l_ahead[q] = dl_ahead[q] = 0.f;
+      if (more) {
+        row_numbers(rows);
+        if (is_q) lse_delta(rows, l, dl);
+      }
+      bool ok = true;
       HA_T_DECL(8)
-      while (more) {
+      while (more && ok) {
         HA_T_MARK(2)
-        const int b = it.b, h = it.h, q_row0 = it.q_row0, box_row = q_row0 + it.q_pos0 + y * TILE + UQ * s;
-        const int c0 = r0, c1 = r1;
-        const float l0 = ld[0], l1 = ld[1], d0 = ld[2], d1 = ld[3];
-        // the next unit's row numbers, lse and delta travel during the wait
+        const int b = it.b, h = it.h, q_row0 = it.q_row0, box_row = q_row0 + it.q_pos0 + y * TILE;
+        const uint16_t* base = tensor + b * sb + h * sh + (int64_t)q_row0 * sn;
+        // The next query tile's row numbers travel while this one's first unit waits for its slot, what they index while the second does.
         advance();
-        if (more) row_numbers(r0, r1, ld);
-        HA_T_MARK(0)
-        if (n >= NU && !wait(b_empty + slot, (lap - 1) & 1)) break;
-        HA_T_MARK(1)
-        const uint32_t full = bar(b_full + slot), dst = ring + slot * 2 * SLAB_U;
-        if (boxed) {
-          const int ur = __shfl_sync(0xffffffffu, box_row, 0), uh = __shfl_sync(0xffffffffu, h, 0), ub = __shfl_sync(0xffffffffu, b, 0);
-          if (elect_one()) {
-            mbar_add_tx(full, 2 * SLAB_U);
-            tma_tile(dst, &maps.tile[is_q ? 0 : 3], 0, ur, uh, ub, full);
-            tma_tile(dst + SLAB_U, &maps.tile[is_q ? 0 : 3], 64, ur, uh, ub, full);
+        if (more) row_numbers(ahead);
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          HA_T_MARK(0)
+          if (ok && n >= NU) ok = wait(b_empty + slot, (lap - 1) & 1);
+          if (!ok) break;
+          HA_T_MARK(1)
+          const uint32_t full = bar(b_full + slot), dst = ring + slot * 2 * SLAB_U;
+          if (boxed) {
+            const int ur = __shfl_sync(0xffffffffu, box_row + UQ * s, 0), uh = __shfl_sync(0xffffffffu, h, 0), ub = __shfl_sync(0xffffffffu, b, 0);
+            if (elect_one()) {
+              mbar_add_tx(full, 2 * SLAB_U);
+              tma_tile(dst, &maps.tile[is_q ? 0 : 3], 0, ur, uh, ub, full);
+              tma_tile(dst + SLAB_U, &maps.tile[is_q ? 0 : 3], 64, ur, uh, ub, full);
+            }
+            __syncwarp();
+            mbar_arrive(full);
+          } else {
+            warp_gather_unit(dst, base, sn, rows[2 * s], rows[2 * s + 1], lane);
+            push_copies(full);
           }
-          __syncwarp();
-          mbar_arrive(full);
-        } else {
-          warp_gather_unit(dst, tensor + b * sb + h * sh + (int64_t)q_row0 * sn, sn, c0, c1, lane);
-          push_copies(full);
+          if (is_q) {
+            float* at = reinterpret_cast<float*>(smem + OFF_LD + slot * 512);
+            at[lane] = -LOG2E * l[2 * s];
+            at[32 + lane] = -LOG2E * l[2 * s + 1];
+            at[UQ + lane] = -p.scale * dl[2 * s];
+            at[UQ + 32 + lane] = -p.scale * dl[2 * s + 1];
+            mbar_arrive(full);
+            if (s == 0 && more) lse_delta(ahead, l_ahead, dl_ahead);
+          }
+          ++n;
+          if (++slot == NU) { slot = 0; ++lap; }
         }
-        if (is_q) {
-          float* at = reinterpret_cast<float*>(smem + OFF_LD + slot * 512);
-          at[lane] = -LOG2E * l0;
-          at[32 + lane] = -LOG2E * l1;
-          at[UQ + lane] = -p.scale * d0;
-          at[UQ + 32 + lane] = -p.scale * d1;
-          mbar_arrive(full);
+        if (!flash && more && e == it.e0) {          // rows met for the first time: into L2
+          const uint16_t* nb = tensor + it.b * sb + it.h * sh + (int64_t)it.q_row0 * sn;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            prefetch_l2(nb + (int64_t)ahead[q] * sn);
+            prefetch_l2(nb + (int64_t)ahead[q] * sn + 64);
+          }
         }
-        ++n;
-        if (++slot == NU) { slot = 0; ++lap; }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) { rows[q] = ahead[q]; l[q] = l_ahead[q]; dl[q] = dl_ahead[q]; }
       }
       HA_T_DUMP(8, (int)blockIdx.x * 8 + 7, lane == 0 && is_q)
       cp_async_commit();
@@ -654,6 +672,7 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
         int ahead[4] = {0, 0, 0, 0};
         if (more) row_numbers(it, e, ahead);
         bool ok = true;
+        const bool fetch = !flash && more && e < it.n_win;      // the next tile's rows into L2
 #pragma unroll 1
         for (int is_k = 0; is_k < 2; ++is_k) {
           HA_T_MARK(0)
@@ -675,6 +694,15 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
             const uint16_t* base = is_k ? (const uint16_t*)p.k + b * p.k_sb + hd * p.k_sh : (const uint16_t*)p.v + b * p.v_sb + hd * p.v_sh;
             warp_gather_tile(dst, base + (int64_t)row0 * sn, sn, 2, r, lane);
             push_copies(full);
+          }
+          if (fetch) {
+            const int64_t sn = is_k ? p.k_sn : p.v_sn;
+            const uint16_t* nb = (is_k ? (const uint16_t*)p.k + it.b * p.k_sb + it.hk * p.k_sh : (const uint16_t*)p.v + it.b * p.v_sb + it.hk * p.v_sh) + (int64_t)it.k_row0 * sn;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              prefetch_l2(nb + (int64_t)ahead[q] * sn);
+              prefetch_l2(nb + (int64_t)ahead[q] * sn + 64);
+            }
           }
         }
         if (!ok) break;
