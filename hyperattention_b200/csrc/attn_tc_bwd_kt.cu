@@ -37,9 +37,9 @@ constexpr int OFF_V = OFF_K + 2 * TILE_B;
 constexpr int OFF_Q = OFF_V + 2 * TILE_B;                      // unit slots: Q
 constexpr int OFF_DO = OFF_Q + NU * 2 * SLAB_U;                // ... dO
 constexpr int OFF_DS = OFF_DO + NU * 2 * SLAB_U;               // dS^T of the two stages: 128 key rows x 64 queries
-constexpr int OFF_ST = OFF_DS + 2 * TILE_B;                    // staging of the drain group: 128 rows x 128 bytes
-constexpr int OFF_LD = OFF_ST + TILE_B;                        // per unit slot: -lse log2e [64], -delta scale [64] (fp32)
-constexpr int SMEM_USED = OFF_LD + NU * 512;
+constexpr int OFF_ST = OFF_DS + 2 * TILE_B;                    // staging of the drain group, 2 x 16 KB (below)
+constexpr int OFF_LD = OFF_ST + 2 * TILE_B;                      // per unit slot: -lse log2e [64], -delta scale [64] (fp32)
+constexpr int SMEM_USED = OFF_LD + NU * 512;                   // from the first 1 KB boundary after the static variables
 constexpr int THREADS = 640;
 constexpr int W_DRAIN = 8, W_MMA = 12, W_Q = 17, W_DO = 18;    // first warp of each role (K and V: 19)
 constexpr int COL_DV = 256, COL_DK = 384;
@@ -62,9 +62,12 @@ enum {
   B_DQ_FREE = 26,     // 2 x 128: ... drained: dP^T may be overwritten
   B_ACC_FULL = 28,    // 2 x 1: dV / dK of a key tile complete
   B_ACC_FREE = 30,    // 2 x 128: ... drained
-  B_D_FULL = 32,      // ND x 1
-  B_D_EMPTY = 32 + ND,
-  N_BARS = 32 + 2 * ND
+  B_ST_FULL = 32,     // 2 x 128: every drain thread has written its column of the staged rows
+  B_ST_IDLE = 34,     // 128: every drain thread is done with a key tile's staging
+  B_ST_FREE = 35,     // 2 x 1: the copy engine has read the staged rows
+  B_D_FULL = 37,      // ND x 1
+  B_D_EMPTY = 37 + ND,
+  N_BARS = 37 + 2 * ND
 };
 __device__ __forceinline__ int bar_count(int i) {
   if (i >= B_D_EMPTY) return CONSUMERS;
@@ -72,12 +75,12 @@ __device__ __forceinline__ int bar_count(int i) {
   if (i == B_K_FULL || i == B_V_FULL || (i >= B_DO_FULL && i < B_DO_EMPTY)) return 32;
   if (i >= B_Q_FULL && i < B_Q_EMPTY) return 64;
   if (i < B_P_READY) return 2;                       // K_EMPTY, Q_EMPTY, DO_EMPTY, S_READY
-  if (i < B_S_FREE || (i >= B_DQ_FREE && i < B_ACC_FULL) || i >= B_ACC_FREE) return 128;
+  if (i < B_S_FREE || (i >= B_DQ_FREE && i < B_ACC_FULL) || (i >= B_ACC_FREE && i < B_ST_FREE)) return 128;
   return 1;
 }
 }  // namespace bkt
 
-enum { KT_HYPER = 0, KT_FLASH = 1, KT_ANY = 2 };               // the plain hyper pattern, exact attention, any call
+enum { KT_HYPER = 0, KT_FLASH = 1, KT_ANY = 2 };               // the plain hyper pattern, exact attention, the hyper pattern in any form
 struct KtMaps { CUtensorMap tile[4]; };                        // tiles of q, k, v, dO
 
 // Entries [e0, e1) of the list of key tiles, each with the query tiles [y0, y1) it meets.
@@ -112,9 +115,13 @@ __device__ __forceinline__ KtItem kt_item(const ha_attn_params& p, const AttnPla
   return it;
 }
 
-__device__ __forceinline__ void red_add_f32_if(bool there, float* addr, float v) {
-  asm volatile("{\n .reg .pred p;\n setp.ne.s32 p, %0, 0;\n @p red.global.add.f32 [%1], %2;\n}\n" ::"r"((int)there), "l"(addr), "f"(v) : "memory");
+// `bytes` of fp32 in shared memory -> added to global memory; the four below concern the calling thread's copies
+__device__ __forceinline__ void bulk_add_f32(float* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void red_add_f32(float* addr, float v) { asm volatile("red.global.add.f32 [%0], %1;" ::"l"(addr), "f"(v) : "memory"); }
 // the 64 rows of a unit's operand, gathered by one warp: rows[q] = source row of unit row 32 q + lane (-1: zero fill)
 __device__ __forceinline__ void warp_gather_unit(uint32_t dst, const uint16_t* __restrict__ base, int64_t row_stride, int r0, int r1, int lane) {
@@ -147,10 +154,19 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
   __shared__ int s_bail;
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  const bool flash = KIND == KT_FLASH || (KIND == KT_ANY && p.mode == HA_MODE_FLASH);
+  constexpr bool flash = KIND == KT_FLASH;
   constexpr bool ANY = KIND == KT_ANY;
 
   if (cta_sees_failure(p.status, &s_bail)) return;   // an earlier CTA gave up: drain quickly (uniform over the CTA)
+  {
+    // Should the dynamic window start somewhere else than assumed, do nothing rather than run over its end.
+    uint32_t dyn;
+    asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+    if ((uint32_t)(smem - smem_raw) + (uint32_t)SMEM_USED > dyn) {      // uniform over the grid
+      if (tid == 0) report_status(p.status, p.status_host, HA_DEV_BAD_LAUNCH);
+      return;
+    }
+  }
   const uint32_t bar0 = smem_u32(bars);
   auto bar = [&](int i) -> uint32_t { return bar0 + 8 * i; };
   if (tid == 0) {
@@ -285,12 +301,13 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
     const uint8_t* warp_rows = smem + OFF_ST + (row & ~31) * 128;
     const bool kv_init = p.flags & HA_FLAG_BWD_KV_INIT;
     uint32_t unit = 0, n_kt = 0;                            // units / key tiles drained so far
+    bool staged = false, last_freed = false;                // a key tile's staging has not been seen idle; (issuer) the last half's rows are known to be read
     bool ok = true;
     HA_T_DECL(8)
     KtItem it;
     while (ok && next_item(it)) {
       const int Hk = p.kv_group > 1 ? pl.by_group(p.H) : p.H;
-      float* dq_base = p.dq_acc + ((long long)(it.b * p.H + it.h) * p.n + it.q_row0) * D + row;      // this lane's element of a row
+      float* dq_base = p.dq_acc + ((long long)(it.b * p.H + it.h) * p.n + it.q_row0) * D + (flash ? 0 : row);      // (scattered rows: this lane's element)
 #pragma unroll 1
       for (int e = it.e0; e < it.e1 && ok; ++e) {
 #pragma unroll 1
@@ -320,11 +337,29 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
               if (flash) {
-                // consecutive rows, `valid` of them
-                const int pos0 = it.q_pos0 + y * TILE + UQ * s + 32 * hf, valid = p.m_q - pos0;
-                float* to = dq_base + (long long)pos0 * D;
+                // 32 consecutive rows: staged as they lie in memory, added by the copy engine
+                const int pos0 = it.q_pos0 + y * TILE + UQ * s + 32 * hf, valid = min(p.m_q - pos0, 32);
+                uint8_t* to = smem + OFF_ST + hf * TILE_B + row * 4;
+                if (hf == 0 && staged && !(ok = wait(B_ST_IDLE, (n_kt - 1) & 1))) break;
+                staged = false;
+                if (unit >= 1 && !(ok = wait(B_ST_FREE + hf, (unit - 1) & 1))) break;
 #pragma unroll
-                for (int i = 0; i < 32; ++i) red_add_f32_if(i < valid, to + i * D, __uint_as_float(r[hf][i]));
+                for (int i = 0; i < 32; ++i) *reinterpret_cast<uint32_t*>(to + i * (D * 4)) = r[hf][i];
+                fence_async_smem();
+                mbar_arrive(bar(B_ST_FULL + hf));
+                if (warp == W_DRAIN) {
+                  if (!(ok = wait(B_ST_FULL + hf, unit & 1))) break;
+                  if (lane == 0) {
+                    if (valid > 0) bulk_add_f32(dq_base + (long long)pos0 * D, s_base + OFF_ST + hf * TILE_B, valid * (D * 4));
+                    bulk_commit();
+                    if (unit + hf > 0) {
+                      bulk_wait_read<1>();          // the half before has been read
+                      if (!last_freed) mbar_arrive(bar(B_ST_FREE + (hf ^ 1)));
+                    }
+                    last_freed = false;
+                  }
+                  __syncwarp();
+                }
               } else {
                 // the row numbers eight at a time: one by one, each addition would wait for a shuffle
 #pragma unroll
@@ -337,11 +372,24 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
                 }
               }
             }
+            if (!ok) break;
             HA_T_MARK(2)
           }
         }
         if (!ok) break;
-        // dV, dK of the key tile
+        // dV, dK of the key tile: 128 rows x 128 bytes staged at a time, a warp's 32 rows in 4 KB of its own
+        if (flash) {
+          if (warp == W_DRAIN) {
+            if (lane == 0) {
+              bulk_wait_read<0>();
+              mbar_arrive(bar(B_ST_FREE + 1));
+              last_freed = true;
+            }
+            __syncwarp();
+          }
+          // (both halves of the last unit: the first was seen free when the second was issued)
+          if (!(ok = wait(B_ST_FREE, (unit - 1) & 1)) || !(ok = wait(B_ST_FREE + 1, (unit - 1) & 1))) break;
+        }
         int local = item_key_row(p, it, e, row, flash);
         if (local >= 0) local += it.k_row0;
         const bool sampled = !flash && e >= it.n_win;
@@ -413,9 +461,14 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
           }
           HA_T_MARK(4)
         }
+        if (flash) {
+          mbar_arrive(bar(B_ST_IDLE));
+          staged = true;
+        }
         ++n_kt;
       }
     }
+    bulk_wait_all();       // nothing of this thread is in flight when the CTA retires
     HA_T_DUMP(8, (int)blockIdx.x * 8 + 2, row == 0)
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
@@ -764,10 +817,16 @@ static int launch_kt_bwd(const ha_attn_params& p, cudaStream_t st) {
              encode_tile_map(&maps.tile[2], p.dtype, p.v, 128, n_k, Hk, p.B, p.v_sn, p.v_sh, p.v_sb, TILE) &&
              (!flash || (encode_tile_map(&maps.tile[0], p.dtype, p.q, 128, n_q, p.H, p.B, p.q_sn, p.q_sh, p.q_sb, bkt::UQ) &&
                          encode_tile_map(&maps.tile[3], p.dtype, p.d_o, 128, n_q, p.H, p.B, p.do_sn, p.do_sh, p.do_sb, bkt::UQ)));
-  constexpr int DYN = bkt::SMEM_USED + 1024;      // (room for the alignment)
-  HA_SMEM_ATTR_ONCE((attn_tc_bwd_kt_kernel<T, KIND>), DYN, "ha_attn_bwd smem attribute");
+  static int dyn_bytes = 0;
+  if (dyn_bytes == 0) {
+    cudaFuncAttributes fa;
+    HA_CUDA_OK(cudaFuncGetAttributes(&fa, attn_tc_bwd_kt_kernel<T, KIND>), "ha_attn_bwd kernel attributes");
+    const int stat = ((int)fa.sharedSizeBytes + 15) / 16 * 16;
+    dyn_bytes = (1024 - stat % 1024) % 1024 + bkt::SMEM_USED;
+  }
+  HA_SMEM_ATTR_ONCE((attn_tc_bwd_kt_kernel<T, KIND>), dyn_bytes, "ha_attn_bwd smem attribute");
   const int sms = sm_count();
-  attn_tc_bwd_kt_kernel<T, KIND><<<(unsigned)(pl.n_items < sms ? pl.n_items : sms), bkt::THREADS, DYN, st>>>(p, pl, maps);
+  attn_tc_bwd_kt_kernel<T, KIND><<<(unsigned)(pl.n_items < sms ? pl.n_items : sms), bkt::THREADS, dyn_bytes, st>>>(p, pl, maps);
   HA_LAUNCHED("ha_attn_bwd (tcgen05, by key tiles)");
   return HA_OK;
 }
