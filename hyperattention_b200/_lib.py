@@ -84,6 +84,7 @@ SIGNATURES = {
     'ha_noncausal_scratch_bytes_ext': (i64, [C.POINTER(CausalParams), vp, vp, i32]),
     'ha_noncausal_fwd_ext': (C.c_int, [C.POINTER(CausalParams), vp, vp, vp]),
     'ha_noncausal_bwd_ext': (C.c_int, [C.POINTER(CausalParams), vp, vp, vp]),
+    'ha_pad_rows': (C.c_int, [i32, vp, vp, vp, vp, vp, i32, i32, i32, i32, vp]),
     'ha_uniform_sample': (C.c_int, [i32, i32, i32, C.c_uint64, vp, vp]),
     'ha_flash_bwd_scratch_bytes': (i64, [C.POINTER(AttnParams), vp]),
     'ha_flash_bwd': (C.c_int, [C.POINTER(AttnParams), vp, vp, vp, vp, i64, vp]),

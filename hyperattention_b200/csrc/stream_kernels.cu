@@ -546,6 +546,37 @@ __global__ void __launch_bounds__(128) sample_weights_kernel(const int32_t* __re
   if (threadIdx.x == 0) tile_logw[seg * T_ + t] = kept > 0 ? logf((float)(m - w.count) / (float)kept) : -INFINITY;
 }
 
+// Rows padded with zero rows, up to four tensors a launch (blockIdx.y): dst [B][H][rows][width] contiguous, of which the first n come from
+// src.  Bound by DRAM: a thread has four 16-byte chunks on the way.  (Eight strided copies and fills of a causal training step at an odd
+// length, 16 heads x 12287 x 64 bf16: 133 us.)
+struct PadJobs {
+  const uint8_t* src[4];
+  uint8_t* dst[4];
+  long long sb[4], sh[4], sn[4], chunks[4];      // strides in bytes; chunks of dst
+  FastDiv by_row[4], by_heads[4];                // chunks per row, heads
+  int heads[4], row_chunks[4];
+};
+template <typename V>
+__global__ void __launch_bounds__(256) pad_rows_kernel(const PadJobs j, const int n, const int rows, const FastDiv by_rows, const int bh0) {
+  const int t = blockIdx.y;
+  const long long total = j.chunks[t], step = (long long)gridDim.x * 256;
+  for (long long i0 = (long long)blockIdx.x * 256 + threadIdx.x; i0 < total; i0 += 4 * step) {
+    V v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const long long i = i0 + u * step;
+      v[u] = V{};
+      if (i >= total) continue;
+      const int row = j.by_row[t]((int)i), c = (int)i - row * j.row_chunks[t];
+      const int at = by_rows(row), r = row - at * rows, bh = bh0 + at, b = j.by_heads[t](bh), h = bh - b * j.heads[t];
+      if (r < n) v[u] = __ldg(reinterpret_cast<const V*>(j.src[t] + b * j.sb[t] + h * j.sh[t] + r * j.sn[t]) + c);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i0 + u * step < total) reinterpret_cast<V*>(j.dst[t])[(long long)bh0 * rows * j.row_chunks[t] + i0 + u * step] = v[u];
+  }
+}
+
 // One slot of one row per thread: stratum [slot n / S, (slot + 1) n / S), 24 uniform bits scaled to its size.
 // Bound by its launch: one instead of the twenty of the same integer arithmetic on tensors, whose launches and host time a call of
 // sampled attention waited for (16 heads x 32768 x 64 training step, with the call's other steps in one library call: 684 -> 615 us).
@@ -562,6 +593,49 @@ __global__ void __launch_bounds__(256) uniform_sample_kernel(long long total, in
 }
 
 extern "C" {
+
+int ha_pad_rows(int32_t count, const void* const* src, const int64_t* strides, const int32_t* heads, const int32_t* widths, void* const* dst, int32_t B,
+                int32_t n, int32_t rows, int32_t elem_size, void* stream) {
+  if (count < 0 || count > 4 || !src || !strides || !heads || !widths || !dst || B < 0 || n < 0 || rows < n || (elem_size != 2 && elem_size != 4))
+    return HA_ERR_INVALID;
+  PadJobs j = {};
+  bool wide = true;
+  for (int t = 0; t < count; ++t) {
+    if (heads[t] < 0 || widths[t] < 0) return HA_ERR_INVALID;
+    if (((long long)B * heads[t] * n * widths[t] > 0 && !src[t]) || ((long long)B * heads[t] * rows * widths[t] > 0 && !dst[t])) return HA_ERR_INVALID;
+    j.src[t] = (const uint8_t*)src[t]; j.dst[t] = (uint8_t*)dst[t];
+    j.sb[t] = strides[3 * t] * elem_size; j.sh[t] = strides[3 * t + 1] * elem_size; j.sn[t] = strides[3 * t + 2] * elem_size;
+    wide = wide && ((uintptr_t)src[t] | (uintptr_t)dst[t] | (uintptr_t)j.sb[t] | (uintptr_t)j.sh[t] | (uintptr_t)j.sn[t] | (uintptr_t)(widths[t] * elem_size)) % 16 == 0;
+  }
+  // 16-byte chunks where every row starts on a 16-byte boundary, elements elsewhere
+  const int chunk = wide ? 16 : elem_size;
+  long long per_head = 1, all = 0;               // chunks of the widest tensor's (batch, head); number of those
+  for (int t = 0; t < count; ++t) {
+    j.heads[t] = heads[t]; j.row_chunks[t] = widths[t] * elem_size / chunk;
+    j.by_row[t] = FastDiv(j.row_chunks[t] > 0 ? j.row_chunks[t] : 1);
+    j.by_heads[t] = FastDiv(heads[t] > 0 ? heads[t] : 1);
+    if ((long long)rows * j.row_chunks[t] > per_head) per_head = (long long)rows * j.row_chunks[t];
+    if ((long long)B * heads[t] > all) all = (long long)B * heads[t];
+  }
+  const long long limit = 0x7fffffffLL - (1 << 26);      // (32-bit indices; a launch takes as many heads as they can count)
+  if (per_head > limit) return HA_ERR_TOO_LARGE;
+  const FastDiv by_rows(rows > 0 ? rows : 1);
+  for (long long bh0 = 0; bh0 < all; bh0 += limit / per_head) {
+    long long most = 0;
+    for (int t = 0; t < count; ++t) {
+      const long long left = (long long)B * heads[t] - bh0, heads_now = left < 0 ? 0 : left < limit / per_head ? left : limit / per_head;
+      j.chunks[t] = heads_now * rows * j.row_chunks[t];
+      if (j.chunks[t] > most) most = j.chunks[t];
+    }
+    if (most == 0) continue;
+    const dim3 grid((unsigned)grid_for(most, 256 * 4), count);
+    if (chunk == 16) pad_rows_kernel<uint4><<<grid, 256, 0, (cudaStream_t)stream>>>(j, n, rows, by_rows, (int)bh0);
+    else if (chunk == 4) pad_rows_kernel<uint32_t><<<grid, 256, 0, (cudaStream_t)stream>>>(j, n, rows, by_rows, (int)bh0);
+    else pad_rows_kernel<uint16_t><<<grid, 256, 0, (cudaStream_t)stream>>>(j, n, rows, by_rows, (int)bh0);
+  }
+  HA_LAUNCHED("ha_pad_rows");
+  return HA_OK;
+}
 
 int ha_uniform_sample(int32_t rows, int32_t n, int32_t sample_size, uint64_t base, int32_t* sample_idx, void* stream) {
   if (rows < 0 || n < 0 || sample_size < 0 || sample_size > n) return HA_ERR_INVALID;

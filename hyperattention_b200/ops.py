@@ -606,12 +606,15 @@ def _call_backward(causal, q, k, v, proj_f32, o, lse, saved, do, cfg, sample=Non
     return dq, dk, dvv
 
 
-def _padded(t, rows):
-    """t [B, H, n, w] with zero rows up to `rows`, contiguous."""
-    B, H, n, w = t.shape
-    out = torch.empty(B, H, rows, w, dtype=t.dtype, device=t.device)
-    out[:, :, :n].copy_(t)
-    out[:, :, n:].zero_()
+def _padded(ts, rows):
+    """Tensors [B, H, n, w] (one type, contiguous rows) with zero rows up to `rows`, contiguous: one launch (ha_pad_rows)."""
+    B, _, n, _ = ts[0].shape
+    out = [torch.empty(B, t.shape[1], rows, t.shape[3], dtype=t.dtype, device=t.device) for t in ts]
+    m = len(ts)
+    ptrs = lambda xs: (C.c_void_p * m)(*[x.data_ptr() for x in xs])
+    st = (C.c_int64 * (3 * m))(*[x for t in ts for x in t.stride()[:3]])
+    L.check(_call(L.load().ha_pad_rows, ts[0].device, m, ptrs(ts), st, (C.c_int32 * m)(*[t.shape[1] for t in ts]),
+                  (C.c_int32 * m)(*[t.shape[3] for t in ts]), ptrs(out), B, n, rows, ts[0].element_size()), 'ha_pad_rows')
     return out
 
 
@@ -636,7 +639,8 @@ class CausalHyperFunc(torch.autograd.Function):
         assert q.dtype == k.dtype == v.dtype, 'All tensors must have the same type'
         n = q.shape[2]
         if n % 2:
-            q, k, v = [_padded(t, n + 1) for t in (q, k, v)]
+            _cuda(q, k, v)
+            q, k, v = _padded((q, k, v), n + 1)
         cfg = (levels, block_size, sample_size, proj_f32.shape[1], int(keep_parts), min_seq_len, scale, flags)
         o, lse, saved = _call_forward(True, q, k, v, proj_f32, cfg)
         return o, lse, saved, (q, k, v), cfg
@@ -647,7 +651,10 @@ class CausalHyperFunc(torch.autograd.Function):
             return (None,) * 11
         q, k, v, o, lse, saved, proj_f32 = ctx.saved_tensors
         n, rows = do.shape[2], q.shape[2]
-        do = do.contiguous() if n == rows else _padded(do, rows)
+        if n != rows:
+            do, = _padded((do if do.stride(-1) == 1 else do.contiguous(),), rows)
+        else:
+            do = do.contiguous()
         dq, dk, dv = _call_backward(True, q, k, v, proj_f32, o, lse, saved, do, ctx.cfg)
         if n != rows:
             dq, dk, dv = dq[:, :, :n], dk[:, :, :n], dv[:, :, :n]

@@ -274,6 +274,11 @@ int64_t ha_noncausal_scratch_bytes_ext(const ha_causal_params* p, const int64_t*
 int ha_noncausal_fwd_ext(const ha_causal_params* p, const int64_t* strides, const int32_t* sample_idx, void* stream);
 int ha_noncausal_bwd_ext(const ha_causal_params* p, const int64_t* strides, const int32_t* sample_idx, void* stream);
 
+/* Up to four [B][heads][n][width] tensors (element strides of batch, head and row: three per tensor; contiguous rows) copied to contiguous
+ * [B][heads][rows][width] ones whose rows past n are zero: the padding of odd lengths (hyper_attention.py:59-61). */
+int ha_pad_rows(int32_t count, const void* const* src, const int64_t* strides, const int32_t* heads, const int32_t* widths, void* const* dst, int32_t B,
+                int32_t n, int32_t rows, int32_t elem_size, void* stream);
+
 /* Distinct sampled rows, one uniform draw from each of sample_size equal strata of [0, n) per row of sample_idx [rows][sample_size]: 24 bits
  * of the splitmix64 finaliser of base + row * sample_size + slot.  No counterpart in the reference. */
 int ha_uniform_sample(int32_t rows, int32_t n, int32_t sample_size, uint64_t base, int32_t* sample_idx, void* stream);

@@ -238,3 +238,13 @@ def test_hyper_backward_by_key_tiles(n, block, S, smooth, weighted):
                                 (L.FLAG_BWD_REF_SMOOTH if smooth else 0) | L.FLAG_NO_WS, weighted)
     ow.backward(T(do.cuda()))
     _check((o, lse, qg.grad, kg.grad, vg.grad), (ow, lw, want[0].grad, want[1].grad, want[2].grad), torch.bfloat16)
+
+
+@pytest.mark.parametrize('dtype,B,n,rows,shapes', [(torch.bfloat16, 2, 1023, 1024, ((3, 64), (3, 64), (1, 128))), (torch.float16, 1, 5, 6, ((2, 20),)),
+                                                   (torch.float32, 3, 130, 133, ((4, 7), (2, 8))), (torch.bfloat16, 1, 1, 2, ((1, 8), (1, 2), (5, 1), (1, 9)))])
+def test_padding_rows(dtype, B, n, rows, shapes):
+    """aligned rows, odd widths, strided sources, one to four tensors: bytes equal to torch's padding"""
+    from hyperattention_b200 import ops
+    ts = [torch.randn(n, B, h, w, device='cuda').to(dtype).permute(1, 2, 0, 3) for h, w in shapes]
+    for t, o in zip(ts, ops._padded(ts, rows)):
+        assert o.is_contiguous() and torch.equal(o, torch.nn.functional.pad(t, (0, 0, 0, rows - n)))
