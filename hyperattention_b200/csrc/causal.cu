@@ -334,6 +334,18 @@ static bool deepest_exact(const ha_causal_params& p, const CausalPlan& pl) { ret
 
 using namespace ha;
 
+// fp32 accumulators -> typed gradients; those that are neighbours on both sides (as the callers lay them out) in one launch
+struct CastJob { const float* src; void* dst; long long count; };
+static int cast_grads(const CastJob* jobs, int n, int dtype, void* stream) {
+  for (int i = 0, j; i < n; i = j) {
+    long long count = jobs[i].count;
+    for (j = i + 1; j < n && jobs[j].src == jobs[i].src + count && (uint8_t*)jobs[j].dst == (uint8_t*)jobs[i].dst + count * dtype_size(dtype); ++j) count += jobs[j].count;
+    const int rc = ha_cast_from_f32(jobs[i].src, jobs[i].dst, count, dtype, stream);
+    if (rc != HA_OK) return rc;
+  }
+  return HA_OK;
+}
+
 extern "C" {
 
 int64_t ha_causal_saved_bytes(const ha_causal_params* p) {
@@ -522,8 +534,9 @@ int ha_causal_bwd_strided(const ha_causal_params* pp, const int64_t* strides, vo
   }
   if (!q_init) HA_CUDA_OK(cudaMemsetAsync(dq_acc, 0, pl.rows * p.d * 4, st), "ha_causal_bwd memset");
   if (!kv_init) {
-    HA_CUDA_OK(cudaMemsetAsync(dk_acc, 0, pl.rows_k * p.d * 4, st), "ha_causal_bwd memset");
-    HA_CUDA_OK(cudaMemsetAsync(dv_acc, 0, pl.rows_k * p.dv * 4, st), "ha_causal_bwd memset");
+    const bool neighbours = dv_acc == dk_acc + pl.rows_k * p.d;
+    HA_CUDA_OK(cudaMemsetAsync(dk_acc, 0, pl.rows_k * (p.d + (neighbours ? p.dv : 0)) * 4, st), "ha_causal_bwd memset");
+    if (!neighbours) HA_CUDA_OK(cudaMemsetAsync(dv_acc, 0, pl.rows_k * p.dv * 4, st), "ha_causal_bwd memset");
   }
   // reference gradient convention: every part uses sum(o_part * dO) of its own output (its d(lse) is dropped);
   // exact convention: sum(o * dO) of the merged output, computed once
@@ -576,11 +589,8 @@ int ha_causal_bwd_strided(const ha_causal_params* pp, const int64_t* strides, vo
     if (rc != HA_OK) return rc;
   }
   if (p.dtype == HA_FP32) return HA_OK;
-  rc = ha_cast_from_f32(dq_acc, p.dq, pl.rows * p.d, p.dtype, stream);
-  if (rc != HA_OK) return rc;
-  rc = ha_cast_from_f32(dk_acc, p.dk, pl.rows_k * p.d, p.dtype, stream);
-  if (rc != HA_OK) return rc;
-  return ha_cast_from_f32(dv_acc, p.dv_out, pl.rows_k * p.dv, p.dtype, stream);
+  const CastJob jobs[3] = {{dq_acc, p.dq, pl.rows * p.d}, {dk_acc, p.dk, pl.rows_k * p.d}, {dv_acc, p.dv_out, pl.rows_k * p.dv}};
+  return cast_grads(jobs, 3, p.dtype, stream);
 }
 
 int ha_causal_bwd(const ha_causal_params* p, void* stream) { return ha_causal_bwd_strided(p, nullptr, stream); }
@@ -594,13 +604,6 @@ int ha_causal_bwd(const ha_causal_params* p, void* stream) { return ha_causal_bw
  * saved: q_idx | k_idx.  scratch: forward = codes of q and k + sort workspace; backward = delta + slot buffers / fp32
  * accumulators as the backward kernel needs them.
  * --------------------------------------------------------------------------------------------------------------- */
-// dk | dv accumulators -> typed gradients: one cast where both pairs are adjacent
-static int cast_kv(const float* dk_acc, const float* dv_acc, void* dk, void* dv, long long count_k, long long count_v, int dtype, void* stream) {
-  if (dv_acc == dk_acc + count_k && (uint8_t*)dv == (uint8_t*)dk + count_k * dtype_size(dtype)) return ha_cast_from_f32(dk_acc, dk, count_k + count_v, dtype, stream);
-  const int rc = ha_cast_from_f32(dk_acc, dk, count_k, dtype, stream);
-  return rc != HA_OK ? rc : ha_cast_from_f32(dv_acc, dv, count_v, dtype, stream);
-}
-
 static int noncausal_check(const ha_causal_params& p, long long& rows, long long& rows_k) {
   if (p.dtype != HA_BF16 && p.dtype != HA_FP16 && p.dtype != HA_FP32) return HA_ERR_DTYPE;
   if (p.B <= 0 || p.H <= 0 || p.n <= 0 || p.d <= 0 || p.dv <= 0 || p.d > 256 || p.dv > 256) return HA_ERR_INVALID;
@@ -738,7 +741,8 @@ int ha_noncausal_bwd_ext(const ha_causal_params* pp, const int64_t* strides, con
     HA_CUDA_OK(cudaMemsetAsync(a.dk_acc, 0, align256(rows_k * p.d * 4) + rows_k * p.dv * 4, st), "ha_noncausal_bwd memset");
     rc = ws_attn_bwd(a, false, st);
     if (rc != HA_OK) return rc;
-    return cast_kv(a.dk_acc, a.dv_acc, p.dk, p.dv_out, rows_k * p.d, rows_k * p.dv, p.dtype, stream);
+    const CastJob jobs[2] = {{a.dk_acc, p.dk, rows_k * p.d}, {a.dv_acc, p.dv_out, rows_k * p.dv}};
+    return cast_grads(jobs, 2, p.dtype, stream);
   }
   if (level >= 1) {
     const long long segs = (long long)p.B * p.H;
@@ -774,11 +778,8 @@ int ha_noncausal_bwd_ext(const ha_causal_params* pp, const int64_t* strides, con
   rc = ha_attn_bwd(&a, stream);
   if (rc != HA_OK) return rc;
   if (p.dtype == HA_FP32) return HA_OK;
-  rc = ha_cast_from_f32(a.dq_acc, p.dq, rows * p.d, p.dtype, stream);
-  if (rc != HA_OK) return rc;
-  rc = ha_cast_from_f32(a.dk_acc, p.dk, rows_k * p.d, p.dtype, stream);
-  if (rc != HA_OK) return rc;
-  return ha_cast_from_f32(a.dv_acc, p.dv_out, rows_k * p.dv, p.dtype, stream);
+  const CastJob jobs[3] = {{a.dq_acc, p.dq, rows * p.d}, {a.dk_acc, p.dk, rows_k * p.d}, {a.dv_acc, p.dv_out, rows_k * p.dv}};
+  return cast_grads(jobs, 3, p.dtype, stream);
 }
 
 int ha_noncausal_bwd(const ha_causal_params* p, void* stream) { return ha_noncausal_bwd_ext(p, nullptr, nullptr, stream); }
@@ -837,9 +838,10 @@ int ha_flash_bwd(const ha_attn_params* pp, void* dq, void* dk, void* dv, void* s
     rc = ws_attn_bwd(a, false, st);
   } else {
     rc = ha_attn_bwd(&a, stream);
-    if (rc == HA_OK) rc = ha_cast_from_f32(a.dq_acc, dq, rows * a.d, a.dtype, stream);
   }
-  return rc != HA_OK ? rc : cast_kv(a.dk_acc, a.dv_acc, dk, dv, rows_k * a.d, rows_k * a.dv, a.dtype, stream);
+  if (rc != HA_OK) return rc;
+  const CastJob jobs[3] = {{a.dq_acc, dq, rows * a.d}, {a.dk_acc, dk, rows_k * a.d}, {a.dv_acc, dv, rows_k * a.dv}};
+  return cast_grads(jobs + typed, 3 - typed, a.dtype, stream);
 }
 
 }  // extern "C"

@@ -248,3 +248,14 @@ def test_padding_rows(dtype, B, n, rows, shapes):
     ts = [torch.randn(n, B, h, w, device='cuda').to(dtype).permute(1, 2, 0, 3) for h, w in shapes]
     for t, o in zip(ts, ops._padded(ts, rows)):
         assert o.is_contiguous() and torch.equal(o, torch.nn.functional.pad(t, (0, 0, 0, rows - n)))
+
+
+@pytest.mark.parametrize('dtype', [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize('count,off', [(1, 0), (7, 0), (8, 0), (100003, 0), (4096, 1)])
+def test_cast_from_f32_at_odd_counts(dtype, count, off):
+    """whole chunks, a tail, less than a chunk, an unaligned source: torch's rounding"""
+    from hyperattention_b200 import _lib as L, ops
+    src = torch.randn(count + off, device='cuda')[off:]
+    dst = torch.full((count + 1,), 7., dtype=dtype, device='cuda')
+    L.check(L.load().ha_cast_from_f32(src.data_ptr(), dst.data_ptr(), count, ops._DT[dtype], ops._stream()), 'ha_cast_from_f32')
+    assert torch.equal(dst[:count], src.to(dtype)) and dst[count] == 7.
