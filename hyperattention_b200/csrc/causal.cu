@@ -211,16 +211,19 @@ struct SavedLayout {
 // utils.py:82-88 of the reference: weights rounded to the tensors' dtype, the merged row rounded after every step), in
 // the same order.  The rectangle launches then run as plain calls that write their part and read nothing back, which
 // costs them a third less time than merging in their epilogue (old rows gathered, two outputs stored).
-// One lane per 16-byte chunk of a row; part = depth, leaves last, as in the saved layout.
-template <typename T>
-__global__ void __launch_bounds__(256) merge_parts_kernel(const uint8_t* __restrict__ parts0, long long part_stride_bytes, long long lse_off_bytes,
+// part = depth, leaves last, as in the saved layout.  A lane takes CH 16-byte chunks of a row: with one, every lane working out the
+// row's weights, the pass was bound by instructions.  64 registers a thread keep enough loads on the way, and the parts are read once
+// (streaming loads): 32 heads x 131072 x 64 652 -> 497 us, x 32768 x 128 225 -> 194 us.
+template <typename T, int CH>
+__global__ void __launch_bounds__(256, 4) merge_parts_kernel(const uint8_t* __restrict__ parts0, long long part_stride_bytes, long long lse_off_bytes,
                                                           int levels, int n, int lpr, T* __restrict__ o, int64_t o_sb, int64_t o_sh, int64_t o_sn,
                                                           FastDiv by_heads, int H, float* __restrict__ lse, long long total_rows, int exact, int log2n) {
+  constexpr int PG = 2;   // parts whose rows are requested together
   const int lane = threadIdx.x & 31;
   const int rpw = 32 / lpr, chunk = lane % lpr, sub = lane / lpr;
   const long long warp_id = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
-  const int dv = lpr * 8;
+  const int dv = lpr * CH * 8;
   const int step = (int)((n_warps * rpw) % n);
   int i = (int)((warp_id * rpw + sub) % n) - step;
   const int step_bh = (int)((n_warps * rpw) / n);
@@ -231,28 +234,30 @@ __global__ void __launch_bounds__(256) merge_parts_kernel(const uint8_t* __restr
     if (i >= n) { i -= n; ++bh; }
     const long long row = base + sub;
     if (row >= total_rows) continue;
-    auto part_row = [&](int part) { return __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(parts0 + part * part_stride_bytes) + row * dv + chunk * 8)); };
+    auto part_row = [&](int part, int c) { return __ldcs(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(parts0 + part * part_stride_bytes) + row * dv) + chunk + c * lpr); };
     auto part_lse = [&](int part) { return __ldg(reinterpret_cast<const float*>(parts0 + part * part_stride_bytes + lse_off_bytes) + row); };
     // every part this row needs is requested before the first merge
-    uint4 cur = part_row(levels);
-    float l1 = part_lse(levels);
-    for (int l0 = levels - 1; l0 >= 0; l0 -= 4) {
-      uint4 nw[4];
-      float l2[4];
-      bool need[4];
+    uint4 cur[CH];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+    for (int c = 0; c < CH; ++c) cur[c] = part_row(levels, c);
+    float l1 = part_lse(levels);
+    for (int l0 = levels - 1; l0 >= 0; l0 -= PG) {
+      uint4 nw[PG][CH];
+      float l2[PG];
+      bool need[PG];
+#pragma unroll
+      for (int j = 0; j < PG; ++j) {
         const int l = l0 - j;
         need[j] = l >= 0 && half_bit(i, n, l, log2n);
-        nw[j] = make_uint4(0, 0, 0, 0);
         l2[j] = 0.f;
         if (need[j]) {
-          nw[j] = part_row(l);
+#pragma unroll
+          for (int c = 0; c < CH; ++c) nw[j][c] = part_row(l, c);
           l2[j] = part_lse(l);
         }
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < PG; ++j) {
         if (!need[j]) continue;
         float w1, w2, lm;
         if (exact) {
@@ -267,19 +272,24 @@ __global__ void __launch_bounds__(256) merge_parts_kernel(const uint8_t* __restr
           w2 = round_to<T>(1.f - cf);
           lm = l1 - __logf(cf + 1.1920929e-07f);
         }
-        const uint32_t ow[4] = {cur.x, cur.y, cur.z, cur.w}, pw[4] = {nw[j].x, nw[j].y, nw[j].z, nw[j].w};
-        uint32_t w[4];
 #pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          const float2 old = unpack2<T>(ow[h]), mine = unpack2<T>(pw[h]);
-          w[h] = pack2<T>(w1 * old.x + w2 * mine.x, w1 * old.y + w2 * mine.y);
+        for (int c = 0; c < CH; ++c) {
+          const uint32_t ow[4] = {cur[c].x, cur[c].y, cur[c].z, cur[c].w}, pw[4] = {nw[j][c].x, nw[j][c].y, nw[j][c].z, nw[j][c].w};
+          uint32_t w[4];
+#pragma unroll
+          for (int h = 0; h < 4; ++h) {
+            const float2 old = unpack2<T>(ow[h]), mine = unpack2<T>(pw[h]);
+            w[h] = pack2<T>(w1 * old.x + w2 * mine.x, w1 * old.y + w2 * mine.y);
+          }
+          cur[c] = make_uint4(w[0], w[1], w[2], w[3]);
         }
-        cur = make_uint4(w[0], w[1], w[2], w[3]);
         l1 = lm;
       }
     }
     const int b = by_heads(bh);
-    *reinterpret_cast<uint4*>(o + b * o_sb + (bh - b * H) * o_sh + i * o_sn + chunk * 8) = cur;
+    uint4* out = reinterpret_cast<uint4*>(o + b * o_sb + (bh - b * H) * o_sh + i * o_sn) + chunk;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) out[c * lpr] = cur[c];
     if (chunk == 0) lse[row] = l1;
   }
 }
@@ -477,18 +487,20 @@ int ha_causal_fwd_strided(const ha_causal_params* pp, const int64_t* strides, vo
     if (rc != HA_OK) return rc;
   }
   if (deferred) {
-    const int lpr = p.dv / 8;
+    const int ch = p.dv >= 16 ? 2 : 1, lpr = p.dv / (8 * ch);
     const long long per_cta = 8LL * (32 / lpr) * 8;
     const long long want = (pl.rows + per_cta - 1) / per_cta;
     const int grid = (int)(want < 148LL * 16 ? want : 148LL * 16);
     const long long part_stride = slot_stride, lse_off = slot_lse;
     const int exact_merge = (p.flags & HA_FLAG_MERGE_EXACT) ? 1 : 0;
-    if (p.dtype == HA_BF16)
-      merge_parts_kernel<__nv_bfloat16><<<grid, 256, 0, main_st>>>((const uint8_t*)slots, part_stride, lse_off, p.levels, p.n, lpr,
-                                                                  (__nv_bfloat16*)p.o, lay.o[0], lay.o[1], lay.o[2], FastDiv(p.H), p.H, p.lse, pl.rows, exact_merge, log2_if_pow2(p.n));
-    else
-      merge_parts_kernel<__half><<<grid, 256, 0, main_st>>>((const uint8_t*)slots, part_stride, lse_off, p.levels, p.n, lpr, (__half*)p.o,
-                                                           lay.o[0], lay.o[1], lay.o[2], FastDiv(p.H), p.H, p.lse, pl.rows, exact_merge, log2_if_pow2(p.n));
+#define HA_MERGE(TT, CH)                                                                                                                               \
+  merge_parts_kernel<TT, CH><<<grid, 256, 0, main_st>>>((const uint8_t*)slots, part_stride, lse_off, p.levels, p.n, lpr, (TT*)p.o, lay.o[0], lay.o[1],  \
+                                                        lay.o[2], FastDiv(p.H), p.H, p.lse, pl.rows, exact_merge, log2_if_pow2(p.n))
+    if (p.dtype == HA_BF16 && ch == 2) HA_MERGE(__nv_bfloat16, 2);
+    else if (p.dtype == HA_BF16) HA_MERGE(__nv_bfloat16, 1);
+    else if (ch == 2) HA_MERGE(__half, 2);
+    else HA_MERGE(__half, 1);
+#undef HA_MERGE
     HA_LAUNCHED("ha_causal_fwd merge");
   }
   return HA_OK;
