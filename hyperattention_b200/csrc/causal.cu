@@ -87,8 +87,7 @@ static int make_plan(const ha_causal_params& p, CausalPlan& pl) {
 
 // delta of every part in one pass: dO is read once per row; the leaf part is needed by every row, the rectangle of
 // depth l only by rows in the second half of their span.  Output delta[part][B*H*n], part = depth, leaves last.
-// Both multi-part passes below are bound by instruction issue, not by DRAM (ncu: issue slots 67-71% busy at 28-35% of the
-// DRAM rate), so the index arithmetic is kept off the loop: a row's position inside its head advances by a constant
+// Both multi-part passes below were bound by instruction issue before DRAM, so the index arithmetic is kept off the loop: a row's position inside its head advances by a constant
 // from one iteration to the next (one conditional subtraction instead of a 64-bit modulo), and with n a power of two
 // (log2n >= 0) the half-span test of a depth is a shift instead of a division.
 __device__ __forceinline__ int half_bit(int i, int n, int depth, int log2n) {
@@ -101,90 +100,79 @@ static int log2_if_pow2(int n) {
   return l;
 }
 
+// A lane takes CH 16-byte chunks of a row (half the shuffles of one chunk a lane), PG parts' rows are requested together, and the parts are
+// read once (streaming loads).  32 heads x 131072 x 64, 7 parts: 802 -> 509 us; 32 x 8192 x 128, 3 parts: 69 -> 48 us.  (PG = 2:
+// 529 us; three CTAs an SM without the few spills: 566 us.)
 template <typename T, int EPC>
-__global__ void __launch_bounds__(256) delta_parts_kernel(const T* __restrict__ d_o, const uint8_t* __restrict__ parts0, long long part_stride_bytes,
-                                                          int levels, int n, int lpr, float* __restrict__ delta, long long total_rows,
-                                                          int log2n) {
+__global__ void __launch_bounds__(256, 4) delta_parts_kernel(const T* __restrict__ d_o, const uint8_t* __restrict__ parts0, long long part_stride_bytes,
+                                                             int levels, int n, int lpr, float* __restrict__ delta, long long total_rows,
+                                                             int log2n) {
+  constexpr int CH = 2, PG = 4;
   const int lane = threadIdx.x & 31;
   const int rpw = 32 / lpr, chunk = lane % lpr, sub = lane / lpr;
   const long long warp_id = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long n_warps = ((long long)gridDim.x * blockDim.x) >> 5;
-  const int dv = lpr * EPC;
-  constexpr int UN = 2;   // row groups per iteration
-  constexpr int PG = 4;   // parts whose rows are requested together: UN * (PG + 1) independent 16-byte loads in flight per lane
-  const int step = (int)((n_warps * rpw * UN) % n);
-  int i[UN];
+  const int chunks = lpr * CH;
+  const int step = (int)((n_warps * rpw) % n);
+  int i = (int)((warp_id * rpw + sub) % n);
+  for (long long base = warp_id * rpw; base < total_rows; base += n_warps * rpw) {
+    const long long row = base + sub;
+    const bool ok = row < total_rows;
+    const long long at = row * chunks + chunk;
+    float gf[CH][8];      // this lane's dO elements, unpacked once for all parts
 #pragma unroll
-  for (int u = 0; u < UN; ++u) i[u] = (int)((warp_id * rpw * UN + u * rpw + sub) % n);
-  for (long long base = warp_id * rpw * UN; base < total_rows; base += n_warps * rpw * UN) {
-    long long row[UN];
-    bool ok[UN];
-    uint4 g[UN];
-#pragma unroll
-    for (int u = 0; u < UN; ++u) {
-      row[u] = base + u * rpw + sub;
-      ok[u] = row[u] < total_rows;
-      g[u] = make_uint4(0, 0, 0, 0);
-      if (ok[u]) g[u] = __ldg(reinterpret_cast<const uint4*>(d_o + row[u] * dv + chunk * EPC));
-    }
-    float gf[UN][8];      // this lane's dO elements, unpacked once for all parts
-#pragma unroll
-    for (int u = 0; u < UN; ++u) {
-      const uint32_t gw[4] = {g[u].x, g[u].y, g[u].z, g[u].w};
+    for (int c = 0; c < CH; ++c) {
+      const uint4 g = ok ? __ldg(reinterpret_cast<const uint4*>(d_o) + at + c * lpr) : make_uint4(0, 0, 0, 0);
+      const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         if constexpr (EPC == 8) {
           const float2 fg = unpack2<T>(gw[w]);
-          gf[u][2 * w] = fg.x;
-          gf[u][2 * w + 1] = fg.y;
+          gf[c][2 * w] = fg.x;
+          gf[c][2 * w + 1] = fg.y;
         } else {
-          gf[u][w] = __uint_as_float(gw[w]);
+          gf[c][w] = __uint_as_float(gw[w]);
         }
       }
     }
     for (int part0 = 0; part0 <= levels; part0 += PG) {
-      bool need[PG][UN];
-      uint4 a[PG][UN];
+      bool need[PG];
+      uint4 a[PG][CH];
 #pragma unroll
       for (int pp = 0; pp < PG; ++pp) {
         const int part = part0 + pp;
+        need[pp] = part <= levels && ok && (part == levels || half_bit(i, n, part, log2n));
 #pragma unroll
-        for (int u = 0; u < UN; ++u) {
-          need[pp][u] = part <= levels && ok[u] && (part == levels || half_bit(i[u], n, part, log2n));
-          a[pp][u] = make_uint4(0, 0, 0, 0);
-          if (need[pp][u])
-            a[pp][u] = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(parts0 + part * part_stride_bytes) + row[u] * dv + chunk * EPC));
+        for (int c = 0; c < CH; ++c) {
+          a[pp][c] = make_uint4(0, 0, 0, 0);
+          if (need[pp]) a[pp][c] = __ldcs(reinterpret_cast<const uint4*>(parts0 + part * part_stride_bytes) + at + c * lpr);
         }
       }
 #pragma unroll
       for (int pp = 0; pp < PG; ++pp) {
-        const int part = part0 + pp;
+        // a warp's rows are consecutive: they nearly always need the same parts, and a part nobody needs is skipped whole
+        if (!__any_sync(0xffffffffu, need[pp])) continue;
+        float s = 0.f;
 #pragma unroll
-        for (int u = 0; u < UN; ++u) {
-          // a warp's rows are consecutive: they nearly always need the same parts, and a part nobody needs is skipped whole
-          if (!__any_sync(0xffffffffu, need[pp][u])) continue;
-          float s = 0.f;
-          const uint32_t aw[4] = {a[pp][u].x, a[pp][u].y, a[pp][u].z, a[pp][u].w};
+        for (int c = 0; c < CH; ++c) {
+          const uint32_t aw[4] = {a[pp][c].x, a[pp][c].y, a[pp][c].z, a[pp][c].w};
 #pragma unroll
           for (int w = 0; w < 4; ++w) {
             if constexpr (EPC == 8) {
               const float2 fa = unpack2<T>(aw[w]);
-              s = fmaf(fa.x, gf[u][2 * w], s);
-              s = fmaf(fa.y, gf[u][2 * w + 1], s);
+              s = fmaf(fa.x, gf[c][2 * w], s);
+              s = fmaf(fa.y, gf[c][2 * w + 1], s);
             } else {
-              s = fmaf(__uint_as_float(aw[w]), gf[u][w], s);
+              s = fmaf(__uint_as_float(aw[w]), gf[c][w], s);
             }
           }
-          for (int off = lpr >> 1; off >= 1; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-          if (need[pp][u] && chunk == 0) delta[(long long)part * total_rows + row[u]] = s;
         }
+        for (int off = lpr >> 1; off >= 1; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+        if (need[pp] && chunk == 0) delta[(long long)(part0 + pp) * total_rows + row] = s;
       }
     }
-#pragma unroll
-    for (int u = 0; u < UN; ++u) {
-      i[u] += step;
-      if (i[u] >= n) i[u] -= n;
-    }
+    i += step;
+    if (i >= n) i -= n;
   }
 }
 
@@ -554,8 +542,8 @@ int ha_causal_bwd_strided(const ha_causal_params* pp, const int64_t* strides, vo
   // exact convention: sum(o * dO) of the merged output, computed once
   bool fused_parts = false;
   if (p.keep_parts && Layout::contiguous(lay.g, p)) {
-    const int es = dtype_size(p.dtype), epc = 16 / es, lpr = p.dv / epc;
-    if (p.dv % epc == 0 && (lpr == 2 || lpr == 4 || lpr == 8 || lpr == 16 || lpr == 32) && (uintptr_t)p.d_o % 16 == 0) {
+    const int es = dtype_size(p.dtype), epc = 16 / es, lpr = p.dv / (2 * epc);
+    if (p.dv % (2 * epc) == 0 && (lpr == 1 || lpr == 2 || lpr == 4 || lpr == 8 || lpr == 16) && (uintptr_t)p.d_o % 16 == 0) {
       const long long part_stride = (uint8_t*)sv.part_o(1) - (uint8_t*)sv.part_o(0);
       const long long per_cta = 8LL * (32 / lpr) * 2;
       long long want = (pl.rows + per_cta - 1) / per_cta;
