@@ -259,3 +259,21 @@ def test_cast_from_f32_at_odd_counts(dtype, count, off):
     dst = torch.full((count + 1,), 7., dtype=dtype, device='cuda')
     L.check(L.load().ha_cast_from_f32(src.data_ptr(), dst.data_ptr(), count, ops._DT[dtype], ops._stream()), 'ha_cast_from_f32')
     assert torch.equal(dst[:count], src.to(dtype)) and dst[count] == 7.
+
+
+def test_host_streams_hand_their_streams_on():
+    """a triple of streams serves one HostStream at a time and then the next one"""
+    import hyperattention_b200 as ha
+    from hyperattention_b200.host import HostStream
+    mod = ha.HyperAttention(input_dim=64, min_seq_len=128, sample_size=128, rng=torch.Generator().manual_seed(3)).to(device='cuda', dtype=torch.bfloat16)
+    q, k, v = [torch.randn(1, 4, 512, 64, dtype=torch.bfloat16).pin_memory() for _ in range(3)]
+    a, b = HostStream(mod), HostStream(mod)
+    oa, ob = a.forward(q, k, v), b.forward(k, q, v)
+    torch.cuda.synchronize()
+    first, other = a._streams, b._streams
+    assert not set(first) & set(other)
+    del a
+    c = HostStream(mod)
+    oc = c.forward(q, k, v)
+    torch.cuda.synchronize()
+    assert c._streams == first and torch.equal(oa, oc) and not torch.equal(oa, ob)
