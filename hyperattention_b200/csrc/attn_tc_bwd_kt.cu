@@ -19,6 +19,10 @@
 // one elected lane issuing from warp-uniform code), three loader warps: Q with lse and delta (ring of three units; also works out the
 // items), dO (ring of three), V and K tiles.
 // TMEM columns: stage s at 128 s: S^T (then P^T) in [0, 64), dP^T (then dQ^T) in [64, 128); dV 256, dK 384.
+// What bounds it: dQ's additions, 64 KB a pair of 128 x 128 tiles.  Scattered, they hold the load/store unit, and with it the loaders (32 heads x
+// 32768, hyper: 1.06 ms, 4600 cycles a pair-half; the kernel that walked query tiles per key tile with dQ, P and dS through shared
+// memory took 1.68 ms).  Consecutive rows, staged and added by the copy engine, are bound by L2 (8 heads x 32768, exact causal: 5.87 ms,
+// 57% of the tensor rate; added from registers 6.27 ms).
 // Hand-offs are mbarriers with bounded waits; a wait that gives up raises the CTA's abort flag, every role leaves its loop at its
 // next wait, and the status words are set at the end.
 #include "attn_items.cuh"
