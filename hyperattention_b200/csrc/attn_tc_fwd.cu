@@ -3,11 +3,13 @@
 //
 // One CTA of 640 threads per SM walks work items; an item is a PAIR of 128-row query tiles of one segment and the list of
 // key tiles the two pair with (AttnItem): every key tile is fetched once for both.  Roles:
-//   * softmax groups 0 / 1 (128 threads each; thread = query row = TMEM lane) of the pair's two query tiles: maximum of the row's 128
-//     scores, then P = exp2(S - reference) back to TMEM in the input dtype and the row's sum.  The reference only moves when
-//     the running maximum has grown by more than 8 (powers of two) beyond it -- any reference gives the same quotient, and
-//     P <= 2^8 is far from either dtype's limits -- so that the accumulator, which lives in TMEM, is hardly ever rescaled; the
-//     group whose reference moved does it, row by row.
+//   * softmax groups 0 / 1 (128 threads each; thread = query row = TMEM lane) of the pair's two query tiles: maximum of the row's 64
+//     scores of a unit, then P = exp2(S - running maximum) back to TMEM in the input dtype and the row's sum.  The accumulator lives in
+//     TMEM; the group whose maximum grew rescales it row by row once its P is stored (the product before has had that long to
+//     complete).  The reference is the exact maximum on purpose: the largest weight of a row is then 1, which a 16-bit P holds
+//     without rounding.  A reference that lags (up to 2^8) saves most of the rescaling -- 32 x 131072 forward 1.06 instead
+//     of 1.14 ms, 16 x 16384 causal 0.58 instead of 0.61 -- but its outputs are 2 to 6% further from 64 bits (32 x 4096: 2.30e-3 instead of
+//     2.17e-3).
 //   * epilogue group (128 threads): O of a finished query tile -> registers -> normalised, merged with the rows already stored
 //     if the call asks for it, stored.  The softmax groups are meanwhile in the next item.
 //   * four MMA warps, S = Q K^T and O += P V of either group, one elected lane issuing from warp-uniform code (descriptors in
@@ -49,7 +51,6 @@ constexpr int ND = 4;                 // descriptor ring
 constexpr int CONSUMERS = 19;         // warps that read every descriptor (all but the one that writes it)
 enum { B_KV_FULL = 0, B_KV_EMPTY = 8, B_Q_FULL = 16, B_Q_EMPTY = 20, B_S_READY = 24, B_PV_DONE = 30, B_O_FULL = 36, B_P_READY = 38, B_O_FREE = 44,
        B_STAT = 46, B_D_FULL = 48, B_D_EMPTY = 48 + ND, N_BARS = 48 + 2 * ND };      // (S ready, P ready, product done: 3 g + buffer)
-constexpr float REF_SLACK = 8.f;
 }  // namespace fw
 
 struct FwdMaps { CUtensorMap tile[3], rows[2]; };    // tiles of q, k, v; rows of q, k
@@ -192,33 +193,12 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
           mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
         }
         const float m_cand = WT ? mx * scale2 + bias2 : mx * scale2;
-        const bool move = m_cand > m_ref + REF_SLACK;        // (the first visible unit always: -inf + 8)
+        const bool move = m_cand > m_ref;
         float alpha = 1.f;
-        if (__any_sync(0xffffffffu, move)) {
-          const float m_new = move ? m_cand : m_ref;
-          if (move) alpha = fast_exp2(m_ref - m_new);        // m_ref = -inf -> 0
-          m_ref = m_new;
-          if (a > 0) {
-            // O is complete up to the previous unit: rescale it
-            const uint32_t pb = buf == 0 ? NB - 1 : buf - 1;
-            if (!(ok = wait(B_PV_DONE + 3 * g + pb, buf == 0 ? par ^ 1 : par))) break;
-            tc_fence_after();
-            const uint64_t al2 = pack_f2(alpha, alpha);
-#pragma unroll 1
-            for (int c = 0; c < DV / 16; ++c) {
-              uint32_t r[16];
-              tmem_ld16(tO + c * 16, r);
-              tmem_ld_fence16(r);
-#pragma unroll
-              for (int i = 0; i < 16; i += 2) {
-                float x, y;
-                unpack_f2(fmul2(pack_u2(r[i], r[i + 1]), al2), x, y);
-                r[i] = __float_as_uint(x);
-                r[i + 1] = __float_as_uint(y);
-              }
-              tmem_st16(tO + c * 16, r);
-            }
-          }
+        const bool moved = __any_sync(0xffffffffu, move);
+        if (move) {
+          alpha = fast_exp2(m_ref - m_cand);
+          m_ref = m_cand;
         }
         HA_T_MARK(2)
         const float m_use = m_ref == -INFINITY ? 0.f : m_ref;
@@ -246,6 +226,31 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
           tmem_st8(tS + c * 8, pk);
         }
         HA_T_MARK(3)
+        if (moved && a > 0) {
+          // O is complete up to the previous unit: rescale it
+          const uint32_t pb = buf == 0 ? NB - 1 : buf - 1;
+          if (!(ok = wait(B_PV_DONE + 3 * g + pb, buf == 0 ? par ^ 1 : par))) break;
+          tc_fence_after();
+          const uint64_t al2 = pack_f2(alpha, alpha);
+#pragma unroll 1
+          for (int c = 0; c < DV / 64; ++c) {
+            uint32_t(&r0)[32] = *reinterpret_cast<uint32_t(*)[32]>(s);
+            uint32_t(&r1)[32] = *reinterpret_cast<uint32_t(*)[32]>(s + 32);
+            tmem_ld32(tO + c * 64, r0);
+            tmem_ld32(tO + c * 64 + 32, r1);
+            tmem_ld_fence(r0);
+            tmem_ld_fence(r1);
+#pragma unroll
+            for (int i = 0; i < 64; i += 2) {
+              float x, y;
+              unpack_f2(fmul2(pack_u2(s[i], s[i + 1]), al2), x, y);
+              s[i] = __float_as_uint(x);
+              s[i + 1] = __float_as_uint(y);
+            }
+            tmem_st32(tO + c * 64, r0);
+            tmem_st32(tO + c * 64 + 32, r1);
+          }
+        }
         tmem_st_wait();
         tc_fence_before();
         mbar_arrive(bar(B_P_READY + 3 * g + buf));

@@ -32,8 +32,8 @@ KT_ROLES = {0: ('elementwise group 0', ['loop, item set-up', 'wait S^T / dP^T re
             6: ('dQ warp', KT_ISSUE), 7: ('Q loader', LOAD)}
 
 # attn_tc_fwd_kernel
-FWD_ROLES = {0: ('softmax group 0', ['loop, item set-up', 'wait S ready', 'scores out of TMEM, maximum, rescale', 'exponentials, P, sum',
-                                     'P store wait, arrival']),
+FWD_ROLES = {0: ('softmax group 0', ['loop, item set-up', 'wait S ready', 'scores out of TMEM, maximum', 'exponentials, P, sum',
+                                     'rescale, P store wait, arrival']),
              1: ('S warp of group 0', ['loop, item set-up', 'wait K tile', 'wait score buffer free', 'issue', 'tile done']),
              6: ('P V warp of group 0', ['loop, item set-up', 'wait V tile', 'wait P ready', 'issue', 'tile done']),
              2: ('K loader', ['index loads', 'wait slot free', 'issue copies']), 3: ('V loader', ['index loads', 'wait slot free', 'issue copies']),

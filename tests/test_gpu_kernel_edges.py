@@ -1,4 +1,6 @@
 """The attention kernels where their tiles, lists of key tiles and loaders change shape, forward and backward, against the oracle."""
+import math
+
 import pytest
 import torch
 
@@ -277,3 +279,24 @@ def test_host_streams_hand_their_streams_on():
     oc = c.forward(q, k, v)
     torch.cuda.synchronize()
     assert c._streams == first and torch.equal(oa, oc) and not torch.equal(oa, ob)
+
+
+@pytest.mark.parametrize('hyper', [False, True])
+@pytest.mark.parametrize('d', [64, 128])
+def test_the_largest_weight_of_a_row_is_exact(d, hyper):
+    """Keys past the first 64 score log(1 + 2^-8) more than those before: weights against the row's maximum are 1 and 0.9961, which a
+    bf16 P holds (to 2e-5), so that a constant V comes back.  Against an earlier, smaller reference they are 1.0039, half a bf16 step
+    above 1."""
+    import hyperattention_b200 as ha
+    n, scale = 1024, math.log1p(2 ** -8)
+    q, k, v = torch.zeros(1, n, 2, d), torch.zeros(1, n, 2, d), torch.ones(1, n, 2, d)
+    q[..., 0] = 1
+    k[:, 64:, :, 0] = 1
+    q, k, v = [t.bfloat16().cuda() for t in (q, k, v)]
+    if hyper:
+        idx = torch.arange(n, device='cuda').view(1, n, 1).expand(1, n, 2)
+        o, lse = ha.hyper_attn_func(q, k, v, idx, idx, 256, 256, scale)
+    else:
+        o, lse = ha.flash_attn_func(q, k, v, None, False, scale)
+        assert rel(lse, torch.full((1, 2, n), math.log(64 + 960 * math.exp(scale)))) < 1e-6
+    assert torch.equal(o, torch.ones_like(o))
