@@ -365,15 +365,21 @@ __device__ __forceinline__ float fast_exp2(float x) {
 }
 
 // 2^x of two values on the FMA and integer pipes, for the share of a softmax's exponentials that the exponential unit (four lanes a clock
-// and scheduler) cannot take: x = n + f with n the nearest integer (Cody-Waite, by adding and subtracting 1.5 * 2^23),
-// 2^f on [-1/2, 1/2] by a degree 5 polynomial with value 1 at 0 whose largest relative error is minimal (found as a linear
-// programme over 4001 Chebyshev points; 1.7e-7 in fp32 arithmetic, the exponential unit's own bound is 2.4e-7), n added to the
-// exponent field.  Arguments below -127, -infinity among them, give 0; arguments are at most about 8 here, 127 in general.
+// and scheduler) cannot take: x = n + f with n the nearest integer (Cody-Waite, by adding and subtracting 1.5 * 2^23 + 127, which
+// leaves n + 127, the exponent field of 2^n, in the low bits), 2^f on [-1/2, 1/2] by a degree 5 polynomial with value 1 at 0 whose
+// largest relative error is minimal (found as a linear programme over 4001 Chebyshev points; 1.7e-7 in fp32 arithmetic, the exponential
+// unit's own bound is 2.4e-7), the two multiplied.  Arguments up to 127; below -127, -infinity among them, they give 0.  A NaN stays
+// one: the clamp hands it on and the product keeps it, whatever its exponent field became.
+__device__ __forceinline__ float max_nan(float a, float b) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+  return d;
+}
 __device__ __forceinline__ void poly_exp2_2(uint64_t x2, float& lo, float& hi) {
   float a, b;
   unpack_f2(x2, a, b);
-  x2 = pack_f2(fmaxf(a, -127.f), fmaxf(b, -127.f));
-  const uint64_t magic = pack_f2(12582912.f, 12582912.f), nmagic = pack_f2(-12582912.f, -12582912.f), mone = pack_f2(-1.f, -1.f);
+  x2 = pack_f2(max_nan(a, -127.f), max_nan(b, -127.f));
+  const uint64_t magic = pack_f2(12583039.f, 12583039.f), nmagic = pack_f2(-12583039.f, -12583039.f), mone = pack_f2(-1.f, -1.f);
   const uint64_t r = fadd2(x2, magic);
   const uint64_t f = ffma2(fadd2(r, nmagic), mone, x2);
   auto c = [](float v) { return pack_f2(v, v); };
@@ -382,11 +388,8 @@ __device__ __forceinline__ void poly_exp2_2(uint64_t x2, float& lo, float& hi) {
   q = ffma2(f, q, c(0x1.ebf9bcp-3f));
   q = ffma2(f, q, c(0x1.62e42ap-1f));
   q = ffma2(f, q, c(1.f));
-  float ra, rb;
-  unpack_f2(r, ra, rb);
-  unpack_f2(q, a, b);
-  lo = __uint_as_float(__float_as_uint(a) + (__float_as_uint(ra) << 23));
-  hi = __uint_as_float(__float_as_uint(b) + (__float_as_uint(rb) << 23));
+  unpack_f2(r, a, b);
+  unpack_f2(fmul2(q, pack_u2(__float_as_uint(a) << 23, __float_as_uint(b) << 23)), lo, hi);
 }
 
 }  // namespace ha

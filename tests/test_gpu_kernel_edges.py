@@ -300,3 +300,21 @@ def test_the_largest_weight_of_a_row_is_exact(d, hyper):
         o, lse = ha.flash_attn_func(q, k, v, None, False, scale)
         assert rel(lse, torch.full((1, 2, n), math.log(64 + 960 * math.exp(scale)))) < 1e-6
     assert torch.equal(o, torch.ones_like(o))
+
+
+@pytest.mark.parametrize('bad', [float('nan'), float('inf')])
+@pytest.mark.parametrize('dtype,d,causal', [(torch.bfloat16, 64, False), (torch.float16, 64, True), (torch.bfloat16, 128, False)])
+def test_a_key_that_is_not_finite_shows_at_every_position(dtype, d, causal, bad):
+    """A NaN key, or one whose score is +infinity, at each of sixteen neighbouring positions (the exponentials of some are polynomials): the
+    rows that see it are not finite, the others are."""
+    import hyperattention_b200 as ha
+    torch.manual_seed(81)
+    n, H, first = 256, 16, 70
+    q, k, v = [torch.randn(1, n, H, d) for _ in range(3)]
+    q[..., 0] = 1
+    for h in range(H):
+        k[0, first + h, h, 0] = bad
+    o, _ = ha.flash_attn_func(*[t.to(dtype).cuda() for t in (q, k, v)], None, causal)
+    sees = torch.arange(n)[:, None] >= first + torch.arange(H) if causal else torch.ones(n, H, dtype=torch.bool)
+    finite = torch.isfinite(o[0].cpu())
+    assert torch.equal(finite.all(-1), ~sees) and torch.equal(finite.any(-1), ~sees)
