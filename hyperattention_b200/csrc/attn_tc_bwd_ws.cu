@@ -57,7 +57,7 @@ enum {
   B_K_EMPTY = 2,      // 2 x 2: the S^T and dQ warps
   B_V_FULL = 4,       // 2 x 32
   B_V_EMPTY = 6,      // 2 x 1: the dP^T warp
-  B_QD_FULL = 8,      // 2 x 32
+  B_QD_FULL = 8,      // 2 x 64: the loader's lanes through their copies, and for what they stored themselves
   B_QD_EMPTY = 10,    // 2 x 4: the S^T, dP^T, dV and dK warps
   B_S_READY = 12,     // 2 x 2: S^T and dP^T of a half are in TMEM
   B_P_READY = 14,     // 2 x 128: its elementwise group has written P^T / dS^T
@@ -80,7 +80,8 @@ __device__ __forceinline__ int bar_count(int i) {
   if (i >= B_D_EMPTY) return CONSUMERS;
   if (i >= B_D_FULL) return 1;
   switch (i >> 1) {
-    case B_K_FULL >> 1: case B_V_FULL >> 1: case B_QD_FULL >> 1: return 32;
+    case B_K_FULL >> 1: case B_V_FULL >> 1: return 32;
+    case B_QD_FULL >> 1: return 64;
     case B_K_EMPTY >> 1: case B_S_READY >> 1: return 2;
     case B_QD_EMPTY >> 1: return 4;
     case B_P_READY >> 1: case B_DQ_FREE >> 1: case B_LDT >> 1: case (B_LDT >> 1) + 1: case B_ACC_FREE >> 1: case B_ST_FULL >> 1: return 128;
@@ -664,6 +665,7 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
           }
         }
         push_copies(full);
+        mbar_arrive(full);       // (the copies' arrivals publish the copies only, not the values of absent rows stored above)
         // the next tile's dO rows into L2 (Q's copies do not mind the latency)
         if (!flash && more) {
           const uint16_t* nb = (const uint16_t*)p.d_o + it.b * p.do_sb + it.h * p.do_sh + (int64_t)it.q_row0 * p.do_sn;

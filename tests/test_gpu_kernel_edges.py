@@ -318,3 +318,24 @@ def test_a_key_that_is_not_finite_shows_at_every_position(dtype, d, causal, bad)
     sees = torch.arange(n)[:, None] >= first + torch.arange(H) if causal else torch.ones(n, H, dtype=torch.bool)
     finite = torch.isfinite(o[0].cpu())
     assert torch.equal(finite.all(-1), ~sees) and torch.equal(finite.any(-1), ~sees)
+
+
+@pytest.mark.parametrize('n,causal', [(130, False), (193, True), (1, False)])
+def test_absent_query_rows_of_many_short_sequences(n, causal):
+    """head dim 64, more sequences than CTAs, the last query tile nearly empty: its absent rows add nothing to any key's gradient, in the
+    first item of a CTA (their slots hold nothing yet) and in later ones (they hold another sequence's)"""
+    import hyperattention_b200 as ha
+    torch.manual_seed(82)
+    q, k, v, do = [torch.randn(2, n, 200, 64).bfloat16() for _ in range(4)]
+    qg, kg, vg = [t.cuda().requires_grad_() for t in (q, k, v)]
+    o, lse = ha.flash_attn_func(qg, kg, vg, None, causal)
+    o.backward(do.cuda())
+    qc, kc, vc = [t.cuda().float().requires_grad_() for t in (q, k, v)]
+    s = T(qc) @ T(kc).transpose(2, 3) * 64 ** -0.5
+    if causal:
+        s = s.masked_fill(torch.ones(n, n, dtype=torch.bool, device='cuda').triu(1), float('-inf'))
+    ow = T(s.softmax(-1) @ T(vc))
+    ow.backward(do.cuda().float())
+    for t, w in ((o, ow), (vg.grad, vc.grad)) + (((qg.grad, qc.grad), (kg.grad, kc.grad)) if n > 1 else ()):
+        per_head = (t.float() - w).norm(dim=(1, 3)) / w.norm(dim=(1, 3))
+        assert per_head.max() < 2e-2, per_head.max()      # (bf16 rounds to 2^-9; gradients are products of three rounded factors)
