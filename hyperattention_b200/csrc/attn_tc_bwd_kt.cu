@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
   __shared__ __align__(16) KtItem s_item[ND];
   __shared__ uint64_t bars[N_BARS];
   __shared__ uint32_t tmem_slot;
+  __shared__ uint32_t s_issued[3];        // units of Q, units of dO, operands of key tiles (V, then K) that the loaders have asked for
   __shared__ int s_abort;
   __shared__ int s_bail;
 
@@ -705,8 +706,9 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
         for (int q = 0; q < 4; ++q) { rows[q] = ahead[q]; l[q] = l_ahead[q]; dl[q] = dl_ahead[q]; }
       }
       HA_T_DUMP(8, (int)blockIdx.x * 8 + 7, lane == 0 && is_q)
+      if (lane == 0) s_issued[warp - W_Q] = n;
       cp_async_commit();
-      cp_async_wait<0>();      // nothing of this warp is in flight when the CTA retires
+      cp_async_wait<0>();
     } else {
       // ===================================================================================================
       // loader of the key side: V and K tiles
@@ -719,7 +721,7 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
       KtItem it;
       bool more = next_item(it);
       int e = more ? it.e0 : 0, rows[4] = {0, 0, 0, 0};
-      uint32_t n = 0;
+      uint32_t n = 0, issued = 0;      // tiles / operands of tiles (V, then K) so far
       HA_T_DECL(8)
       if (more) row_numbers(it, e, rows);
       while (more) {
@@ -752,6 +754,7 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
             warp_gather_tile(dst, base + (int64_t)row0 * sn, sn, 2, r, lane);
             push_copies(full);
           }
+          ++issued;
           if (fetch) {
             const int64_t sn = is_k ? p.k_sn : p.v_sn;
             const uint16_t* nb = (is_k ? (const uint16_t*)p.k + it.b * p.k_sb + it.hk * p.k_sh : (const uint16_t*)p.v + it.b * p.v_sb + it.hk * p.v_sh) + (int64_t)it.k_row0 * sn;
@@ -769,6 +772,7 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
         HA_T_MARK(2)
       }
       HA_T_DUMP(8, (int)blockIdx.x * 8 + 3, lane == 0)
+      if (lane == 0) s_issued[warp - W_Q] = issued;
       cp_async_commit();
       cp_async_wait<0>();
     }
@@ -776,7 +780,29 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
   // every role is done (or has given up); TMEM goes back
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && s_abort) report_timeout(p.status, p.status_host);
+  if (s_abort) {      // (nobody writes it any more)
+    // What is still under way is waited for, with a limit, before TMEM goes and the CTA retires: the last tile of every slot a loader fills, each
+    // MMA warp's products, stores to TMEM.  (The drain group's copies out are through.)  A CTA that gets through its items
+    // has waited for all of it on the way.
+    const uint32_t bar_end = smem_u32(s_item);      // (the descriptors have been used up: their place takes the MMA warps' barriers)
+    if (tid < 5) mbar_init(bar_end + 8 * tid, 1);
+    mbar_fence_init();
+    __syncthreads();
+    if (warp > W_DO) {
+      const uint32_t n = s_issued[2];
+      if (n >= 1) mbar_wait(bar(B_V_FULL), ((n + 1) / 2 - 1) & 1);
+      if (n >= 2) mbar_wait(bar(B_K_FULL), (n / 2 - 1) & 1);
+    } else if (warp >= W_Q) {
+      const uint32_t n = s_issued[warp - W_Q];
+      for (uint32_t back = 1; back <= NU && n >= back; ++back) mbar_wait(bar((warp == W_Q ? B_Q_FULL : B_DO_FULL) + (n - back) % NU), ((n - back) / NU) & 1);
+    } else if (warp >= W_MMA) {
+      mma_settle(bar_end + 8 * (warp - W_MMA));
+    } else {
+      tmem_st_wait();
+    }
+    __syncthreads();
+    if (tid == 0) report_timeout(p.status, p.status_host);
+  }
   if (warp == W_MMA) tmem_dealloc(tmem, 512);
 }
 

@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
   __shared__ __align__(16) AttnItem s_item[ND];
   __shared__ uint64_t bars[N_BARS];
   __shared__ uint32_t tmem_slot;
+  __shared__ uint32_t s_issued[4];        // query tiles 0 and 1, K tiles, V tiles that the loaders have asked for
   __shared__ int s_abort;
   __shared__ int s_bail;
 
@@ -679,8 +680,9 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
         HA_T_MARK(2)
       }
       HA_T_DUMP(8, (int)blockIdx.x * 8 + 7, lane == 0)
+      if (lane == 0) { s_issued[0] = n_y0; s_issued[1] = n_y1; }
       cp_async_commit();
-      cp_async_wait<0>();      // nothing of this warp is in flight when the CTA retires
+      cp_async_wait<0>();
     } else {
       // ===================================================================================================
       // loaders of the key side: K tiles (warp 18), V tiles (warp 19)
@@ -737,6 +739,7 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
         HA_T_MARK(2)
       }
       HA_T_DUMP(8, (int)blockIdx.x * 8 + 3, lane == 0 && !is_v)
+      if (lane == 0) s_issued[2 + is_v] = n;
       cp_async_commit();
       cp_async_wait<0>();
     }
@@ -744,7 +747,28 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
   // every role is done (or has given up); TMEM goes back
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && s_abort) report_timeout(p.status, p.status_host);
+  if (s_abort) {      // (nobody writes it any more)
+    // What is still under way is waited for, with a limit, before TMEM goes and the CTA retires: the last tile of every slot a loader fills, each
+    // MMA warp's products, stores to TMEM.  (The drain group's copies out are through.)  A CTA that gets through its items
+    // has waited for all of it on the way.
+    const uint32_t bar_end = smem_u32(s_item);      // (the descriptors have been used up: their place takes the MMA warps' barriers)
+    if (tid < 5) mbar_init(bar_end + 8 * tid, 1);
+    mbar_fence_init();
+    __syncthreads();
+    if (warp == W_QD) {
+      for (int y = 0; y < 2; ++y)
+        if (s_issued[y] > 0) mbar_wait(bar(B_QD_FULL + y), (s_issued[y] - 1) & 1);
+    } else if (warp > W_QD) {
+      const uint32_t n = s_issued[warp - W_QD + 1];
+      for (uint32_t back = 1; back <= 2 && n >= back; ++back) mbar_wait(bar((warp == W_K ? B_K_FULL : B_V_FULL) + ((n - back) & 1)), ((n - back) >> 1) & 1);
+    } else if (warp >= W_MMA) {
+      mma_settle(bar_end + 8 * (warp - W_MMA));
+    } else {
+      tmem_st_wait();
+    }
+    __syncthreads();
+    if (tid == 0) report_timeout(p.status, p.status_host);
+  }
   if (warp == W_MMA) tmem_dealloc(tmem, 512);
 }
 

@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
   __shared__ __align__(16) AttnItem s_item[ND];
   __shared__ uint64_t bars[N_BARS];
   __shared__ uint32_t tmem_slot;
+  __shared__ uint32_t s_issued[4];        // ring positions the loaders have got to
   __shared__ int s_abort;
   __shared__ int s_bail;
 
@@ -606,14 +607,35 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
         for (int q = 0; q < 4; ++q) rows[q] = ahead[q];
       }
       HA_T_DUMP(8, (int)blockIdx.x * 8 + (is_k ? 2 : is_q ? 4 : 3), lane == 0 && (warp <= W_K + 1))
+      if (lane == 0) s_issued[warp - W_Q] = n;
       cp_async_commit();
-      cp_async_wait<0>();      // nothing of this warp is in flight when the CTA retires
+      cp_async_wait<0>();
     }
   }
   // every role is done (or has given up); TMEM goes back
   tc_fence_before();
   __syncthreads();
-  if (tid == 0 && s_abort) report_timeout(p.status, p.status_host);
+  if (s_abort) {      // (nobody writes it any more)
+    // What is still under way is waited for, with a limit, before TMEM goes and the CTA retires: the last tile of every slot a loader fills,
+    // each MMA warp's products, stores to TMEM.  A CTA that gets through its items has waited for all of it on the way.
+    const uint32_t bar_end = smem_u32(s_item);      // (the descriptors have been used up: their place takes the MMA warps' barriers)
+    if (tid < 4) mbar_init(bar_end + 8 * tid, 1);
+    mbar_fence_init();
+    __syncthreads();
+    if (warp >= W_Q) {
+      const uint32_t ring = warp == W_Q ? NQ : NKV, step = warp == W_Q ? 1 : warp == W_K ? 2 : 4, first = warp <= W_K ? 0 : 2 * (warp & 1) + 1;
+      const uint32_t n = s_issued[warp - W_Q];
+#pragma unroll 1
+      for (uint32_t back = step; back <= ring && n >= first + back; back += step)
+        mbar_wait(bar((warp == W_Q ? B_Q_FULL : B_KV_FULL) + (n - back) % ring), ((n - back) / ring) & 1);
+    } else if (warp >= W_S) {
+      mma_settle(bar_end + 8 * (warp - W_S));
+    } else {
+      tmem_st_wait();
+    }
+    __syncthreads();
+    if (tid == 0) report_timeout(p.status, p.status_host);
+  }
   if (warp == W_S) tmem_dealloc(tmem, 512);
 }
 

@@ -225,6 +225,13 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
+// For a CTA that gave up: waits (bounded) for the products that this warp's elected lane has issued.  `bar`: one arrival, used for nothing else.
+__device__ __forceinline__ void mma_settle(uint32_t bar) {
+  __syncwarp();
+  if (elect_one()) mma_commit(bar);
+  __syncwarp();
+  mbar_wait(bar, 0);
+}
 
 // 32 consecutive fp32 columns of this thread's TMEM lane
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
