@@ -302,6 +302,10 @@ struct Layout {
     set(o, p.H, p.dv);
     set(g, p.H, p.dv);
   }
+  // do the rows of a 16-bit tensor start on 16-byte boundaries?  (a dimension of extent 1 is never stepped through)
+  static bool aligned(const void* base, const int64_t (&s)[3], const ha_causal_params& p) {
+    return (uintptr_t)base % 16 == 0 && s[2] % 8 == 0 && (p.H == 1 || s[1] % 8 == 0) && (p.B == 1 || s[0] % 8 == 0);
+  }
   static bool contiguous(const int64_t (&s)[3], const ha_causal_params& p) {
     return s[2] == p.dv && (p.H == 1 || s[1] == (int64_t)p.n * p.dv) && (p.B == 1 || s[0] == (int64_t)p.n * p.dv * p.H);
   }
@@ -388,6 +392,13 @@ int ha_causal_fwd_strided(const ha_causal_params* pp, const int64_t* strides, vo
   void* sort_ws = (uint8_t*)p.scratch + 2 * align256(pl.rows * 4);
 
   const Layout lay(p, strides);
+  // A call that keeps the parts (16-bit tensors, tensor-core kernels) writes every part straight into its slot and merges
+  // them in one pass at the end; otherwise every rectangle merges into (o, lse) in its epilogue.  The pass stores 16 bytes at a time: an
+  // output whose rows do not start on such boundaries is left to the epilogues.
+  const long long in_scratch = scratch_part_bytes(p, pl);
+  const bool deferred = merges_deferrable(p) && Layout::aligned(p.o, lay.o, p) && (p.keep_parts || in_scratch > 0);
+  // (un-merged rows beside the merged ones have the layout of o: only where that is the slots' own)
+  if (p.keep_parts && !deferred && !Layout::contiguous(lay.o, p)) return HA_ERR_INVALID;
   rc = hash_pair(p.q, lay.q, p.H, codes_q, p.k, lay.k, pl.Hk, codes_k, p.B, p.n, p.d, p.dtype, p.proj, p.lsh_bits, (cudaStream_t)stream);
   if (rc != HA_OK) return rc;
 
@@ -439,20 +450,11 @@ int ha_causal_fwd_strided(const ha_causal_params* pp, const int64_t* strides, vo
   a.flags = HA_FLAG_CAUSAL | (p.flags & HA_FLAG_FORCE_SIMT);
   a.segs_per_head = 1 << p.levels;
   a.span = pl.leaf; a.q_off = 0; a.k_off = 0; a.m_q = pl.leaf; a.m_k = pl.leaf;
-  // A call that keeps the parts (16-bit tensors, tensor-core kernels) writes every part straight into its slot and merges
-  // them in one pass at the end; otherwise every rectangle merges into (o, lse) in its epilogue.
-  const long long in_scratch = scratch_part_bytes(p, pl);
-  const bool deferred = merges_deferrable(p) && (p.keep_parts || in_scratch > 0);
   // the parts' slots: in the saved buffer (kept for the backward) or, for a call that keeps nothing, in the scratch
   uint8_t* const slots = !deferred ? nullptr : p.keep_parts ? (uint8_t*)sv.part_o(0) : (uint8_t*)p.scratch + 2 * align256(pl.rows * 4) + align256(pl.sort_ws);
   const long long slot_stride = align256(pl.part_o_bytes) + align256(pl.part_lse_bytes), slot_lse = align256(pl.part_o_bytes);
   auto slot_o = [&](int part) -> void* { return slots + part * slot_stride; };
   auto slot_lse_of = [&](int part) -> float* { return (float*)(slots + part * slot_stride + slot_lse); };
-  // (un-merged rows beside the merged ones have the layout of o: only where that is the slots' own)
-  if (p.keep_parts && !deferred && !Layout::contiguous(lay.o, p)) {
-    if (side) { cudaStreamWaitEvent(main_st, side->join, 0); side_lock.unlock(); }
-    return HA_ERR_INVALID;
-  }
   if (deferred) { a.o = slot_o(p.levels); a.lse = slot_lse_of(p.levels); a.o_sn = p.dv; a.o_sh = (int64_t)p.n * p.dv; a.o_sb = a.o_sh * p.H; }
   else if (p.keep_parts) { a.part_o = sv.part_o(p.levels); a.part_lse = sv.part_lse(p.levels); }
   rc = ha_attn_fwd(&a, stream);

@@ -262,8 +262,8 @@ int ha_noncausal_bwd(const ha_causal_params* p, void* stream);
 
 /* The same calls on strided tensors.  strides: 15 element strides, (batch, head, row) of q, k, v, o, dO in this order, the last
  * dimension contiguous (dO's are looked at by the backward only); NULL = contiguous.  The gradients stay contiguous.  (A causal
- * call that keeps its parts on the CUDA-core kernels takes a contiguous o only.)  The reference copies its inputs instead
- * (hyper_attention.py:38-40). */
+ * call that keeps its parts takes a strided o only if the merges run as one pass: 16-bit tensors, dv 8, 16, ... 256, o and its
+ * strides multiples of 16 bytes.)  The reference copies its inputs instead (hyper_attention.py:38-40). */
 int ha_causal_fwd_strided(const ha_causal_params* p, const int64_t* strides, void* stream);
 int ha_causal_bwd_strided(const ha_causal_params* p, const int64_t* strides, void* stream);
 /* ... and the non-causal one with sampled rows of the caller's choice: sample_idx (int32 [B*H][sample_size], distinct rows) makes the sampled

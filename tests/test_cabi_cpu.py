@@ -159,3 +159,19 @@ def test_counter_based_sample_indices_agree_with_the_oracle():
         assert torch.equal(idx, want)
         assert int(idx.min()) >= 0 and int(idx.max()) < n and bool((idx[:, 1:] > idx[:, :-1]).all())      # distinct, in range
     assert 0.45 < float(u.float().mean()) / 2 ** 24 < 0.55
+
+
+def test_causal_call_that_keeps_parts_rejects_an_output_it_cannot_store(lib):
+    """the merging pass stores 16 bytes at a time; an o that is strided and not aligned for it has no other path when the parts are kept"""
+    from hyperattention_b200 import _lib
+    p = _lib.CausalParams()
+    p.dtype, p.B, p.H, p.n, p.d, p.dv, p.levels, p.block_size, p.sample_size, p.lsh_bits = _lib.BF16, 1, 2, 1024, 64, 64, 1, 256, 256, 8
+    p.keep_parts, p.min_seq_len, p.scale = 1, 512, 0.125
+    p.q = p.k = p.v = p.proj = p.o = p.lse = p.saved = p.scratch = 256
+    p.saved_bytes, p.scratch_bytes = lib.ha_causal_saved_bytes(C.byref(p)), lib.ha_causal_scratch_bytes(C.byref(p), 0)
+    rows = [2 * 1024 * 64, 1024 * 64, 64]
+    odd = [2 * 1024 * 68, 1024 * 68, 68]
+    assert lib.ha_causal_fwd_strided(C.byref(p), (C.c_int64 * 15)(*rows * 3, *odd, 0, 0, 0), None) == -1
+    p.o = 258
+    wide = [2 * 1024 * 128, 1024 * 128, 128]
+    assert lib.ha_causal_fwd_strided(C.byref(p), (C.c_int64 * 15)(*rows * 3, *wide, 0, 0, 0), None) == -1

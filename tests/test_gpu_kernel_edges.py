@@ -339,3 +339,32 @@ def test_absent_query_rows_of_many_short_sequences(n, causal):
     for t, w in ((o, ow), (vg.grad, vc.grad)) + (((qg.grad, qc.grad), (kg.grad, kc.grad)) if n > 1 else ()):
         per_head = (t.float() - w).norm(dim=(1, 3)) / w.norm(dim=(1, 3))
         assert per_head.max() < 2e-2, per_head.max()      # (bf16 rounds to 2^-9; gradients are products of three rounded factors)
+
+
+@pytest.mark.parametrize('keep,stride,off', [(0, 68, 0), (0, 64, 1), (1, 64, 1), (1, 72, 8)])
+def test_causal_outputs_that_vector_stores_do_not_fit(keep, stride, off):
+    """C entry point: output rows 136 bytes apart, or starting one element into an allocation (no 16-byte boundaries: the merges run in the
+    epilogues), and aligned ones with a gap; against the module's own contiguous call"""
+    import ctypes as C
+    import hyperattention_b200 as ha
+    from hyperattention_b200 import _lib as L, ops
+    torch.manual_seed(83)
+    B, H, n, d = 1, 2, 1024, 64
+    q, k, v = [torch.randn(B, H, n, d, device='cuda').bfloat16() for _ in range(3)]
+    mod = ha.HyperAttention(input_dim=d, min_seq_len=512, sample_size=128, rng=torch.Generator().manual_seed(6)).to(device='cuda', dtype=torch.bfloat16)
+    want, lse_want = mod(q, k, v, causal=True, return_lse=True)
+    mem = torch.full((off + B * H * n * stride + 64,), 7., device='cuda', dtype=torch.bfloat16)
+    o, lse = mem[off:off + B * H * n * stride].view(B, H, n, stride)[..., :d], torch.empty(B, H, n, device='cuda')
+    p, lib = L.CausalParams(), L.load()
+    p.dtype, p.B, p.H, p.n, p.d, p.dv, p.levels, p.block_size, p.sample_size, p.lsh_bits = L.BF16, B, H, n, d, d, 1, 256, 128, 8
+    p.keep_parts, p.min_seq_len, p.scale = keep, 512, d ** -0.5
+    p.q, p.k, p.v, p.o, p.lse, p.proj = [t.data_ptr() for t in (q, k, v, o, lse, mod.lsh.proj_f32())]
+    saved = ops._buffer(p, 'saved', lib.ha_causal_saved_bytes(C.byref(p)), 'cuda')
+    scratch = ops._buffer(p, 'scratch', lib.ha_causal_scratch_bytes(C.byref(p), 0), 'cuda')
+    st = (C.c_int64 * 15)(*q.stride()[:3], *k.stride()[:3], *v.stride()[:3], *o.stride()[:3], 0, 0, 0)
+    L.check(lib.ha_causal_fwd_strided(C.byref(p), st, ops._stream()), 'ha_causal_fwd_strided')
+    assert rel(o, want) < 1e-2 and rel(lse, lse_want[..., 0]) < 1e-4        # (bf16 weights on one side, fp32 ones on the other)
+    gaps = torch.ones_like(mem, dtype=torch.bool)
+    gaps[off:off + B * H * n * stride].view(B, H, n, stride)[..., :d] = False
+    assert (mem[gaps] == 7).all()
+    del saved, scratch
