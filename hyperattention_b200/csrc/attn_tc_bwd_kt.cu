@@ -847,13 +847,8 @@ static int launch_kt_bwd(const ha_attn_params& p, cudaStream_t st) {
              encode_tile_map(&maps.tile[2], p.dtype, p.v, 128, n_k, Hk, p.B, p.v_sn, p.v_sh, p.v_sb, TILE) &&
              (!flash || (encode_tile_map(&maps.tile[0], p.dtype, p.q, 128, n_q, p.H, p.B, p.q_sn, p.q_sh, p.q_sb, bkt::UQ) &&
                          encode_tile_map(&maps.tile[3], p.dtype, p.d_o, 128, n_q, p.H, p.B, p.do_sn, p.do_sh, p.do_sb, bkt::UQ)));
-  static int dyn_bytes = 0;
-  if (dyn_bytes == 0) {
-    cudaFuncAttributes fa;
-    HA_CUDA_OK(cudaFuncGetAttributes(&fa, attn_tc_bwd_kt_kernel<T, KIND>), "ha_attn_bwd kernel attributes");
-    const int stat = ((int)fa.sharedSizeBytes + 15) / 16 * 16;
-    dyn_bytes = (1024 - stat % 1024) % 1024 + bkt::SMEM_USED;
-  }
+  int dyn_bytes;
+  HA_WINDOW_BYTES(dyn_bytes, (attn_tc_bwd_kt_kernel<T, KIND>), bkt::SMEM_USED, "ha_attn_bwd kernel attributes");
   HA_SMEM_ATTR_ONCE((attn_tc_bwd_kt_kernel<T, KIND>), dyn_bytes, "ha_attn_bwd smem attribute");
   const int sms = sm_count();
   attn_tc_bwd_kt_kernel<T, KIND><<<(unsigned)(pl.n_items < sms ? pl.n_items : sms), bkt::THREADS, dyn_bytes, st>>>(p, pl, maps);

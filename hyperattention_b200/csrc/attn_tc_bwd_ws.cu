@@ -814,13 +814,8 @@ static int launch_ws_bwd(const ha_attn_params& p, bool store_dq, cudaStream_t st
       encode_acc_map(&maps.acc[2], p.dk_acc, 64, p.n, (long long)p.B * Hk))
     out.bulk |= 2;
   out.store_dq = store_dq;
-  static int dyn_bytes = 0;
-  if (dyn_bytes == 0) {
-    cudaFuncAttributes fa;
-    HA_CUDA_OK(cudaFuncGetAttributes(&fa, attn_tc_bwd_ws_kernel<T, KIND>), "ha_attn_bwd kernel attributes");
-    const int stat = ((int)fa.sharedSizeBytes + 15) / 16 * 16;
-    dyn_bytes = (1024 - stat % 1024) % 1024 + bws::SMEM_USED;
-  }
+  int dyn_bytes;
+  HA_WINDOW_BYTES(dyn_bytes, (attn_tc_bwd_ws_kernel<T, KIND>), bws::SMEM_USED, "ha_attn_bwd kernel attributes");
   HA_SMEM_ATTR_ONCE((attn_tc_bwd_ws_kernel<T, KIND>), dyn_bytes, "ha_attn_bwd smem attribute");
   const int sms = sm_count();
   attn_tc_bwd_ws_kernel<T, KIND><<<(unsigned)(pl.n_items < sms ? pl.n_items : sms), bws::THREADS, dyn_bytes, st>>>(p, pl, out, maps);

@@ -655,13 +655,8 @@ static int launch_fwd(const ha_attn_params& p, cudaStream_t st) {
              encode_tile_map(&maps.tile[2], p.dtype, p.v, DV, n_k, Hk, p.B, p.v_sn, p.v_sh, p.v_sb, TILE);
   plan_row_maps(pl, p, maps.rows, n_q, n_k);
   // the tiles start at the first 1 KB boundary after the static variables; at head dim 128 they end with the CTA's last byte
-  static int dyn_bytes = 0;
-  if (dyn_bytes == 0) {
-    cudaFuncAttributes fa;
-    HA_CUDA_OK(cudaFuncGetAttributes(&fa, attn_tc_fwd_kernel<T, D, DV, KIND>), "ha_attn_fwd kernel attributes");
-    const int stat = ((int)fa.sharedSizeBytes + 15) / 16 * 16;
-    dyn_bytes = (1024 - stat % 1024) % 1024 + Cfg::SMEM_USED;
-  }
+  int dyn_bytes;
+  HA_WINDOW_BYTES(dyn_bytes, (attn_tc_fwd_kernel<T, D, DV, KIND>), Cfg::SMEM_USED, "ha_attn_fwd kernel attributes");
   HA_SMEM_ATTR_ONCE((attn_tc_fwd_kernel<T, D, DV, KIND>), dyn_bytes, "ha_attn_fwd smem attribute");
   const int sms = sm_count();
   attn_tc_fwd_kernel<T, D, DV, KIND><<<(unsigned)(pl.n_items < sms ? pl.n_items : sms), fw::THREADS, dyn_bytes, st>>>(p, pl, maps);

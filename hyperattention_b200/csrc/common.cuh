@@ -75,6 +75,21 @@ inline int sm_count() {
     }                                                                                                  \
   } while (0)
 
+// Dynamic shared memory of a kernel whose layout of `used` bytes starts at the first 1 KB boundary after its static variables: looked up at the
+// first launch (by whichever host thread comes first; they all find the same).
+#define HA_WINDOW_BYTES(bytes, kernel, used, where)                                                    \
+  do {                                                                                                 \
+    static std::atomic<int> _bytes{0};                                                                 \
+    bytes = _bytes.load(std::memory_order_relaxed);                                                    \
+    if (bytes == 0) {                                                                                  \
+      cudaFuncAttributes _fa;                                                                          \
+      HA_CUDA_OK(cudaFuncGetAttributes(&_fa, kernel), where);                                          \
+      const int _stat = ((int)_fa.sharedSizeBytes + 15) / 16 * 16;                                     \
+      bytes = (1024 - _stat % 1024) % 1024 + (used);                                                   \
+      _bytes.store(bytes, std::memory_order_relaxed);                                                  \
+    }                                                                                                  \
+  } while (0)
+
 // ---------------------------------------------------------------------------------------------------
 // element access
 // ---------------------------------------------------------------------------------------------------

@@ -1,5 +1,6 @@
 """The attention kernels where their tiles, lists of key tiles and loaders change shape, forward and backward, against the oracle."""
 import math
+import os
 
 import pytest
 import torch
@@ -368,3 +369,33 @@ def test_causal_outputs_that_vector_stores_do_not_fit(keep, stride, off):
     gaps[off:off + B * H * n * stride].view(B, H, n, stride)[..., :d] = False
     assert (mem[gaps] == 7).all()
     del saved, scratch
+
+
+def test_first_calls_from_many_threads():
+    """the first launches of a process, made by eight host threads at once on streams of their own: every thread's results are one thread's"""
+    import subprocess
+    import sys
+    code = '''
+import threading, torch, hyperattention_b200 as ha
+torch.manual_seed(0)
+ts = [torch.randn(1, 2, 1024, 64, device='cuda').bfloat16() for _ in range(4)]
+mod = ha.HyperAttention(input_dim=64, min_seq_len=256, sample_size=128, rng=torch.Generator().manual_seed(1)).to(device='cuda', dtype=torch.bfloat16)
+torch.cuda.synchronize()
+out, gate = [None] * 8, threading.Barrier(8)
+def work(i):
+    with torch.cuda.stream(torch.cuda.Stream()):
+        q, k, v = [t.clone().requires_grad_() for t in ts[:3]]
+        gate.wait()
+        o = mod(q, k, v, causal=i % 2 == 0)
+        out[i] = (o.detach(),) + torch.autograd.grad(o, (q, k, v), ts[3])
+        torch.cuda.current_stream().synchronize()
+threads = [threading.Thread(target=work, args=(i,)) for i in range(8)]
+[t.start() for t in threads]
+[t.join() for t in threads]
+for i in range(2, 8):
+    assert torch.equal(out[i][0], out[i % 2][0]), i
+    for a, b in zip(out[i][1:], out[i % 2][1:]):
+        assert (a.float() - b.float()).norm() < 1e-3 * b.float().norm(), i      # (fp32 additions in no fixed order, rounded to bf16)
+ha.check_device_status()
+'''
+    subprocess.run([sys.executable, '-c', code], check=True, timeout=120, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
