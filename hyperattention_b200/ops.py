@@ -637,7 +637,9 @@ class CausalHyperFunc(torch.autograd.Function):
     @staticmethod
     def run(q, k, v, proj_f32, levels, block_size, sample_size, scale, flags, keep_parts, min_seq_len):
         assert q.dtype == k.dtype == v.dtype, 'All tensors must have the same type'
-        n = q.shape[2]
+        B, H, n, d = q.shape
+        assert k.shape[0] == B and k.shape[2:] == (n, d), 'query and key sequence lengths must be equal'
+        assert H % k.shape[1] == 0 and v.shape[:3] == k.shape[:3], 'query heads must be a multiple of the key/value heads'
         if n % 2:
             _cuda(q, k, v)
             q, k, v = _padded((q, k, v), n + 1)

@@ -175,3 +175,14 @@ def test_causal_call_that_keeps_parts_rejects_an_output_it_cannot_store(lib):
     p.o = 258
     wide = [2 * 1024 * 128, 1024 * 128, 128]
     assert lib.ha_causal_fwd_strided(C.byref(p), (C.c_int64 * 15)(*rows * 3, *wide, 0, 0, 0), None) == -1
+
+
+@pytest.mark.parametrize('n', [1024, 1023])
+@pytest.mark.parametrize('k,v', [((1, 2, 0, 64), (1, 2, 0, 64)), ((2, 2, 0, 64), (1, 2, 0, 64)), ((2, 2, 0, 32), (2, 2, 0, 64)), ((2, 2, 0, 64), (2, 1, 0, 64)),
+                                 ((2, 2, 0, 64), (2, 2, -128, 64)), ((2, 3, 0, 64), (2, 3, 0, 64))])
+def test_causal_call_looks_at_every_shape(n, k, v):
+    """batch, heads, rows and width of k and v are compared with q's before anything is read (kernels take them from q)"""
+    from hyperattention_b200 import ops
+    at = lambda s: torch.zeros(s[0], s[1], n + s[2], s[3])
+    with pytest.raises(AssertionError, match='lengths must be equal|multiple of the key'):
+        ops.causal_hyper(torch.zeros(2, 4, n, 64), at(k), at(v), torch.zeros(64, 8), 1, 256, 256, 0.125, 0, True, 512)
