@@ -37,7 +37,8 @@ def _wants_grad(*ts):
 
 
 # Parameter structs of earlier calls by shape, strides and options (everything but the pointers): filling one field by field costs more
-# host time than the launch.  Bounded; entries are immutable bytes.
+# host time than the launch.  Bounded; entries are immutable bytes, keys are plain values (a tensor or array as the scale would be found by its
+# identity, whatever it holds by then: callers of _flash_params and _plan turn it into a float).
 _TEMPLATES = {}
 
 
@@ -433,7 +434,7 @@ def _flash_forward(q, k, v, causal, softmax_scale, flags):
     assert q.dtype == k.dtype == v.dtype, 'All tensors must have the same type'
     o = _rows_like(q.transpose(1, 2), v.shape[-1]).transpose(1, 2)
     lse = torch.empty(B, H, nq, dtype=torch.float32, device=q.device)
-    p = _flash_params(q, k, v, o, lse, causal, softmax_scale or 1.0 / math.sqrt(d), flags)
+    p = _flash_params(q, k, v, o, lse, causal, float(softmax_scale or 1.0 / math.sqrt(d)), flags)
     L.check(_call(L.load().ha_attn_fwd, q.device, C.byref(p)), 'ha_attn_fwd')
     return o, lse
 
@@ -449,7 +450,7 @@ class FlashAttnFunc(torch.autograd.Function):
         q, k, v = [x if x.stride(-1) == 1 else x.contiguous() for x in (q, k, v)]
         o, lse = _flash_forward(q, k, v, causal, softmax_scale, flags)
         ctx.save_for_backward(q, k, v, o, lse)
-        ctx.cfg = (causal, softmax_scale or 1.0 / math.sqrt(q.shape[-1]), flags)
+        ctx.cfg = (causal, float(softmax_scale or 1.0 / math.sqrt(q.shape[-1])), flags)
         ctx.set_materialize_grads(False)          # the gradient of lse is never used: no zero tensor for it
         return o, _pad_lse(lse) if pad_lse else lse
 
@@ -643,7 +644,7 @@ class CausalHyperFunc(torch.autograd.Function):
         if n % 2:
             _cuda(q, k, v)
             q, k, v = _padded((q, k, v), n + 1)
-        cfg = (levels, block_size, sample_size, proj_f32.shape[1], int(keep_parts), min_seq_len, scale, flags)
+        cfg = (levels, block_size, sample_size, proj_f32.shape[1], int(keep_parts), min_seq_len, float(scale), flags)
         o, lse, saved = _call_forward(True, q, k, v, proj_f32, cfg)
         return o, lse, saved, (q, k, v), cfg
 
@@ -686,7 +687,7 @@ class NonCausalHyperFunc(torch.autograd.Function):
         assert H % k.shape[1] == 0 and v.shape[:3] == k.shape[:3], 'query heads must be a multiple of the key/value heads'
         assert n % 128 == 0, 'keys sequence length must be divisible by 128'
         assert sample_size % 128 == 0
-        cfg = (0, block_size, sample_size, proj_f32.shape[1], 0, 0, scale, flags)
+        cfg = (0, block_size, sample_size, proj_f32.shape[1], 0, 0, float(scale), flags)
         return _call_forward(False, q, k, v, proj_f32, cfg, sample), cfg
 
     @staticmethod

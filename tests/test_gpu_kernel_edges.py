@@ -399,3 +399,23 @@ for i in range(2, 8):
 ha.check_device_status()
 '''
     subprocess.run([sys.executable, '-c', code], check=True, timeout=120, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+
+
+@pytest.mark.parametrize('n,causal', [(300, True), (512, False), (1024, True)])
+@pytest.mark.parametrize('kind', ['tensor', 'cuda', 'numpy'])
+def test_a_scale_that_changes_between_calls(n, causal, kind):
+    """a 0-dim tensor or array as the scale, rewritten in place: every call takes its value of that moment, forward and backward"""
+    import numpy as np
+    import hyperattention_b200 as ha
+    torch.manual_seed(84)
+    mod = ha.HyperAttention(input_dim=64, min_seq_len=512, sample_size=128, rng=torch.Generator().manual_seed(7)).to(device='cuda', dtype=torch.bfloat16)
+    q, k, v = [torch.randn(1, 2, n, 64, device='cuda').bfloat16().requires_grad_() for _ in range(3)]
+    scale = np.array(0.) if kind == 'numpy' else torch.zeros((), device='cuda' if kind == 'cuda' else 'cpu')
+    for value in (0.0625, 0.25):
+        scale[...] = value
+        got, want = mod(q, k, v, scale=scale, causal=causal), mod(q, k, v, scale=value, causal=causal)
+        with torch.no_grad():
+            assert torch.equal(mod(q, k, v, scale=scale, causal=causal), want)
+        assert torch.equal(got, want)
+        for a, b in zip(torch.autograd.grad(got, (q, k, v), v), torch.autograd.grad(want, (q, k, v), v)):
+            assert rel(a, b) < 1e-3        # (fp32 additions in no fixed order, rounded to bf16)
