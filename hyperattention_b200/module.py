@@ -42,9 +42,18 @@ class AngularLSH(torch.nn.Module):
         """proj_dir as a contiguous float32 [d, r] tensor (values exactly those of the stored dtype)."""
         pd = self.proj_dir
         key = (pd.data_ptr(), pd._version, pd.dtype, pd.device)
-        if self._proj_cache is None or self._proj_cache[0] != key:
-            self._proj_cache = (key, pd.detach().reshape(pd.shape[-2], pd.shape[-1]).to(torch.float32).contiguous())
-        return self._proj_cache[1]
+        cache = self._proj_cache
+        if cache is None or cache[0] != key:
+            cache = (key, pd.detach().reshape(pd.shape[-2], pd.shape[-1]).to(torch.float32).contiguous())
+            if pd.is_cuda:
+                # Other streams and threads read it without asking this one: kept only once it is there.  A capture is not waited for;
+                # its copy is written at every replay, and belongs to the graph.
+                stream = torch.cuda.current_stream(pd.device)
+                if torch.cuda.is_current_stream_capturing():
+                    return cache[1]
+                stream.synchronize()
+            self._proj_cache = cache
+        return cache[1]
 
     def hash_torch(self, mat):
         """The reference's PyTorch formulation (src/angular_lsh_triton.py:175-179), kept for comparisons."""

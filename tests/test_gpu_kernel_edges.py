@@ -419,3 +419,38 @@ def test_a_scale_that_changes_between_calls(n, causal, kind):
         assert torch.equal(got, want)
         for a, b in zip(torch.autograd.grad(got, (q, k, v), v), torch.autograd.grad(want, (q, k, v), v)):
             assert rel(a, b) < 1e-3        # (fp32 additions in no fixed order, rounded to bf16)
+
+
+def test_projection_copy_is_there_for_other_streams():
+    """the fp32 copy of the projection is made behind other work of one stream; a call on another stream right after it uses the finished one"""
+    import hyperattention_b200 as ha
+    torch.manual_seed(85)
+    q, k, v = [torch.randn(1, 2, 1024, 64, device='cuda').bfloat16() for _ in range(3)]
+    new = lambda: ha.HyperAttention(input_dim=64, min_seq_len=256, sample_size=128, rng=torch.Generator().manual_seed(8)).to(device='cuda', dtype=torch.bfloat16)
+    want, mod, a, b = new()(q, k, v), new(), torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(a):
+        stale = torch.full((64, 8), float('nan'), device='cuda')      # (what the copy's memory holds until it is written)
+    torch.cuda.synchronize()
+    del stale
+    with torch.cuda.stream(a):
+        torch.cuda._sleep(200_000_000)
+        mod(q, k, v)
+    with torch.cuda.stream(b):
+        got = mod(q, k, v)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+
+
+def test_projection_copy_of_a_capture_stays_in_its_graph():
+    """a module whose first call is captured: eager calls before a replay have a copy of their own"""
+    import hyperattention_b200 as ha
+    torch.manual_seed(86)
+    q, k, v = [torch.randn(1, 2, 1024, 64, device='cuda').bfloat16() for _ in range(3)]
+    new = lambda: ha.HyperAttention(input_dim=64, min_seq_len=256, sample_size=128, rng=torch.Generator().manual_seed(8)).to(device='cuda', dtype=torch.bfloat16)
+    want, mod, graph = new()(q, k, v), new(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = mod(q, k, v)
+    assert torch.equal(mod(q, k, v), want)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(captured, want)
