@@ -7,6 +7,7 @@ Secondary API names mirror the reference's: hyper_attn_func (src/hyper_attn_trit
 """
 import ctypes as C
 import math
+import threading
 
 import torch
 
@@ -69,6 +70,7 @@ def _ptr(t):
 
 _STATUS = {}
 _STATUS_RAW = {}        # the words' addresses, and the host word as the processor sees it
+_STATUS_LOCK = threading.Lock()
 
 
 def _status_words(device):
@@ -77,10 +79,14 @@ def _status_words(device):
     kernels write as well and the host can read without synchronising."""
     key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
     if key not in _STATUS:
-        _STATUS[key] = (torch.zeros(1, dtype=torch.int32, device=f'cuda:{key}'),
-                        torch.zeros(1, dtype=torch.int32).pin_memory())
-        dev_w, host_w = _STATUS[key]
-        _STATUS_RAW[key] = (dev_w.data_ptr(), host_w.data_ptr(), C.c_int32.from_address(host_w.data_ptr()))
+        with _STATUS_LOCK:          # one pair a device, whichever threads come first: launches under way hold its addresses
+            if key not in _STATUS:
+                dev_w, host_w = torch.zeros(1, dtype=torch.int32, device=f'cuda:{key}'), torch.zeros(1, dtype=torch.int32).pin_memory()
+                # kernels on any stream look at the word, and take what is not 0 for a failure
+                if not torch.cuda.is_current_stream_capturing():
+                    torch.cuda.current_stream(key).synchronize()
+                _STATUS_RAW[key] = (dev_w.data_ptr(), host_w.data_ptr(), C.c_int32.from_address(host_w.data_ptr()))
+                _STATUS[key] = (dev_w, host_w)
     return _STATUS[key]
 
 

@@ -454,3 +454,27 @@ def test_projection_copy_of_a_capture_stays_in_its_graph():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(captured, want)
+
+
+def test_status_word_is_there_for_other_streams(monkeypatch):
+    """the device's status word is made behind other work of one stream; a call on another stream right after it does not take what its memory
+    held for a failure"""
+    import hyperattention_b200 as ha
+    from hyperattention_b200 import ops
+    torch.manual_seed(87)
+    q, k, v = [torch.randn(1, 300, 2, 64, device='cuda').bfloat16() for _ in range(3)]
+    want, a, b = ha.flash_attn_func(q, k, v, None, True)[0], torch.cuda.Stream(), torch.cuda.Stream()
+    monkeypatch.setattr(ops, '_STATUS', {})
+    monkeypatch.setattr(ops, '_STATUS_RAW', {})
+    with torch.cuda.stream(a):
+        stale = torch.ones(1, dtype=torch.int32, device='cuda')
+    torch.cuda.synchronize()
+    del stale
+    with torch.cuda.stream(a):
+        torch.cuda._sleep(200_000_000)
+        first = ha.flash_attn_func(q, k, v, None, True)[0]
+    with torch.cuda.stream(b):
+        got = ha.flash_attn_func(q, k, v, None, True)[0]
+    torch.cuda.synchronize()
+    assert torch.equal(got, want) and torch.equal(first, want)
+    ha.check_device_status()
