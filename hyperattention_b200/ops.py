@@ -10,6 +10,7 @@ import math
 import threading
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib as L
 
@@ -34,7 +35,10 @@ def _call(fn, device, *args):
 
 
 def _wants_grad(*ts):
-    return torch.is_grad_enabled() and any(t.requires_grad for t in ts)
+    """Does the call go through its autograd Function?  Under forward-mode differentiation and function transforms, too: the Function says
+    there that it has no rule for them, where the bare call would lose the tangents without a word."""
+    return (torch.is_grad_enabled() and any(t.requires_grad for t in ts)) or forward_ad._current_level >= 0 or \
+        torch._C._are_functorch_transforms_active()
 
 
 # Parameter structs of earlier calls by shape, strides and options (everything but the pointers): filling one field by field costs more

@@ -478,3 +478,22 @@ def test_status_word_is_there_for_other_streams(monkeypatch):
     torch.cuda.synchronize()
     assert torch.equal(got, want) and torch.equal(first, want)
     ha.check_device_status()
+
+
+@pytest.mark.parametrize('n,causal', [(300, True), (512, False), (1024, True)])
+def test_forward_mode_and_transforms_are_refused(n, causal):
+    """there is no rule for tangents or batches: an error, also where no input requires a gradient; other tensors in a dual level pass"""
+    import torch.autograd.forward_ad as fwd
+    import hyperattention_b200 as ha
+    torch.manual_seed(88)
+    mod = ha.HyperAttention(input_dim=64, min_seq_len=512, sample_size=128, rng=torch.Generator().manual_seed(9)).to(device='cuda', dtype=torch.bfloat16)
+    q, k, v = [torch.randn(1, 2, n, 64, device='cuda').bfloat16() for _ in range(3)]
+    call = lambda t: mod(t, k, v, causal=causal)
+    want = call(q)
+    with torch.no_grad(), fwd.dual_level():
+        with pytest.raises(NotImplementedError):
+            call(fwd.make_dual(q, torch.ones_like(q)))
+        assert torch.equal(call(q), want)
+    for run in (lambda: torch.func.jvp(call, (q,), (torch.ones_like(q),)), lambda: torch.func.vmap(call)(q[None])):
+        with pytest.raises(RuntimeError):
+            run()
