@@ -148,6 +148,11 @@ inline bool plan_items(AttnPlan& pl, const ha_attn_params& p) {
   pl.by_block = FastDiv(p.mode == HA_MODE_HYPER ? (p.block_size + TILE - 1) / TILE : 1);
   return true;
 }
+// May tiles of contiguous rows come as TMA boxes?  A box that runs past the end of a segment brings the next segment's rows, where cp.async
+// fills with zeros: hidden weights are 0, but 0 times a row that is not finite is not.  (Past the last row of all, the map
+// fills with zeros itself.)
+inline bool boxes_end_with_segments(const ha_attn_params& p) { return p.segs_per_head == 1 || (p.m_q % TILE == 0 && p.m_k % TILE == 0); }
+
 // Row maps of q (0) and k (1) for tile::gather4.
 inline void plan_row_maps(AttnPlan& pl, const ha_attn_params& p, CUtensorMap (&maps)[2], long long n_q, long long n_k) {
   pl.rows = 0;

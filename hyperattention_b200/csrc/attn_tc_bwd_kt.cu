@@ -843,7 +843,7 @@ static int launch_kt_bwd(const ha_attn_params& p, cudaStream_t st) {
   const long long n_k = p.segs_per_head > 1 ? (long long)p.segs_per_head * p.span : p.k_off + p.m_k;
   const bool boxed_samples = p.sample_size > 0 && !p.sample_idx;
   pl.rows = 0;
-  pl.tiles = (flash || boxed_samples) && encode_tile_map(&maps.tile[1], p.dtype, p.k, 128, n_k, Hk, p.B, p.k_sn, p.k_sh, p.k_sb, TILE) &&
+  pl.tiles = (flash || boxed_samples) && boxes_end_with_segments(p) && encode_tile_map(&maps.tile[1], p.dtype, p.k, 128, n_k, Hk, p.B, p.k_sn, p.k_sh, p.k_sb, TILE) &&
              encode_tile_map(&maps.tile[2], p.dtype, p.v, 128, n_k, Hk, p.B, p.v_sn, p.v_sh, p.v_sb, TILE) &&
              (!flash || (encode_tile_map(&maps.tile[0], p.dtype, p.q, 128, n_q, p.H, p.B, p.q_sn, p.q_sh, p.q_sb, bkt::UQ) &&
                          encode_tile_map(&maps.tile[3], p.dtype, p.d_o, 128, n_q, p.H, p.B, p.do_sn, p.do_sh, p.do_sb, bkt::UQ)));

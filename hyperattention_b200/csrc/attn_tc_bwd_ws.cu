@@ -803,7 +803,7 @@ static int launch_ws_bwd(const ha_attn_params& p, bool store_dq, cudaStream_t st
   const long long n_q = p.segs_per_head > 1 ? (long long)p.segs_per_head * p.span : p.q_off + p.m_q;
   const long long n_k = p.segs_per_head > 1 ? (long long)p.segs_per_head * p.span : p.k_off + p.m_k;
   const bool flash = p.mode == HA_MODE_FLASH, boxed_samples = p.sample_size > 0 && !p.sample_idx;
-  pl.tiles = (flash || boxed_samples) && encode_tile_map(&maps.tile[1], p.dtype, p.k, 64, n_k, Hk, p.B, p.k_sn, p.k_sh, p.k_sb, TILE) &&
+  pl.tiles = (flash || boxed_samples) && boxes_end_with_segments(p) && encode_tile_map(&maps.tile[1], p.dtype, p.k, 64, n_k, Hk, p.B, p.k_sn, p.k_sh, p.k_sb, TILE) &&
              encode_tile_map(&maps.tile[2], p.dtype, p.v, 64, n_k, Hk, p.B, p.v_sn, p.v_sh, p.v_sb, TILE) &&
              (!flash || (encode_tile_map(&maps.tile[0], p.dtype, p.q, 64, n_q, p.H, p.B, p.q_sn, p.q_sh, p.q_sb, TILE) &&
                          encode_tile_map(&maps.tile[3], p.dtype, p.d_o, 64, n_q, p.H, p.B, p.do_sn, p.do_sh, p.do_sb, TILE)));

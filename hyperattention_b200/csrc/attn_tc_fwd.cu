@@ -650,7 +650,7 @@ static int launch_fwd(const ha_attn_params& p, cudaStream_t st) {
   // rows a head really has on either side (a single-segment call may have fewer or more keys than queries)
   const long long n_q = p.segs_per_head > 1 ? (long long)p.segs_per_head * p.span : p.q_off + p.m_q;
   const long long n_k = p.segs_per_head > 1 ? (long long)p.segs_per_head * p.span : p.k_off + p.m_k;
-  pl.tiles = encode_tile_map(&maps.tile[0], p.dtype, p.q, D, n_q, p.H, p.B, p.q_sn, p.q_sh, p.q_sb, TILE) &&
+  pl.tiles = boxes_end_with_segments(p) && encode_tile_map(&maps.tile[0], p.dtype, p.q, D, n_q, p.H, p.B, p.q_sn, p.q_sh, p.q_sb, TILE) &&
              encode_tile_map(&maps.tile[1], p.dtype, p.k, D, n_k, Hk, p.B, p.k_sn, p.k_sh, p.k_sb, TILE) &&
              encode_tile_map(&maps.tile[2], p.dtype, p.v, DV, n_k, Hk, p.B, p.v_sn, p.v_sh, p.v_sb, TILE);
   plan_row_maps(pl, p, maps.rows, n_q, n_k);

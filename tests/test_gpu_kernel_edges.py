@@ -497,3 +497,30 @@ def test_forward_mode_and_transforms_are_refused(n, causal):
     for run in (lambda: torch.func.jvp(call, (q,), (torch.ones_like(q),)), lambda: torch.func.vmap(call)(q[None])):
         with pytest.raises(RuntimeError):
             run()
+
+
+@pytest.mark.parametrize('m,causal', [(200, True), (72, False), (330, True)])
+@pytest.mark.parametrize('d', [64, 128])
+def test_segments_of_any_length_keep_to_themselves(d, m, causal):
+    """C entry points: two segments a head that end inside a tile; the second one's rows are all NaN, the first one's results are not"""
+    import ctypes as C
+    from hyperattention_b200 import _lib as L, ops
+    torch.manual_seed(89)
+    H, n, lib = 3, 2 * m, L.load()
+    q, k, v, do = [torch.randn(1, n, H, d, device='cuda').bfloat16() for _ in range(4)]
+    for t in (q, k, v, do):
+        t[:, m:] = float('nan')
+    o, lse = torch.empty_like(q), torch.empty(1, H, n, device='cuda')
+    acc, delta = torch.zeros(3, 1, H, n, d, device='cuda'), torch.empty(1, H, n, device='cuda')
+    p = ops._flash_params(q, k, v, o, lse, causal, d ** -0.5, 0)
+    p.segs_per_head, p.span, p.m_q, p.m_k = 2, m, m, m
+    L.check(lib.ha_attn_fwd(C.byref(p), ops._stream()), 'ha_attn_fwd')
+    L.check(lib.ha_delta(o.data_ptr(), *ops._bhn(o), do.data_ptr(), *ops._bhn(do), 1, H, n, d, L.BF16, delta.data_ptr(), ops._stream()), 'ha_delta')
+    p.d_o, p.delta, p.dq_acc, p.dk_acc, p.dv_acc = do.data_ptr(), delta.data_ptr(), acc[0].data_ptr(), acc[1].data_ptr(), acc[2].data_ptr()
+    p.do_sb, p.do_sh, p.do_sn = ops._bhn(do)
+    L.check(lib.ha_attn_bwd(C.byref(p), ops._stream()), 'ha_attn_bwd')
+    ref = [t[:, :m].float().cpu().requires_grad_() for t in (q, k, v)]
+    ow, lw = O.flash_attn_func(*ref, None, causal)
+    ow.backward(do[:, :m].float().cpu())
+    _check((o[:, :m], lse[:, :, :m]) + tuple(T(a[:, :, :m]) for a in acc), (ow, lw[:, :, :m]) + tuple(t.grad for t in ref), torch.bfloat16)
+    assert torch.isnan(o[:, m:]).all()
