@@ -796,7 +796,9 @@ static bool flash_typed_dq(const ha_attn_params& p, const void* dq) {
 }
 static bool flash_bwd_shape(const ha_attn_params* p, long long& rows, long long& rows_k) {
   if (!p || p->mode != HA_MODE_FLASH || p->segs_per_head != 1 || p->q_off || p->k_off || p->m_q != p->n || p->m_k != p->n || p->span != p->n) return false;
-  if (p->B <= 0 || p->H <= 0 || p->n <= 0 || p->d <= 0 || p->dv <= 0 || p->kv_group < 0 || (p->kv_group > 1 && p->H % p->kv_group != 0)) return false;
+  if (p->B <= 0 || p->H <= 0 || p->n <= 0 || p->d <= 0 || p->dv <= 0 || p->d > 256 || p->dv > 256 || p->kv_group < 0 ||
+      (p->kv_group > 1 && p->H % p->kv_group != 0))
+    return false;
   if (p->dtype != HA_BF16 && p->dtype != HA_FP16 && p->dtype != HA_FP32) return false;
   rows = (long long)p->B * p->H * p->n;
   rows_k = p->kv_group > 1 ? rows / p->kv_group : rows;
@@ -813,7 +815,7 @@ int64_t ha_flash_bwd_scratch_bytes(const ha_attn_params* p, const void* dq) {
 
 int ha_flash_bwd(const ha_attn_params* pp, void* dq, void* dk, void* dv, void* scratch, int64_t scratch_bytes, void* stream) {
   long long rows, rows_k;
-  if (!flash_bwd_shape(pp, rows, rows_k) || !pp->o || !pp->d_o || !pp->lse || !dq || !dk || !dv) return HA_ERR_INVALID;
+  if (!flash_bwd_shape(pp, rows, rows_k) || !pp->q || !pp->k || !pp->v || !pp->o || !pp->d_o || !pp->lse || !dq || !dk || !dv) return HA_ERR_INVALID;
   if (!scratch || scratch_bytes < ha_flash_bwd_scratch_bytes(pp, dq)) return HA_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   ha_attn_params a = *pp;

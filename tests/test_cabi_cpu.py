@@ -186,3 +186,21 @@ def test_causal_call_looks_at_every_shape(n, k, v):
     at = lambda s: torch.zeros(s[0], s[1], n + s[2], s[3])
     with pytest.raises(AssertionError, match='lengths must be equal|multiple of the key'):
         ops.causal_hyper(torch.zeros(2, 4, n, 64), at(k), at(v), torch.zeros(64, 8), 1, 256, 256, 0.125, 0, True, 512)
+
+
+def test_exact_backward_call_looks_at_its_arguments(lib):
+    """ha_flash_bwd launches the backward kernel itself: every tensor is there and every width one the kernels have before anything runs"""
+    from hyperattention_b200 import _lib
+    def call(**over):
+        p = _lib.AttnParams()
+        p.mode, p.dtype, p.B, p.H, p.n, p.d, p.dv, p.segs_per_head, p.span, p.m_q, p.m_k, p.scale = _lib.MODE_FLASH, _lib.BF16, 1, 2, 256, 64, 64, 1, 256, 256, 256, 0.125
+        for name in ('q', 'k', 'v', 'o', 'd_o'):
+            setattr(p, name, 256)
+            setattr(p, name + '_sn' if name != 'd_o' else 'do_sn', 64)
+        p.lse = 256
+        for name, value in over.items():
+            setattr(p, name, value)
+        return lib.ha_flash_bwd(C.byref(p), 256, 256, 256, 256, 1 << 40, None)
+    for name in ('q', 'k', 'v', 'o', 'd_o', 'lse'):
+        assert call(**{name: None}) == -1, name
+    assert call(d=264, dv=264) == -1 and call(dv=512) == -1
