@@ -6,9 +6,14 @@
 // a warp fall into distinct banks: per 4 steps of the contraction a thread of the forward reads 8 + 4 vectors for 128 FMAs, 16
 // shared-memory cycles against 32 of the FMA pipe.  64-key tiles also make every window boundary a tile boundary (windows
 // start at multiples of 64).
-// Bound by the FMA pipe.  Against one warp per query / key with lane-wise dot products (4 heads x 4096 x 64, block 256, sample 256):
-// forward 2440 us, backward 5130 us there.
+// Every product is summed in short chains (32 columns, or a tile of 64 keys or queries, by themselves, then added as a whole), which keeps the
+// errors below those of one warp per query / key with lane-wise dot products (32-bit sums over all keys in one chain were 15 to
+// 35% above: o 5.2e-7 instead of 4.5e-7 at 4 heads x 4096 x 64, now 2.4e-7).  The extra additions cost 3% of a training step, 7% of a causal one.
+// 4 heads x 4096 x 64, block 256, sample 256: step 326 us (one warp per query / key: 7780 us), about a third of the FMA pipe's rate: 256
+// CTAs of four warps on 148 SMs leave each scheduler one or two warps to hide shared memory behind, and a half-empty last wave.
 #include "attn_index.cuh"
+
+#include <type_traits>
 
 namespace ha {
 
@@ -114,22 +119,35 @@ __global__ void __launch_bounds__(128) attn_f32_fwd_kernel(const ha_attn_params 
     for (int i = 0; i < 8; ++i)
 #pragma unroll
       for (int c = 0; c < 4; ++c) s[i][c] = 0.f;
+    // 32 columns are summed by themselves and added as a whole: a chain of 32 + D / 32 roundings instead of D
+#pragma unroll 1
+    for (int k0 = 0; k0 < D; k0 += 32) {
+      float t[8][4];
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) t[i][c] = 0.f;
 #pragma unroll 2
-    for (int k = 0; k < D; k += 4) {
-      float4 b[4];
+      for (int k = k0; k < k0 + 32; k += 4) {
+        float4 b[4];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) b[c] = lds4(sK + (tn + 16 * c) * (D + 4) + k);
+        for (int c = 0; c < 4; ++c) b[c] = lds4(sK + (tn + 16 * c) * (D + 4) + k);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 a = lds4(sQ + (tm + 8 * i) * (D + 4) + k);
+        for (int i = 0; i < 8; ++i) {
+          const float4 a = lds4(sQ + (tm + 8 * i) * (D + 4) + k);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          s[i][c] = fmaf(a.x, b[c].x, s[i][c]);
-          s[i][c] = fmaf(a.y, b[c].y, s[i][c]);
-          s[i][c] = fmaf(a.z, b[c].z, s[i][c]);
-          s[i][c] = fmaf(a.w, b[c].w, s[i][c]);
+          for (int c = 0; c < 4; ++c) {
+            t[i][c] = fmaf(a.x, b[c].x, t[i][c]);
+            t[i][c] = fmaf(a.y, b[c].y, t[i][c]);
+            t[i][c] = fmaf(a.z, b[c].z, t[i][c]);
+            t[i][c] = fmaf(a.w, b[c].w, t[i][c]);
+          }
         }
       }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) s[i][c] += t[i][c];
     }
     __syncthreads();                       // K is read: its place takes the next tile
     if (j + 1 < n_tiles) load_tile<D, 128>(sK, kb, p.k_sn, s_krow[(j + 1) & 1]);
@@ -147,6 +165,7 @@ __global__ void __launch_bounds__(128) attn_f32_fwd_kernel(const ha_attn_params 
       }
     }
     const bool edge = (j + 1) * BT > n_keys || (causal && j == qt) || weighted;
+    float alphas[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       float mx = -INFINITY;
@@ -174,11 +193,16 @@ __global__ void __launch_bounds__(128) attn_f32_fwd_kernel(const ha_attn_params 
       for (int off = 8; off >= 1; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
       l[i] = l[i] * alpha + sum;
       m[i] = mnew;
-#pragma unroll
-      for (int c = 0; c < NC; ++c) { o[i][c].x *= alpha; o[i][c].y *= alpha; o[i][c].z *= alpha; o[i][c].w *= alpha; }
+      alphas[i] = alpha;
     }
     cp_async_wait<1>();
     __syncthreads();
+    // a tile's product is summed by itself and added as a whole: the chain of roundings is 64 + tiles long instead of a row's keys
+    float4 t[8][NC];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) t[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 2
     for (int k = 0; k < BT; k += 4) {
       float4 a[8];
@@ -192,13 +216,22 @@ __global__ void __launch_bounds__(128) attn_f32_fwd_kernel(const ha_attn_params 
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
             const float x = at(a[i], kk);
-            o[i][c].x = fmaf(x, b.x, o[i][c].x);
-            o[i][c].y = fmaf(x, b.y, o[i][c].y);
-            o[i][c].z = fmaf(x, b.z, o[i][c].z);
-            o[i][c].w = fmaf(x, b.w, o[i][c].w);
+            t[i][c].x = fmaf(x, b.x, t[i][c].x);
+            t[i][c].y = fmaf(x, b.y, t[i][c].y);
+            t[i][c].z = fmaf(x, b.z, t[i][c].z);
+            t[i][c].w = fmaf(x, b.w, t[i][c].w);
           }
         }
     }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        o[i][c].x = fmaf(o[i][c].x, alphas[i], t[i][c].x);
+        o[i][c].y = fmaf(o[i][c].y, alphas[i], t[i][c].y);
+        o[i][c].z = fmaf(o[i][c].z, alphas[i], t[i][c].z);
+        o[i][c].w = fmaf(o[i][c].w, alphas[i], t[i][c].w);
+      }
     __syncthreads();
     if (j + 1 < n_tiles) load_tile<DV, 128>(sV, vb, p.v_sn, s_krow[(j + 1) & 1]);
     cp_async_commit();
@@ -377,23 +410,36 @@ __global__ void __launch_bounds__(256, D + DV <= 128 ? 2 : 1) attn_f32_bwd_kerne
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int c = 0; c < 4; ++c) s[i][c] = dp[i][c] = 0.f;
+    // 32 columns are summed by themselves, as in the forward
     auto product = [&](float (&acc)[4][4], const float* A, const float* B, int W) {
+#pragma unroll 1
+      for (int k0 = 0; k0 < W; k0 += 32) {
+        float t[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) t[i][c] = 0.f;
 #pragma unroll 2
-      for (int k = 0; k < W; k += 4) {
-        float4 b[4];
+        for (int k = k0; k < k0 + 32; k += 4) {
+          float4 b[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) b[c] = lds4(B + (tn + 16 * c) * (W + 4) + k);
+          for (int c = 0; c < 4; ++c) b[c] = lds4(B + (tn + 16 * c) * (W + 4) + k);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 x = lds4(A + (tm + 16 * i) * (W + 4) + k);
+          for (int i = 0; i < 4; ++i) {
+            const float4 x = lds4(A + (tm + 16 * i) * (W + 4) + k);
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            acc[i][c] = fmaf(x.x, b[c].x, acc[i][c]);
-            acc[i][c] = fmaf(x.y, b[c].y, acc[i][c]);
-            acc[i][c] = fmaf(x.z, b[c].z, acc[i][c]);
-            acc[i][c] = fmaf(x.w, b[c].w, acc[i][c]);
+            for (int c = 0; c < 4; ++c) {
+              t[i][c] = fmaf(x.x, b[c].x, t[i][c]);
+              t[i][c] = fmaf(x.y, b[c].y, t[i][c]);
+              t[i][c] = fmaf(x.z, b[c].z, t[i][c]);
+              t[i][c] = fmaf(x.w, b[c].w, t[i][c]);
+            }
           }
         }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[i][c] += t[i][c];
       }
     };
     product(s, sQ, sK, D);
@@ -423,35 +469,37 @@ __global__ void __launch_bounds__(256, D + DV <= 128 ? 2 : 1) attn_f32_bwd_kerne
       }
     }
     __syncthreads();
-    // ---- dV += P^T dO, dK += dS^T Q ----
+    // ---- dV += P^T dO, dK += dS^T Q: a tile's product is summed by itself, as in the forward ----
+    auto fold = [&](auto& acc, const float* weights, const float* rows, auto chunks) {
+      constexpr int N = decltype(chunks)::value;
+      float4 t[4][N];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < N; ++c) t[i][c] = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
-    for (int q = 0; q < BT; ++q) {
-      const float4 x = lds4(sP + q * LDP + tm * 4), y = lds4(sS + q * LDP + tm * 4);
+      for (int q = 0; q < BT; ++q) {
+        const float4 x = lds4(weights + q * LDP + tm * 4);
 #pragma unroll
-      for (int c = 0; c < NV; ++c) {
-        const float4 b = lds4(sG + q * (DV + 4) + tn * 4 + 64 * c);
+        for (int c = 0; c < N; ++c) {
+          const float4 b = lds4(rows + q * (64 * N + 4) + tn * 4 + 64 * c);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float f = at(x, i);
-          dv[i][c].x = fmaf(f, b.x, dv[i][c].x);
-          dv[i][c].y = fmaf(f, b.y, dv[i][c].y);
-          dv[i][c].z = fmaf(f, b.z, dv[i][c].z);
-          dv[i][c].w = fmaf(f, b.w, dv[i][c].w);
+          for (int i = 0; i < 4; ++i) {
+            const float f = at(x, i);
+            t[i][c].x = fmaf(f, b.x, t[i][c].x);
+            t[i][c].y = fmaf(f, b.y, t[i][c].y);
+            t[i][c].z = fmaf(f, b.z, t[i][c].z);
+            t[i][c].w = fmaf(f, b.w, t[i][c].w);
+          }
         }
       }
 #pragma unroll
-      for (int c = 0; c < NK; ++c) {
-        const float4 b = lds4(sQ + q * (D + 4) + tn * 4 + 64 * c);
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float f = at(y, i);
-          dk[i][c].x = fmaf(f, b.x, dk[i][c].x);
-          dk[i][c].y = fmaf(f, b.y, dk[i][c].y);
-          dk[i][c].z = fmaf(f, b.z, dk[i][c].z);
-          dk[i][c].w = fmaf(f, b.w, dk[i][c].w);
-        }
-      }
-    }
+        for (int c = 0; c < N; ++c) { acc[i][c].x += t[i][c].x; acc[i][c].y += t[i][c].y; acc[i][c].z += t[i][c].z; acc[i][c].w += t[i][c].w; }
+    };
+    fold(dv, sP, sG, std::integral_constant<int, NV>{});
+    fold(dk, sS, sQ, std::integral_constant<int, NK>{});
     // ---- dQ rows tm + 16 i += dS K ----
     {
       float4 dq[4][NK];

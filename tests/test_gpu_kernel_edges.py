@@ -524,3 +524,20 @@ def test_segments_of_any_length_keep_to_themselves(d, m, causal):
     ow.backward(do[:, :m].float().cpu())
     _check((o[:, :m], lse[:, :, :m]) + tuple(T(a[:, :, :m]) for a in acc), (ow, lw[:, :, :m]) + tuple(t.grad for t in ref), torch.bfloat16)
     assert torch.isnan(o[:, m:]).all()
+
+
+@pytest.mark.parametrize('d', [64, 128])
+def test_fp32_sums_are_made_of_short_chains(d):
+    """exact attention in fp32 against 64 bits.  A chain of L roundings of 2^-24 is off by about 2^-24 / sqrt(3) sqrt(L / 2): 2.2e-7 where tiles of
+    64 are summed by themselves and then added (L = 64 + 16 here), 7.7e-7 where a sum runs over all 1000 keys.  Two products in a row: 3.1e-7."""
+    import hyperattention_b200 as ha
+    torch.manual_seed(90)
+    q, k, v, do = [torch.randn(1, 1000, 4, d, device='cuda') for _ in range(4)]
+    qg, kg, vg = [t.clone().requires_grad_() for t in (q, k, v)]
+    o, _ = ha.flash_attn_func(qg, kg, vg)
+    o.backward(do)
+    qe, ke, ve = [t.double().requires_grad_() for t in (q, k, v)]
+    oe = T((T(qe) @ T(ke).transpose(2, 3) * d ** -0.5).softmax(-1) @ T(ve))
+    oe.backward(do.double())
+    err = [((a.double() - b).norm() / b.norm()).item() for a, b in ((o, oe), (qg.grad, qe.grad), (kg.grad, ke.grad), (vg.grad, ve.grad))]
+    assert max(err) < 4.5e-7, err
