@@ -467,7 +467,7 @@ int ha_causal_fwd_strided(const ha_causal_params* pp, const int64_t* strides, vo
     const bool exact = exact_deepest && l == p.levels - 1;
     a.mode = exact ? HA_MODE_FLASH : HA_MODE_HYPER;
     a.flags = (deferred ? 0 : HA_FLAG_MERGE | (p.flags & HA_FLAG_MERGE_EXACT)) | (p.flags & HA_FLAG_FORCE_SIMT) |
-              (exact ? 0 : (p.flags & (HA_FLAG_SMOOTH | HA_FLAG_NO_WS)));
+              (exact ? 0 : (p.flags & HA_FLAG_SMOOTH));
     a.segs_per_head = 1 << l;
     a.span = span; a.q_off = m; a.k_off = 0; a.m_q = m; a.m_k = m;
     a.q_idx = exact ? nullptr : sv.q_idx(l); a.k_idx = exact ? nullptr : sv.k_idx(l); a.sample_idx = nullptr;

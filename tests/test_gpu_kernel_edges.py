@@ -10,7 +10,10 @@ from oracle import hyper_oracle as O
 pytestmark = pytest.mark.gpu
 
 T = lambda x: x.transpose(1, 2)
-TOL = {torch.float32: (1e-4, 2e-4), torch.bfloat16: (2e-2, 3e-2), torch.float16: (2e-2, 3e-2)}
+# Outputs and log-sum-exps, gradients: twice what roundings to 16 bits make of them.  Outputs: weights and result, 2^-9 / sqrt(3) each in bf16, with one
+# more a merge: 1.6e-3 to 2.6e-3; gradients: weights, dS, output and result: 2.3e-3 to 2.9e-3.  fp32: the reference's merges have
+# an eps in their logarithm (2^-23 a merge, which the gradients' exponentials repeat for every row).
+TOL = {torch.float32: (2e-6, 5e-5), torch.bfloat16: (5e-3, 6e-3), torch.float16: (6.5e-4, 7.5e-4)}
 
 
 def rel(a, b):
@@ -86,7 +89,7 @@ def test_exact_attention_unequal_lengths_and_layouts(nq, nk):
     k, v = [torch.randn(B, nk, 1, d).bfloat16().expand(-1, -1, H, -1) for _ in range(2)]
     o, lse = ha.flash_attn_func(q.cuda(), k.cuda()[:, :, :1].expand(-1, -1, H, -1), v.cuda()[:, :, :1].expand(-1, -1, H, -1))
     ow, lw = O.flash_attn_func(q.float(), k.float(), v.float())
-    assert rel(o, ow) < 2e-2 and rel(lse[:, :, :nq], lw[:, :, :nq]) < 2e-2
+    _check((o, lse[:, :, :nq]), (ow, lw[:, :, :nq]), torch.bfloat16)
     qs, ks, vs = [t.contiguous().permute(1, 0, 2, 3).contiguous().cuda().permute(1, 0, 2, 3) for t in (q, k, v)]     # [n, B, H, d] memory
     o2, lse2 = ha.flash_attn_func(qs, ks, vs)
     assert torch.equal(o2, o) and torch.equal(lse2, lse)
@@ -102,7 +105,7 @@ def test_rows_that_see_no_key_of_a_tile():
     sidx = ki[:, :, :128].contiguous()                  # the first window tile's keys: dropped for the first block, kept for the second
     o, lse = ha.hyper_attn_func(T(q.cuda()), T(k.cuda()), T(v.cuda()), T(qi.cuda()), T(ki.cuda()), 256, 128, None, False, sidx.cuda(), 0, True)
     ow, lw = O.hyper_attn_func(T(q.float()), T(k.float()), T(v.float()), T(qi), T(ki), 256, 128, None, False, sidx, False, True)
-    assert rel(o, ow) < 2e-2 and rel(lse, lw) < 2e-2
+    _check((o, lse), (ow, lw), torch.bfloat16)
 
 
 @pytest.mark.parametrize('n,dtype,train', [(1023, torch.bfloat16, True), (2047, torch.float32, True), (1535, torch.bfloat16, False)])
@@ -200,9 +203,9 @@ def test_uniform_sample_draws_the_oracles_rows(rows, n, S):
     assert torch.equal(got, torch.as_tensor(O.uniform_sample_idx(2024, 3, rows, S, n)).long())
 
 
-@pytest.mark.parametrize('n,causal,H', [(1, True, 2), (63, False, 1), (64, True, 2), (65, True, 1), (193, True, 3), (1000, False, 1), (2176, True, 1), (384, True, 80)])
+@pytest.mark.parametrize('n,causal,H', [(1000, False, 1), (2176, True, 1), (384, True, 80)])
 def test_exact_backward_by_key_tiles(n, causal, H):
-    """head dim 128: steps of 64 query rows and key tiles of 128, cut anywhere; more key tiles than CTAs"""
+    """head dim 128: many key tiles (shorter sequences: test_exact_attention_lengths), more of them than CTAs"""
     import hyperattention_b200 as ha
     torch.manual_seed(78)
     q, k, v, do = [torch.randn(1, n, H, 128).bfloat16() for _ in range(4)]
@@ -215,32 +218,54 @@ def test_exact_backward_by_key_tiles(n, causal, H):
         s = s.masked_fill(torch.ones(n, n, dtype=torch.bool).triu(1), float('-inf'))
     ow = T(s.softmax(-1) @ T(vc))
     ow.backward(do.float())
-    if n == 1:                                          # (one key: its weight is one, so q and k have no gradient)
-        assert rel(vg.grad, vc.grad) < 2e-2 and qg.grad.abs().max() < 0.1 and kg.grad.abs().max() < 0.1
-    else:
-        _check((o, lse[:, :, :n], qg.grad, kg.grad, vg.grad), (ow, s.logsumexp(-1), qc.grad, kc.grad, vc.grad), torch.bfloat16)
+    _check((o, lse[:, :, :n], qg.grad, kg.grad, vg.grad), (ow, s.logsumexp(-1), qc.grad, kc.grad, vc.grad), torch.bfloat16)
 
 
-@pytest.mark.parametrize('n,block,S,smooth,weighted', [(896, 384, 128, False, False), (512, 256, 128, False, True), (768, 256, 256, True, True)])
-def test_hyper_backward_by_key_tiles(n, block, S, smooth, weighted):
-    """head dim 128: key tiles that one query tile of a pair meets, weighted samples with dropped slots, smooth windows; against the kernel that
-    takes the other shapes"""
-    import hyperattention_b200 as ha
-    from hyperattention_b200 import _lib as L
+@pytest.mark.parametrize('direct', [None, False])
+@pytest.mark.parametrize('n,block,S,smooth,weighted', [(896, 384, 128, False, False), (512, 256, 128, False, True), (768, 256, 256, True, True), (512, 512, 0, True, False)])
+def test_hyper_backward_by_key_tiles(n, block, S, smooth, weighted, direct):
+    """head dim 128: key tiles that one query tile of a pair meets, weighted samples with dropped slots, smooth windows.  direct=False (fp32
+    accumulators) is what the kernel by key tiles takes in all of these; the default leaves those without whole blocks to the earlier one."""
+    from hyperattention_b200 import _lib as L, ops
     torch.manual_seed(79)
     B, H, d = 1, 2, 128
     q, k, v, do = [torch.randn(B, H, n, d).bfloat16() for _ in range(4)]
     qi, ki = [torch.sort(torch.randint(0, 4, (B, H, n)), dim=2, stable=True)[1] for _ in range(2)]
     sidx = ki[:, :, 64:64 + S].contiguous() if weighted else None
-    qg, kg, vg = [T(t.cuda()).requires_grad_() for t in (q, k, v)]
-    o, lse = ha.hyper_attn_func(qg, kg, vg, T(qi.cuda()), T(ki.cuda()), block, S, None, smooth, sidx.cuda() if weighted else None,
-                                L.FLAG_BWD_REF_SMOOTH if smooth else 0, weighted)
-    o.backward(T(do.cuda()))
-    want = [t.detach().requires_grad_() for t in (qg, kg, vg)]
-    ow, lw = ha.hyper_attn_func(*want, T(qi.cuda()), T(ki.cuda()), block, S, None, smooth, sidx.cuda() if weighted else None,
-                                (L.FLAG_BWD_REF_SMOOTH if smooth else 0) | L.FLAG_NO_WS, weighted)
-    ow.backward(T(do.cuda()))
-    _check((o, lse, qg.grad, kg.grad, vg.grad), (ow, lw, want[0].grad, want[1].grad, want[2].grad), torch.bfloat16)
+    qc, kc, vc = [t.float().requires_grad_() for t in (q, k, v)]
+    ow, lw = O.hyper_attn_func(T(qc), T(kc), T(vc), T(qi), T(ki), block, S, None, smooth, sidx, False, weighted)
+    T(ow).backward(do.float())
+    qg, kg, vg, og, dg = [T(t.cuda()) for t in (q, k, v, T(ow).detach().bfloat16(), do)]
+    qr, kr = [t.cuda().int().view(B * H, n) for t in (qi, ki)]
+    sr = sidx.cuda().int().view(B * H, S) if weighted else None
+    delta = T((og.float() * dg.float()).sum(-1)).contiguous()
+    flags = (L.FLAG_SMOOTH | L.FLAG_BWD_REF_SMOOTH) if smooth else 0
+    weights = ops.sample_weights(kr, sr, n, block, S, smooth) if weighted else None
+    got = ops.hyper_bwd(qg, kg, vg, qr, kr, sr, og, lw.detach().cuda().contiguous(), dg, delta, block, S, d ** -0.5, flags, weights, direct)
+    errs = [rel(T(g), w) for g, w in zip(got, (qc.grad, kc.grad, vc.grad))]
+    assert max(errs) < TOL[torch.bfloat16][1], errs
+
+
+@pytest.mark.parametrize('block,smooth', [(256, True), (384, False), (512, True)])
+def test_causal_training_at_head_dim_128(block, smooth):
+    """the kernel by key tiles in the causal schedule, which adds to fp32 accumulators: smooth windows of two and four tiles, blocks of three
+    tiles (cut at the ends of the rectangles)"""
+    import hyperattention_b200 as ha
+    torch.manual_seed(91)
+    n, d = 2048, 128
+    proj = torch.randn(1, 1, d, 8).bfloat16().float()
+    q, k, v, do = [torch.randn(1, 2, n, d).bfloat16() for _ in range(4)]
+    mod = ha.HyperAttention(input_dim=d, block_size=block, sample_size=128, min_seq_len=512, smooth_block=smooth)
+    mod.lsh.proj_dir.copy_(proj)
+    mod = mod.to(device='cuda', dtype=torch.bfloat16)
+    assert mod._regular_causal(n)
+    qg, kg, vg = [t.cuda().requires_grad_() for t in (q, k, v)]
+    o, lse = mod(qg, kg, vg, causal=True, return_lse=True)
+    o.backward(do.cuda())
+    qc, kc, vc = [t.float().requires_grad_() for t in (q, k, v)]
+    ow, lw = O.HyperAttentionOracle(proj, block, 128, 512, smooth)(qc, kc, vc, causal=True, return_lse=True)
+    ow.backward(do.float())
+    _check((o, lse, qg.grad, kg.grad, vg.grad), (ow, lw, qc.grad, kc.grad, vc.grad), torch.bfloat16)
 
 
 @pytest.mark.parametrize('dtype,B,n,rows,shapes', [(torch.bfloat16, 2, 1023, 1024, ((3, 64), (3, 64), (1, 128))), (torch.float16, 1, 5, 6, ((2, 20),)),
