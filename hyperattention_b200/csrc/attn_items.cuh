@@ -38,7 +38,10 @@ __device__ __forceinline__ AttnItem attn_item(const ha_attn_params& p, const Att
   const int n_qt = (p.m_q + TILE - 1) / TILE;
   if (flash && (p.flags & HA_FLAG_CAUSAL)) {
     // Items grow with the pair.  Long pairs first; with few pairs the order is turned by the segment, so that a CTA, which
-    // takes every 148th item, meets all lengths.
+    // takes every 148th item, meets all lengths.  Exact causal attention, turned against not (forward): 64 x 32 heads x 2048 rows 1.79 against
+    // 2.35 ms, 8 x 32 x 1024 82 against 113 us, where items outnumber CTAs many times; 32 heads x 2048 66 against 53 us, x 4096 168
+    // against 150, x 8192 567 against 473, where they do not; 8 heads x 16384 (64 pairs) 545 against 590.  The line at 32 pairs serves the leaves
+    // of causal calls (up to 2048 rows, many segments).
     pr = pl.pairs - 1 - pr;
     if (pl.pairs <= 32) pr += it.seg - pl.by_pairs(pr + it.seg) * pl.pairs;
   }

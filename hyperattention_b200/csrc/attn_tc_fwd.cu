@@ -66,8 +66,8 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
   const bool flash = KIND == FWD_FLASH || (KIND == FWD_ANY && p.mode == HA_MODE_FLASH);
   constexpr bool WT = KIND == FWD_ANY;                 // weighted sampling / merging possible
   // Pairs of every eight whose exponentials go to the FMA pipe.  It pays where the chain is bound by the exponential unit, i.e. in exact
-  // attention (32 x 2048-row leaves, head dim 64: 1.67 -> 1.60 ms); the hyper pattern is bound by its gathers and by the
-  // instruction caches before that (0.79 ms without, 0.83 ms with).
+  // attention (64 x 32 heads x 2048 rows, head dim 64: 1.85 -> 1.79 ms; 32 x 4096: 178 -> 168 us; head dim 128, 8 x 32768: 2.09 -> 2.05 ms); the
+  // hyper pattern is bound by its gathers and its rescaling before that (call at 32 x 131072: 1.151 ms without, 1.156 with).
   constexpr int POLY = KIND == FWD_FLASH ? 2 : 0;
   const bool merge = KIND == FWD_ANY && (p.flags & HA_FLAG_MERGE);
   extern __shared__ uint8_t smem_raw[];

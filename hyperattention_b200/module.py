@@ -10,8 +10,7 @@ Additional keyword arguments (all optional, accepted through **kwargs like the r
   fused_causal  True (default): run regular causal shapes through the single-call schedule; False: always use the
               per-level path built from the individual operators.
   fused_calls True (default): a non-causal call is one library call each way (hash, sort and attention;
-              delta, backward and finishing pass); False: one call per operator, as the uniform sampling mode always
-              does.
+              delta, backward and finishing pass); False: one call per operator.
 """
 import math
 
