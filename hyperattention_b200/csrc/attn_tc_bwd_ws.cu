@@ -13,21 +13,23 @@
 // goes to shared memory ([key][query] rows, an MN-major A operand) for  dQ += dS K.  A (key tile, query tile) pair is two halves of
 // 64 query columns on two TMEM stages, so that the elementwise phase of one half runs underneath the tensor work of the other.
 //
-// Roles (640 threads):
-//   * elementwise groups g = 0, 1 (128 threads each, thread = key row = TMEM lane): half g of every pair (= TMEM stage g).
-//   * drain group (128 threads, thread = TMEM lane): finished accumulators -> global memory.  Rows that lie scattered are transposed
-//     through a staging tile and leave coalesced (typed rows, fp32 reductions); tiles of contiguous rows leave as TMA
-//     additions of 32 x 128 floats, two in flight.
+// Roles (768 threads):
+//   * elementwise groups g = 0, 1 (128 threads each, thread = key row = TMEM lane): queries 32 g .. 32 g + 31 of every half.  Both work on one
+//     half while the tensor core works for the other; with a half each they met in their waits (1882 pairs of 2048-row leaves: 52% of a
+//     group's time waiting for scores, now 22%).
+//   * two drain groups (128 threads each, thread = TMEM lane): finished accumulators -> global memory, dV and dQ of query tile 0 by one, dK and
+//     dQ of query tile 1 by the other.  A key tile's accumulators are wanted again right away, and with one group dK waited until
+//     dV had left.  Rows that lie scattered are transposed through a staging tile and leave coalesced (typed rows, fp32
+//     reductions); tiles of contiguous rows leave as TMA additions of 32 x 128 floats.
 //   * five MMA warps, one product each (S^T, dP^T, dV, dK of every half, dQ of every pair), one elected lane issuing from
 //     warp-uniform code.
 //   * three loader warps: (Q, dO, lse, delta) of the item's query tiles, K tiles (ring of two), V tiles (ring of two); the first also
 //     works out the items and publishes their descriptors.
 // The roles' loops are rolled and small on purpose: the kernel this one replaced, most of it tcgen05.mma from divergent lanes, spent
 // its time on instruction fetch and issue.
-// What bounds it now (32 heads x 131072, 6400 -> 5000 cycles a pair of 128 x 128): the chain S^T -> elementwise -> dV / dK -> S^T of a
-// stage.  With one piece taken out at a time (2.30 ms with all): no elementwise phase 1.76 ms, an eighth of the MMAs 2.04, nothing
-// written out 2.06.
-// TMEM columns: stage s at 128 s: S^T in [0, 64), dP^T in [64, 128); P^T / dS^T packed over their first halves.  dV 256, dK 320, dQ of
+// What bounds it: the chain S^T -> elementwise -> dV / dK -> S^T of a stage, 4000 cycles a pair of 128 x 128, of which the tensor core is busy 1620.  32 heads
+// x 131072 (step): 3.60 -> 3.54 ms; 128 x 1920 rows exact causal (step): 500 -> 459 us; decoder 16 heads x 12287: 988 -> 929 us.
+// TMEM columns: stage s at 128 s: S^T in [0, 64), dP^T in [64, 128); P^T / dS^T packed over the first halves of a group's 32 columns.  dV 256, dK 320, dQ of
 // query tile 0 / 1 at 384 / 448.
 // Hand-offs are mbarriers with bounded waits; a wait that gives up raises the CTA's abort flag, every role leaves its loop at its
 // next wait, and the status words are set at the end.
@@ -45,12 +47,12 @@ constexpr int OFF_V = OFF_K + 2 * TILE_B;                      // V ring (2)
 constexpr int OFF_QD = OFF_V + 2 * TILE_B;                     // query tile y of the item: Q, then dO
 constexpr int OFF_DS = OFF_QD + 2 * 2 * TILE_B;                // two buffers (pairs alternate) of two slabs (halves)
 constexpr int OFF_LD = OFF_DS + 2 * 2 * TILE_B;                // per query tile: lse[128], delta[128] (fp32)
-constexpr int OFF_ST = OFF_LD + 2 * 1024;                      // two staging tiles of the drain group: 128 rows x 128 bytes
+constexpr int OFF_ST = OFF_LD + 2 * 1024;                      // a staging tile for each drain group: 128 rows x 128 bytes
 constexpr int SMEM_USED = OFF_ST + 2 * TILE * 128;             // from the first 1 KB boundary after the static variables: all a CTA has
-constexpr int THREADS = 640;
-constexpr int W_DRAIN = 8, W_MMA = 12, W_QD = 17, W_K = 18;    // first warp of each role (V: 19)
+constexpr int THREADS = 768;
+constexpr int W_DRAIN = 8, W_MMA = 16, W_QD = 21, W_K = 22;    // first warp of each role (V: 23)
 constexpr int COL_DV = 256, COL_DK = 320, COL_DQ = 384;
-constexpr int ND = 4, CONSUMERS = 19;                          // descriptor ring; warps that read every descriptor (all but the writer)
+constexpr int ND = 4, CONSUMERS = 23;                          // descriptor ring; warps that read every descriptor (all but the writer)
 // barrier slots (index + stage / buffer / query tile) and their arrivals per phase
 enum {
   B_K_FULL = 0,       // 2 x 32: every lane of the loader, through its copies
@@ -70,7 +72,7 @@ enum {
   B_LDT = 28,         // (2 query tiles x 2 groups) x 128: an elementwise group has scaled the lse / delta of its own columns
   B_ACC_FULL = 32,    // 2 x 1: dV / dK of a key tile complete
   B_ACC_FREE = 34,    // 2 x 128: ... drained
-  B_ST_FULL = 36,     // 2 x 128: every drain thread has written its row of the staging tile
+  B_ST_FULL = 36,     // 2 x 128: every thread of a drain group has written its row of the staging tile
   B_ST_FREE = 38,     // 2 x 1: the copy engine has read it
   B_D_FULL = 40,      // ND x 1
   B_D_EMPTY = 40 + ND,
@@ -84,8 +86,8 @@ __device__ __forceinline__ int bar_count(int i) {
     case B_QD_FULL >> 1: return 64;
     case B_K_EMPTY >> 1: case B_S_READY >> 1: return 2;
     case B_QD_EMPTY >> 1: return 4;
-    case B_P_READY >> 1: case B_DQ_FREE >> 1: case B_LDT >> 1: case (B_LDT >> 1) + 1: case B_ACC_FREE >> 1: case B_ST_FULL >> 1: return 128;
-    case B_DS_FULL >> 1: return 256;
+    case B_DQ_FREE >> 1: case B_LDT >> 1: case (B_LDT >> 1) + 1: case B_ACC_FREE >> 1: case B_ST_FULL >> 1: return 128;
+    case B_P_READY >> 1: case B_DS_FULL >> 1: return 256;
     default: return 1;
   }
 }
@@ -165,14 +167,14 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
   };
   constexpr float LOG2E = 1.4426950408889634f;
 
-  // Register budget: 640 threads x 96 at launch = 61440 = 256 x 128 (elementwise) + 128 x 96 (drain) + 256 x 64 (the rest).
+  // Register budget: 768 threads x 80 at launch = 61440 = 256 x 104 (elementwise) + 256 x 72 (drain) + 256 x 64 (the rest).
   if (warp < W_DRAIN) {
     // =====================================================================================================
     // elementwise groups: P^T = exp2(S^T scale log2e - lse log2e), dS^T = P^T (dP^T - delta) scale
     // =====================================================================================================
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 128;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     const int g = warp >> 2, row = tid & 127;
-    const uint32_t tS = tmem + 128 * g + ((uint32_t)((warp & 3) * 32) << 16), tDP = tS + 64;
+    const uint32_t tG = tmem + 32 * g + ((uint32_t)((warp & 3) * 32) << 16);      // this group's columns of stage 0's S^T (dP^T: 64 further on)
     const uint64_t sc2 = pack_f2(p.scale * LOG2E, p.scale * LOG2E), scl = pack_f2(p.scale, p.scale);
     const bool causal = flash && (p.flags & HA_FLAG_CAUSAL);
     uint32_t pair = 0, n_y0 = 0, n_y1 = 0;      // pairs so far; items that had query tile 0 / 1
@@ -183,90 +185,95 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
 #pragma unroll 1
       for (int e = 0; e < it.n_list && ok; ++e) {
 #pragma unroll 1
-        for (int y = 0; y < 2; ++y) {
+        for (int y = 0; y < 2 && ok; ++y) {
           if (!it.active(y, e)) continue;
-          HA_T_MARK(0)
-          if (!(ok = wait(B_S_READY + g, pair & 1))) break;
-          HA_T_MARK(1)
-          float* ld = reinterpret_cast<float*>(smem + OFF_LD + y * 1024) + 64 * g;      // this half's lse; delta 128 floats on
-          if (e == it.first_entry(y)) {
-            // lse / delta of the query tile have landed: the group scales those of its half once for all pairs of the item
-            const uint32_t par = (y ? n_y1 : n_y0) & 1;
-            if (!(ok = wait(B_QD_FULL + y, par))) break;
-            ld[(row >> 6) * TILE + (row & 63)] *= row < 64 ? -LOG2E : -p.scale;
-            mbar_arrive(bar(B_LDT + 2 * y + g));
-            if (!(ok = wait(B_LDT + 2 * y + g, par))) break;
-          }
-          if (pair >= 2 && !(ok = wait(B_DS_FREE + (pair & 1), ((pair >> 1) - 1) & 1))) break;   // dQ of pair - 2 has read the buffer
-          HA_T_MARK(2)
-          tc_fence_after();
-          // columns [0, hidden) of the half do not count for this key row
-          int hidden = 0;
-          float bias2 = 0.f;
-          if (flash) {
-            if (causal && e == it.qt0 + y) hidden = row - 64 * g;              // queries before the key
-            if (e * TILE + row >= p.m_k) hidden = 64;                          // past the last key
-          } else if (ANY && p.sample_logw && e >= it.n_win) {
-            int pos = it.q_pos0 + y * TILE + 64 * g;
-            if (pos >= p.m_q) pos -= p.m_q;
-            const long long qtile = (long long)it.seg * (p.m_q / TILE) + pos / TILE;
-            const int s = (e - it.n_win) * TILE + row;
-            bias2 = p.sample_logw[qtile] * LOG2E;
-            if ((p.sample_mask[qtile * (p.sample_size / 32) + (s >> 5)] >> (s & 31)) & 1u) hidden = 64;
-          }
-          const bool masked = KIND != BWD_HYPER && __any_sync(0xffffffffu, hidden > 0);
-          const uint64_t bias = pack_f2(bias2, bias2);
-          uint8_t* ds_row = smem + OFF_DS + (pair & 1) * 2 * TILE_B + g * TILE_B + row * 128;
-          // 16 query columns a turn; requesting the next turn's scores ahead measured slower (2.30 against 2.21 ms)
+          float* ld = reinterpret_cast<float*>(smem + OFF_LD + y * 1024) + 32 * g;      // lse of this group's columns; delta 128 floats on
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
-            uint32_t rs[16], rp[16], pk[8], dk[8];
-            tmem_ld16(tS + c * 16, rs);
-            tmem_ld16(tDP + c * 16, rp);
-            tmem_ld_fence16(rs);
-            tmem_ld_fence16(rp);
-#pragma unroll
-            for (int i = 0; i < 16; i += 4) {
-              // four query columns: their (scaled) lse and delta, the same for every thread: broadcast reads
-              ulonglong2 L = *reinterpret_cast<const ulonglong2*>(ld + c * 16 + i);
-              const ulonglong2 Dl = *reinterpret_cast<const ulonglong2*>(ld + TILE + c * 16 + i);
-              if (ANY) { L.x = fadd2(L.x, bias); L.y = fadd2(L.y, bias); }
-              float p0, p1, p2, p3, d0, d1, d2, d3;
-              unpack_f2(ffma2(pack_u2(rs[i], rs[i + 1]), sc2, L.x), p0, p1);
-              unpack_f2(ffma2(pack_u2(rs[i + 2], rs[i + 3]), sc2, L.y), p2, p3);
-              p0 = fast_exp2(p0); p1 = fast_exp2(p1); p2 = fast_exp2(p2); p3 = fast_exp2(p3);
-              if (masked) {
-                const int at = c * 16 + i;
-                if (at < hidden) p0 = 0.f;
-                if (at + 1 < hidden) p1 = 0.f;
-                if (at + 2 < hidden) p2 = 0.f;
-                if (at + 3 < hidden) p3 = 0.f;
+          for (int s = 0; s < 2; ++s, ld += 64) {
+            HA_T_MARK(0)
+            if (!(ok = wait(B_S_READY + s, pair & 1))) break;
+            HA_T_MARK(1)
+            if (s == 0) {
+              if (e == it.first_entry(y)) {
+                // lse / delta of the query tile have landed: the group scales those of its columns once for all pairs of the item
+                const uint32_t par = (y ? n_y1 : n_y0) & 1;
+                if (!(ok = wait(B_QD_FULL + y, par))) break;
+                ld[(row >> 6) * TILE + ((row >> 5) & 1) * 64 + (row & 31)] *= row < 64 ? -LOG2E : -p.scale;
+                mbar_arrive(bar(B_LDT + 2 * y + g));
+                if (!(ok = wait(B_LDT + 2 * y + g, par))) break;
               }
-              // ds = p * (dp - delta) * scale
-              unpack_f2(fmul2(pack_f2(p0, p1), ffma2(pack_u2(rp[i], rp[i + 1]), scl, Dl.x)), d0, d1);
-              unpack_f2(fmul2(pack_f2(p2, p3), ffma2(pack_u2(rp[i + 2], rp[i + 3]), scl, Dl.y)), d2, d3);
-              pk[i >> 1] = pack2<T>(p0, p1);
-              pk[(i >> 1) + 1] = pack2<T>(p2, p3);
-              dk[i >> 1] = pack2<T>(d0, d1);
-              dk[(i >> 1) + 1] = pack2<T>(d2, d3);
+              if (pair >= 2 && !(ok = wait(B_DS_FREE + (pair & 1), ((pair >> 1) - 1) & 1))) break;   // dQ of pair - 2 has read the buffer
             }
-            // P^T / dS^T of the chunk (8 packed columns) over columns this thread has already consumed
-            tmem_st8(tS + c * 8, pk);
-            tmem_st8(tDP + c * 8, dk);
+            HA_T_MARK(2)
+            tc_fence_after();
+            // queries [0, hidden) of the group's do not count for this key row
+            int hidden = 0;
+            float bias2 = 0.f;
+            if (flash) {
+              if (causal && e == it.qt0 + y) hidden = row - 64 * s - 32 * g;              // queries before the key
+              if (e * TILE + row >= p.m_k) hidden = 32;                                   // past the last key
+            } else if (ANY && p.sample_logw && e >= it.n_win) {
+              int pos = it.q_pos0 + y * TILE + 64 * s;
+              if (pos >= p.m_q) pos -= p.m_q;
+              const long long qtile = (long long)it.seg * (p.m_q / TILE) + pos / TILE;
+              const int sl = (e - it.n_win) * TILE + row;
+              bias2 = p.sample_logw[qtile] * LOG2E;
+              if ((p.sample_mask[qtile * (p.sample_size / 32) + (sl >> 5)] >> (sl & 31)) & 1u) hidden = 32;
+            }
+            const bool masked = KIND != BWD_HYPER && __any_sync(0xffffffffu, hidden > 0);
+            const uint64_t bias = pack_f2(bias2, bias2);
+            const uint32_t tS = tG + 128 * s, tDP = tS + 64;
+            uint8_t* ds_row = smem + OFF_DS + (pair & 1) * 2 * TILE_B + s * TILE_B + row * 128;
+#pragma unroll 1
+            for (int c = 0; c < 2; ++c) {
+              uint32_t rs[16], rp[16], pk[8], dk[8];
+              tmem_ld16(tS + c * 16, rs);
+              tmem_ld16(tDP + c * 16, rp);
+              tmem_ld_fence16(rs);
+              tmem_ld_fence16(rp);
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
-              *reinterpret_cast<uint4*>(ds_row + (((c * 2 + j) ^ (row & 7)) << 4)) = make_uint4(dk[4 * j], dk[4 * j + 1], dk[4 * j + 2], dk[4 * j + 3]);
+              for (int i = 0; i < 16; i += 4) {
+                // four query columns: their (scaled) lse and delta, the same for every thread: broadcast reads
+                ulonglong2 L = *reinterpret_cast<const ulonglong2*>(ld + c * 16 + i);
+                const ulonglong2 Dl = *reinterpret_cast<const ulonglong2*>(ld + TILE + c * 16 + i);
+                if (ANY) { L.x = fadd2(L.x, bias); L.y = fadd2(L.y, bias); }
+                float p0, p1, p2, p3, d0, d1, d2, d3;
+                unpack_f2(ffma2(pack_u2(rs[i], rs[i + 1]), sc2, L.x), p0, p1);
+                unpack_f2(ffma2(pack_u2(rs[i + 2], rs[i + 3]), sc2, L.y), p2, p3);
+                p0 = fast_exp2(p0); p1 = fast_exp2(p1); p2 = fast_exp2(p2); p3 = fast_exp2(p3);
+                if (masked) {
+                  const int at = c * 16 + i;
+                  if (at < hidden) p0 = 0.f;
+                  if (at + 1 < hidden) p1 = 0.f;
+                  if (at + 2 < hidden) p2 = 0.f;
+                  if (at + 3 < hidden) p3 = 0.f;
+                }
+                // ds = p * (dp - delta) * scale
+                unpack_f2(fmul2(pack_f2(p0, p1), ffma2(pack_u2(rp[i], rp[i + 1]), scl, Dl.x)), d0, d1);
+                unpack_f2(fmul2(pack_f2(p2, p3), ffma2(pack_u2(rp[i + 2], rp[i + 3]), scl, Dl.y)), d2, d3);
+                pk[i >> 1] = pack2<T>(p0, p1);
+                pk[(i >> 1) + 1] = pack2<T>(p2, p3);
+                dk[i >> 1] = pack2<T>(d0, d1);
+                dk[(i >> 1) + 1] = pack2<T>(d2, d3);
+              }
+              // P^T / dS^T of the chunk (8 packed columns) over columns this thread has already consumed
+              tmem_st8(tS + c * 8, pk);
+              tmem_st8(tDP + c * 8, dk);
+#pragma unroll
+              for (int j = 0; j < 2; ++j)
+                *reinterpret_cast<uint4*>(ds_row + (((4 * g + c * 2 + j) ^ (row & 7)) << 4)) = make_uint4(dk[4 * j], dk[4 * j + 1], dk[4 * j + 2], dk[4 * j + 3]);
+            }
+            HA_T_MARK(3)
+            tmem_st_wait();
+            fence_async_smem();       // the dS rows are read by the tensor core (async proxy)
+            tc_fence_before();
+            mbar_arrive(bar(B_P_READY + s));
+            // The dQ warp follows the dS buffers, not the TMEM stages: it may run up to two pairs behind this thread, and a parity wait
+            // must never fall two phases behind its barrier; the buffer's own barrier cannot run ahead of it.
+            if (s == 1) mbar_arrive(bar(B_DS_FULL + (pair & 1)));
+            HA_T_MARK(4)
           }
-          HA_T_MARK(3)
-          tmem_st_wait();
-          fence_async_smem();       // the dS rows are read by the tensor core (async proxy)
-          tc_fence_before();
-          mbar_arrive(bar(B_P_READY + g));
-          // The dQ warp follows the dS buffers, not the TMEM stages: it may run up to two pairs behind this thread, and a parity wait
-          // must never fall two phases behind its barrier; the buffer's own barrier cannot run ahead of it.
-          mbar_arrive(bar(B_DS_FULL + (pair & 1)));
           ++pair;
-          HA_T_MARK(4)
         }
       }
       ++n_y0;
@@ -277,13 +284,15 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
     // =====================================================================================================
     // drain group: finished accumulators -> global memory
     // =====================================================================================================
-    const int row = tid & 127, rot = row & 7;
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    const int row = tid & 127, rot = row & 7, grp = (warp - W_DRAIN) >> 2;
     const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
-    uint8_t* const stage = smem + OFF_ST;                   // scattered rows: the warp's own 4 KB of tile 0
-    uint8_t* my_row = stage + row * 128;
-    const uint8_t* warp_rows = stage + (row & ~31) * 128;
-    uint32_t n_kt = 0, n_y0 = 0, n_y1 = 0;                  // key tiles / query tiles 0, 1 drained so far
-    uint32_t ops = 0, freed = 0;                            // tile additions issued; of those, known to have left their staging tile
+    const uint32_t s_stage = OFF_ST + grp * (TILE * 128);   // scattered rows: the warp's own 4 KB
+    uint8_t* my_row = smem + s_stage + row * 128;
+    const uint8_t* warp_rows = smem + s_stage + (row & ~31) * 128;
+    uint32_t n_kt = 0, n_y = 0;                             // key tiles / query tiles drained so far
+    uint32_t ops = 0;                                       // tile additions issued
+    bool reading = false;                                   // the last of them may still be reading the staging tile
     bool ok = true;
     HA_T_DECL(8)
     AttnItem it;
@@ -291,12 +300,10 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
       const int Hk = p.kv_group > 1 ? pl.by_group(p.H) : p.H;
 #pragma unroll 1
       for (int e = 0; e < it.n_list && ok; ++e) {
-        // dQ of query tile 0 (complete one pair before the key tile), dV, dK, dQ of query tile 1
+        // dV (dK) of the key tile, then dQ of query tile 0 (1) if the tile was its last
 #pragma unroll 1
-        for (int job = 0; job < 4; ++job) {
-          const bool is_q = job == 0 || job == 3;
-          const int y = job == 3;
-          if (is_q && ((y && !it.has1) || e != it.last_entry(y))) continue;
+        for (int is_q = 0; is_q < 2; ++is_q) {
+          if (is_q && ((grp && !it.has1) || e != it.last_entry(grp))) continue;
           HA_T_MARK(0)
           // where this lane's row goes, and how
           enum { TYPED, ROWS_ADD, ROWS_STORE, TILE_ADD, TILE_STORE, SLOTS };
@@ -306,51 +313,39 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
           float* acc;
           const bool sampled = !flash && e >= it.n_win;
           if (is_q) {
-            int pos = it.q_pos0 + y * TILE + row;
+            int pos = it.q_pos0 + grp * TILE + row;
             if (pos >= p.m_q && !flash) pos -= p.m_q;
             local = flash ? (pos < p.m_q ? pos : -1) : p.q_idx[(long long)it.seg * p.m_q + pos];
             if (local >= 0) local += it.q_row0;
             map = 0;
-            tile_row = it.q_row0 + it.q_pos0 + y * TILE;
+            tile_row = it.q_row0 + it.q_pos0 + grp * TILE;
             typed = (T*)p.dq_out;
             acc = p.dq_acc;
             mode = p.dq_out ? TYPED : flash && (out.bulk & 1) ? (out.store_dq ? TILE_STORE : TILE_ADD) : out.store_dq ? ROWS_STORE : ROWS_ADD;
-            full = B_DQ_FULL + y;
-            free_bar = B_DQ_FREE + y;
-            par = (y ? n_y1 : n_y0) & 1;
-            taddr = COL_DQ + 64 * y;
+            full = B_DQ_FULL + grp;
+            free_bar = B_DQ_FREE + grp;
+            par = n_y & 1;
+            taddr = COL_DQ + 64 * grp;
           } else {
-            const bool is_k = job == 2;
             local = item_key_row(p, it, e, row, flash);
             if (local >= 0) local += it.k_row0;
-            map = is_k ? 2 : 1;                                   // (accumulator maps: dq, dv, dk)
+            map = 1 + grp;                                        // (accumulator maps: dq, dv, dk)
             tile_row = it.k_row0 + (flash ? e : e - it.n_win) * TILE;
-            typed = (T*)(is_k ? p.dk_out : p.dv_out);
-            acc = is_k ? p.dk_acc : p.dv_acc;
+            typed = (T*)(grp ? p.dk_out : p.dv_out);
+            acc = grp ? p.dk_acc : p.dv_acc;
             if (p.dk_out) {
               mode = sampled ? SLOTS : TYPED;
-              if (sampled) acc = (is_k ? p.dk_sacc : p.dv_sacc) + ((long long)it.kseg * p.sample_size + (e - it.n_win) * TILE) * D;
+              if (sampled) acc = (grp ? p.dk_sacc : p.dv_sacc) + ((long long)it.kseg * p.sample_size + (e - it.n_win) * TILE) * D;
             } else {
               mode = (out.bulk & 2) && (flash || (sampled && !p.sample_idx)) ? TILE_ADD : ROWS_ADD;
             }
-            full = B_ACC_FULL + is_k;
-            free_bar = B_ACC_FREE + is_k;
+            full = B_ACC_FULL + grp;
+            free_bar = B_ACC_FREE + grp;
             par = n_kt & 1;
-            taddr = is_k ? COL_DK : COL_DV;
+            taddr = grp ? COL_DK : COL_DV;
           }
           const int head = is_q ? it.b * p.H + it.h : it.b * Hk + it.hk;
-          const long long rid = (long long)head * p.n + local;
           const bool by_tile = mode >= TILE_ADD;
-          // scattered rows use a staging tile that an addition may still be reading
-          if (!by_tile && freed < ops) {
-            if (row == 0) {
-              bws_bulk_wait_read<0>();
-              mbar_arrive(bar(B_ST_FREE + ((ops - 1) & 1)));
-            }
-            __syncwarp();
-            freed = ops;
-            if (!(ok = wait(B_ST_FREE + ((ops - 1) & 1), ((ops - 1) >> 1) & 1))) break;
-          }
           HA_T_MARK(1)
           if (!(ok = wait(full, par))) break;
           HA_T_MARK(2)
@@ -364,6 +359,15 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
               tc_fence_before();
               mbar_arrive(bar(free_bar));
             }
+            if (reading) {
+              if (row == 0) {
+                bws_bulk_wait_read<0>();
+                mbar_arrive(bar(B_ST_FREE + grp));
+              }
+              __syncwarp();
+              if (!(ok = wait(B_ST_FREE + grp, (ops - 1) & 1))) break;
+              reading = false;
+            }
             if (mode == TYPED) {
               // both halves of a row fill its 128 bytes
 #pragma unroll
@@ -375,33 +379,24 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
               }
               if (hf == 0) continue;
             } else {
-              uint8_t* dst = my_row;
-              if (by_tile) {
-                dst += (ops & 1) * (TILE * 128);
-                if (ops >= 2 && !(ok = wait(B_ST_FREE + (ops & 1), ((ops - 2) >> 1) & 1))) break;
-              }
 #pragma unroll
-              for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(dst + ((i ^ rot) << 4)) = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+              for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(my_row + ((i ^ rot) << 4)) = make_uint4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
             }
             if (by_tile) {
               fence_async_smem();
-              mbar_arrive(bar(B_ST_FULL + (ops & 1)));
-              if (warp == W_DRAIN) {
-                if (!(ok = wait(B_ST_FULL + (ops & 1), (ops >> 1) & 1))) break;
+              mbar_arrive(bar(B_ST_FULL + grp));
+              if (warp == W_DRAIN + 4 * grp) {
+                if (!(ok = wait(B_ST_FULL + grp, ops & 1))) break;
                 if (lane == 0) {
-                  const uint32_t src = s_base + OFF_ST + (ops & 1) * (TILE * 128);
+                  const uint32_t src = s_base + s_stage;
                   if (mode == SLOTS) bws_bulk_add_f32(acc + hf * (TILE * 32), src, TILE * 128);
                   else if (mode == TILE_ADD) tma_add_tile(&maps.acc[map], hf * 32, tile_row, head, src);
                   else tma_store_tile(&maps.acc[map], hf * 32, tile_row, head, src);
                   bws_bulk_commit();
-                  if (freed < ops) {
-                    bws_bulk_wait_read<1>();          // the one before has been read
-                    mbar_arrive(bar(B_ST_FREE + ((ops - 1) & 1)));
-                  }
                 }
                 __syncwarp();
               }
-              freed = ops;
+              reading = true;
               ++ops;
             } else {
               // eight lanes cover the 128 contiguous bytes of a row
@@ -424,16 +419,16 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
                 for (int j = 0; j < 8; ++j)
                   if (to[j] >= 0) red_add_v4(dst_rows + (long long)to[j] * D, v[j]);
               } else {
+                const long long row0 = (long long)head * p.n;
 #pragma unroll 2
                 for (int j = 0; j < 8; ++j) {
                   const int rl = 4 * j + (lane >> 3);
                   const float4 v = *reinterpret_cast<const float4*>(warp_rows + rl * 128 + ((c ^ (rl & 7)) << 4));
-                  const long long rr = __shfl_sync(0xffffffffu, rid, rl);
-                  const bool there = __shfl_sync(0xffffffffu, local, rl) >= 0;
-                  if (there) {
-                    if (mode == TYPED) *reinterpret_cast<float4*>(typed + rr * D + c * 8) = v;
-                    else if (mode == ROWS_ADD) red_add_v4(acc + rr * D + hf * 32 + c * 4, v);
-                    else *reinterpret_cast<float4*>(acc + rr * D + hf * 32 + c * 4) = v;
+                  const int to = __shfl_sync(0xffffffffu, local, rl);
+                  if (to >= 0) {
+                    if (mode == TYPED) *reinterpret_cast<float4*>(typed + (row0 + to) * D + c * 8) = v;
+                    else if (mode == ROWS_ADD) red_add_v4(acc + (row0 + to) * D + hf * 32 + c * 4, v);
+                    else *reinterpret_cast<float4*>(acc + (row0 + to) * D + hf * 32 + c * 4) = v;
                   }
                 }
               }
@@ -442,17 +437,13 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
           }
           if (!ok) break;
           HA_T_MARK(3)
-          if (is_q) {
-            if (y) ++n_y1;
-            else ++n_y0;
-          } else if (job == 2) {
-            ++n_kt;
-          }
+          if (is_q) ++n_y;
+          else ++n_kt;
         }
       }
     }
     bws_bulk_wait_all();       // nothing of this thread is in flight when the CTA retires
-    HA_T_DUMP(8, (int)blockIdx.x * 8 + 2, row == 0)
+    HA_T_DUMP(8, (int)blockIdx.x * 8 + 2, row == 0 && grp == 0)
   } else {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     if (warp < W_QD) {
@@ -522,7 +513,7 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
                 if (elect_one()) {
 #pragma unroll
                   for (int kk = 0; kk < 4; ++kk)
-                    mma_ts(tmem + (is_k ? COL_DK : COL_DV), tmem + 128 * s + is_k * 64 + kk * 8, dB + s * (TILE_B / 2 >> 4) + kk * (2048 >> 4), idesc,
+                    mma_ts(tmem + (is_k ? COL_DK : COL_DV), tmem + 128 * s + is_k * 64 + (kk >> 1) * 32 + (kk & 1) * 8, dB + s * (TILE_B / 2 >> 4) + kk * (2048 >> 4), idesc,
                            !fresh | (s + kk > 0));
                   mma_commit(bar((is_k ? B_SF_P : B_SF_S) + s));
                   if (s == 1 && tile_done) mma_commit(bar(B_ACC_FULL + is_k));
