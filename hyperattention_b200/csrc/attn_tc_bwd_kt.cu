@@ -208,12 +208,12 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
     // elementwise groups: P^T = exp2(S^T scale log2e - lse log2e), dS^T = P^T (dP^T - delta) scale
     // =====================================================================================================
     asm volatile("setmaxnreg.inc.sync.aligned.u32 128;");
-    const int g = warp >> 2, row = tid & 127;
+    const int g = warp >> 2;
     const uint32_t tS = tmem + 128 * g + ((uint32_t)((warp & 3) * 32) << 16), tDP = tS + 64;
     const uint64_t sc2 = pack_f2(p.scale * LOG2E, p.scale * LOG2E), scl = pack_f2(p.scale, p.scale);
     const bool causal = flash && (p.flags & HA_FLAG_CAUSAL);
     uint32_t pair = 0, slot = g, lap = 0;       // units of this group so far; unit slot and its lap round the ring
-    uint8_t* ds_row = smem + OFF_DS + g * TILE_B + row * 128;
+    const uint32_t ds_rows = s_base + OFF_DS + g * TILE_B + (32 * (warp & 3) + (lane & 7)) * 128;
     bool ok = true;
     HA_T_DECL(8)
     KtItem it;
@@ -231,58 +231,74 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
           HA_T_MARK(2)
           tc_fence_after();
           const float* ld = reinterpret_cast<const float*>(smem + OFF_LD + slot * 512);      // lse; delta 64 floats on
-          // columns [0, hidden) of the unit do not count for this key row
-          int hidden = 0;
           float bias2 = 0.f;
-          if (flash) {
-            if (causal && e == y) hidden = row - UQ * g;                       // queries before the key
-            if (e * TILE + row >= p.m_k) hidden = UQ;                          // past the last key
-          } else if (ANY && p.sample_logw && e >= it.n_win) {
+          const bool weighted = ANY && p.sample_logw && e >= it.n_win;
+          const uint32_t* drop = nullptr;
+          if (weighted) {
             int pos = it.q_pos0 + y * TILE + UQ * g;
             if (pos >= p.m_q) pos -= p.m_q;
             const long long qtile = (long long)it.seg * (p.m_q / TILE) + pos / TILE;
-            const int s = (e - it.n_win) * TILE + row;
             bias2 = p.sample_logw[qtile] * LOG2E;
-            if ((p.sample_mask[qtile * (p.sample_size / 32) + (s >> 5)] >> (s & 31)) & 1u) hidden = UQ;
+            drop = p.sample_mask + qtile * (p.sample_size / 32) + (e - it.n_win) * (TILE / 32) + (warp & 3);
           }
-          const bool masked = KIND != KT_HYPER && __any_sync(0xffffffffu, hidden > 0);
+          const bool diag = causal && e == y, masked = KIND != KT_HYPER && (weighted || diag || (flash && (e + 1) * TILE > p.m_k));
           const uint64_t bias = pack_f2(bias2, bias2);
+          // Fragments of 16 keys x 8 queries, two keys and two neighbouring queries a thread, 16 keys x 32 queries at a time: the thread
+          // needs the lse and delta of 8 queries, where with a key a thread it needed those of all of them, as broadcast reads (decoder 2 x 16 x 8192:
+          // 1400 -> 1360 us, 8 x 32 x 2047 exact causal 1580 -> 1538, 32 x 32768 hyper 1964 -> 1933).
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
-            uint32_t rs[16], rp[16], pk[8], dk[8];
-            tmem_ld16(tS + c * 16, rs);
-            tmem_ld16(tDP + c * 16, rp);
-            tmem_ld_fence16(rs);
-            tmem_ld_fence16(rp);
+          for (int c = 0; c < 2; ++c) {
+            const uint32_t ds_to = ds_rows + (((4 * c + (lane >> 3)) ^ (lane & 7)) << 4);
+            uint64_t L[4], Dl[4];
 #pragma unroll
-            for (int i = 0; i < 16; i += 4) {
-              // four query columns: their (scaled) lse and delta, the same for every thread: broadcast reads
-              ulonglong2 L = *reinterpret_cast<const ulonglong2*>(ld + c * 16 + i);
-              const ulonglong2 Dl = *reinterpret_cast<const ulonglong2*>(ld + UQ + c * 16 + i);
-              if (ANY) { L.x = fadd2(L.x, bias); L.y = fadd2(L.y, bias); }
-              float p0, p1, p2, p3, d0, d1, d2, d3;
-              unpack_f2(ffma2(pack_u2(rs[i], rs[i + 1]), sc2, L.x), p0, p1);
-              unpack_f2(ffma2(pack_u2(rs[i + 2], rs[i + 3]), sc2, L.y), p2, p3);
-              p0 = fast_exp2(p0); p1 = fast_exp2(p1); p2 = fast_exp2(p2); p3 = fast_exp2(p3);
-              if (masked) {
-                const int at = c * 16 + i;
-                if (at < hidden) p0 = 0.f;
-                if (at + 1 < hidden) p1 = 0.f;
-                if (at + 2 < hidden) p2 = 0.f;
-                if (at + 3 < hidden) p3 = 0.f;
-              }
-              // ds = p * (dp - delta) * scale
-              unpack_f2(fmul2(pack_f2(p0, p1), ffma2(pack_u2(rp[i], rp[i + 1]), scl, Dl.x)), d0, d1);
-              unpack_f2(fmul2(pack_f2(p2, p3), ffma2(pack_u2(rp[i + 2], rp[i + 3]), scl, Dl.y)), d2, d3);
-              pk[i >> 1] = pack2<T>(p0, p1);
-              pk[(i >> 1) + 1] = pack2<T>(p2, p3);
-              dk[i >> 1] = pack2<T>(d0, d1);
-              dk[(i >> 1) + 1] = pack2<T>(d2, d3);
+            for (int j = 0; j < 4; ++j) {
+              L[j] = *reinterpret_cast<const uint64_t*>(ld + 32 * c + 8 * j + 2 * (lane & 3));
+              Dl[j] = *reinterpret_cast<const uint64_t*>(ld + UQ + 32 * c + 8 * j + 2 * (lane & 3));
+              if (ANY) L[j] = fadd2(L[j], bias);
             }
-            tmem_st8(tS + c * 8, pk);          // P^T of the chunk (8 packed columns) over columns this thread has already consumed
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
-              *reinterpret_cast<uint4*>(ds_row + (((c * 2 + j) ^ (row & 7)) << 4)) = make_uint4(dk[4 * j], dk[4 * j + 1], dk[4 * j + 2], dk[4 * j + 3]);
+            for (int h = 0; h < 2; ++h) {
+              uint32_t rs[16], rp[16], pk[8], dk[8];
+              tmem_ld_16x256(tS + 32 * c + (h << 20), rs);
+              tmem_ld_16x256(tDP + 32 * c + (h << 20), rp);
+              tmem_ld_fence16(rs);
+              tmem_ld_fence16(rp);
+              // queries [0, hidden) of these 32 do not count for a key row
+              int hidden[2] = {0, 0};
+              if (masked) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                  const int row = 32 * (warp & 3) + 16 * h + 8 * k + (lane >> 2);
+                  if (flash) {
+                    if (diag) hidden[k] = row - UQ * g - 32 * c;               // queries before the key
+                    if (e * TILE + row >= p.m_k) hidden[k] = 32;               // past the last key
+                  } else if ((*drop >> (row & 31)) & 1u) {
+                    hidden[k] = 32;
+                  }
+                }
+              }
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                  const int i = 4 * j + 2 * k, at = 8 * j + 2 * (lane & 3);
+                  float p0, p1, d0, d1;
+                  unpack_f2(ffma2(pack_u2(rs[i], rs[i + 1]), sc2, L[j]), p0, p1);
+                  p0 = fast_exp2(p0); p1 = fast_exp2(p1);
+                  if (masked) {
+                    if (at < hidden[k]) p0 = 0.f;
+                    if (at + 1 < hidden[k]) p1 = 0.f;
+                  }
+                  // ds = p * (dp - delta) * scale
+                  unpack_f2(fmul2(pack_f2(p0, p1), ffma2(pack_u2(rp[i], rp[i + 1]), scl, Dl[j])), d0, d1);
+                  pk[2 * j + k] = pack2<T>(p0, p1);
+                  dk[2 * j + k] = pack2<T>(d0, d1);
+                }
+              }
+              tmem_st_16x128(tS + 32 * c + (h << 20), pk);      // P^T (16 packed columns) over columns this warp has consumed
+#pragma unroll
+              for (int k = 0; k < 2; ++k) store_matrix_x4(ds_to + (16 * h + 8 * k) * 128, dk[k], dk[2 + k], dk[4 + k], dk[6 + k]);
+            }
           }
           HA_T_MARK(3)
           tmem_st_wait();
@@ -539,7 +555,7 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
                   const uint64_t dB = smem_desc(sDO, SLAB_U, 1024);
                   if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) mma_ts(tmem + COL_DV, tmem + 128 * s + kk * 8, dB + kk * (2048 >> 4), idesc, !fresh | (kk > 0));
+                    for (int kk = 0; kk < 4; ++kk) mma_ts(tmem + COL_DV, tmem + 128 * s + (kk >> 1) * 32 + (kk & 1) * 8, dB + kk * (2048 >> 4), idesc, !fresh | (kk > 0));
                     mma_commit(bar(B_S_FREE + s));
                     mma_commit(bar(B_DO_EMPTY + slot));
                     if (s == 1 && tile_done) mma_commit(bar(B_ACC_FULL));

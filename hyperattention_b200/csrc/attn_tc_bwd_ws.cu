@@ -14,9 +14,9 @@
 // 64 query columns on two TMEM stages, so that the elementwise phase of one half runs underneath the tensor work of the other.
 //
 // Roles (768 threads):
-//   * elementwise groups g = 0, 1 (128 threads each, thread = key row = TMEM lane): queries 32 g .. 32 g + 31 of every half.  Both work on one
-//     half while the tensor core works for the other; with a half each they met in their waits (1882 pairs of 2048-row leaves: 52% of a
-//     group's time waiting for scores, now 22%).
+//   * elementwise groups g = 0, 1 (128 threads each): queries 32 g .. 32 g + 31 of every half.  Both work on one half while the tensor core
+//     works for the other; with a half each they met in their waits (32 x 131072: half of a group's time waiting for scores, then a
+//     third).  A warp's 32 keys x 32 queries come as MMA fragments (16 x 8, two keys and two queries a thread).
 //   * two drain groups (128 threads each, thread = TMEM lane): finished accumulators -> global memory, dV and dQ of query tile 0 by one, dK and
 //     dQ of query tile 1 by the other.  A key tile's accumulators are wanted again right away, and with one group dK waited until
 //     dV had left.  Rows that lie scattered are transposed through a staging tile and leave coalesced (typed rows, fp32
@@ -27,8 +27,11 @@
 //     works out the items and publishes their descriptors.
 // The roles' loops are rolled and small on purpose: the kernel this one replaced, most of it tcgen05.mma from divergent lanes, spent
 // its time on instruction fetch and issue.
-// What bounds it: the chain S^T -> elementwise -> dV / dK -> S^T of a stage, 4000 cycles a pair of 128 x 128, of which the tensor core is busy 1620.  32 heads
-// x 131072 (step): 3.60 -> 3.54 ms; 128 x 1920 rows exact causal (step): 500 -> 459 us; decoder 16 heads x 12287: 988 -> 929 us.
+// What bounds it: the chain S^T -> elementwise -> dV / dK -> S^T of a stage, 3800 cycles a pair of 128 x 128, of which the tensor core is busy 1620
+// (shared memory, which feeds it 6 KB an instruction of 48 cycles, about 2500).  With one piece taken out at a time (128 x 1920 rows exact causal,
+// backward 278 us): no elementwise phase 218, nothing written out 238, a quarter of the MMAs 265, none of the three 108.  Measured and not
+// kept: P^T handed over before dP^T is awaited, with dK out of shared memory (442 -> 459 us the step), one arrival a warp instead of a thread (no
+// difference), test_wait instead of try_wait (8% slower), Q, dO and (K, V) as the loaders' shares (no difference; smooth windows 3% slower).
 // TMEM columns: stage s at 128 s: S^T in [0, 64), dP^T in [64, 128); P^T / dS^T packed over the first halves of a group's 32 columns.  dV 256, dK 320, dQ of
 // query tile 0 / 1 at 384 / 448.
 // Hand-offs are mbarriers with bounded waits; a wait that gives up raises the CTA's abort flag, every role leaves its loop at its
@@ -206,62 +209,75 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
             }
             HA_T_MARK(2)
             tc_fence_after();
-            // queries [0, hidden) of the group's do not count for this key row
-            int hidden = 0;
             float bias2 = 0.f;
-            if (flash) {
-              if (causal && e == it.qt0 + y) hidden = row - 64 * s - 32 * g;              // queries before the key
-              if (e * TILE + row >= p.m_k) hidden = 32;                                   // past the last key
-            } else if (ANY && p.sample_logw && e >= it.n_win) {
+            const bool weighted = ANY && !flash && p.sample_logw && e >= it.n_win;
+            const uint32_t* drop = nullptr;
+            if (weighted) {
               int pos = it.q_pos0 + y * TILE + 64 * s;
               if (pos >= p.m_q) pos -= p.m_q;
               const long long qtile = (long long)it.seg * (p.m_q / TILE) + pos / TILE;
-              const int sl = (e - it.n_win) * TILE + row;
               bias2 = p.sample_logw[qtile] * LOG2E;
-              if ((p.sample_mask[qtile * (p.sample_size / 32) + (sl >> 5)] >> (sl & 31)) & 1u) hidden = 32;
+              drop = p.sample_mask + qtile * (p.sample_size / 32) + (e - it.n_win) * (TILE / 32) + (warp & 3);
             }
-            const bool masked = KIND != BWD_HYPER && __any_sync(0xffffffffu, hidden > 0);
+            const bool diag = causal && e == it.qt0 + y, masked = KIND != BWD_HYPER && (weighted || diag || (flash && (e + 1) * TILE > p.m_k));
             const uint64_t bias = pack_f2(bias2, bias2);
             const uint32_t tS = tG + 128 * s, tDP = tS + 64;
-            uint8_t* ds_row = smem + OFF_DS + (pair & 1) * 2 * TILE_B + s * TILE_B + row * 128;
-#pragma unroll 1
-            for (int c = 0; c < 2; ++c) {
+            uint8_t* ds_rows = smem + OFF_DS + (pair & 1) * 2 * TILE_B + s * TILE_B + (32 * (warp & 3) + (lane & 7)) * 128;
+            // Two keys and two neighbouring queries a fragment and thread: it needs the lse and delta of 8 queries.  With a key a thread it needed
+            // those of all 32, and the broadcast reads, four cycles of the shared memory each, held up the tensor core's operands: exact causal 128 x 1920
+            // rows 459 -> 442 us (step), 16 x 12287 929 -> 886, smooth 32 x 16384 644 -> 621, 32 x 131072 3.54 -> 3.41 ms.
+            const uint32_t ds_to = smem_u32(ds_rows) + (((4 * g + (lane >> 3)) ^ (lane & 7)) << 4);
+            uint64_t L[4], Dl[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              L[j] = *reinterpret_cast<const uint64_t*>(ld + 8 * j + 2 * (lane & 3));
+              Dl[j] = *reinterpret_cast<const uint64_t*>(ld + TILE + 8 * j + 2 * (lane & 3));
+              if (ANY) L[j] = fadd2(L[j], bias);
+            }
+#pragma unroll 2
+            for (int h = 0; h < 2; ++h) {
               uint32_t rs[16], rp[16], pk[8], dk[8];
-              tmem_ld16(tS + c * 16, rs);
-              tmem_ld16(tDP + c * 16, rp);
+              tmem_ld_16x256(tS + (h << 20), rs);
+              tmem_ld_16x256(tDP + (h << 20), rp);
               tmem_ld_fence16(rs);
               tmem_ld_fence16(rp);
+              // queries [0, hidden) of the group's do not count for a key row
+              int hidden[2] = {0, 0};
+              if (masked) {
 #pragma unroll
-              for (int i = 0; i < 16; i += 4) {
-                // four query columns: their (scaled) lse and delta, the same for every thread: broadcast reads
-                ulonglong2 L = *reinterpret_cast<const ulonglong2*>(ld + c * 16 + i);
-                const ulonglong2 Dl = *reinterpret_cast<const ulonglong2*>(ld + TILE + c * 16 + i);
-                if (ANY) { L.x = fadd2(L.x, bias); L.y = fadd2(L.y, bias); }
-                float p0, p1, p2, p3, d0, d1, d2, d3;
-                unpack_f2(ffma2(pack_u2(rs[i], rs[i + 1]), sc2, L.x), p0, p1);
-                unpack_f2(ffma2(pack_u2(rs[i + 2], rs[i + 3]), sc2, L.y), p2, p3);
-                p0 = fast_exp2(p0); p1 = fast_exp2(p1); p2 = fast_exp2(p2); p3 = fast_exp2(p3);
-                if (masked) {
-                  const int at = c * 16 + i;
-                  if (at < hidden) p0 = 0.f;
-                  if (at + 1 < hidden) p1 = 0.f;
-                  if (at + 2 < hidden) p2 = 0.f;
-                  if (at + 3 < hidden) p3 = 0.f;
+                for (int k = 0; k < 2; ++k) {
+                  const int row = 32 * (warp & 3) + 16 * h + 8 * k + (lane >> 2);
+                  if (flash) {
+                    if (diag) hidden[k] = row - 64 * s - 32 * g;               // queries before the key
+                    if (e * TILE + row >= p.m_k) hidden[k] = 32;               // past the last key
+                  } else if ((*drop >> (row & 31)) & 1u) {
+                    hidden[k] = 32;
+                  }
                 }
-                // ds = p * (dp - delta) * scale
-                unpack_f2(fmul2(pack_f2(p0, p1), ffma2(pack_u2(rp[i], rp[i + 1]), scl, Dl.x)), d0, d1);
-                unpack_f2(fmul2(pack_f2(p2, p3), ffma2(pack_u2(rp[i + 2], rp[i + 3]), scl, Dl.y)), d2, d3);
-                pk[i >> 1] = pack2<T>(p0, p1);
-                pk[(i >> 1) + 1] = pack2<T>(p2, p3);
-                dk[i >> 1] = pack2<T>(d0, d1);
-                dk[(i >> 1) + 1] = pack2<T>(d2, d3);
               }
-              // P^T / dS^T of the chunk (8 packed columns) over columns this thread has already consumed
-              tmem_st8(tS + c * 8, pk);
-              tmem_st8(tDP + c * 8, dk);
 #pragma unroll
-              for (int j = 0; j < 2; ++j)
-                *reinterpret_cast<uint4*>(ds_row + (((4 * g + c * 2 + j) ^ (row & 7)) << 4)) = make_uint4(dk[4 * j], dk[4 * j + 1], dk[4 * j + 2], dk[4 * j + 3]);
+              for (int j = 0; j < 4; ++j) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                  const int i = 4 * j + 2 * k, at = 8 * j + 2 * (lane & 3);
+                  float p0, p1, d0, d1;
+                  unpack_f2(ffma2(pack_u2(rs[i], rs[i + 1]), sc2, L[j]), p0, p1);
+                  p0 = fast_exp2(p0); p1 = fast_exp2(p1);
+                  if (masked) {
+                    if (at < hidden[k]) p0 = 0.f;
+                    if (at + 1 < hidden[k]) p1 = 0.f;
+                  }
+                  // ds = p * (dp - delta) * scale
+                  unpack_f2(fmul2(pack_f2(p0, p1), ffma2(pack_u2(rp[i], rp[i + 1]), scl, Dl[j])), d0, d1);
+                  pk[2 * j + k] = pack2<T>(p0, p1);
+                  dk[2 * j + k] = pack2<T>(d0, d1);
+                }
+              }
+              // P^T / dS^T (16 packed columns) over columns this warp has consumed
+              tmem_st_16x128(tS + (h << 20), pk);
+              tmem_st_16x128(tDP + (h << 20), dk);
+#pragma unroll
+              for (int k = 0; k < 2; ++k) store_matrix_x4(ds_to + (16 * h + 8 * k) * 128, dk[k], dk[2 + k], dk[4 + k], dk[6 + k]);
             }
             HA_T_MARK(3)
             tmem_st_wait();
