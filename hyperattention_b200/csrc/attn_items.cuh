@@ -8,7 +8,10 @@ namespace ha {
 
 struct AttnPlan {
   FastDiv by_pairs, by_segs, by_heads, by_group, by_block;     // pairs, segs_per_head, H, kv_group, window tiles per block
-  int n_items, pairs;                 // items = pairs of query tiles x segments
+  int n_items, pairs;                 // items = pairs of query tiles (or key tiles) x segments
+  // exact causal attention (plan_order): items of a round, its segments, the segments after the whole rounds; by_length = 0: no rounds
+  FastDiv by_round, by_round_segs, by_rest;
+  int by_length, round_segs, whole_items, whole_segs, rest_segs;
   int tiles, rows;                    // contiguous rows may be loaded as TMA boxes / indexed rows of q (1) and k (2) by gather4
   int row_sb[2], row_sh[2], row_sn[2];   // row maps of q, k: steps of the row number per batch, head and row
 };
@@ -28,23 +31,49 @@ struct AttnItem {
   __device__ __forceinline__ int count(int g) const { return (g == 0 || has1) ? hi(g) - lo(g) + n_list - n_win : 0; }
 };
 
+// Exact causal attention: the items of a segment differ in length (place 0: the longest), and CTA c takes items c, c + grid, ... of one
+// order.  That order is by length over a round of segments -- as many as make whole turns of the grid (37 for 4, 8, 12 or 16 places and 148
+// CTAs) --, then over the segments that are left; every other turn the CTAs take theirs in the opposite direction
+// (item_of_turn).  Lengths are dealt out evenly that way: the longest CTA has 0 to 7% more than the average, where the segments' own order
+// gave 4 to 50% (segments x places: 64 x 8 4 for 50%, 128 x 6 6 for 40, 128 x 8 6 for 23, 256 x 8 1 for 10, 128 x 16 1 for 16).
+// Training steps: 16 heads x 12287 x 64 (128 x 6) 889 -> 840 us, 128 x 1920 x 64 442 -> 420, 2 x 16 heads x 8192 x 128 (128 x 8, x 16 in the backward)
+// 1360 -> 1337, 256 x 2047 x 128 1538 -> 1514.
+__device__ __forceinline__ int item_of_turn(const AttnPlan& pl, int turn) {
+  return turn * gridDim.x + (pl.by_length && (turn & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+}
+__device__ __forceinline__ int causal_place(const AttnPlan& pl, int item, int& seg) {
+  int place;
+  if (!pl.by_length) {
+    // the segments' own order; with few places turned by the segment, so that a CTA, which takes every 148th item, meets all lengths
+    seg = pl.by_pairs(item);
+    place = item - seg * pl.pairs;
+    if (pl.pairs <= 32) place += seg - pl.by_pairs(place + seg) * pl.pairs;
+  } else if (item < pl.whole_items) {
+    const int round = pl.by_round(item);
+    item -= round * pl.round_segs * pl.pairs;
+    place = pl.by_round_segs(item);
+    seg = round * pl.round_segs + item - place * pl.round_segs;
+  } else {
+    item -= pl.whole_items;
+    place = pl.by_rest(item);
+    seg = pl.whole_segs + item - place * pl.rest_segs;
+  }
+  return place;
+}
+
 // by_keys: enumerate the pairs of smooth windows per KEY tile with the forward's window formula, as the reference's backward does
 // (src/hyper_attn_triton.py:290-325): key tile t meets the sorted queries [128 t - 64 (bs - 1), ...); the query tiles are then
 // shifted by half a tile when bs is even.  Needs whole blocks (m_k a multiple of bs tiles).
 __device__ __forceinline__ AttnItem attn_item(const ha_attn_params& p, const AttnPlan& pl, int item, bool flash, bool by_keys = false) {
   AttnItem it;
-  it.seg = pl.by_pairs(item);
-  int pr = item - it.seg * pl.pairs;
-  const int n_qt = (p.m_q + TILE - 1) / TILE;
+  int pr;
   if (flash && (p.flags & HA_FLAG_CAUSAL)) {
-    // Items grow with the pair.  Long pairs first; with few pairs the order is turned by the segment, so that a CTA, which
-    // takes every 148th item, meets all lengths.  Exact causal attention, turned against not (forward): 64 x 32 heads x 2048 rows 1.79 against
-    // 2.35 ms, 8 x 32 x 1024 82 against 113 us, where items outnumber CTAs many times; 32 heads x 2048 66 against 53 us, x 4096 168
-    // against 150, x 8192 567 against 473, where they do not; 8 heads x 16384 (64 pairs) 545 against 590.  The line at 32 pairs serves the leaves
-    // of causal calls (up to 2048 rows, many segments).
-    pr = pl.pairs - 1 - pr;
-    if (pl.pairs <= 32) pr += it.seg - pl.by_pairs(pr + it.seg) * pl.pairs;
+    pr = pl.pairs - 1 - causal_place(pl, item, it.seg);
+  } else {
+    it.seg = pl.by_pairs(item);
+    pr = item - it.seg * pl.pairs;
   }
+  const int n_qt = (p.m_q + TILE - 1) / TILE;
   it.qt0 = 2 * pr;
   it.q_pos0 = it.qt0 * TILE;
   it.has1 = it.qt0 + 1 < n_qt;
@@ -150,6 +179,29 @@ inline bool plan_items(AttnPlan& pl, const ha_attn_params& p) {
   pl.by_group = FastDiv(p.kv_group > 1 ? p.kv_group : 1);
   pl.by_block = FastDiv(p.mode == HA_MODE_HYPER ? (p.block_size + TILE - 1) / TILE : 1);
   return true;
+}
+// The order of the items (causal_place) for a launch of `grid` CTAs; after n_items and pairs.  Rounds whose segments leave L2 (126 MB) lose more
+// than the balance gives: with all segments as one round, 8 x 32 heads x 2047 x 128 took 1807 instead of 1600 us (537 MB of fp32 dK / dV and
+// their like), 128 x 2048 x 128 1459 instead of 1404 (268 MB), 128 x 1536 x 64 925 instead of 990 (100 MB).  With more than two segments a CTA the
+// segments' own order is even enough: rounds cost 1 to 3% there (2048 x 2048 x 64, step of 32 heads x 131072: 18.97 -> 19.56 ms; 512 x 2048 x 128,
+// forward: 1795 -> 1814 us).
+inline void plan_order(AttnPlan& pl, const ha_attn_params& p, int grid) {
+  pl.by_length = 0;
+  if (p.mode != HA_MODE_FLASH || !(p.flags & HA_FLAG_CAUSAL) || grid <= 0) return;
+  int a = grid, b = pl.pairs;
+  while (b) { const int r = a % b; a = b; b = r; }          // a: greatest common divisor
+  const int segs = pl.n_items / pl.pairs;
+  pl.round_segs = grid / a;
+  const long long round_items = (long long)pl.round_segs * pl.pairs, over = (long long)pl.n_items - 2 * grid;      // (two turns at least stay for the rest)
+  const int rounds = over > 0 ? (int)(over / round_items) : 0;
+  pl.whole_segs = rounds * pl.round_segs;
+  pl.whole_items = pl.whole_segs * pl.pairs;
+  pl.rest_segs = segs - pl.whole_segs;
+  pl.by_round = FastDiv((uint32_t)round_items);
+  pl.by_round_segs = FastDiv(pl.round_segs);
+  pl.by_rest = FastDiv(pl.rest_segs);
+  const long long at_a_time = rounds > 0 ? pl.round_segs : pl.rest_segs;
+  pl.by_length = segs <= 2 * grid && at_a_time * p.m_k * (p.d + p.dv) * 4 / (p.kv_group > 1 ? p.kv_group : 1) <= (126LL << 20);
 }
 // May tiles of contiguous rows come as TMA boxes?  A box that runs past the end of a segment brings the next segment's rows, where cp.async
 // fills with zeros: hidden weights are 0, but 0 times a row that is not finite is not.  (Past the last row of all, the map

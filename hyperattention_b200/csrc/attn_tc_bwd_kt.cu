@@ -99,13 +99,15 @@ __device__ __forceinline__ KtItem kt_item(const ha_attn_params& p, const AttnPla
     it.y0 = 0; it.y1 = 2;
     return it;
   }
-  // Key tile kt of its segment.  Causal items shrink with kt: long ones first; with few of them the order is turned by the segment, so
-  // that a CTA, which takes every 148th item, meets all lengths (the line as in attn_item, where it is measured; here 32 heads x 2048 take 214 us
-  // turned against 194, 32 x 4096 541 against 525, 8 x 8192 no difference).
+  // Key tile kt of its segment; causal items shrink with kt
   const bool causal = p.flags & HA_FLAG_CAUSAL;
-  it.seg = pl.by_pairs(item);
-  int kt = item - it.seg * pl.pairs;
-  if (causal && pl.pairs <= 32) kt += it.seg - pl.by_pairs(kt + it.seg) * pl.pairs;
+  int kt;
+  if (causal) {
+    kt = causal_place(pl, item, it.seg);
+  } else {
+    it.seg = pl.by_pairs(item);
+    kt = item - it.seg * pl.pairs;
+  }
   it.qt0 = 0; it.has1 = 1; it.q_pos0 = 0; it.first = 0; it.lo1 = 0;
   it.hi0 = it.hi1 = it.n_win = it.n_list = kt + 1;
   it.e0 = kt; it.e1 = kt + 1;
@@ -608,7 +610,7 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
         for (; published <= (int)n_item + 2; ++published) {
           const uint32_t at = published % ND;
           it.n_list = 0;
-          const int item = blockIdx.x + published * gridDim.x;
+          const int item = item_of_turn(pl, published);
           if (item < pl.n_items) it = kt_item(p, pl, item, flash, by_keys);
           if (published >= ND && !wait(B_D_EMPTY + at, (published / ND - 1) & 1)) return false;
           if (lane == 0) {
@@ -867,8 +869,9 @@ static int launch_kt_bwd(const ha_attn_params& p, cudaStream_t st) {
   int dyn_bytes;
   HA_WINDOW_BYTES(dyn_bytes, (attn_tc_bwd_kt_kernel<T, KIND>), bkt::SMEM_USED, "ha_attn_bwd kernel attributes");
   HA_SMEM_ATTR_ONCE((attn_tc_bwd_kt_kernel<T, KIND>), dyn_bytes, "ha_attn_bwd smem attribute");
-  const int sms = sm_count();
-  attn_tc_bwd_kt_kernel<T, KIND><<<(unsigned)(pl.n_items < sms ? pl.n_items : sms), bkt::THREADS, dyn_bytes, st>>>(p, pl, maps);
+  const int sms = sm_count(), grid = pl.n_items < sms ? pl.n_items : sms;
+  plan_order(pl, p, grid);
+  attn_tc_bwd_kt_kernel<T, KIND><<<grid, bkt::THREADS, dyn_bytes, st>>>(p, pl, maps);
   HA_LAUNCHED("ha_attn_bwd (tcgen05, by key tiles)");
   return HA_OK;
 }

@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
         for (; published <= (int)n_item + 2; ++published) {
           const uint32_t slot = published % ND;
           it.n_list = 0;
-          const int item = blockIdx.x + published * gridDim.x;
+          const int item = item_of_turn(pl, published);
           if (item < pl.n_items) it = attn_item(p, pl, item, flash, by_keys);
           if (published >= ND && !wait(B_D_EMPTY + slot, (published / ND - 1) & 1)) return false;
           if (lane == 0) {
@@ -824,8 +824,9 @@ static int launch_ws_bwd(const ha_attn_params& p, bool store_dq, cudaStream_t st
   int dyn_bytes;
   HA_WINDOW_BYTES(dyn_bytes, (attn_tc_bwd_ws_kernel<T, KIND>), bws::SMEM_USED, "ha_attn_bwd kernel attributes");
   HA_SMEM_ATTR_ONCE((attn_tc_bwd_ws_kernel<T, KIND>), dyn_bytes, "ha_attn_bwd smem attribute");
-  const int sms = sm_count();
-  attn_tc_bwd_ws_kernel<T, KIND><<<(unsigned)(pl.n_items < sms ? pl.n_items : sms), bws::THREADS, dyn_bytes, st>>>(p, pl, out, maps);
+  const int sms = sm_count(), grid = pl.n_items < sms ? pl.n_items : sms;
+  plan_order(pl, p, grid);
+  attn_tc_bwd_ws_kernel<T, KIND><<<grid, bws::THREADS, dyn_bytes, st>>>(p, pl, out, maps);
   HA_LAUNCHED("ha_attn_bwd (tcgen05, warp-specialised)");
   return HA_OK;
 }

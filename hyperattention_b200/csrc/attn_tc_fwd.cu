@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
         for (; published <= (int)n_item + 2; ++published) {
           const uint32_t slot = published % ND;
           it.n_list = 0;
-          const int item = blockIdx.x + published * gridDim.x;
+          const int item = item_of_turn(pl, published);
           if (item < pl.n_items) it = attn_item(p, pl, item, flash);
           if (published >= ND && !wait(B_D_EMPTY + slot, (published / ND - 1) & 1)) return false;
           if (lane == 0) {
@@ -658,8 +658,9 @@ static int launch_fwd(const ha_attn_params& p, cudaStream_t st) {
   int dyn_bytes;
   HA_WINDOW_BYTES(dyn_bytes, (attn_tc_fwd_kernel<T, D, DV, KIND>), Cfg::SMEM_USED, "ha_attn_fwd kernel attributes");
   HA_SMEM_ATTR_ONCE((attn_tc_fwd_kernel<T, D, DV, KIND>), dyn_bytes, "ha_attn_fwd smem attribute");
-  const int sms = sm_count();
-  attn_tc_fwd_kernel<T, D, DV, KIND><<<(unsigned)(pl.n_items < sms ? pl.n_items : sms), fw::THREADS, dyn_bytes, st>>>(p, pl, maps);
+  const int sms = sm_count(), grid = pl.n_items < sms ? pl.n_items : sms;
+  plan_order(pl, p, grid);
+  attn_tc_fwd_kernel<T, D, DV, KIND><<<grid, fw::THREADS, dyn_bytes, st>>>(p, pl, maps);
   HA_LAUNCHED("ha_attn_fwd (tcgen05)");
   return HA_OK;
 }

@@ -566,3 +566,24 @@ def test_fp32_sums_are_made_of_short_chains(d):
     oe.backward(do.double())
     err = [((a.double() - b).norm() / b.norm()).item() for a, b in ((o, oe), (qg.grad, qe.grad), (kg.grad, ke.grad), (vg.grad, ve.grad))]
     assert max(err) < 4.5e-7, err
+
+
+@pytest.mark.parametrize('d', [64, 128])
+@pytest.mark.parametrize('n,H', [(600, 5), (512, 230), (640, 250), (330, 300)])
+def test_causal_items_are_dealt_out_once_each(d, n, H):
+    """exact causal attention with fewer items than CTAs, whole rounds of segments and a rest (even and odd numbers of pairs), more than two segments
+    a CTA (the segments' own order): every head's outputs and gradients"""
+    import hyperattention_b200 as ha
+    torch.manual_seed(95)
+    q, k, v, do = [torch.randn(1, n, H, d, device='cuda').bfloat16() for _ in range(4)]
+    qg, kg, vg = [t.clone().requires_grad_() for t in (q, k, v)]
+    o, lse = ha.flash_attn_func(qg, kg, vg, None, True)
+    o.backward(do)
+    qc, kc, vc = [T(t).double().requires_grad_() for t in (q, k, v)]
+    s = (qc @ kc.transpose(2, 3) * d ** -0.5).masked_fill(torch.ones(n, n, dtype=torch.bool, device='cuda').triu(1), float('-inf'))
+    ow = s.softmax(-1) @ vc
+    ow.backward(T(do).double())
+    for got, want, tol in ((o, ow, 0), (qg.grad, qc.grad, 1), (kg.grad, kc.grad, 1), (vg.grad, vc.grad, 1)):
+        err = (T(got).double() - want).flatten(2).norm(dim=2) / want.flatten(2).norm(dim=2)
+        assert err.max() < TOL[torch.bfloat16][tol], (err.max(), err.argmax())
+    assert (lse[:, :, :n].double() - s.logsumexp(-1)).abs().max() < 1e-4
