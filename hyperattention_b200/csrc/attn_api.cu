@@ -63,6 +63,7 @@ static int check_common(const ha_attn_params& p, bool backward) {
 
 template <typename T>
 __global__ void bwd_finish_kernel(const ha_attn_params p, long long total, const bool tiled) {
+  chain_begin();
   // one thread per (segment, slot, 8 elements of dk | dv)
   const int cpr_k = p.d / 8, cpr = cpr_k + p.dv / 8;
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -209,8 +210,8 @@ int ha_attn_bwd_finish(const ha_attn_params* p, void* stream) {
   if ((total + 255) / 256 > 0x7fffffffLL) return HA_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
   const bool tiled = !(p->flags & HA_FLAG_FORCE_SIMT) && ws_bwd_supported(*p);     // which kernel filled the slot buffers
-  if (p->dtype == HA_BF16) bwd_finish_kernel<__nv_bfloat16><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(*p, total, tiled);
-  else bwd_finish_kernel<__half><<<(unsigned)((total + 255) / 256), 256, 0, st>>>(*p, total, tiled);
+  if (p->dtype == HA_BF16) launch_chained(bwd_finish_kernel<__nv_bfloat16>, (unsigned)((total + 255) / 256), 256, 0, st, *p, total, tiled);
+  else launch_chained(bwd_finish_kernel<__half>, (unsigned)((total + 255) / 256), 256, 0, st, *p, total, tiled);
   HA_LAUNCHED("ha_attn_bwd_finish");
   return HA_OK;
 }

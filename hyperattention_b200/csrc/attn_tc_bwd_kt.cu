@@ -150,6 +150,7 @@ __device__ __forceinline__ void warp_gather_unit(uint32_t dst, const uint16_t* _
 
 template <typename T, int KIND>
 __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const ha_attn_params p, const AttnPlan pl, const __grid_constant__ KtMaps maps) {
+  chain_begin();
   using namespace bkt;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -871,7 +872,7 @@ static int launch_kt_bwd(const ha_attn_params& p, cudaStream_t st) {
   HA_SMEM_ATTR_ONCE((attn_tc_bwd_kt_kernel<T, KIND>), dyn_bytes, "ha_attn_bwd smem attribute");
   const int sms = sm_count(), grid = pl.n_items < sms ? pl.n_items : sms;
   plan_order(pl, p, grid);
-  attn_tc_bwd_kt_kernel<T, KIND><<<grid, bkt::THREADS, dyn_bytes, st>>>(p, pl, maps);
+  launch_chained((attn_tc_bwd_kt_kernel<T, KIND>), grid, bkt::THREADS, dyn_bytes, st, p, pl, maps);
   HA_LAUNCHED("ha_attn_bwd (tcgen05, by key tiles)");
   return HA_OK;
 }

@@ -116,6 +116,7 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src) {
 template <typename T, int KIND>
 __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const ha_attn_params p, const AttnPlan pl, const BwdOut out,
                                                                          const __grid_constant__ BwdMaps maps) {
+  chain_begin();
   using namespace bws;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -826,7 +827,7 @@ static int launch_ws_bwd(const ha_attn_params& p, bool store_dq, cudaStream_t st
   HA_SMEM_ATTR_ONCE((attn_tc_bwd_ws_kernel<T, KIND>), dyn_bytes, "ha_attn_bwd smem attribute");
   const int sms = sm_count(), grid = pl.n_items < sms ? pl.n_items : sms;
   plan_order(pl, p, grid);
-  attn_tc_bwd_ws_kernel<T, KIND><<<grid, bws::THREADS, dyn_bytes, st>>>(p, pl, out, maps);
+  launch_chained((attn_tc_bwd_ws_kernel<T, KIND>), grid, bws::THREADS, dyn_bytes, st, p, pl, out, maps);
   HA_LAUNCHED("ha_attn_bwd (tcgen05, warp-specialised)");
   return HA_OK;
 }

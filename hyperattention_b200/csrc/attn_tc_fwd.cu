@@ -60,6 +60,7 @@ struct FwdMaps { CUtensorMap tile[3], rows[2]; };    // tiles of q, k, v; rows o
 enum { FWD_HYPER = 0, FWD_FLASH = 1, FWD_ANY = 2 };
 template <typename T, int D, int DV, int KIND>
 __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_attn_params p, const AttnPlan pl, const __grid_constant__ FwdMaps maps) {
+  chain_begin();
   using namespace fw;
   using Cfg = FwdCfg<D, DV>;
   constexpr int NQ = Cfg::NQ, NKV = Cfg::NKV, NB = Cfg::NB;
@@ -660,7 +661,7 @@ static int launch_fwd(const ha_attn_params& p, cudaStream_t st) {
   HA_SMEM_ATTR_ONCE((attn_tc_fwd_kernel<T, D, DV, KIND>), dyn_bytes, "ha_attn_fwd smem attribute");
   const int sms = sm_count(), grid = pl.n_items < sms ? pl.n_items : sms;
   plan_order(pl, p, grid);
-  attn_tc_fwd_kernel<T, D, DV, KIND><<<grid, fw::THREADS, dyn_bytes, st>>>(p, pl, maps);
+  launch_chained((attn_tc_fwd_kernel<T, D, DV, KIND>), grid, fw::THREADS, dyn_bytes, st, p, pl, maps);
   HA_LAUNCHED("ha_attn_fwd (tcgen05)");
   return HA_OK;
 }

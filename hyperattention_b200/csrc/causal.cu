@@ -107,6 +107,7 @@ template <typename T, int EPC>
 __global__ void __launch_bounds__(256, 4) delta_parts_kernel(const T* __restrict__ d_o, const uint8_t* __restrict__ parts0, long long part_stride_bytes,
                                                              int levels, int n, int lpr, float* __restrict__ delta, long long total_rows,
                                                              int log2n) {
+  chain_release();
   constexpr int CH = 2, PG = 4;
   const int lane = threadIdx.x & 31;
   const int rpw = 32 / lpr, chunk = lane % lpr, sub = lane / lpr;
@@ -206,6 +207,7 @@ template <typename T, int CH>
 __global__ void __launch_bounds__(256, 4) merge_parts_kernel(const uint8_t* __restrict__ parts0, long long part_stride_bytes, long long lse_off_bytes,
                                                           int levels, int n, int lpr, T* __restrict__ o, int64_t o_sb, int64_t o_sh, int64_t o_sn,
                                                           FastDiv by_heads, int H, float* __restrict__ lse, long long total_rows, int exact, int log2n) {
+  chain_begin();
   constexpr int PG = 2;   // parts whose rows are requested together
   const int lane = threadIdx.x & 31;
   const int rpw = 32 / lpr, chunk = lane % lpr, sub = lane / lpr;
@@ -484,7 +486,7 @@ int ha_causal_fwd_strided(const ha_causal_params* pp, const int64_t* strides, vo
     const long long part_stride = slot_stride, lse_off = slot_lse;
     const int exact_merge = (p.flags & HA_FLAG_MERGE_EXACT) ? 1 : 0;
 #define HA_MERGE(TT, CH)                                                                                                                               \
-  merge_parts_kernel<TT, CH><<<grid, 256, 0, main_st>>>((const uint8_t*)slots, part_stride, lse_off, p.levels, p.n, lpr, (TT*)p.o, lay.o[0], lay.o[1],  \
+  launch_chained((merge_parts_kernel<TT, CH>), grid, 256, 0, main_st, (const uint8_t*)slots, part_stride, lse_off, p.levels, p.n, lpr, (TT*)p.o, lay.o[0], lay.o[1],  \
                                                         lay.o[2], FastDiv(p.H), p.H, p.lse, pl.rows, exact_merge, log2_if_pow2(p.n))
     if (p.dtype == HA_BF16 && ch == 2) HA_MERGE(__nv_bfloat16, 2);
     else if (p.dtype == HA_BF16) HA_MERGE(__nv_bfloat16, 1);

@@ -131,6 +131,7 @@ __device__ __forceinline__ const SortJob& job_of(const SortJobs& jobs, int block
 
 // digit counts of every chunk; grid: chunks
 __global__ void __launch_bounds__(512) sort_chunk_hist_kernel(const SortJobs jobs, int chunk) {
+  chain_begin();
   __shared__ uint32_t cnt[256];
   const SortJob& jb = job_of(jobs, blockIdx.x, &SortJob::first);
   const int at = blockIdx.x - jb.first, seg = at / jb.chunks, c = at - seg * jb.chunks, row = seg / jb.parts;
@@ -155,6 +156,7 @@ __global__ void __launch_bounds__(512) sort_chunk_hist_kernel(const SortJobs job
 
 // counts -> first slot of every (chunk, digit) run inside the segment; grid: segments
 __global__ void __launch_bounds__(256) sort_chunk_scan_kernel(const SortJobs jobs) {
+  chain_begin();
   __shared__ uint32_t wsum[8];
   const SortJob& jb = job_of(jobs, blockIdx.x, &SortJob::first_seg);
   uint32_t* h = jobs.hist + ((long long)jb.first + (long long)(blockIdx.x - jb.first_seg) * jb.chunks) * 256 + threadIdx.x;
@@ -185,6 +187,7 @@ __global__ void __launch_bounds__(256) sort_chunk_scan_kernel(const SortJobs job
 
 template <int W>
 __global__ void __launch_bounds__(W * 32) sort_chunk_kernel(const SortJobs jobs) {
+  chain_begin();
   constexpr int UN = 8, CHUNK = W * 32 * UN;
   extern __shared__ uint32_t sort_smem[];
   uint32_t (*cnt)[256] = reinterpret_cast<uint32_t (*)[256]>(sort_smem);
@@ -285,19 +288,19 @@ int SortJobs::run(uint32_t* workspace, cudaStream_t st) {
   if (chunks > 0x7fffffffLL) return HA_ERR_TOO_LARGE;
   hist = workspace;
   if (several) {
-    sort_chunk_hist_kernel<<<(unsigned)chunks, 512, 0, st>>>(*this, chunk);
+    launch_chained(sort_chunk_hist_kernel, (unsigned)chunks, 512, 0, st, *this, chunk);
     HA_LAUNCHED("ha_seg_sort hist");
-    sort_chunk_scan_kernel<<<(unsigned)segs, 256, 0, st>>>(*this);
+    launch_chained(sort_chunk_scan_kernel, (unsigned)segs, 256, 0, st, *this);
     HA_LAUNCHED("ha_seg_sort scan");
   }
   const int smem = 2 * chunk * 4;
   if (warps == 8) {
-    sort_chunk_kernel<8><<<(unsigned)chunks, 256, smem, st>>>(*this);
+    launch_chained(sort_chunk_kernel<8>, (unsigned)chunks, 256, smem, st, *this);
   } else if (warps == 16) {
-    sort_chunk_kernel<16><<<(unsigned)chunks, 512, smem, st>>>(*this);
+    launch_chained(sort_chunk_kernel<16>, (unsigned)chunks, 512, smem, st, *this);
   } else {
     HA_SMEM_ATTR_ONCE(sort_chunk_kernel<32>, smem, "ha_seg_sort smem attribute");
-    sort_chunk_kernel<32><<<(unsigned)chunks, 1024, smem, st>>>(*this);
+    launch_chained(sort_chunk_kernel<32>, (unsigned)chunks, 1024, smem, st, *this);
   }
   HA_LAUNCHED("ha_seg_sort");
   return HA_OK;

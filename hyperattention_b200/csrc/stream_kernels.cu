@@ -67,6 +67,7 @@ template <typename T, int RP, int UNROLL>
 __global__ void __launch_bounds__(256) lsh_hash_vec_kernel(const T* __restrict__ x, int64_t sb, int64_t sh, int64_t sn, int H, int n,
                                                            int d, const float* __restrict__ proj, int r, int32_t* __restrict__ codes,
                                                            long long total_rows) {
+  chain_release();
   constexpr int EPC = Vec16<T>::N;
   const int lane = threadIdx.x & 31;
   const int lpr = d / EPC;            // lanes per row: 8, 16 or 32
@@ -161,6 +162,7 @@ struct HashSrc {
 template <typename T, int CH, int NSET, int UNROLL>
 __global__ void __launch_bounds__(256, 4) lsh_hash_mma_kernel(const HashSrc src0, const HashSrc src1, FastDiv by_n, int n,
                                                            const float* __restrict__ proj, int r) {
+  chain_release();
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   // B fragments: for chunk c, MMA m (0/1), register j (0/1): projection column (set*8 + g), rows c*32 + 8t + 4m + 2j + {0,1}
@@ -414,6 +416,7 @@ template <typename T>
 __global__ void __launch_bounds__(256, 4) delta_vec_kernel(const T* __restrict__ o, int64_t osb, int64_t osh, int64_t osn, const T* __restrict__ go,
                                                            int64_t gsb, int64_t gsh, int64_t gsn, FastDiv by_n, FastDiv by_heads, int H, int n, int lpr,
                                                            float* __restrict__ delta, int total_rows) {
+  chain_release();
   constexpr int EPC = Vec16<T>::N, UN = 2;
   const int lane = threadIdx.x & 31;
   const int rpw = 32 / lpr, chunk = lane % lpr, sub = lane / lpr;
@@ -549,6 +552,7 @@ using namespace ha;
 // (keys already inside the tile's block window) and the log importance weight of the kept ones.
 // ---------------------------------------------------------------------------------------------------
 __global__ void invert_perm_kernel(const int32_t* __restrict__ idx, int32_t* __restrict__ inv, int m, long long total) {
+  chain_begin();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const long long seg = i / m;
@@ -558,6 +562,7 @@ __global__ void invert_perm_kernel(const int32_t* __restrict__ idx, int32_t* __r
 __global__ void __launch_bounds__(128) sample_weights_kernel(const int32_t* __restrict__ inv, const int32_t* __restrict__ sample_idx,
                                                              int m, int bs, int S, int smooth, float* __restrict__ tile_logw,
                                                              uint32_t* __restrict__ tile_mask) {
+  chain_begin();
   const int t = blockIdx.x, T_ = gridDim.x;
   const long long seg = blockIdx.y;
   const ha::Window w = ha::block_window(t, bs, m, smooth != 0);
@@ -804,9 +809,9 @@ int ha_sample_weights(const int32_t* k_idx, const int32_t* sample_idx, int32_t s
   cudaStream_t st = (cudaStream_t)stream;
   const long long total = (long long)segs * m;
   if ((total + 255) / 256 > 0x7fffffffLL) return HA_ERR_TOO_LARGE;
-  invert_perm_kernel<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(k_idx, inv_workspace, m, total);
+  launch_chained(invert_perm_kernel, (unsigned)((total + 255) / 256), 256, 0, st, k_idx, inv_workspace, m, total);
   HA_LAUNCHED("ha_sample_weights (invert)");
-  sample_weights_kernel<<<dim3(m / TILE, segs), 128, 0, st>>>(inv_workspace, sample_idx, m, (block_size + TILE - 1) / TILE,
+  launch_chained(sample_weights_kernel, dim3(m / TILE, segs), 128, 0, st, inv_workspace, sample_idx, m, (block_size + TILE - 1) / TILE,
                                                              sample_size, smooth, tile_logw, tile_mask);
   HA_LAUNCHED("ha_sample_weights");
   return HA_OK;
