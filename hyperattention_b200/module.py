@@ -178,9 +178,7 @@ class HyperAttention(torch.nn.Module):
         if causal is False:
             attn, lse = self.forward_no_causal_mask(query, key, value, scale)
         elif n_key <= self.min_seq_len:
-            attn, lse = ops.flash_attn_func(query.transpose(1, 2), key.transpose(1, 2), value.transpose(1, 2), None, True,
-                                            scale, self.kernel_flags & L.FLAG_FORCE_SIMT, return_lse)
-            attn = attn.transpose(1, 2)
+            attn, lse = ops.exact_causal(query, key, value, scale, self.kernel_flags & L.FLAG_FORCE_SIMT, return_lse)
         elif self.fused_causal and self.sampling == 'reference' and self._regular_causal(n_key):
             attn, lse = ops.causal_hyper(query, key, value, self.lsh.proj_f32(), self._causal_levels(n_key + n_key % 2),
                                          self.block_size, self.sample_size, scale, self._flags(),

@@ -433,18 +433,20 @@ def hyper_attn_func(q, k, v, q_sort_idx, k_sort_idx, block_size, sample_size=0, 
                                sample_idx, flags, weighted)
 
 
-def _flash_forward(q, k, v, causal, softmax_scale, flags):
-    """Exact attention on [B, n, H, *] views with contiguous rows: o [B, n_q, H, dv] (in the memory order of q) and lse [B, H, n_q]."""
+def _flash_forward(q, k, v, causal, softmax_scale, flags, heads_first=False):
+    """Exact attention on [B, n, H, *] views (heads_first: [B, H, n, *] tensors) with contiguous rows: o of the same layout (in the memory order of q)
+    and lse [B, H, n_q]."""
     _cuda(q, k, v)
     B, nq, H, d = q.shape
-    nk = k.shape[1]
-    Hk = k.shape[2]              # fewer key / value heads: consecutive query heads share one
-    assert k.shape == (B, nk, Hk, d) and H % Hk == 0
-    assert v.shape[:3] == (B, nk, Hk)
+    _, nk, Hk, _ = k.shape
+    assert k.shape == (B, nk, Hk, d) and v.shape[:3] == (B, nk, Hk)
+    if heads_first:
+        nq, H, Hk = H, nq, nk
+    assert H % Hk == 0              # fewer key / value heads: consecutive query heads share one
     assert q.dtype == k.dtype == v.dtype, 'All tensors must have the same type'
-    o = _rows_like(q.transpose(1, 2), v.shape[-1]).transpose(1, 2)
+    o = _rows_like(q, v.shape[-1]) if heads_first else _rows_like(q.transpose(1, 2), v.shape[-1]).transpose(1, 2)
     lse = torch.empty(B, H, nq, dtype=torch.float32, device=q.device)
-    p = _flash_params(q, k, v, o, lse, causal, float(softmax_scale or 1.0 / math.sqrt(d)), flags)
+    p = _flash_params(q, k, v, o, lse, causal, float(softmax_scale or 1.0 / math.sqrt(d)), flags, heads_first)
     L.check(_call(L.load().ha_attn_fwd, q.device, C.byref(p)), 'ha_attn_fwd')
     return o, lse
 
@@ -497,24 +499,35 @@ def _pad_lse(lse):
     return lse if nq_r == nq else torch.nn.functional.pad(lse, (0, nq_r - nq))
 
 
-def _flash_params(q, k, v, o, lse, causal, scale, flags):
+def _flash_params(q, k, v, o, lse, causal, scale, flags, heads_first=False):
     def fill(p):
-        B, nq, H, d = q.shape
-        nk, dv = k.shape[1], v.shape[-1]
+        rows = [x.transpose(1, 2) if heads_first else x for x in (q, k, v, o)]
+        B, nq, H, d = rows[0].shape
+        nk, dv = rows[1].shape[1], v.shape[-1]
         p.mode, p.dtype = L.MODE_FLASH, _dtype_id(q)
         p.flags = (L.FLAG_CAUSAL if causal else 0) | flags
         p.B, p.H, p.n, p.d, p.dv = B, H, nq, d, dv
         p.segs_per_head, p.span, p.q_off, p.k_off, p.m_q, p.m_k = 1, nq, 0, 0, nq, nk
         p.scale = scale
-        p.kv_group = H // k.shape[2]
-        p.q_sb, p.q_sh, p.q_sn = _bhn(q)
-        p.k_sb, p.k_sh, p.k_sn = _bhn(k)
-        p.v_sb, p.v_sh, p.v_sn = _bhn(v)
-        p.o_sb, p.o_sh, p.o_sn = _bhn(o)
-    p = _template(L.AttnParams, (0, q.dtype, q.shape, k.shape[1:3], v.shape[-1], q.stride(), k.stride(), v.stride(), o.stride(), causal, scale, flags), fill)
+        p.kv_group = H // rows[1].shape[2]
+        p.q_sb, p.q_sh, p.q_sn = _bhn(rows[0])
+        p.k_sb, p.k_sh, p.k_sn = _bhn(rows[1])
+        p.v_sb, p.v_sh, p.v_sn = _bhn(rows[2])
+        p.o_sb, p.o_sh, p.o_sn = _bhn(rows[3])
+    p = _template(L.AttnParams, (heads_first, q.dtype, q.shape, k.shape[1:3], v.shape[-1], q.stride(), k.stride(), v.stride(), o.stride(), causal, scale, flags), fill)
     p.q, p.k, p.v, p.o, p.lse = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr()
     _set_status(p, q.device)
     return p
+
+
+def exact_causal(q, k, v, scale, flags, pad_lse):
+    """Exact causal attention on [B, H, n, *] tensors with contiguous rows: (o [B, H, n, dv], lse).  Without a gradient to keep the tensors go
+    to the kernel as they are: the six views that flash_attn_func's layout takes were a seventh of a short call's host time (@@M@@)."""
+    if _wants_grad(q, k, v):
+        o, lse = flash_attn_func(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), None, True, scale, flags, pad_lse)
+        return o.transpose(1, 2), lse
+    o, lse = _flash_forward(q, k, v, True, scale, flags, True)
+    return o, _pad_lse(lse) if pad_lse else lse
 
 
 def flash_attn_func(q, k, v, bias=None, causal=False, softmax_scale=None, flags=0, pad_lse=True):
