@@ -522,7 +522,7 @@ def _flash_params(q, k, v, o, lse, causal, scale, flags, heads_first=False):
 
 def exact_causal(q, k, v, scale, flags, pad_lse):
     """Exact causal attention on [B, H, n, *] tensors with contiguous rows: (o [B, H, n, dv], lse).  Without a gradient to keep the tensors go
-    to the kernel as they are: the six views that flash_attn_func's layout takes were a seventh of a short call's host time (@@M@@)."""
+    to the kernel as they are: the six views that flash_attn_func's layout takes were a seventh of a short call's host time."""
     if _wants_grad(q, k, v):
         o, lse = flash_attn_func(q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), None, True, scale, flags, pad_lse)
         return o.transpose(1, 2), lse
