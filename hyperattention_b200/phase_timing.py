@@ -21,7 +21,7 @@ EW = ['loop, item set-up', 'wait S^T / dP^T ready', 'lse / delta scaling, wait d
 ISSUE = ['loop, item set-up', 'wait operand tile', 'wait inputs / accumulator', 'issue', 'tile done']
 LOAD = ['row numbers', 'wait slot free', 'issue copies']
 ROLES = {0: ('elementwise group 0', EW), 1: ('elementwise group 1', EW),
-         2: ('drain group', ['loop, item set-up', 'row numbers, wait staging tile', 'wait accumulator complete', 'out of TMEM, staged, stored']),
+         2: ('drain group of dV', ['loop, item set-up', 'row numbers', 'wait accumulator complete', 'out of TMEM, staged, stored']),
          3: ('K loader', LOAD), 4: ('S^T warp', ISSUE), 5: ('dV warp', ISSUE), 6: ('dQ warp', ISSUE), 7: ('Q / dO loader', LOAD)}
 
 # attn_tc_bwd_kt_kernel (head dim 128)
