@@ -65,7 +65,7 @@ enum {
   B_QD_FULL = 8,      // 2 x 64: the loader's lanes through their copies, and for what they stored themselves
   B_QD_EMPTY = 10,    // 2 x 4: the S^T, dP^T, dV and dK warps
   B_S_READY = 12,     // 2 x 2: S^T and dP^T of a half are in TMEM
-  B_P_READY = 14,     // 2 x 128: its elementwise group has written P^T / dS^T
+  B_P_READY = 14,     // 2 x 256: both elementwise groups have written P^T / dS^T of the half
   B_SF_S = 16,        // 2 x 1: dV of the stage's half completed: its S^T columns may be overwritten
   B_SF_P = 18,        // 2 x 1: dK ...: its dP^T columns
   B_DS_FULL = 20,     // 2 x 256: both halves' dS slabs of a pair are in the buffer
