@@ -9,9 +9,10 @@ namespace ha {
 struct AttnPlan {
   FastDiv by_pairs, by_segs, by_heads, by_group, by_block;     // pairs, segs_per_head, H, kv_group, window tiles per block
   int n_items, pairs;                 // items = pairs of query tiles (or key tiles) x segments
-  // exact causal attention (plan_order): items of a round, its segments, the segments after the whole rounds; by_length = 0: no rounds
+  // exact causal attention (plan_order): items of a round, its segments, the segments after the whole rounds; by_length = 0: no rounds, the
+  // segments' own order, a segment's places turned by turn times its number
   FastDiv by_round, by_round_segs, by_rest;
-  int by_length, round_segs, whole_items, whole_segs, rest_segs;
+  int by_length, turn, round_segs, whole_items, whole_segs, rest_segs;
   int tiles, rows;                    // contiguous rows may be loaded as TMA boxes / indexed rows of q (1) and k (2) by gather4
   int row_sb[2], row_sh[2], row_sn[2];   // row maps of q, k: steps of the row number per batch, head and row
 };
@@ -38,16 +39,19 @@ struct AttnItem {
 // gave 4 to 50% (segments x places: 64 x 8 4 for 50%, 128 x 6 6 for 40, 128 x 8 6 for 23, 256 x 8 1 for 10, 128 x 16 1 for 16).
 // Training steps: 16 heads x 12287 x 64 (128 x 6) 889 -> 840 us, 128 x 1920 x 64 442 -> 420, 2 x 16 heads x 8192 x 128 (128 x 8, x 16 in the backward)
 // 1360 -> 1337, 256 x 2047 x 128 1538 -> 1514.
-__device__ __forceinline__ int item_of_turn(const AttnPlan& pl, int turn) {
-  return turn * gridDim.x + (pl.by_length && (turn & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+__host__ __device__ __forceinline__ int item_of_turn(const AttnPlan& pl, int turn, int cta, int grid) {
+  return turn * grid + (pl.by_length && (turn & 1) ? grid - 1 - cta : cta);
 }
-__device__ __forceinline__ int causal_place(const AttnPlan& pl, int item, int& seg) {
+__host__ __device__ __forceinline__ int causal_place(const AttnPlan& pl, int item, int& seg) {
   int place;
   if (!pl.by_length) {
-    // the segments' own order; with few places turned by the segment, so that a CTA, which takes every 148th item, meets all lengths
     seg = pl.by_pairs(item);
     place = item - seg * pl.pairs;
-    if (pl.pairs <= 32) place += seg - pl.by_pairs(place + seg) * pl.pairs;
+    if (pl.turn) {
+      const int by = seg - pl.by_pairs(seg) * pl.pairs;
+      place += pl.turn > 0 ? by : -by;
+      place += place < 0 ? pl.pairs : place >= pl.pairs ? -pl.pairs : 0;
+    }
   } else if (item < pl.whole_items) {
     const int round = pl.by_round(item);
     item -= round * pl.round_segs * pl.pairs;
@@ -180,6 +184,18 @@ inline bool plan_items(AttnPlan& pl, const ha_attn_params& p) {
   pl.by_block = FastDiv(p.mode == HA_MODE_HYPER ? (p.block_size + TILE - 1) / TILE : 1);
   return true;
 }
+// The segments' own order: by how much a segment's places are turned against the segment's before.  A CTA takes every 148th item, and should meet all
+// lengths on its way.  Unturned, its place advances by 148 mod places a turn, which goes evenly round all of an odd number of places, but only meets
+// one in 2 or 4 of an even one.  Turned, the place advances by some fraction more or less, and what decides between up and down is whether a few
+// such steps come back to where they began (22 places, up: 22.7 a turn, which is no step at all; 16, down: three steps are one round).  Longest CTA
+// over the average, mean of 297 to 1024 segments, down / up / unturned: 5 places 1.15 / 1.18 / 1.07, 7 1.10 / 1.11 / 1.08, 8 1.07 / 1.07 / 1.35, 14
+// 1.05 / 1.09 / 1.10, 16 1.10 / 1.05 / 1.20, 19 1.04 / 1.16 / 1.03, 22 1.04 / 1.09 / 1.07.  Forward of 512 x 1152 x 128 239 / 245 / 237 us, of
+// 320 x 4864 x 128 1930 / 2228 / 1903, of 320 x 4096 x 128 1577 / 1370 down / up.  Beyond 32 places: unturned.
+inline int own_order_turn(int places) {
+  if (places > 32 || (places % 2 == 1 && places < 20)) return 0;
+  constexpr uint32_t DOWN = 1u << 14 | 1u << 18 | 1u << 22 | 1u << 23 | 1u << 31;
+  return places < 32 && (DOWN >> places & 1) ? -1 : 1;
+}
 // The order of the items (causal_place) for a launch of `grid` CTAs; after n_items and pairs.  Rounds whose segments leave L2 (126 MB) lose more
 // than the balance gives: with all segments as one round, 8 x 32 heads x 2047 x 128 took 1807 instead of 1600 us (537 MB of fp32 dK / dV and
 // their like), 128 x 2048 x 128 1459 instead of 1404 (268 MB), 128 x 1536 x 64 925 instead of 990 (100 MB).  With more than two segments a CTA the
@@ -187,6 +203,7 @@ inline bool plan_items(AttnPlan& pl, const ha_attn_params& p) {
 // forward: 1795 -> 1814 us).
 inline void plan_order(AttnPlan& pl, const ha_attn_params& p, int grid) {
   pl.by_length = 0;
+  pl.turn = own_order_turn(pl.pairs);
   if (p.mode != HA_MODE_FLASH || !(p.flags & HA_FLAG_CAUSAL) || grid <= 0) return;
   int a = grid, b = pl.pairs;
   while (b) { const int r = a % b; a = b; b = r; }          // a: greatest common divisor

@@ -1,0 +1,79 @@
+"""The order in which the tensor-core kernels' CTAs take the items of an exact causal launch (csrc/attn_items.cuh), worked out on the host by the
+kernels' own functions."""
+import ctypes as C
+import os
+import subprocess
+import sys
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), 'hyperattention_b200', 'csrc')
+SOURCE = r'''
+#include "attn_items.cuh"
+using namespace ha;
+// places and segments of the items in the order of turns (places[turn * grid + cta]; -1: none); returns the number of turns
+extern "C" int deal(int places, int segs, int rows, int d, int sms, int* place, int* seg, int* meta) {
+  ha_attn_params p{};
+  p.mode = HA_MODE_FLASH; p.flags = HA_FLAG_CAUSAL; p.dtype = HA_BF16;
+  p.B = 1; p.H = segs; p.n = p.m_q = p.m_k = rows; p.span = rows; p.segs_per_head = 1; p.d = p.dv = d;
+  AttnPlan pl;
+  pl.pairs = places; pl.n_items = segs * places; pl.by_pairs = FastDiv(places);
+  const int grid = pl.n_items < sms ? pl.n_items : sms;
+  PLAN_ORDER
+  const int turns = (pl.n_items + grid - 1) / grid;
+  for (int t = 0; t < turns; ++t)
+    for (int c = 0; c < grid; ++c) {
+      const int item = item_of_turn(pl, t, c, grid);
+      place[t * grid + c] = -1;
+      if (item < pl.n_items) place[t * grid + c] = causal_place(pl, item, seg[t * grid + c]);
+    }
+  meta[0] = grid; meta[1] = pl.by_length; meta[2] = pl.by_length ? pl.round_segs : 0; meta[3] = pl.by_length ? pl.rest_segs : 0;
+  meta[4] = pl.by_length ? pl.whole_segs : 0;
+  return turns;
+}
+'''
+SMS = 148
+
+
+@pytest.fixture(scope='module')
+def deal(tmp_path_factory):
+    sys.path.insert(0, CSRC)
+    import build
+    src = tmp_path_factory.mktemp('order') / 'order.cu'
+    src.write_text(SOURCE.replace('PLAN_ORDER', 'plan_order(pl, p, grid);'))
+    lib = str(src)[:-3] + '.so'
+    subprocess.run([os.environ.get('NVCC', 'nvcc')] + build.NVCC_FLAGS + ['-shared', str(src), '-o', lib], check=True, timeout=300)
+    lib = C.CDLL(lib)
+
+    def run(places, segs, rows, d):
+        n = segs * places + SMS
+        place, seg, meta = (C.c_int * n)(), (C.c_int * n)(), (C.c_int * 5)()
+        turns = lib.deal(places, segs, rows, d, SMS, place, seg, meta)
+        grid = meta[0]
+        ctas = [[(place[t * grid + c], seg[t * grid + c]) for t in range(turns) if place[t * grid + c] >= 0] for c in range(grid)]
+        return ctas, meta
+    return run
+
+
+def longest(ctas, places):
+    """key tiles of the longest CTA over the average of all SMs (an item of place p: 2 (places - p) of them, and one for its start)"""
+    loads = [sum(2 * (places - p) + 1 for p, _ in items) for items in ctas]
+    return max(loads) / (sum(loads) / SMS)
+
+
+@pytest.mark.parametrize('d', [64, 128])
+@pytest.mark.parametrize('places', [1, 2, 3, 4, 5, 7, 8, 9, 13, 16, 22, 32, 33, 64])
+def test_every_item_is_taken_once(deal, places, d):
+    for segs in (1, 2, 5, 18, 32, 37, 74, 104, 148, 149, 230, 295, 296, 297, 400, 513):
+        ctas, _ = deal(places, segs, 256 * places, d)
+        items = [x for items in ctas for x in items]
+        assert sorted(items) == [(p, s) for p in range(places) for s in range(segs)], (places, segs)
+
+
+@pytest.mark.parametrize('places,segs,bound', [(3, 400, 1.12), (5, 400, 1.08), (5, 512, 1.08), (7, 400, 1.07), (8, 400, 1.07), (14, 320, 1.11), (16, 320, 1.04),
+                                               (19, 320, 1.05), (22, 320, 1.07), (23, 320, 1.06), (31, 320, 1.04)])
+def test_own_order_is_turned_so_that_a_cta_meets_all_lengths(deal, places, segs, bound):
+    """launches that keep the segments' own order (more than two segments a CTA): the longest CTA stays near the average"""
+    ctas, meta = deal(places, segs, 256 * places, 128)
+    assert not meta[1]
+    assert longest(ctas, places) < bound
