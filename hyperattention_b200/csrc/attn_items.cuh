@@ -196,12 +196,16 @@ inline int own_order_turn(int places) {
   constexpr uint32_t DOWN = 1u << 14 | 1u << 18 | 1u << 22 | 1u << 23 | 1u << 31;
   return places < 32 && (DOWN >> places & 1) ? -1 : 1;
 }
-// The order of the items (causal_place) for a launch of `grid` CTAs; after n_items and pairs.  Rounds whose segments leave L2 (126 MB) lose more
-// than the balance gives: with all segments as one round, 8 x 32 heads x 2047 x 128 took 1807 instead of 1600 us (537 MB of fp32 dK / dV and
-// their like), 128 x 2048 x 128 1459 instead of 1404 (268 MB), 128 x 1536 x 64 925 instead of 990 (100 MB).  With more than two segments a CTA the
-// segments' own order is even enough: rounds cost 1 to 3% there (2048 x 2048 x 64, step of 32 heads x 131072: 18.97 -> 19.56 ms; 512 x 2048 x 128,
-// forward: 1795 -> 1814 us).
-inline void plan_order(AttnPlan& pl, const ha_attn_params& p, int grid) {
+// The order of the items (causal_place) for a launch of `grid` CTAs; after n_items and pairs.  width: bytes of an element of the rows that the items of
+// a segment share: K and V (2) in the forward, fp32 sums (4) in the backward.  All of a round, and all that is left after the rounds, is live at once,
+// and what leaves L2 (126 MB) costs more than the balance gives.  By length against the segments' own order: forward of 64 x 2048 x 128 (67 MB)
+// 82 / 111 us, 32 x 4096 x 128 (67) 141 / 204, 32 x 8192 x 128 (134) 507 / 590, 64 x 8192 x 128 (155, one round of 37) 1012 / 1065; backward of 38 x
+// 4096 x 128 (159) 546 / 635, 85 x 3072 x 128 (151, after the rounds) 747 / 795, 85 x 6144 x 64 (151, so too) 1394 / 1537, 64 x 8192 x 64 (155) 1785 /
+// 1944; 128 x 1920 x 128 (251) 679 / 619, 230 x 1920 x 128 (291) 1244 / 1063.  Odd numbers of places are even enough in the segments' own order to
+// want a lower line: forward of 140 x 1664 x 128 (119) 134 / 125, 128 x 1152 x 128 (75) 66 / 70, 64 x 1152 x 128 (38) 40 / 60.  With more than two
+// segments a CTA the segments' own order is even enough: rounds cost 1 to 3% there (2048 x 2048 x 64, step of 32 heads x 131072:
+// 18.97 -> 19.56 ms; 512 x 2048 x 128, forward: 1795 -> 1814 us).
+inline void plan_order(AttnPlan& pl, const ha_attn_params& p, int grid, int width) {
   pl.by_length = 0;
   pl.turn = own_order_turn(pl.pairs);
   if (p.mode != HA_MODE_FLASH || !(p.flags & HA_FLAG_CAUSAL) || grid <= 0) return;
@@ -217,8 +221,9 @@ inline void plan_order(AttnPlan& pl, const ha_attn_params& p, int grid) {
   pl.by_round = FastDiv((uint32_t)round_items);
   pl.by_round_segs = FastDiv(pl.round_segs);
   pl.by_rest = FastDiv(pl.rest_segs);
-  const long long at_a_time = rounds > 0 ? pl.round_segs : pl.rest_segs;
-  pl.by_length = segs <= 2 * grid && at_a_time * p.m_k * (p.d + p.dv) * 4 / (p.kv_group > 1 ? p.kv_group : 1) <= (126LL << 20);
+  const long long at_a_time = rounds > 0 && pl.round_segs > pl.rest_segs ? pl.round_segs : pl.rest_segs;
+  const long long shared = at_a_time * p.m_k * (p.d + p.dv) * width / (p.kv_group > 1 ? p.kv_group : 1);
+  pl.by_length = segs <= 2 * grid && shared <= (long long)(pl.pairs % 2 ? 32 * width : 160) << 20;
 }
 // May tiles of contiguous rows come as TMA boxes?  A box that runs past the end of a segment brings the next segment's rows, where cp.async
 // fills with zeros: hidden weights are 0, but 0 times a row that is not finite is not.  (Past the last row of all, the map

@@ -871,7 +871,7 @@ static int launch_kt_bwd(const ha_attn_params& p, cudaStream_t st) {
   HA_WINDOW_BYTES(dyn_bytes, (attn_tc_bwd_kt_kernel<T, KIND>), bkt::SMEM_USED, "ha_attn_bwd kernel attributes");
   HA_SMEM_ATTR_ONCE((attn_tc_bwd_kt_kernel<T, KIND>), dyn_bytes, "ha_attn_bwd smem attribute");
   const int sms = sm_count(), grid = pl.n_items < sms ? pl.n_items : sms;
-  plan_order(pl, p, grid);
+  plan_order(pl, p, grid, 4);
   launch_chained((attn_tc_bwd_kt_kernel<T, KIND>), grid, bkt::THREADS, dyn_bytes, st, p, pl, maps);
   HA_LAUNCHED("ha_attn_bwd (tcgen05, by key tiles)");
   return HA_OK;

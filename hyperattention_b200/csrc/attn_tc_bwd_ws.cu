@@ -826,7 +826,7 @@ static int launch_ws_bwd(const ha_attn_params& p, bool store_dq, cudaStream_t st
   HA_WINDOW_BYTES(dyn_bytes, (attn_tc_bwd_ws_kernel<T, KIND>), bws::SMEM_USED, "ha_attn_bwd kernel attributes");
   HA_SMEM_ATTR_ONCE((attn_tc_bwd_ws_kernel<T, KIND>), dyn_bytes, "ha_attn_bwd smem attribute");
   const int sms = sm_count(), grid = pl.n_items < sms ? pl.n_items : sms;
-  plan_order(pl, p, grid);
+  plan_order(pl, p, grid, 4);
   launch_chained((attn_tc_bwd_ws_kernel<T, KIND>), grid, bws::THREADS, dyn_bytes, st, p, pl, out, maps);
   HA_LAUNCHED("ha_attn_bwd (tcgen05, warp-specialised)");
   return HA_OK;

@@ -660,7 +660,7 @@ static int launch_fwd(const ha_attn_params& p, cudaStream_t st) {
   HA_WINDOW_BYTES(dyn_bytes, (attn_tc_fwd_kernel<T, D, DV, KIND>), Cfg::SMEM_USED, "ha_attn_fwd kernel attributes");
   HA_SMEM_ATTR_ONCE((attn_tc_fwd_kernel<T, D, DV, KIND>), dyn_bytes, "ha_attn_fwd smem attribute");
   const int sms = sm_count(), grid = pl.n_items < sms ? pl.n_items : sms;
-  plan_order(pl, p, grid);
+  plan_order(pl, p, grid, 2);
   launch_chained((attn_tc_fwd_kernel<T, D, DV, KIND>), grid, fw::THREADS, dyn_bytes, st, p, pl, maps);
   HA_LAUNCHED("ha_attn_fwd (tcgen05)");
   return HA_OK;
