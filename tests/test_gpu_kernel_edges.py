@@ -587,3 +587,72 @@ def test_causal_items_are_dealt_out_once_each(d, n, H):
         err = (T(got).double() - want).flatten(2).norm(dim=2) / want.flatten(2).norm(dim=2)
         assert err.max() < TOL[torch.bfloat16][tol], (err.max(), err.argmax())
     assert (lse[:, :, :n].double() - s.logsumexp(-1)).abs().max() < 1e-4
+
+
+@pytest.mark.parametrize('dtype,d', [(torch.bfloat16, 64), (torch.bfloat16, 128), (torch.float32, 64)])
+@pytest.mark.parametrize('n', [1, 515, 640])
+def test_exact_causal_call_without_a_gradient(dtype, d, n):
+    """short causal calls that keep nothing for a backward hand [batch, heads, rows, width] tensors to the kernel as they are: fewer K/V heads than query
+    heads, tensors that lie as [n, B, heads, d] in memory, rows padded and not; the same bits as the call that keeps them"""
+    import hyperattention_b200 as ha
+    torch.manual_seed(96)
+    B, H, Hk = 2, 6, 2
+    q, k, v = [torch.randn(n, B, h, d, device='cuda').to(dtype).permute(1, 2, 0, 3) for h in (H, Hk, Hk)]
+    mod = ha.HyperAttention(input_dim=d, min_seq_len=2048, rng=torch.Generator().manual_seed(10)).to(device='cuda', dtype=dtype)
+    with torch.no_grad():
+        o, lse = mod(q, k, v, causal=True, return_lse=True)
+        assert torch.equal(mod(q, k, v, causal=True), o)
+        assert torch.equal(mod(*[t.contiguous() for t in (q, k, v)], causal=True), o)
+    og, lg = mod(*[t.detach().requires_grad_() for t in (q, k, v)], causal=True, return_lse=True)
+    assert torch.equal(o, og) and torch.equal(lse, lg) and o.stride() == og.stride() and lse.shape == (B, H, -(-n // 128) * 128)
+    s = (q.double() @ k.double().repeat_interleave(H // Hk, 1).transpose(2, 3) * d ** -0.5).masked_fill(torch.ones(n, n, dtype=torch.bool, device='cuda').triu(1), float('-inf'))
+    assert rel(o, s.softmax(-1) @ v.double().repeat_interleave(H // Hk, 1)) < TOL[dtype][0]
+    assert (lse[:, :, :n].double() - s.logsumexp(-1)).abs().max() < 1e-4 and not lse[:, :, n:].any()
+
+
+@pytest.mark.parametrize('causal,smooth,dtype,d', [(True, False, torch.bfloat16, 64), (True, False, torch.bfloat16, 128), (False, False, torch.bfloat16, 64),
+                                                   (False, True, torch.float16, 64), (False, False, torch.bfloat16, 128), (True, False, torch.float32, 64)])
+def test_captured_step_repeats_the_eager_one(causal, smooth, dtype, d):
+    """forward alone, forward and backward, recorded as graphs (a side stream and its join, zero-fills and launches that overlap the one before) and replayed
+    on other inputs, several times in a row"""
+    import hyperattention_b200 as ha
+    torch.manual_seed(97)
+    n = 2048
+    mod = ha.HyperAttention(input_dim=d, min_seq_len=512, sample_size=128, smooth_block=smooth, rng=torch.Generator().manual_seed(11)).to(device='cuda', dtype=dtype)
+    new = lambda: [torch.randn(1, 3, n, d, device='cuda').to(dtype) for _ in range(4)]
+    held = new()
+    q, k, v = [t.requires_grad_() for t in held[:3]]
+    do = held[3]
+
+    def forward():
+        with torch.no_grad():
+            return mod(q, k, v, causal=causal, return_lse=True)
+
+    def step():
+        o = mod(q, k, v, causal=causal)
+        return (o.detach(),) + torch.autograd.grad(o, (q, k, v), do)
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        forward(), step()
+    torch.cuda.current_stream().wait_stream(side)
+    graphs = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graphs[0]):
+        kept = forward()
+    with torch.cuda.graph(graphs[1]):
+        grads = step()
+    for times in (1, 3):
+        with torch.no_grad():
+            for t, x in zip(held, new()):
+                t.copy_(x)
+        for _ in range(times):
+            for g in graphs:
+                g.replay()
+        torch.cuda.synchronize()
+        for got, want in zip(kept, forward()):
+            assert torch.equal(got, want)
+        want = step()
+        assert torch.equal(grads[0], want[0])
+        for got, w in zip(grads[1:], want[1:]):       # (fp32 additions in no fixed order, rounded to 16 bits)
+            assert rel(got, w) < (1e-3 if dtype != torch.float32 else 1e-6)
