@@ -39,8 +39,12 @@ struct AttnItem {
 // gave 4 to 50% (segments x places: 64 x 8 4 for 50%, 128 x 6 6 for 40, 128 x 8 6 for 23, 256 x 8 1 for 10, 128 x 16 1 for 16).
 // Training steps: 16 heads x 12287 x 64 (128 x 6) 889 -> 840 us, 128 x 1920 x 64 442 -> 420, 2 x 16 heads x 8192 x 128 (128 x 8, x 16 in the backward)
 // 1360 -> 1337, 256 x 2047 x 128 1538 -> 1514.
+// EXACT: may the launch be exact attention?  Kernels of the hyper pattern, whose items are of one length, are compiled without the order: its few
+// instructions in the warp that works the items out cost them 0.5 to 3% (32 x 131072 x 64, step: 3286 -> 3250 us; smooth 32 x 16384 630 -> 609;
+// weighted 16 x 32768 590 -> 570; forward of 32 x 131072 1124 -> 1118).
+template <bool EXACT>
 __host__ __device__ __forceinline__ int item_of_turn(const AttnPlan& pl, int turn, int cta, int grid) {
-  return turn * grid + (pl.by_length && (turn & 1) ? grid - 1 - cta : cta);
+  return turn * grid + (EXACT && pl.by_length && (turn & 1) ? grid - 1 - cta : cta);
 }
 __host__ __device__ __forceinline__ int causal_place(const AttnPlan& pl, int item, int& seg) {
   int place;

@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
         for (; published <= (int)n_item + 2; ++published) {
           const uint32_t at = published % ND;
           it.n_list = 0;
-          const int item = item_of_turn(pl, published, blockIdx.x, gridDim.x);
+          const int item = item_of_turn<KIND == KT_FLASH>(pl, published, blockIdx.x, gridDim.x);
           if (item < pl.n_items) it = kt_item(p, pl, item, flash, by_keys);
           if (published >= ND && !wait(B_D_EMPTY + at, (published / ND - 1) & 1)) return false;
           if (lane == 0) {

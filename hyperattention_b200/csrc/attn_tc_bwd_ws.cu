@@ -101,7 +101,7 @@ struct BwdOut {
   int bulk;           // accumulators that take TMA additions: 1 = dq, 2 = dk and dv
   int store_dq;       // fp32 dq rows are stored, not added
 };
-enum { BWD_HYPER = 0, BWD_FLASH = 1, BWD_ANY = 2 };            // the plain hyper pattern, exact attention, any call
+enum { BWD_HYPER = 0, BWD_FLASH = 1, BWD_ANY = 2 };            // the plain hyper pattern, exact attention, the hyper pattern with smooth windows or weights
 
 __device__ __forceinline__ void bws_bulk_add_f32(float* dst, uint32_t src, uint32_t bytes) {
   asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
   __shared__ int s_bail;
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-  const bool flash = KIND == BWD_FLASH || (KIND == BWD_ANY && p.mode == HA_MODE_FLASH);
+  constexpr bool flash = KIND == BWD_FLASH;
   constexpr bool ANY = KIND == BWD_ANY;
 
   if (cta_sees_failure(p.status, &s_bail)) return;   // an earlier CTA gave up: drain quickly (uniform over the CTA)
@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
         for (; published <= (int)n_item + 2; ++published) {
           const uint32_t slot = published % ND;
           it.n_list = 0;
-          const int item = item_of_turn(pl, published, blockIdx.x, gridDim.x);
+          const int item = item_of_turn<KIND == BWD_FLASH>(pl, published, blockIdx.x, gridDim.x);
           if (item < pl.n_items) it = attn_item(p, pl, item, flash, by_keys);
           if (published >= ND && !wait(B_D_EMPTY + slot, (published / ND - 1) & 1)) return false;
           if (lane == 0) {

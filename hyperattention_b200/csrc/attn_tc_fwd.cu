@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(fw::THREADS, 1) attn_tc_fwd_kernel(const ha_at
         for (; published <= (int)n_item + 2; ++published) {
           const uint32_t slot = published % ND;
           it.n_list = 0;
-          const int item = item_of_turn(pl, published, blockIdx.x, gridDim.x);
+          const int item = item_of_turn<KIND != FWD_HYPER>(pl, published, blockIdx.x, gridDim.x);
           if (item < pl.n_items) it = attn_item(p, pl, item, flash);
           if (published >= ND && !wait(B_D_EMPTY + slot, (published / ND - 1) & 1)) return false;
           if (lane == 0) {

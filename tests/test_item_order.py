@@ -23,7 +23,7 @@ extern "C" int deal(int places, int segs, int rows, int d, int width, int sms, i
   const int turns = (pl.n_items + grid - 1) / grid;
   for (int t = 0; t < turns; ++t)
     for (int c = 0; c < grid; ++c) {
-      const int item = item_of_turn(pl, t, c, grid);
+      const int item = item_of_turn<true>(pl, t, c, grid);
       place[t * grid + c] = -1;
       if (item < pl.n_items) place[t * grid + c] = causal_place(pl, item, seg[t * grid + c]);
     }
