@@ -35,10 +35,11 @@ struct AttnItem {
 // Exact causal attention: the items of a segment differ in length (place 0: the longest), and CTA c takes items c, c + grid, ... of one
 // order.  That order is by length over a round of segments -- as many as make whole turns of the grid (37 for 4, 8, 12 or 16 places and 148
 // CTAs) --, then over the segments that are left; every other turn the CTAs take theirs in the opposite direction
-// (item_of_turn).  Lengths are dealt out evenly that way: the longest CTA has 0 to 7% more than the average, where the segments' own order
-// gave 4 to 50% (segments x places: 64 x 8 4 for 50%, 128 x 6 6 for 40, 128 x 8 6 for 23, 256 x 8 1 for 10, 128 x 16 1 for 16).
-// Training steps: 16 heads x 12287 x 64 (128 x 6) 889 -> 840 us, 128 x 1920 x 64 442 -> 420, 2 x 16 heads x 8192 x 128 (128 x 8, x 16 in the backward)
-// 1360 -> 1337, 256 x 2047 x 128 1538 -> 1514.
+// (item_of_turn).  How much more the longest CTA has than the average (up to 32 places and 295 segments, worked out on the host): with six turns of the
+// grid or more 1% in half of the cases, 14% at most; with three to six 6% in half of them, 32% at most; below three turns 10 to 90%, where little can be
+// dealt out.  Against the segments' own order (segments x places): 64 x 8 4 for 50%, 128 x 6 6 for 40, 128 x 8 6 for 23, 256 x 8 1 for 10, 128 x
+// 16 1 for 17.  Training steps, in turn: 16 heads x 12287 x 64 (128 x 6) 894 -> 856 us, 128 x 1920 x 64 442 -> 425, 2 x 16 heads x 8192 x 128 (128 x 8,
+// x 16 in the backward) 1355 -> 1309, 256 x 2047 x 128 1488 -> 1446.
 // EXACT: may the launch be exact attention?  Kernels of the hyper pattern, whose items are of one length, are compiled without the order: its few
 // instructions in the warp that works the items out cost them 0.5 to 3% (32 x 131072 x 64, step: 3286 -> 3250 us; smooth 32 x 16384 630 -> 609;
 // weighted 16 x 32768 590 -> 570; forward of 32 x 131072 1124 -> 1118).

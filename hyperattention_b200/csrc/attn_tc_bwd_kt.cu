@@ -247,8 +247,8 @@ __global__ void __launch_bounds__(bkt::THREADS, 1) attn_tc_bwd_kt_kernel(const h
           const bool diag = causal && e == y, masked = KIND != KT_HYPER && (weighted || diag || (flash && (e + 1) * TILE > p.m_k));
           const uint64_t bias = pack_f2(bias2, bias2);
           // Fragments of 16 keys x 8 queries, two keys and two neighbouring queries a thread, 16 keys x 32 queries at a time: the thread
-          // needs the lse and delta of 8 queries, where with a key a thread it needed those of all of them, as broadcast reads (decoder 2 x 16 x 8192:
-          // 1400 -> 1360 us, 8 x 32 x 2047 exact causal 1580 -> 1538, 32 x 32768 hyper 1964 -> 1933).
+          // needs the lse and delta of 8 queries, where with a key a thread it needed those of all of them, as broadcast reads (steps: decoder 2 x 16 x
+          // 8192 1388 -> 1355 us, 8 x 32 x 2047 exact causal 1532 -> 1488, 32 x 32768 hyper 1868 -> 1827).
 #pragma unroll 1
           for (int c = 0; c < 2; ++c) {
             const uint32_t ds_to = ds_rows + (((4 * c + (lane >> 3)) ^ (lane & 7)) << 4);

@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
             uint8_t* ds_rows = smem + OFF_DS + (pair & 1) * 2 * TILE_B + s * TILE_B + (32 * (warp & 3) + (lane & 7)) * 128;
             // Two keys and two neighbouring queries a fragment and thread: it needs the lse and delta of 8 queries.  With a key a thread it needed
             // those of all 32, and the broadcast reads, four cycles of the shared memory each, held up the tensor core's operands: exact causal 128 x 1920
-            // rows 459 -> 442 us (step), 16 x 12287 929 -> 886, smooth 32 x 16384 644 -> 621, 32 x 131072 3.54 -> 3.41 ms.
+            // rows 458 -> 442 us (step), 16 x 12287 934 -> 894, smooth 32 x 16384 642 -> 621, 32 x 131072 3398 -> 3256.
             const uint32_t ds_to = smem_u32(ds_rows) + (((4 * g + (lane >> 3)) ^ (lane & 7)) << 4);
             uint64_t L[4], Dl[4];
 #pragma unroll
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
     HA_T_DUMP(8, (int)blockIdx.x * 8 + g, row == 0)
   } else if (warp < W_MMA) {
     // =====================================================================================================
-    // drain group: finished accumulators -> global memory
+    // drain groups: finished accumulators -> global memory
     // =====================================================================================================
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     const int row = tid & 127, rot = row & 7, grp = (warp - W_DRAIN) >> 2;
@@ -420,9 +420,9 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
               __syncwarp();
               const int c = lane & 7;
               if (KIND != BWD_FLASH && mode == ROWS_ADD) {
-                // all reads, then all additions: a branch a row made smooth windows (32 heads x 16384) 7% slower.  Typed rows measured
-                // the other way round (2.22 against 2.28 ms at 32 x
-                // 131072), and exact attention, whose tiles rarely leave this way, without this branch (4.46 against 4.50 ms).
+                // all reads, then all additions: a branch a row made smooth windows (32 heads x 16384) 7% slower.  Typed rows measured the
+                // other way round (2.22 against 2.28 ms at 32 x 131072), and exact attention, whose tiles rarely leave this way, is
+                // faster without this branch (4.46 against 4.50 ms, leaves of 32 x 131072).
                 float4 v[8];
                 int to[8];
 #pragma unroll
@@ -693,7 +693,7 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
       cp_async_wait<0>();
     } else {
       // ===================================================================================================
-      // loaders of the key side: K tiles (warp 18), V tiles (warp 19)
+      // loaders of the key side: K tiles (warp W_K), V tiles (the warp after it)
       // ===================================================================================================
       const bool is_v = warp != W_K;
       const uint16_t* tensor = (const uint16_t*)(is_v ? p.v : p.k);
@@ -757,7 +757,7 @@ __global__ void __launch_bounds__(bws::THREADS, 1) attn_tc_bwd_ws_kernel(const h
   __syncthreads();
   if (s_abort) {      // (nobody writes it any more)
     // What is still under way is waited for, with a limit, before TMEM goes and the CTA retires: the last tile of every slot a loader fills, each
-    // MMA warp's products, stores to TMEM.  (The drain group's copies out are through.)  A CTA that gets through its items
+    // MMA warp's products, stores to TMEM.  (The drain groups' copies out are through.)  A CTA that gets through its items
     // has waited for all of it on the way.
     const uint32_t bar_end = smem_u32(s_item);      // (the descriptors have been used up: their place takes the MMA warps' barriers)
     if (tid < 5) mbar_init(bar_end + 8 * tid, 1);
