@@ -207,8 +207,8 @@ inline int own_order_turn(int places) {
 // 82 / 111 us, 32 x 4096 x 128 (67) 141 / 204, 32 x 8192 x 128 (134) 507 / 590, 64 x 8192 x 128 (155, one round of 37) 1012 / 1065; backward of 38 x
 // 4096 x 128 (159) 546 / 635, 85 x 3072 x 128 (151, after the rounds) 747 / 795, 85 x 6144 x 64 (151, so too) 1394 / 1537, 64 x 8192 x 64 (155) 1785 /
 // 1944; 128 x 1920 x 128 (251) 679 / 619, 230 x 1920 x 128 (291) 1244 / 1063.  Odd numbers of places are even enough in the segments' own order to
-// want a lower line: forward of 140 x 1664 x 128 (119) 134 / 125, 128 x 1152 x 128 (75) 66 / 70, 64 x 1152 x 128 (38) 40 / 60.  With more than two
-// segments a CTA the segments' own order is even enough: rounds cost 1 to 3% there (2048 x 2048 x 64, step of 32 heads x 131072:
+// want a lower line: forward of 140 x 1664 x 128 (119) 134 / 125, 128 x 1152 x 128 (75) 66 / 70.  With more than two segments a CTA the segments'
+// own order is even enough: rounds cost 1 to 3% there (2048 x 2048 x 64, step of 32 heads x 131072:
 // 18.97 -> 19.56 ms; 512 x 2048 x 128, forward: 1795 -> 1814 us).
 inline void plan_order(AttnPlan& pl, const ha_attn_params& p, int grid, int width) {
   pl.by_length = 0;
